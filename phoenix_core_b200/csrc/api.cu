@@ -183,6 +183,14 @@ int run_pass(Pass pass, int dtype, int variant, int engine, const Geom& g, const
     return simt_launch(pass, dtype, variant, g, a, b, bias, out, scratch, stream);
 }
 
+// Whether a dense call runs on the kernels that take the caller's tensors as they are (qgemm_tc.cu). `tensors`: the OR of all
+// tensor addresses of the call. The workspace must be what the size query asks for, as for every other path.
+bool dense_direct(const pcb_dense_desc* desc, const Geom& g, uintptr_t tensors, void* workspace, size_t ws_bytes, size_t need) {
+    const int tv = tensor_variant(variant_for(g, desc->variant), desc->engine);
+    return desc->engine != PCB_ENGINE_SIMT && workspace && ws_bytes >= need && ((tensors | reinterpret_cast<uintptr_t>(workspace)) & 15u) == 0 &&
+           dense_tc_supported(desc->dtype, tv, g);
+}
+
 // Grouped convolution (reference: the groups argument of the scalar convolutions, src/backend/cudnn/conv2d.hpp:126-127):
 // one pass per group on the CUDA-core kernels, which address every tensor through strides -- a group is a channel slice
 // of x, y and the filters. The filter gradient of a group is produced contiguously in the workspace and copied into its
@@ -466,6 +474,11 @@ int pcb_qdense_fwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     if (!x || !w || !y || (g.has_bias && !bias)) { set_error("null tensor pointer"); return PCB_ERR_INVALID_ARGUMENT; }
     rc = reset_status(workspace, workspace_bytes_, (cudaStream_t)stream);
     if (rc != PCB_OK) return rc;
+    const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
+    if (dense_direct(desc, g, all, workspace, workspace_bytes_, pcb_qdense_fwd_workspace_size(desc))) {
+        forget_kept(workspace);
+        return dense_tc_fwd(desc->dtype, g, x, w, bias, y, static_cast<int*>(workspace), (cudaStream_t)stream);
+    }
     return run_pass(PASS_FWD, desc->dtype, variant_for(g, desc->variant), desc->engine, g, w, x, bias, y, workspace, workspace_bytes_, (cudaStream_t)stream);
 }
 
@@ -482,6 +495,13 @@ int pcb_qdense_bwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     if (!x || !w || !dy || (desc->require_input_grad && !dx)) { set_error("null tensor pointer"); return PCB_ERR_INVALID_ARGUMENT; }
     rc = reset_status(workspace, workspace_bytes_, (cudaStream_t)stream);
     if (rc != PCB_OK) return rc;
+    void* gx = desc->require_input_grad ? dx : nullptr;
+    const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(dy) |
+                          reinterpret_cast<uintptr_t>(dw) | reinterpret_cast<uintptr_t>(gx);
+    if (dense_direct(desc, g, all, workspace, workspace_bytes_, pcb_qdense_bwd_workspace_size(desc))) {
+        forget_kept(workspace);
+        return dense_tc_bwd(desc->dtype, g, x, w, dy, dw, gx, static_cast<int*>(workspace), (cudaStream_t)stream);
+    }
     rc = run_pass(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g, dy, x, nullptr, dw, workspace, workspace_bytes_, (cudaStream_t)stream);
     if (rc != PCB_OK) return rc;
     if (desc->require_input_grad)

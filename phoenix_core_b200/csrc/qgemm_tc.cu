@@ -1,0 +1,546 @@
+// Quaternion matrix products on the tensor cores straight from the caller's tensors: dense layers (forward, backward-data and
+// filter gradient, any feature counts, fp16 / bf16 / fp32).
+//
+// One output tile of the product is 128 rows of one operand (A) by NT columns of the other (B) for all four output
+// components: D[m][(c, n)] = sum over (kc, k) of A[kc][m][k] * s(kc, c) B[c ^ kc][n][k]. A is multiplied as it lies in memory;
+// the signed / permuted quaternion block is expanded on B alone while its tile is written to shared memory: component
+// c ^ kc of B, with its sign, goes to block c of the stage (kc, k chunk). So a stage is ONE real product 128 x (4 NT) x 64 and the
+// expanded 4 x 4 block never exists in global memory. Roles:
+//     forward        m = output feature, n = batch row, k = input feature:   A[kc] = w_kc,  B = x,  s = s(c ^ kc, c)
+//     backward-data  m = input feature,  n = batch row, k = output feature:  A[kc] = w_kc,  B = dy, s = s(c, c ^ kc)
+//     filter grad.   m = output feature, n = input feature, k = batch row:   A[kc] = dy_kc, B = x,  s = s(c ^ kc, kc)
+// The rows m are contiguous in the output of every pass, so the 32 lanes of an epilogue warp store 32 consecutive elements.
+// (replaces the 16 GEMM calls and accumulate passes of the reference, src/dense.hpp:21-379, src/backend/cudnn/dense.hpp:20-218.)
+//
+// Three groups of four warps load (plain loads of the widest type that the rows' alignment allows: feature counts need no
+// alignment, which a tensor map would ask for), expand and store the operands in the tcgen05 layouts, each group its own stages;
+// one thread of a thirteenth warp issues the MMAs. fp32 operands are split into hi + lo TF32 numbers on their way
+// (three MMAs per product, as in conv_tf32.cu). The reduced dimension of a tile is cut over the CTAs of a cluster, which add
+// their partial tiles through distributed shared memory in a fixed order (results do not depend on timing, nothing is zeroed or
+// cast in a second pass). What bounds a dense layer of a few hundred features is the latency of this chain (load, expand, MMA,
+// exchange, store), not bandwidth: hence one launch per call, no staging kernels, and a cluster split that fills the machine.
+// All mbarrier waits are bounded.
+#include "tc_common.cuh"
+#include "tensor_path.cuh"
+
+namespace pcb {
+namespace {
+
+using namespace umma;
+using namespace tc;
+
+constexpr int QM = 128;                               // rows of a tile
+constexpr int Q_GROUP = 128, Q_GROUPS = 3;             // loader threads: groups that fill stages in turn
+constexpr int Q_LOADERS = Q_GROUP * Q_GROUPS, Q_THREADS = Q_LOADERS + 32;
+constexpr int Q_MAX_STAGES = 6;
+constexpr int Q_ROW_BYTES = 128;                      // bytes of one K row of an operand tile: 64 16-bit or 32 fp32 elements
+constexpr int ST_Q_LOADER = 0x1000, ST_Q_MMA = 0x2000, ST_Q_EPILOGUE = 0x4000;
+// MMAs that may be added into one fp32 accumulator of the fp32 path (each truncates when it adds: conv_tf32.cu), and how many
+// accumulators there are. 8 stages of 12 MMAs in each of 4 accumulators.
+constexpr int Q_F32_STAGES_PER_ACC = 8, Q_F32_ACCS = 4;
+
+// One operand: element (component, u, v) lies at component * cs + u + v * ld, u being the contiguous index.
+struct QOperand {
+    const void* p;
+    int cs, ld;
+    int nu, nv;          // extents of u and v
+    int chunk;           // bytes per load: the largest of 16, 8, 4, 2 that divides every row start
+};
+struct QProblem {
+    QOperand a, b;
+    void* out;
+    const void* bias;    // [4][M] or null
+    int M, N, K;
+    int o_c, o_n;        // output element (c, n, m) at c * o_c + n * o_n + m
+    int tiles_m, tiles_n;
+    int chunks;          // K chunks of 64 (fp32: 32) elements
+    int split;           // CTAs that share a tile, neighbours in a cluster: slices of the K chunks
+    uint32_t neg;        // bit 4 * kc + c: component c ^ kc of B enters block c negated
+};
+struct QParams {
+    QProblem prob[2];
+    int first_blocks;    // CTAs of prob[0]; the rest work on prob[1]
+    int cluster;         // CTAs of a cluster (the larger of the two splits)
+    int fmt;             // 0 = fp16, 1 = bf16, 2 = fp32 as TF32
+};
+
+__device__ __forceinline__ uint32_t q_cluster_rank() {
+    uint32_t r;
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
+    return r;
+}
+__device__ __forceinline__ void q_cluster_sync() {
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+    asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+__device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, uint32_t rank) {
+    uint32_t a;
+    float v;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"(local_addr), "r"(rank));
+    asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
+    return v;
+}
+__device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
+__device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t b) {
+    asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
+}
+
+// ---- operand tiles ----------------------------------------------------------------------------------------------------------
+// ROWS (m or n) x 128 bytes of K (64 16-bit or 32 fp32 elements), moved by the 128 threads of a loader group in chunks of CB bytes.
+//   KMAJ: u = k. Chunk i of thread t: row t / PER + i * STEP, byte (t % PER) * CB of that row's 128.
+//   else: u = m or n, v = k. Chunk i: k row t / PER + i * STEP, byte (t % PER) * CB of the ROWS elements.
+template <bool F32, bool KMAJ, int ROWS, int CB>
+struct QChunks {
+    static constexpr int EB = F32 ? 4 : 2;
+    static constexpr int PER = (KMAJ ? Q_ROW_BYTES : ROWS * EB) / CB, STEP = Q_GROUP / PER;
+    static constexpr int COUNT = ROWS * Q_ROW_BYTES / CB / Q_GROUP;
+    static_assert(Q_GROUP % PER == 0 && COUNT >= 1, "chunks");
+};
+template <bool F32, bool KMAJ, int ROWS, int CB>
+__device__ __forceinline__ void load_chunks(uint32_t (&r)[ROWS / 4], const QOperand& o, int comp, int row0, int k0, int t) {
+    typedef QChunks<F32, KMAJ, ROWS, CB> C;
+    const int u = (KMAJ ? k0 : row0) + (t % C::PER) * (CB / C::EB), v0 = (KMAJ ? row0 : k0) + t / C::PER;
+    const bool u_ok = u < o.nu;
+    const char* src = static_cast<const char*>(o.p) + ((size_t)comp * o.cs + (size_t)v0 * o.ld + u) * C::EB;
+    const size_t step = (size_t)C::STEP * o.ld * C::EB;
+#pragma unroll
+    for (int i = 0; i < C::COUNT; ++i) {
+        const bool ok = u_ok && v0 + i * C::STEP < o.nv;
+        const char* q = src + i * step;
+        if (CB == 16) {
+            uint4 w = make_uint4(0u, 0u, 0u, 0u);
+            if (ok) w = __ldg(reinterpret_cast<const uint4*>(q));
+            r[4 * i] = w.x; r[4 * i + 1] = w.y; r[4 * i + 2] = w.z; r[4 * i + 3] = w.w;
+        } else if (CB == 8) {
+            uint2 w = make_uint2(0u, 0u);
+            if (ok) w = __ldg(reinterpret_cast<const uint2*>(q));
+            r[2 * i] = w.x; r[2 * i + 1] = w.y;
+        } else if (CB == 4) {
+            r[i] = ok ? __ldg(reinterpret_cast<const uint32_t*>(q)) : 0u;
+        } else {
+            const uint32_t w = ok ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(q)) : 0u;
+            if (i & 1) r[i / 2] |= w << 16; else r[i / 2] = w;
+        }
+    }
+}
+__device__ __forceinline__ uint32_t tf32_hi(uint32_t x) { return x & 0xFFFFE000u; }
+__device__ __forceinline__ uint32_t tf32_lo(uint32_t x) { return __float_as_uint(__uint_as_float(x) - __uint_as_float(x & 0xFFFFE000u)); }
+// Writes the chunks to rows row_base .. of an operand tile, every element's sign flipped by `flip`; fp32: hi parts to `tile`, lo
+// parts to `tile` + lo_ofs.
+template <bool F32, bool KMAJ, int ROWS, int CB>
+__device__ __forceinline__ void store_chunks(const uint32_t (&r)[ROWS / 4], uint32_t tile, uint32_t lo_ofs, int row_base, uint32_t flip, int t) {
+    typedef QChunks<F32, KMAJ, ROWS, CB> C;
+    const int ub = (t % C::PER) * CB, v0 = t / C::PER;
+#pragma unroll
+    for (int i = 0; i < C::COUNT; ++i) {
+        const int v = v0 + i * C::STEP;
+        uint32_t dst;
+        if (KMAJ) {
+            const int row = row_base + v;
+            dst = tile + (uint32_t)row * Q_ROW_BYTES + (uint32_t)(((ub >> 4) ^ (row & 7)) << 4) + (uint32_t)(ub & 15);
+        } else {
+            // blocks of 128 bytes of rows, K rows of 128 bytes inside; 16-byte units swizzled over 8 K rows (16-bit elements),
+            // 32-byte units over 4 K rows (fp32)
+            const int b = row_base * C::EB + ub, in = b & 127;
+            dst = tile + (uint32_t)(b >> 7) * (F32 ? 32 : 64) * Q_ROW_BYTES + (uint32_t)v * Q_ROW_BYTES +
+                  (F32 ? (uint32_t)(((in >> 5) ^ (v & 3)) << 5) + (uint32_t)(in & 31) : (uint32_t)(((in >> 4) ^ (v & 7)) << 4) + (uint32_t)(in & 15));
+        }
+        uint32_t w[4], lo[4];
+        constexpr int W = CB >= 4 ? CB / 4 : 1;
+#pragma unroll
+        for (int j = 0; j < W; ++j) {
+            w[j] = (CB >= 4 ? r[W * i + j] : ((i & 1) ? r[i / 2] >> 16 : r[i / 2])) ^ flip;
+            if (F32) { lo[j] = tf32_lo(w[j]); w[j] = tf32_hi(w[j]); }
+        }
+        if (CB == 16) { st_shared_v4(dst, w[0], w[1], w[2], w[3]); if (F32) st_shared_v4(dst + lo_ofs, lo[0], lo[1], lo[2], lo[3]); }
+        else if (CB == 8) { st_shared_v2(dst, w[0], w[1]); if (F32) st_shared_v2(dst + lo_ofs, lo[0], lo[1]); }
+        else if (CB == 4) { st_shared_u32(dst, w[0]); if (F32) st_shared_u32(dst + lo_ofs, lo[0]); }
+        else st_shared_u16(dst, (uint16_t)(w[0] & 0xffffu));
+    }
+}
+template <bool F32, bool KMAJ, int ROWS>
+__device__ __forceinline__ void load_tile(uint32_t (&r)[ROWS / 4], const QOperand& o, int comp, int row0, int k0, int t) {
+    if (o.chunk == 16) load_chunks<F32, KMAJ, ROWS, 16>(r, o, comp, row0, k0, t);
+    else if (o.chunk == 8) load_chunks<F32, KMAJ, ROWS, 8>(r, o, comp, row0, k0, t);
+    else if (F32 || o.chunk == 4) load_chunks<F32, KMAJ, ROWS, 4>(r, o, comp, row0, k0, t);
+    else load_chunks<false, KMAJ, ROWS, 2>(r, o, comp, row0, k0, t);
+}
+template <bool F32, bool KMAJ, int ROWS>
+__device__ __forceinline__ void store_tile(const uint32_t (&r)[ROWS / 4], const QOperand& o, uint32_t tile, uint32_t lo_ofs, int row_base, uint32_t flip, int t) {
+    if (o.chunk == 16) store_chunks<F32, KMAJ, ROWS, 16>(r, tile, lo_ofs, row_base, flip, t);
+    else if (o.chunk == 8) store_chunks<F32, KMAJ, ROWS, 8>(r, tile, lo_ofs, row_base, flip, t);
+    else if (F32 || o.chunk == 4) store_chunks<F32, KMAJ, ROWS, 4>(r, tile, lo_ofs, row_base, flip, t);
+    else store_chunks<false, KMAJ, ROWS, 2>(r, tile, lo_ofs, row_base, flip, t);
+}
+// fp32 operand with its rows contiguous along m or n: blocks of 32 rows `block_bytes` apart, groups of 4 K rows 512 bytes apart.
+__device__ __forceinline__ uint64_t make_desc_mn_f32(uint32_t addr, uint32_t block_bytes) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((block_bytes >> 4) & 0x3FFFu) << 16) | ((uint64_t)(512u >> 4) << 32) |
+           DESC_VERSION_SM100 | (1ull << 61);
+}
+
+template <bool F32, int NT>
+struct QLayout {
+    static constexpr int N = 4 * NT;
+    static constexpr uint32_t A_TILE = QM * Q_ROW_BYTES, B_TILE = N * Q_ROW_BYTES;
+    static constexpr uint32_t STAGE = (A_TILE + B_TILE) * (F32 ? 2 : 1);
+    static constexpr int STAGES_FIT = (int)((216 * 1024) / STAGE);
+    static constexpr int STAGES = STAGES_FIT < Q_MAX_STAGES ? STAGES_FIT : Q_MAX_STAGES;
+    static constexpr int ACCS = F32 ? Q_F32_ACCS : 2;                 // accumulators of N columns, used in turn
+    static constexpr uint32_t PARTIAL = (uint32_t)N * QM * 4;         // the exchanged partial tile, in the stages' memory
+    static constexpr uint32_t BODY = STAGES * STAGE > PARTIAL ? STAGES * STAGE : PARTIAL;
+    static constexpr size_t SMEM = 1024 + BODY + 256;
+    static_assert(ACCS * N <= 512, "tensor memory");
+};
+
+__device__ __forceinline__ void q_store(void* out, size_t at, float v, int fmt) {
+    if (fmt == 2) static_cast<float*>(out)[at] = v;
+    else if (fmt == 0) static_cast<__half*>(out)[at] = __float2half_rn(v);
+    else static_cast<__nv_bfloat16*>(out)[at] = __float2bfloat16_rn(v);
+}
+__device__ __forceinline__ float q_bias(const void* bias, size_t at, int fmt) {
+    if (fmt == 2) return static_cast<const float*>(bias)[at];
+    if (fmt == 0) return __half2float(static_cast<const __half*>(bias)[at]);
+    return __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[at]);
+}
+
+template <bool F32, int NT, bool AK, bool BK>
+__device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster, int fmt, uint32_t tmem_base, uint32_t tiles, uint32_t full_bar,
+                                       uint32_t empty_bar, uint32_t done_bar, int* status) {
+    typedef QLayout<F32, NT> L;
+    constexpr int KC = F32 ? 32 : 64;
+    const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int split = p.split, tile = block / split, rank = block - tile * split;
+    const int m0 = (tile % p.tiles_m) * QM, n0 = (tile / p.tiles_m) * NT;
+    const int per = (p.chunks + split - 1) / split;
+    const int c_beg = min(p.chunks, rank * per), c_end = min(p.chunks, c_beg + per);
+    // stage st: chunk c_beg + st / 4, component st % 4 of A. (The grid is padded to whole clusters: CTAs past the last tile do nothing.)
+    const int n_stages = tile < p.tiles_m * p.tiles_n ? (c_end - c_beg) * 4 : 0;
+
+    bool ok = true;
+    if (t < Q_LOADERS) {
+        // ------------------------------------------------------------------------------------------ loaders
+        // group g fills stages g, g + Q_GROUPS, ...: while one group waits for its loads the others write theirs
+        const int tg = t % Q_GROUP;
+        constexpr int HALF = NT == 32 ? 4 : 2;                     // components of B in registers at a time
+        for (int st = t / Q_GROUP; st < n_stages && ok; st += Q_GROUPS) {
+            const int kc = st & 3, k0 = (c_beg + (st >> 2)) * KC, s = st % L::STAGES;
+            uint32_t ra[QM / 4], rb[HALF][NT / 4];
+            load_tile<F32, AK, QM>(ra, p.a, kc, m0, k0, tg);
+#pragma unroll
+            for (int c = 0; c < HALF; ++c) load_tile<F32, BK, NT>(rb[c], p.b, c ^ kc, n0, k0, tg);
+            ok = mbar_wait_bounded(empty_bar + 8 * s, (st / L::STAGES + 1) & 1, status, ST_Q_LOADER);
+            if (ok) {
+                const uint32_t a_tile = tiles + s * L::STAGE, b_tile = a_tile + L::A_TILE * (F32 ? 2 : 1);
+                constexpr uint32_t SIGN = F32 ? 0x80000000u : 0x80008000u;
+                const uint32_t neg = p.neg >> (4 * kc);
+                store_tile<F32, AK, QM>(ra, p.a, a_tile, L::A_TILE, 0, 0u, tg);
+#pragma unroll
+                for (int h = 0; h < 4; h += HALF) {
+                    if (h > 0) {
+#pragma unroll
+                        for (int c = 0; c < HALF; ++c) load_tile<F32, BK, NT>(rb[c], p.b, (h + c) ^ kc, n0, k0, tg);
+                    }
+#pragma unroll
+                    for (int c = 0; c < HALF; ++c)
+                        store_tile<F32, BK, NT>(rb[c], p.b, b_tile, L::B_TILE, (h + c) * NT, ((neg >> (h + c)) & 1u) ? SIGN : 0u, tg);
+                }
+                fence_proxy_async_smem();
+            }
+            __syncwarp();
+            if (lane == 0) mbar_arrive(full_bar + 8 * s);          // also after an expired wait: the MMA thread sees the status word
+        }
+    } else if (lane == 0 && n_stages > 0) {
+        // ------------------------------------------------------------------------------------------ MMA issuer
+        const uint32_t idesc = make_idesc_f16(F32 ? 2 : fmt, QM, L::N, !AK, !BK);
+        constexpr uint32_t KROWS = F32 ? 32 : 64, KSTEP = F32 ? 8 : 16;          // K rows of a stage, K of one MMA
+        constexpr uint32_t AS = (AK ? 32 : KSTEP * Q_ROW_BYTES) >> 4, BS = (BK ? 32 : KSTEP * Q_ROW_BYTES) >> 4;
+        auto desc = [](uint32_t addr, bool kmajor) {
+            return kmajor ? make_desc_kmajor(addr) : (F32 ? make_desc_mn_f32(addr, KROWS * Q_ROW_BYTES) : make_desc_mnmajor(addr, KROWS * Q_ROW_BYTES));
+        };
+        int s = 0, phase = 0;
+        for (int st = 0; st < n_stages; ++st) {
+            if (!mbar_wait_bounded(full_bar + 8 * s, phase, status, ST_Q_MMA)) break;
+            tc_fence_after_sync();
+            const uint32_t a_tile = tiles + s * L::STAGE, b_tile = a_tile + L::A_TILE * (F32 ? 2 : 1);
+            const uint64_t ah = desc(a_tile, AK), bh = desc(b_tile, BK);
+            if (F32) {
+                // stage st adds into accumulator st mod 4; small terms first
+                const uint32_t d = tmem_base + (uint32_t)((st % L::ACCS) * L::N);
+                const uint64_t al = desc(a_tile + L::A_TILE, AK), bl = desc(b_tile + L::B_TILE, BK);
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    mma_tf32_ss(d, al + AS * j, bh + BS * j, idesc, (st >= L::ACCS || j > 0) ? 1u : 0u);
+                    mma_tf32_ss(d, ah + AS * j, bl + BS * j, idesc, 1u);
+                    mma_tf32_ss(d, ah + AS * j, bh + BS * j, idesc, 1u);
+                }
+            } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j)                            // two accumulators in turn
+                    mma_f16_ss(tmem_base + (uint32_t)((j & 1) * L::N), ah + AS * j, bh + BS * j, idesc, (st > 0 || j > 1) ? 1u : 0u);
+            }
+            mma_commit(empty_bar + 8 * s);
+            if (st == n_stages - 1) mma_commit(done_bar);
+            if (++s == L::STAGES) { s = 0; phase ^= 1; }
+        }
+    }
+    __syncwarp();
+
+    // ---------------------------------------------------------------------------------------------- epilogue
+    const int q = warp & 3, half = warp >> 2;                          // TMEM lane quadrant, half of the columns (warps 0 .. 7)
+    if (warp < 8) {
+        if (n_stages > 0) ok = mbar_wait_bounded(done_bar, 0, status, ST_Q_EPILOGUE) && ok;
+        ok = __all_sync(0xffffffffu, ok);
+        tc_fence_after_sync();
+        const int row = q * 32 + lane, m = m0 + row;
+#pragma unroll 1
+        for (int cb = 0; cb < L::N / 2; cb += 32) {
+            const int col0 = half * (L::N / 2) + cb;
+            float sum[32];
+#pragma unroll
+            for (int e = 0; e < 32; ++e) sum[e] = 0.f;
+            if (ok && n_stages > 0) {
+#pragma unroll
+                for (int acc = 0; acc < L::ACCS; ++acc) {
+                    if (F32 && acc >= n_stages) break;                 // fewer stages than accumulators (n_stages is a multiple of 4)
+                    uint32_t v[32];
+                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * L::N) + col0, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) sum[e] += __uint_as_float(v[e]);
+                }
+            }
+            if (split > 1) {
+                // the stages are drained (every MMA has completed), their memory takes the partial tile [column][row]
+#pragma unroll
+                for (int e = 0; e < 32; ++e) st_shared_u32(tiles + (uint32_t)((col0 + e) * QM + row) * 4u, __float_as_uint(sum[e]));
+            } else if (ok && m < p.M) {
+                const int c = col0 / NT, nb = n0 + col0 - c * NT;      // 32 columns lie in one component
+                const float badd = p.bias ? q_bias(p.bias, (size_t)c * p.M + m, fmt) : 0.f;
+#pragma unroll
+                for (int e = 0; e < 32; ++e)
+                    if (nb + e < p.N) q_store(p.out, (size_t)c * p.o_c + (size_t)(nb + e) * p.o_n + m, sum[e] + badd, fmt);
+            }
+        }
+        tc_fence_before_sync();
+    }
+    if (cluster > 1) {
+        q_cluster_sync();
+        if (split > 1 && t < Q_LOADERS) {
+            // every CTA of the tile finishes N / split columns: the partial tiles are added in rank order, four columns at a time
+            // so that their reads from the other SMs overlap
+            const bool good = *reinterpret_cast<volatile int*>(status) == 0;
+            const int row = t % QM, m = m0 + row, cols = L::N / split, col_beg = rank * cols;
+            const uint32_t peer0 = q_cluster_rank() - (uint32_t)rank;
+            constexpr int BATCH = 4;
+            if (good && m < p.M) {
+                for (int col = col_beg + (t / QM) * BATCH; col < col_beg + cols; col += Q_GROUPS * BATCH) {
+                    float v[BATCH][8];
+#pragma unroll
+                    for (int e = 0; e < BATCH; ++e)
+#pragma unroll
+                        for (int r = 0; r < 8; ++r)
+                            v[e][r] = r < split ? ld_cluster_f32(tiles + (uint32_t)((col + e) * QM + row) * 4u, peer0 + r) : 0.f;
+                    const int c = col / NT;                            // cols and NT are multiples of BATCH: one component
+                    const float badd = p.bias ? q_bias(p.bias, (size_t)c * p.M + m, fmt) : 0.f;
+#pragma unroll
+                    for (int e = 0; e < BATCH; ++e) {
+                        const int n = n0 + col + e - c * NT;
+                        float sum = badd;
+#pragma unroll
+                        for (int r = 0; r < 8; ++r) sum += v[e][r];
+                        if (n < p.N) q_store(p.out, (size_t)c * p.o_c + (size_t)n * p.o_n + m, sum, fmt);
+                    }
+                }
+            }
+        }
+        q_cluster_sync();                                              // nobody leaves while its partial tile is still read
+    }
+}
+
+// PAIR: prob[0] has layouts (AK, BK), prob[1] (AK1, BK1) -- both gradients of a dense layer in one launch.
+template <bool F32, int NT, bool AK, bool BK, bool PAIR, bool AK1, bool BK1>
+__global__ void __launch_bounds__(Q_THREADS, 1) qgemm_tc_kernel(const __grid_constant__ QParams p, int* __restrict__ status) {
+    typedef QLayout<F32, NT> L;
+    extern __shared__ uint8_t smem_raw[];
+    const int t = threadIdx.x, warp = t >> 5;
+    uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::BODY);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * Q_MAX_STAGES + 1);
+    const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + Q_MAX_STAGES), done_bar = smem_u32(bars + 2 * Q_MAX_STAGES);
+    if (t == 0) {
+        for (int s = 0; s < L::STAGES; ++s) { mbar_init(full_bar + 8 * s, Q_GROUP / 32); mbar_init(empty_bar + 8 * s, 1); }
+        mbar_init(done_bar, 1);
+        fence_barrier_init();
+    }
+    if (warp == Q_LOADERS / 32) tmem_alloc(smem_u32(tmem_slot), L::ACCS * L::N);
+    tc_fence_before_sync();
+    __syncthreads();
+    tc_fence_after_sync();
+    const uint32_t tmem_base = *tmem_slot;
+    const int block = blockIdx.x;
+    if (!PAIR || block < p.first_blocks)
+        q_tile<F32, NT, AK, BK>(p.prob[0], block, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, status);
+    else
+        q_tile<F32, NT, AK1, BK1>(p.prob[1], block - p.first_blocks, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, status);
+    tc_fence_before_sync();
+    __syncthreads();
+    if (warp == Q_LOADERS / 32) tmem_dealloc(tmem_base, L::ACCS * L::N);
+}
+
+template <bool F32, int NT, bool AK, bool BK, bool PAIR, bool AK1, bool BK1>
+int q_launch(const QParams& p, int blocks, int* status, cudaStream_t stream) {
+    typedef QLayout<F32, NT> L;
+    auto* kernel = qgemm_tc_kernel<F32, NT, AK, BK, PAIR, AK1, BK1>;
+    PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM));
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)blocks);
+    cfg.blockDim = dim3(Q_THREADS);
+    cfg.dynamicSmemBytes = L::SMEM;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)p.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    PCB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, status));
+    return PCB_OK;
+}
+
+// Bytes per load of an operand whose rows start `ld` elements apart and whose components lie `cs` elements apart.
+int q_chunk(const void* ptr, int ld, int cs, int es) {
+    int c = 16;
+    while (c > es && ((size_t)ld * es % c != 0 || (size_t)cs * es % c != 0 || reinterpret_cast<uintptr_t>(ptr) % c != 0)) c >>= 1;
+    return c;
+}
+QOperand q_operand(const void* ptr, int cs, int ld, int nu, int nv, int f32) {
+    QOperand o;
+    o.p = ptr; o.cs = cs; o.ld = ld; o.nu = nu; o.nv = nv; o.chunk = q_chunk(ptr, ld, cs, f32 ? 4 : 2);
+    return o;
+}
+void q_finish(QProblem& p, int NT, int f32, uint32_t neg) {
+    p.tiles_m = (p.M + QM - 1) / QM;
+    p.tiles_n = (p.N + NT - 1) / NT;
+    p.chunks = (p.K + (f32 ? 32 : 64) - 1) / (f32 ? 32 : 64);
+    p.neg = neg;
+}
+uint32_t q_signs(Pass pass) {
+    uint32_t neg = 0;
+    for (int kc = 0; kc < 4; ++kc)
+        for (int c = 0; c < 4; ++c) {
+            const bool n = pass == PASS_FWD ? quat_negative(c ^ kc, c) : (pass == PASS_BWD_DATA ? quat_negative(c, c ^ kc) : quat_negative(c ^ kc, kc));
+            if (n) neg |= 1u << (4 * kc + c);
+        }
+    return neg;
+}
+// Picks the slices of the reduced dimension of the one or two problems of a launch, and the cluster that holds them: powers of
+// two up to 8 (a portable cluster). The cost of a choice is rounds of the machine x (stages of the longest CTA + the fixed part
+// of a CTA, about as long as 6 stages). A cluster lies inside one group of 16 to 20 SMs and every CTA takes an SM, so clusters
+// of 4 and 8 fill only about 7/8 of the SMs at once. fp32: every slice short enough for its accumulators.
+int q_plan(QParams& p, bool two, int f32) {
+    long long best = -1;
+    int blocks = 0;
+    QProblem &a = p.prob[0], &b = p.prob[1];
+    const int most = Q_F32_STAGES_PER_ACC * Q_F32_ACCS / 4;            // chunks of an fp32 slice
+    const int ta = a.tiles_m * a.tiles_n, tb = two ? b.tiles_m * b.tiles_n : 0;
+    int sa_best = 1, sb_best = 1;
+    for (int sa = 1; sa <= 8; sa *= 2)
+        for (int sb = 1; sb <= (two ? 8 : 1); sb *= 2) {
+            const int la = (a.chunks + sa - 1) / sa, lb = two ? (b.chunks + sb - 1) / sb : 0;
+            if ((sa > 1 && sa > a.chunks) || (two && sb > 1 && sb > b.chunks)) continue;
+            if (f32 && (la > most || lb > most)) continue;
+            const int cl = sa > sb ? sa : sb;
+            const int na = round_up(ta * sa, cl), nb = round_up(tb * sb, cl), slots = cl > 2 ? sm_count() * 7 / 8 / cl * cl : sm_count() / cl * cl;
+            if (slots < cl) continue;
+            const long long cost = (long long)((na + nb + slots - 1) / slots) * ((la > lb ? la : lb) * 4 + 6 + (cl > 1 ? 1 : 0));
+            if (best < 0 || cost < best) { best = cost; sa_best = sa; sb_best = sb; p.cluster = cl; p.first_blocks = na; blocks = na + nb; }
+        }
+    a.split = sa_best;
+    b.split = sb_best;
+    return blocks;
+}
+
+QProblem dense_problem(Pass pass, const Geom& g, const void* x, const void* w, const void* dy, const void* bias, void* out, int NT, int f32) {
+    QProblem p;
+    const int I = g.Ci, O = g.Co, B = g.Nb;
+    p.out = out; p.bias = nullptr;
+    if (pass == PASS_FWD) {
+        p.M = O; p.N = B; p.K = I;
+        p.a = g.w_io ? q_operand(w, I * O, O, O, I, f32) : q_operand(w, I * O, I, I, O, f32);
+        p.b = q_operand(x, B * I, I, I, B, f32);
+        p.o_c = B * O; p.o_n = O;
+        p.bias = g.has_bias ? bias : nullptr;
+    } else if (pass == PASS_BWD_DATA) {
+        p.M = I; p.N = B; p.K = O;
+        p.a = g.w_io ? q_operand(w, I * O, O, O, I, f32) : q_operand(w, I * O, I, I, O, f32);
+        p.b = q_operand(dy, B * O, O, O, B, f32);
+        p.o_c = B * I; p.o_n = I;
+    } else {
+        p.M = O; p.N = I; p.K = B;
+        p.a = q_operand(dy, B * O, O, O, B, f32);
+        p.b = q_operand(x, B * I, I, I, B, f32);
+        p.o_c = I * O; p.o_n = O;
+    }
+    p.split = 1;
+    q_finish(p, NT, f32, q_signs(pass));
+    return p;
+}
+int q_tiles(const QProblem& p) { return p.tiles_m * p.tiles_n; }
+
+}  // namespace
+
+// fp32: a slice of the reduced dimension is at most 8 chunks of 32 long (q_plan), and there are at most 8 slices.
+bool dense_tc_supported(int dtype, int variant, const Geom& g) {
+    if (variant != PCB_VARIANT_16_PRODUCT || g.nc != 4 || g.real_in) return false;
+    if (g.H != 1 || g.W != 1 || g.KH != 1 || g.KW != 1 || !g.dw_io || g.groups != 1) return false;
+    const int most = 8 * Q_F32_STAGES_PER_ACC * Q_F32_ACCS / 4 * 32;
+    if (dtype == PCB_F32 && (g.Ci > most || g.Co > most || g.Nb > most)) return false;
+    return true;
+}
+
+int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream) {
+    const int f32 = dtype == PCB_F32;
+    QParams p;
+    p.fmt = f32 ? 2 : (dtype == PCB_F16 ? 0 : 1);
+    p.prob[0] = dense_problem(PASS_FWD, g, x, w, nullptr, bias, y, 32, f32);
+    const bool wide = !f32 && q_tiles(p.prob[0]) > sm_count();
+    if (wide) p.prob[0] = dense_problem(PASS_FWD, g, x, w, nullptr, bias, y, 64, f32);
+    p.prob[1] = p.prob[0];
+    const int blocks = q_plan(p, false, f32);
+    if (blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
+    if (f32) return g.w_io ? q_launch<true, 32, false, true, false, false, false>(p, blocks, status, stream)
+                           : q_launch<true, 32, true, true, false, false, false>(p, blocks, status, stream);
+    if (wide) return g.w_io ? q_launch<false, 64, false, true, false, false, false>(p, blocks, status, stream)
+                            : q_launch<false, 64, true, true, false, false, false>(p, blocks, status, stream);
+    return g.w_io ? q_launch<false, 32, false, true, false, false, false>(p, blocks, status, stream)
+                  : q_launch<false, 32, true, true, false, false, false>(p, blocks, status, stream);
+}
+
+// dw, and dx unless it is null, in one launch.
+int dense_tc_bwd(int dtype, const Geom& g, const void* x, const void* w, const void* dy, void* dw, void* dx, int* status, cudaStream_t stream) {
+    const int f32 = dtype == PCB_F32;
+    QParams p;
+    p.fmt = f32 ? 2 : (dtype == PCB_F16 ? 0 : 1);
+    auto build = [&](int NT) {
+        p.prob[0] = dense_problem(PASS_BWD_FILTER, g, x, w, dy, nullptr, dw, NT, f32);
+        p.prob[1] = dx ? dense_problem(PASS_BWD_DATA, g, x, w, dy, nullptr, dx, NT, f32) : p.prob[0];
+        return q_tiles(p.prob[0]) + (dx ? q_tiles(p.prob[1]) : 0);
+    };
+    int tiles = build(32);
+    const bool wide = !f32 && tiles > sm_count();
+    if (wide) tiles = build(64);
+    const int blocks = q_plan(p, dx != nullptr, f32);
+    if (blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
+    if (!dx) {
+        if (f32) return q_launch<true, 32, false, false, false, false, false>(p, blocks, status, stream);
+        return wide ? q_launch<false, 64, false, false, false, false, false>(p, blocks, status, stream)
+                    : q_launch<false, 32, false, false, false, false, false>(p, blocks, status, stream);
+    }
+    if (f32) return g.w_io ? q_launch<true, 32, false, false, true, true, true>(p, blocks, status, stream)
+                           : q_launch<true, 32, false, false, true, false, true>(p, blocks, status, stream);
+    if (wide) return g.w_io ? q_launch<false, 64, false, false, true, true, true>(p, blocks, status, stream)
+                            : q_launch<false, 64, false, false, true, false, true>(p, blocks, status, stream);
+    return g.w_io ? q_launch<false, 32, false, false, true, true, true>(p, blocks, status, stream)
+                  : q_launch<false, 32, false, false, true, false, true>(p, blocks, status, stream);
+}
+
+}  // namespace pcb
