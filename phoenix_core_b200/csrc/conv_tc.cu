@@ -59,7 +59,9 @@ struct GParams {
     int bias_ld;                 // bias is [components][bias_ld]
     int exact;                   // plane mode with a tile box of exactly PN whole planes (WO x HO x PN pixels, any plane size up to
                                  // 256 pixels): the MMAs are n_cols = PN * WO * HO rounded up to 16 columns wide
-    uint32_t b_tx;               // bytes one activation box brings (plain form)
+    uint32_t b_tx;               // bytes one activation box brings (plain and DUAL forms)
+    int rows_epi;                // NCHW output whose image rows are not 16-byte aligned: stored through shared memory (store_rows)
+    int PT, PL;                  // DUAL form: padding of the strided layer
 };
 constexpr uint32_t G_PLANE_BYTES = GM * GN * 2;      // staging buffer of the plane-mode epilogue
 
@@ -126,16 +128,27 @@ __device__ __forceinline__ void plane_pack_exact(const uint32_t (&v)[32], int co
     }
 }
 
+// 192 KB of operand stages, at most 12
+template <int KS, bool DUAL> constexpr int G_MAX_STAGES = KS == 64 ? (DUAL ? 6 : 4) : (KS == 32 ? (DUAL ? 12 : 8) : 12);
+
 // HALO (KS == 32, stride-1 correlation, tile = 8 x PH pixels of one image): a stage is one 32-channel slice of one
 // component -- the halo tile [Ht][Wt][32 channels] of the output tile and the filter slices of ALL taps -- and every
 // tap's MMAs read the same halo tile at a shifted start address. Per MMA the kernel then moves 5 KB from L2 instead
 // of 12 KB, which is what bounds the plain form.
-template <int KS, bool HALO>
+//
+// DUAL (backward-data of a layer with strides 2 x 2): the input pixels fall into four classes by the parity of row and column,
+// and with r = (a + PT) mod 2, c = (a + PT) div 2 the gradient of row class a is dx[2 i + a] = sum over k of dy[i + c - k] w[r + 2 k]
+// (columns alike) -- every class takes its own taps of the same dy and filters. A tile is one row class and BOTH column
+// classes of 128 x 128 class pixels: a tap kw belongs to column class (kw + PL) mod 2 and its MMAs go to that class's accumulator,
+// and the epilogue interleaves the two accumulators into runs of neighbouring pixels of dx. The layer's FLOPs are executed once
+// (a convolution of a zero-inserted dy executes four times as many) from one compact copy of dy, in one launch. Bound by the
+// operand traffic from L2: 32 KB per four MMAs of 128 x 128 x 16.
+template <int KS, bool HALO, bool DUAL>
 __global__ void __launch_bounds__(G_THREADS, 1)
 qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GParams p,
                         const uint16_t* __restrict__ bias, uint16_t* __restrict__ out, int* __restrict__ status) {
-    constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = GN * KS * 2;
-    constexpr int MAX_STAGES = KS == 64 ? 4 : (KS == 32 ? 8 : 12);     // 192 KB of operand stages
+    constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = (DUAL ? GN / 2 : GN) * KS * 2;
+    constexpr int MAX_STAGES = G_MAX_STAGES<KS, DUAL>;
     const uint32_t STAGE = HALO ? p.stage_bytes : A_BYTES + B_BYTES;
     const int STAGES = p.n_stages;
     const int taps = p.KH * p.KW;
@@ -151,8 +164,10 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     uint8_t* plane_buf = base + STAGES * STAGE + 512;              // plane mode only: [image][128 rows][HO * WO]
 
     const int tiles_px = p.tiles_w * p.tiles_h * p.tiles_n;
-    const int n_tiles = tiles_px * p.tiles_m;
+    const int n_tiles = tiles_px * p.tiles_m * (DUAL ? 2 : 1);
     const int c_steps = p.Cp / KS;
+    // DUAL: the row class with more taps comes first in the tile order
+    const int first_class = p.PT & 1;               // (a + PT) mod 2 == 0: taps 0, 2, ...
     const int n_k = (HALO ? 1 : taps) * p.LK * c_steps;           // stages per tile
 
     if (t == 0) {
@@ -178,6 +193,28 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 const int tw = rest % p.tiles_w; rest /= p.tiles_w;
                 const int th = rest % p.tiles_h;
                 const int tn = rest / p.tiles_h;
+                if (DUAL) {
+                    const int cls = tn / p.tiles_n, a = first_class ^ cls, n0 = (tn - cls * p.tiles_n) * p.PN, m0 = tm * GM;
+                    for (int kh = (a + p.PT) & 1; kh < p.KH && ok; kh += 2) {
+                        const int row = th * p.PH + ((a + p.PT) >> 1) - (kh >> 1);
+                        for (int kw = 0; kw < p.KW && ok; ++kw) {
+                            const int b = (kw + p.PL) & 1, col = tw * p.PW + ((b + p.PL) >> 1) - (kw >> 1);
+                            const int tap = taps - 1 - (kh * p.KW + kw);             // the packed filters hold the taps flipped
+                            for (int l = 0; l < p.LK && ok; ++l) {
+                                for (int cs = 0; cs < c_steps; ++cs) {
+                                    ok = mbar_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+                                    if (!ok) break;
+                                    const uint32_t a_dst = tiles_addr + s * STAGE, bar = full_bar + 8 * s;
+                                    mbar_arrive_expect_tx(bar, A_BYTES + p.b_tx);
+                                    tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, bar);
+                                    tma_load_5d(a_dst + A_BYTES, &map_x, cs * KS, col, row, n0, l, bar);
+                                    if (++s == STAGES) { s = 0; phase ^= 1; }
+                                }
+                            }
+                        }
+                    }
+                    continue;
+                }
                 const int m0 = tm * GM, ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
                 if (HALO) {
                     for (int l = 0; l < p.LK && ok; ++l) {
@@ -217,7 +254,7 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         // time the tensor pipe idles, so there is no warp synchronisation inside and a stage's two descriptors are built once
         // and stepped by adding to the address field of their low words (16-byte units, never carrying out of the field).
         if (lane == 0) {
-            const uint32_t idesc = make_idesc_f16(p.fmt, GM, (HALO || p.exact) ? p.n_cols : GN, false, false);
+            const uint32_t idesc = make_idesc_f16(p.fmt, GM, DUAL ? GN / 2 : ((HALO || p.exact) ? p.n_cols : GN), false, false);
             int s = 0, phase = 0, local_tile = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local_tile) {
@@ -228,6 +265,29 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     tc_fence_after_sync();
                 }
                 const uint32_t d_tmem = tmem_base + buf * GN;
+                if (DUAL) {
+                    const int a = first_class ^ (tile / (tiles_px * p.tiles_m)), kh0 = (a + p.PT) & 1;
+                    const int inner = p.LK * c_steps, steps = (p.KH - kh0 + 1) / 2 * p.KW * inner;
+                    int kw = 0, left = inner, b = p.PL & 1;
+                    uint32_t started = 0;                              // bit b: column class b's accumulator has been written
+                    for (int k = 0; k < steps; ++k) {
+                        ok = mbar_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA);
+                        if (!ok) break;
+                        tc_fence_after_sync();
+                        const uint32_t a_addr = tiles_addr + s * STAGE;
+                        const uint64_t ad = make_desc_kmajor_rows<KS>(a_addr), bd = make_desc_kmajor_rows<KS>(a_addr + A_BYTES);
+#pragma unroll
+                        for (int j = 0; j < KS / 16; ++j)
+                            mma_f16_ss_words(d_tmem + b * (GN / 2), (uint32_t)ad + 2 * j, (uint32_t)(ad >> 32), (uint32_t)bd + 2 * j, (uint32_t)(bd >> 32),
+                                             idesc, (j > 0 || ((started >> b) & 1u)) ? 1u : 0u);
+                        started |= 1u << b;
+                        mma_commit(empty_bar + 8 * s);
+                        if (k == steps - 1) mma_commit(tmem_full + 8 * buf);
+                        if (++s == STAGES) { s = 0; phase ^= 1; }
+                        if (--left == 0) { left = inner; b ^= 1; if (++kw == p.KW) { kw = 0; b = p.PL & 1; } }
+                    }
+                    continue;
+                }
                 for (int k = 0; k < n_k && ok; ++k) {
                     ok = mbar_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA);
                     if (!ok) break;
@@ -267,9 +327,10 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         const int q = warp & 3;                    // TMEM lane quadrant
         const int chalf = (warp - 2) >> 2;         // which 128 of the 256 columns
         const int sv = p.store_vec;                // pixels per store instruction: 16, 8, 4, 2 or 1
-        const bool vec_ok = sv >= 8;
         const bool issuer = warp == 2 && lane == 0;
         const int HWo = p.HO * p.WO;
+        const int ePW = DUAL ? 2 * p.PW : p.PW, eLW = DUAL ? p.lw + 1 : p.lw;
+        constexpr int ROW_STEP = DUAL ? 2 : 1;
         int local_tile = 0, epi_phase = 0;
         bool ok = true;
         // all eight warps meet; bounded like every other wait of the kernel
@@ -286,8 +347,10 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             int rest = tile / p.tiles_m;
             const int tw = rest % p.tiles_w; rest /= p.tiles_w;
             const int th = rest % p.tiles_h;
-            const int tn = rest / p.tiles_h;
-            const int ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
+            int tn = rest / p.tiles_h, cls = 0;
+            if (DUAL) { cls = tn / p.tiles_n; tn -= cls * p.tiles_n; }
+            // DUAL: the two accumulators interleave to rows of 2 PW output pixels, two output rows apart
+            const int ow0 = tw * ePW, oh0 = DUAL ? 2 * th * p.PH + (first_class ^ cls) : th * p.PH, n0 = tn * p.PN;
             const int m = tm * GM + q * 32 + lane;
             const bool row_ok = m < p.Mvalid;
             const int d = row_ok ? m / p.Cout : 0, co = m - d * p.Cout;
@@ -339,9 +402,19 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             for (int cb = 0; cb < 4; ++cb) {
                 uint32_t v[32];
                 const int col0 = chalf * 128 + cb * 32;
-                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * GN + col0, v);
-                tmem_ld_wait();
-                if (!row_ok) continue;
+                if (DUAL) {
+                    uint32_t even[16], odd[16];
+                    const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + buf * GN + col0 / 2;
+                    tmem_ld_32x32b_x16(at, even);
+                    tmem_ld_32x32b_x16(at + GN / 2, odd);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) { v[2 * e] = even[e]; v[2 * e + 1] = odd[e]; }
+                } else {
+                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * GN + col0, v);
+                    tmem_ld_wait();
+                }
+                if (!row_ok && !p.rows_epi) continue;
                 // convert the 32 columns once, then store runs of 16 pixels (32 bytes) where a run stays inside one
                 // output row and rows are 32-byte aligned, runs of 8 pixels (16 bytes) where rows are 16-byte aligned,
                 // single elements otherwise
@@ -351,6 +424,18 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     const float f0 = __uint_as_float(v[2 * e]) + badd, f1 = __uint_as_float(v[2 * e + 1]) + badd;
                     if (p.fmt == 0) { const __half2 h = __floats2half2_rn(f0, f1); packed[e] = *reinterpret_cast<const uint32_t*>(&h); }
                     else { const __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1); packed[e] = *reinterpret_cast<const uint32_t*>(&h); }
+                }
+                if (p.rows_epi) {
+                    const uint32_t tbuf = smem_u32(plane_buf) + (uint32_t)(warp - 2) * EPI_ROWS_BYTES;
+                    const int row_off = row_ok ? (d * p.Nb * p.Cout + co) * HWo : -1;
+                    const int je = col0 + (sv == 1 ? lane : (sv == 2 ? (lane & 15) * 2 : (lane & 7) * 4));
+                    const int wl = je & (ePW - 1), hl = p.lh >= 0 ? ((je >> eLW) & (p.PH - 1)) : (je >> eLW), nl = p.lh >= 0 ? (je >> (eLW + p.lh)) : 0;
+                    const int ow = ow0 + wl, oh = oh0 + hl * ROW_STEP, img = n0 + nl;
+                    const int pix_off = (je < p.n_cols && ow < p.WO && oh < p.HO && img < p.Nb) ? (img * p.Cout * p.HO + oh) * p.WO + ow : -1;
+                    if (sv == 1) store_rows<1>(tbuf, packed, out, row_off, pix_off, lane);
+                    else if (sv == 2) store_rows<2>(tbuf, packed, out, row_off, pix_off, lane);
+                    else store_rows<4>(tbuf, packed, out, row_off, pix_off, lane);
+                    continue;
                 }
                 if (p.o_cl32) {
                     // channels-last output, 32 consecutive channels per warp: the 32 x 32 block goes through 2 KB of shared memory
@@ -369,15 +454,15 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     for (int it = 0; it < 4; ++it) {
                         const int px = it * 8 + (lane >> 2), je = col0 + px;
                         if (je >= p.n_cols) continue;
-                        const int wl = je & (p.PW - 1), hl = p.lh >= 0 ? ((je >> p.lw) & (p.PH - 1)) : (je >> p.lw), nl = p.lh >= 0 ? (je >> (p.lw + p.lh)) : 0;
-                        const int ow = ow0 + wl, oh = oh0 + hl, img = n0 + nl;
+                        const int wl = je & (ePW - 1), hl = p.lh >= 0 ? ((je >> eLW) & (p.PH - 1)) : (je >> eLW), nl = p.lh >= 0 ? (je >> (eLW + p.lh)) : 0;
+                        const int ow = ow0 + wl, oh = oh0 + hl * ROW_STEP, img = n0 + nl;
                         if (ow >= p.WO || oh >= p.HO || img >= p.Nb) continue;
                         const uint4 val = ld_shared_v4(tbuf + px * 64 + (lane & 3) * 16);
                         *reinterpret_cast<uint4*>(out + (size_t)(d0 * p.Nb + img) * p.o_p + (size_t)oh * p.o_h + (size_t)ow * p.o_w + cch) = val;
                     }
                     continue;
                 }
-                const bool wide = !p.o_generic && sv >= 16 && (p.PW % 16) == 0;
+                const bool wide = !p.o_generic && sv >= 16 && (ePW % 16) == 0;
 #pragma unroll
                 for (int g8 = 0; g8 < 4; ++g8) {
                     if (wide && (g8 & 1)) continue;                      // the odd groups were written with their even neighbours
@@ -392,8 +477,8 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                         for (int e = 0; e < 8; ++e) {
                             const int je = j + e;
                             if (je >= p.n_cols) continue;
-                            const int wl = je & (p.PW - 1), hl = p.lh >= 0 ? ((je >> p.lw) & (p.PH - 1)) : (je >> p.lw), nl = p.lh >= 0 ? (je >> (p.lw + p.lh)) : 0;
-                            const int ow = ow0 + wl, oh = oh0 + hl, img = n0 + nl;
+                            const int wl = je & (ePW - 1), hl = p.lh >= 0 ? ((je >> eLW) & (p.PH - 1)) : (je >> eLW), nl = p.lh >= 0 ? (je >> (eLW + p.lh)) : 0;
+                            const int ow = ow0 + wl, oh = oh0 + hl * ROW_STEP, img = n0 + nl;
                             if (ow >= p.WO || oh >= p.HO || img >= p.Nb) continue;
                             out[(size_t)(d * p.Nb + img) * p.o_p + (size_t)co * p.o_c + (size_t)oh * p.o_h + (size_t)ow * p.o_w] =
                                 (uint16_t)((packed[4 * g8 + (e >> 1)] >> ((e & 1) * 16)) & 0xffffu);
@@ -401,26 +486,14 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                         continue;
                     }
                     // PW is a power of two; PH too unless the tile is one image tall (PN == 1, halo mode)
-                    const int wl = j & (p.PW - 1), hl = p.lh >= 0 ? ((j >> p.lw) & (p.PH - 1)) : (j >> p.lw), nl = p.lh >= 0 ? (j >> (p.lw + p.lh)) : 0;
-                    const int ow = ow0 + wl, oh = oh0 + hl, img = n0 + nl;
+                    const int wl = j & (ePW - 1), hl = p.lh >= 0 ? ((j >> eLW) & (p.PH - 1)) : (j >> eLW), nl = p.lh >= 0 ? (j >> (eLW + p.lh)) : 0;
+                    const int ow = ow0 + wl, oh = oh0 + hl * ROW_STEP, img = n0 + nl;
                     if (ow >= p.WO || oh >= p.HO || img >= p.Nb) continue;
                     uint16_t* dst = out + (((size_t)(d * p.Nb + img) * p.Cout + co) * p.HO + oh) * p.WO + ow;
                     if (wide) {
                         st_global_v8(dst, &packed[4 * g8]);
-                    } else if (vec_ok) {
+                    } else {                       // rows are 16-byte aligned (all others: store_rows)
                         *reinterpret_cast<uint4*>(dst) = make_uint4(packed[4 * g8], packed[4 * g8 + 1], packed[4 * g8 + 2], packed[4 * g8 + 3]);
-                    } else if (sv == 4) {          // rows are 8-byte aligned: two 4-pixel stores
-#pragma unroll
-                        for (int h = 0; h < 2; ++h)
-                            if (ow + 4 * h < p.WO) *reinterpret_cast<uint2*>(dst + 4 * h) = make_uint2(packed[4 * g8 + 2 * h], packed[4 * g8 + 2 * h + 1]);
-                    } else if (sv == 2) {          // rows are 4-byte aligned: pixel pairs
-#pragma unroll
-                        for (int h = 0; h < 4; ++h)
-                            if (ow + 2 * h < p.WO) *reinterpret_cast<uint32_t*>(dst + 2 * h) = packed[4 * g8 + h];
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 8; ++e)
-                            if (ow + e < p.WO) dst[e] = (uint16_t)((packed[4 * g8 + (e >> 1)] >> ((e & 1) * 16)) & 0xffffu);
                     }
                 }
             }
@@ -1033,8 +1106,14 @@ struct Plan {
     int Cp, Hp, Wp, Mp, Kp;
     int LK;                        // components of the convolved tensor (1 for a real-valued input)
     int KS;
+    int dual;                      // backward-data with strides 2 x 2 by pixel classes (the kernel's DUAL form)
     size_t xp_bytes, w_bytes;
 };
+
+// Both row and column classes need taps of their own.
+bool dual_classes(Pass pass, const Geom& g) {
+    return pass == PASS_BWD_DATA && g.SH == 2 && g.SW == 2 && g.DH == 1 && g.DW == 1 && g.KH >= 2 && g.KW >= 2;
+}
 
 Plan make_plan(Pass pass, const Geom& g) {
     Plan pl;
@@ -1047,11 +1126,14 @@ Plan make_plan(Pass pass, const Geom& g) {
         pl.pad_top = (g.KH - 1) * g.DH - g.PT; pl.pad_left = (g.KW - 1) * g.DW - g.PL; pl.SH = 1; pl.SW = 1;
         pl.ins_h = g.SH; pl.ins_w = g.SW;
     }
+    pl.dual = dual_classes(pass, g) ? 1 : 0;
+    if (pl.dual) { pl.ins_h = pl.ins_w = 1; pl.pad_top = pl.pad_left = 0; }   // dy as it is: taps past its edges read zeros
     pl.LK = (pass == PASS_FWD && g.real_in) ? 1 : g.nc;
     pl.Cp = round_up(pl.Cin, 16);
     pl.KS = (pl.Cp % 64 == 0) ? 64 : ((pl.Cp % 32 == 0) ? 32 : 16);   // the widest slice: a TMA copy costs about the same whatever its size
     pl.Hp = (pl.Hout - 1) * pl.SH + (g.KH - 1) * g.DH + 1;
     pl.Wp = (pl.Wout - 1) * pl.SW + (g.KW - 1) * g.DW + 1;
+    if (pl.dual) { pl.Hp = pl.Hin; pl.Wp = pl.Win; }
     pl.Mp = round_up(g.nc * pl.Cout, GM);
     pl.Kp = pl.LK * pl.Cp;
     pl.xp_bytes = ((size_t)pl.LK * g.Nb * pl.Hp * pl.Wp * pl.Cp * 2 + 1023) / 1024 * 1024;
@@ -1060,6 +1142,8 @@ Plan make_plan(Pass pass, const Geom& g) {
 }
 
 }  // namespace
+
+bool conv_tc_dual_classes(Pass pass, const Geom& g) { return dual_classes(pass, g); }
 
 bool conv_tc_supported(Pass pass, int dtype, int variant, const Geom& g) {
     if (pass != PASS_FWD && pass != PASS_BWD_DATA) return false;
@@ -1124,9 +1208,20 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         PCB_CUDA_TRY(cudaGetLastError());
     }
 
-    // pick the output tile box (PW x PH x PN = 256 pixels) that wastes the fewest MMA columns
     GParams p;
-    {
+    p.store_vec = 1;
+    while (p.store_vec < 16 && pl.Wout % (p.store_vec * 2) == 0 && (reinterpret_cast<uintptr_t>(out) % (size_t)(p.store_vec * 4)) == 0) p.store_vec *= 2;
+    // pick the output tile box (PW x PH x PN = 256 pixels, DUAL: 128 pixels of a class) that wastes the fewest MMA columns
+    const int Wc = pl.dual ? (pl.Wout + 1) / 2 : pl.Wout, Hc = pl.dual ? (pl.Hout + 1) / 2 : pl.Hout;
+    if (pl.dual) {
+        long long best = -1;
+        for (int pw = 4; pw <= 64; pw *= 2)
+            for (int ph = 1; ph * pw <= GN / 2; ph *= 2) {
+                const int pn = GN / 2 / (pw * ph);
+                const long long vol = (long long)round_up(Wc, pw) * round_up(Hc, ph) * round_up(g.Nb, pn);
+                if (best < 0 || vol < best || (vol == best && pw > p.PW)) { best = vol; p.PW = pw; p.PH = ph; p.PN = pn; }
+            }
+    } else {
         long long best = -1;
         // (dense layers are 1 x 1 images: their box is 1 x 1 x 256, so that the columns of a tile are batch rows and none is wasted)
         const bool dense_like = pl.Wout == 1 && pl.Hout == 1;
@@ -1145,22 +1240,25 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         int pw = 8, ph = 1;
         while (pw < pl.Wout) pw *= 2;
         while (ph < pl.Hout) ph *= 2;
-        if (pw * ph <= 256 && pl.Cout % GM == 0 && pl.Wout % 8 != 0 && !(pl.Wout == 1 && pl.Hout == 1)) { p.PW = pw; p.PH = ph; p.PN = 256 / (pw * ph); }
+        if (!pl.dual && pw * ph <= 256 && pl.Cout % GM == 0 && pl.Wout % 8 != 0 && !(pl.Wout == 1 && pl.Hout == 1)) { p.PW = pw; p.PH = ph; p.PN = 256 / (pw * ph); }
     }
     // Halo mode (see the kernel): stride-1 correlation, 32-channel slices, several taps, and an image tall enough for
     // tiles of 8 x PH >= 192 pixels (smaller tiles re-read the filter slices too often to gain anything).
     // channels-last output with a multiple of 32 channels and 16-byte aligned pixels: the transposing epilogue (16 KB of shared memory)
     const bool cl32 = !g.plain && so.c == 1 && pl.Cout % 32 == 0 && so.w % 8 == 0 && so.h % 8 == 0 && so.p % 8 == 0 &&
                       (reinterpret_cast<uintptr_t>(out) & 15u) == 0;
-    constexpr int CL32_BYTES = 8 * 2048;
+    constexpr int CL32_BYTES = 8 * 2048, ROWS_BYTES = 8 * EPI_ROWS_BYTES;
+    // shared memory of the epilogue beside the operand stages (plane mode has its own)
+    const bool unaligned_rows = g.plain && p.store_vec < 8;
+    const int epi_bytes = cl32 ? CL32_BYTES : (unaligned_rows ? ROWS_BYTES : 0);
     bool halo = false;
     p.n_cols = 256; p.Wt = p.Ht = 0; p.n_stages = 0; p.stage_bytes = 0;
-    if (pl.Cp % 32 == 0 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
+    if (!pl.dual && pl.Cp % 32 == 0 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
         const int rows = (pl.Hout + 31) / 32;
         const int ph = (((pl.Hout + rows - 1) / rows) + 1) & ~1;
         const int wt = 8 + (g.KW - 1) * g.DW, ht = ph + (g.KH - 1) * g.DH;
         const uint32_t stage = ((uint32_t)taps * GM * 32 * 2 + (uint32_t)wt * ht * 64 + 1023) / 1024 * 1024;
-        const int n_stages = (int)((227 * 1024 - 1024 - 512 - (cl32 ? CL32_BYTES : 0)) / stage);
+        const int n_stages = (int)((227 * 1024 - 1024 - 512 - epi_bytes) / stage);
         if (ph >= 24 && wt <= 256 && ht <= 256 && taps <= 256 && n_stages >= 2) {
             halo = true;
             p.PW = 8; p.PH = ph; p.PN = 1; p.n_cols = 8 * ph; p.Wt = wt; p.Ht = ht;
@@ -1173,18 +1271,18 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     }
     // plane mode (see the epilogue): whole output planes per tile, 128 rows = 128 consecutive channels of one component
     // strided output: anything but a dense NCHW tensor, and the narrow boxes of dense layers
-    p.o_generic = (!g.plain || p.lw < 3) ? 1 : 0;
+    p.o_generic = (!g.plain || p.lw + pl.dual < 3) ? 1 : 0;
     p.o_cl32 = (cl32 && p.o_generic && p.lw >= 0) ? 1 : 0;
     p.o_p = (int)so.p; p.o_c = (int)so.c; p.o_h = (int)so.h; p.o_w = (int)so.w;
     p.bias_ld = g.bias_ld;
     p.off_w = direct ? -pl.pad_left : 0; p.off_h = direct ? -pl.pad_top : 0;
-    p.plane_mode = (!p.o_generic && !halo && p.PW >= pl.Wout && p.PH >= pl.Hout && pl.Cout % GM == 0 && p.lh >= 0 && (p.lw == 3 || p.lw == 4) &&
+    p.plane_mode = (!p.o_generic && !halo && !pl.dual && p.PW >= pl.Wout && p.PH >= pl.Hout && pl.Cout % GM == 0 && p.lh >= 0 && (p.lw == 3 || p.lw == 4) &&
                     (reinterpret_cast<uintptr_t>(out) & 15u) == 0) ? 1 : 0;
     // Planes of at most 256 pixels: the box is exactly PN whole planes (7 x 7 x 5 = 245 of 256 columns instead of 8 x 8 x 4 with
     // 49 of every 64 in use; 14 x 14 x 1 = 196 columns in MMAs 208 wide instead of 256), and the tile still leaves as one bulk
     // copy per image.
     p.exact = 0;
-    if (!p.o_generic && !halo && pl.Cout % GM == 0 && pl.Hout * pl.Wout <= 256 && pl.Wout <= 256 && pl.Hout <= 256 &&
+    if (!p.o_generic && !halo && !pl.dual && pl.Cout % GM == 0 && pl.Hout * pl.Wout <= 256 && pl.Wout <= 256 && pl.Hout <= 256 &&
         (pl.Wout - 1) * pl.SW + 1 <= 256 && (pl.Hout - 1) * pl.SH + 1 <= 256 && (reinterpret_cast<uintptr_t>(out) & 15u) == 0) {
         const int HWo = pl.Hout * pl.Wout;
         int pn = 256 / HWo;
@@ -1199,20 +1297,23 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
             p.lw = p.lh = 0;
         }
     }
-    p.b_tx = (uint32_t)(p.exact ? p.PW * p.PH * p.PN : GN) * (uint32_t)pl.KS * 2u;
+    p.rows_epi = (unaligned_rows && !p.o_generic && !p.plane_mode) ? 1 : 0;
+    const int b_rows = pl.dual ? GN / 2 : GN;
+    p.b_tx = (uint32_t)(p.exact ? p.PW * p.PH * p.PN : b_rows) * (uint32_t)pl.KS * 2u;
+    const int tail_bytes = p.plane_mode ? (int)G_PLANE_BYTES : (p.o_cl32 ? CL32_BYTES : (p.rows_epi ? ROWS_BYTES : 0));
     if (!halo) {
-        const int max_stages = pl.KS == 64 ? 4 : (pl.KS == 32 ? 8 : 12);
-        const int fit = (int)((227 * 1024 - 1024 - 512 - (p.plane_mode ? G_PLANE_BYTES : (p.o_cl32 ? CL32_BYTES : 0))) / ((GM + GN) * pl.KS * 2));
+        const int max_stages = pl.KS == 64 ? G_MAX_STAGES<64, false> + 2 * pl.dual : (pl.KS == 32 ? G_MAX_STAGES<32, false> + 4 * pl.dual : G_MAX_STAGES<16, false>);
+        const int fit = (int)((227 * 1024 - 1024 - 512 - tail_bytes) / ((GM + b_rows) * pl.KS * 2));
         p.n_stages = fit < max_stages ? fit : max_stages;
+        p.stage_bytes = (uint32_t)(GM + b_rows) * pl.KS * 2;
     }
     p.Nb = g.Nb; p.Cout = pl.Cout; p.Mvalid = g.nc * pl.Cout; p.HO = pl.Hout; p.WO = pl.Wout; p.Cp = pl.Cp;
     p.KH = g.KH; p.KW = g.KW; p.SH = pl.SH; p.SW = pl.SW; p.DH = g.DH; p.DW = g.DW;
-    p.tiles_w = (pl.Wout + p.PW - 1) / p.PW; p.tiles_h = (pl.Hout + p.PH - 1) / p.PH; p.tiles_n = (g.Nb + p.PN - 1) / p.PN;
+    p.tiles_w = (Wc + p.PW - 1) / p.PW; p.tiles_h = (Hc + p.PH - 1) / p.PH; p.tiles_n = (g.Nb + p.PN - 1) / p.PN;
     p.tiles_m = pl.Mp / GM;
+    p.PT = g.PT; p.PL = g.PL;
     p.fmt = fmt; p.has_bias = (pass == PASS_FWD && g.has_bias) ? 1 : 0;
     p.LK = pl.LK;
-    p.store_vec = 1;
-    while (p.store_vec < 16 && pl.Wout % (p.store_vec * 2) == 0 && (reinterpret_cast<uintptr_t>(out) % (size_t)(p.store_vec * 4)) == 0) p.store_vec *= 2;
 
     const CUtensorMapDataType dt = fmt == 0 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16;
     const int ks = halo ? 32 : pl.KS;
@@ -1242,25 +1343,19 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (activations) failed with code %d", (int)r); return PCB_ERR_CUDA; }
     }
 
-    const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m;
+    const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * (pl.dual ? 2 : 1);
     const int grid = n_tiles < sm_count() ? n_tiles : sm_count();
-    if (halo) {
-        const size_t smem = 1024 + (size_t)p.n_stages * p.stage_bytes + 512 + (p.o_cl32 ? CL32_BYTES : 0);
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tc_kernel<32, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        qconv_general_tc_kernel<32, true><<<grid, G_THREADS, smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
-    } else if (pl.KS == 64) {
-        const size_t smem = 1024 + (size_t)p.n_stages * (GM + GN) * 64 * 2 + 512 + (p.plane_mode ? G_PLANE_BYTES : (p.o_cl32 ? CL32_BYTES : 0));
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tc_kernel<64, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        qconv_general_tc_kernel<64, false><<<grid, G_THREADS, smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
-    } else if (pl.KS == 32) {
-        const size_t smem = 1024 + (size_t)p.n_stages * (GM + GN) * 32 * 2 + 512 + (p.plane_mode ? G_PLANE_BYTES : (p.o_cl32 ? CL32_BYTES : 0));
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tc_kernel<32, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        qconv_general_tc_kernel<32, false><<<grid, G_THREADS, smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
-    } else {
-        const size_t smem = 1024 + (size_t)p.n_stages * (GM + GN) * 16 * 2 + 512 + (p.plane_mode ? G_PLANE_BYTES : (p.o_cl32 ? CL32_BYTES : 0));
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tc_kernel<16, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        qconv_general_tc_kernel<16, false><<<grid, G_THREADS, smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
-    }
+    const size_t smem = 1024 + (size_t)p.n_stages * p.stage_bytes + 512 + tail_bytes;
+    auto run = [&](auto* kernel) -> int {
+        PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        kernel<<<grid, G_THREADS, smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
+        return PCB_OK;
+    };
+    int rc;
+    if (pl.dual) rc = pl.KS == 64 ? run(qconv_general_tc_kernel<64, false, true>) : (pl.KS == 32 ? run(qconv_general_tc_kernel<32, false, true>) : run(qconv_general_tc_kernel<16, false, true>));
+    else if (halo) rc = run(qconv_general_tc_kernel<32, true, false>);
+    else rc = pl.KS == 64 ? run(qconv_general_tc_kernel<64, false, false>) : (pl.KS == 32 ? run(qconv_general_tc_kernel<32, false, false>) : run(qconv_general_tc_kernel<16, false, false>));
+    if (rc != PCB_OK) return rc;
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
@@ -1317,10 +1412,10 @@ bool conv_filter_tc_stages_like_forward(const Geom& g) {
 }
 
 bool conv_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes) {
-    if (!g.plain || g.SH != 1 || g.SW != 1) return false;       // strided layers: backward-data reads a zero-inserted copy
+    const Plan pl = make_plan(PASS_BWD_DATA, g);
+    if (!g.plain || pl.ins_h != 1 || pl.ins_w != 1) return false;   // backward-data reads a zero-inserted copy
     const FilterPlan f = make_filter_plan(g);
     if (channel_block(f.Cop) != f.Cop) return false;            // the filter gradient would block the channels
-    const Plan pl = make_plan(PASS_BWD_DATA, g);
     if (pl.Cp != f.Cop || pl.pad_top < 0 || pl.pad_left < 0) return false;
     view->Hp = pl.Hp; view->Wp = pl.Wp; view->pad_top = pl.pad_top; view->pad_left = pl.pad_left;
     *bytes = pl.xp_bytes;

@@ -500,6 +500,8 @@ int stride_classes(const Geom& g, int dtype, StrideClass* cls, size_t* bytes) {
 
 bool strided_classes_supported(int dtype, int variant, const Geom& g) {
     if (!strided_taps(g)) return false;
+    // 16-bit layers with strides 2 x 2: one launch over all classes (the general kernel's DUAL form)
+    if (dtype != PCB_F32 && conv_tc_dual_classes(PASS_BWD_DATA, g) && conv_tc_supported(PASS_BWD_DATA, dtype, variant, g)) return false;
     StrideClass cls[4];
     size_t bytes;
     const int n = stride_classes(g, dtype, cls, &bytes);
@@ -694,7 +696,8 @@ bool forward_keeps_staged_input(int dtype, int variant, const Geom& g) {
 
 bool backward_shares_staged_dy(int dtype, int variant, const Geom& g, StagedView* view, size_t* bytes) {
     if ((dtype != PCB_F16 && dtype != PCB_BF16) || variant != PCB_VARIANT_16_PRODUCT || !g.plain || g.groups != 1 || g.real_in) return false;
-    if (g.KH * g.KW == 1 || g.SH != 1 || g.SW != 1) return false;
+    if (g.KH * g.KW == 1) return false;
+    if ((g.SH != 1 || g.SW != 1) && !conv_tc_dual_classes(PASS_BWD_DATA, g)) return false;
     // the same order of preference as tensor_launch, for both passes
     if (pointwise_filter_tc_supported(dtype, variant, g)) return false;
     const bool narrow_dat = narrow_tc_supported(PASS_BWD_DATA, dtype, variant, g), narrow_flt = narrow_filter_tc_supported(dtype, variant, g);

@@ -1,0 +1,87 @@
+"""16-bit convolutions at the sizes where two forms of the general kernel end: output planes whose rows are not 16-byte aligned
+(stored through shared memory, 1, 2 or 4 pixels per lane) and the backward-data pass of layers with strides 2 x 2 (pixel
+classes: odd and even planes, every parity of the padding, filters of 2 to 7 taps per axis, classes with few taps)."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import normal, rel_err, uniform
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"f16": 2.0 ** -10, "bf16": 2.0 ** -7}      # half a unit in the last place of max|ref|, twice for the sums' own error
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import gpu_util
+    return gpu_util
+
+
+def _case(gpu, oracle, n, ci, co, h, w, kh, kw, stride, pad, dtype):
+    x = gpu.rounded(uniform(81, (4 * n, ci, h, w)), dtype)
+    f = gpu.rounded(normal(82, (4, co, ci, kh, kw), std=(2.0 / (4 * ci * kh * kw)) ** 0.5), dtype)
+    b = gpu.rounded(uniform(83, (4, co)), dtype)
+    ref = oracle.conv2d_fwd(x, f, b, stride, (1, 1), pad)
+    y = gpu.run_conv_fwd(x, f, b, stride, pad, dtype, "16p", "tensor")
+    dy = gpu.rounded(normal(84, ref.shape), dtype)
+    rdw, rdx = oracle.conv2d_bwd(x, f, dy, stride, (1, 1), pad)
+    dw, dx = gpu.run_conv_bwd(x, f, dy, stride, pad, dtype, "16p", "tensor", True)
+    for got, want, what in ((y, ref, "y"), (dx, rdx, "dx"), (dw, rdw, "dw")):
+        assert np.all(np.isfinite(got)), what
+        assert rel_err(got, want) <= TOL[dtype], (what, rel_err(got, want))
+
+
+# n, ci, co, h, w: widths 1 .. 4 modulo 8, several images per tile, rows past the last output channel, one to three row tiles
+@pytest.mark.parametrize("k", [1, 3])
+@pytest.mark.parametrize("shape", [(1, 24, 40, 45, 37), (3, 32, 17, 27, 26), (2, 64, 33, 30, 44), (5, 40, 48, 9, 11), (7, 20, 24, 5, 7), (2, 80, 100, 13, 19),
+                                   (1, 32, 32, 33, 129), (4, 24, 24, 3, 2)])
+def test_unaligned_rows(gpu, oracle, shape, k):
+    n, ci, co, h, w = shape
+    p = k // 2
+    _case(gpu, oracle, n, ci, co, h, w, k, k, (1, 1), (p, p, p, p), "f16" if k == 3 else "bf16")
+
+
+@pytest.mark.parametrize("pad", [(0, 0, 0, 0), (1, 1, 1, 1), (0, 1, 1, 0), (1, 0, 0, 1)])
+@pytest.mark.parametrize("shape", [(2, 24, 40, 14, 14), (1, 64, 32, 15, 9), (3, 20, 48, 8, 13), (1, 130, 72, 28, 20)])
+def test_stride_two_classes_3x3(gpu, oracle, shape, pad):
+    n, ci, co, h, w = shape
+    _case(gpu, oracle, n, ci, co, h, w, 3, 3, (2, 2), pad, "f16")
+
+
+@pytest.mark.parametrize("taps,pad", [((2, 2), (0, 0, 0, 0)), ((2, 3), (1, 1, 0, 1)), ((5, 5), (2, 2, 2, 2)), ((5, 2), (1, 0, 2, 1)), ((7, 7), (2, 2, 3, 3)),
+                                      ((4, 6), (3, 2, 0, 3))])
+def test_stride_two_classes_filters(gpu, oracle, taps, pad):
+    _case(gpu, oracle, 2, 36, 40, 17, 22, taps[0], taps[1], (2, 2), pad, "bf16")
+
+
+def test_stride_two_classes_channels_last_and_groups(gpu, oracle):
+    import phoenix_core_b200 as pcb
+    n, ci, co, h, w = 2, 32, 48, 13, 18
+    x = gpu.rounded(uniform(91, (4 * n, ci, h, w)), "f16")
+    f = gpu.rounded(normal(92, (4, co, ci, 3, 3), std=0.04), "f16")
+    pad = (1, 1, 1, 1)
+    dy = gpu.rounded(normal(93, oracle.conv2d_fwd(x, f, None, (2, 2), (1, 1), pad).shape), "f16")
+    rdw, rdx = oracle.conv2d_bwd(x, f, dy, (2, 2), (1, 1), pad)
+
+    def last(a):
+        return torch.from_numpy(a).permute(0, 2, 3, 1).contiguous().half().cuda()
+
+    wd = torch.from_numpy(f).permute(0, 1, 3, 4, 2).contiguous().half().cuda()
+    xd, gd = last(x), last(dy)
+    desc = pcb.Conv2DBwdDescriptor(tuple(xd.shape), tuple(wd.shape), 2, 1, pcb.Padding.EXPLICIT, pad, 1, pcb.Algebra.QUATERNION, pcb.DataFormat.NHWC,
+                                   pcb.FilterLayout.OHWI, True)
+    dw, dx = torch.full_like(wd, float("nan")), torch.full_like(xd, float("nan"))
+    pcb.conv2DBwd(xd, wd, gd, dw, dx, desc, gpu.context("16p"), gpu.ENGINES["tensor"])
+    assert rel_err(dx.float().cpu().permute(0, 3, 1, 2).numpy(), rdx) <= TOL["f16"]
+    assert rel_err(dw.float().cpu().permute(0, 1, 4, 2, 3).numpy(), rdw) <= TOL["f16"]
+
+    # two groups: each half of the channels on its own (channel slices of NCHW tensors)
+    fg = np.ascontiguousarray(f[:, :, :ci // 2])
+    dwg, dxg = gpu.run_conv_bwd(x, fg, dy, (2, 2), pad, "f16", "16p", "tensor", True, groups=2)
+    for g in range(2):
+        ic, oc = slice(g * ci // 2, (g + 1) * ci // 2), slice(g * co // 2, (g + 1) * co // 2)
+        rdw, rdx = oracle.conv2d_bwd(np.ascontiguousarray(x[:, ic]), np.ascontiguousarray(fg[:, oc]), np.ascontiguousarray(dy[:, oc]), (2, 2), (1, 1), pad)
+        assert rel_err(dxg[:, ic], rdx) <= TOL["f16"] and rel_err(dwg[:, oc], rdw) <= TOL["f16"]
