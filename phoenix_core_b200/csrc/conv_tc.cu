@@ -4,13 +4,13 @@
 // The reference layout (NCHW, components stacked on the batch axis) cannot feed tap-shifted TMA boxes: the
 // innermost TMA coordinate must be a multiple of 16 bytes, and a filter tap shifts the pixel axis by single
 // elements. So a convolution with taps first stages two small-or-cheap things in the caller's workspace:
-//   * the activations, channels-last and zero-padded:  xp[comp][img][hp][wp][c16]   (pack_activations_kernel)
+//   * the activations, channels-last:  xp[comp][img][h][w][c16]   (stage_compact_kernel and others)
 //   * the filters as the signed, permuted real matrix of the Hamilton product, one slab per tap:
 //       Wexp[tap][(d,co)][(l,ci)] = s(l,d) * w[l^d][co][ci][tap]                    (pack_filters_kernel)
 //     (reference sign table src/algebras.cc:28-49; for backward-data the transposed block with flipped taps)
 // and then runs ONE implicit-GEMM kernel: D[(d,co), pixel] = sum over (tap, l, ci). With channels innermost a
 // tap is a shift of the *outer* TMA coordinates (free), stride 2 is the tensor map's element stride, and
-// padding is materialised zeros or TMA out-of-bounds fill. This replaces the 8/16 cuDNN calls and their
+// padding is TMA out-of-bounds fill. This replaces the 8/16 cuDNN calls and their
 // crop / insert / accumulate kernels (src/conv2d.hpp:167-275, :433-562; src/backend/cudnn/conv2d.hpp:280-309,
 // :447-488; src/backend/cudnn/kernels.cu:39-156).
 //
@@ -50,8 +50,8 @@ struct GParams {
     // halo mode
     int Wt, Ht;
     uint32_t stage_bytes;
-    int off_w, off_h;            // added to the pixel coordinates of every activation box: 0 for a staged (padded) copy, minus the
-                                 // padding when the caller's channels-last tensor is read in place (the padding is TMA zero fill)
+    int off_w, off_h;            // added to the pixel coordinates of every activation box: minus the padding (out-of-range coordinates
+                                 // read zeros); 0 for a zero-inserted copy, which holds its padding
     int o_generic;               // the output is addressed through the element strides below (channels-last tensors, channel
     int o_p, o_c, o_h, o_w;      // slices of grouped layers, boxes narrower than 8 pixels): one 16-bit store per element
     int o_cl32;                  // channels-last output whose channel count is a multiple of 32: a warp transposes its 32 rows x 32
@@ -613,23 +613,97 @@ pack_activations_smem_kernel(const T* __restrict__ x, T* __restrict__ xp, int C,
     }
 }
 
-// Host dispatch of the activation staging: the 4- or 2-pixel form where it applies, the general form otherwise.
-// cb > 0 selects the channel-block layout of the filter-gradient kernels (Nb images per component).
-// `ss` = nullptr: a dense NCHW source (the fast forms apply); otherwise its element strides.
+// The staging of dense NCHW tensors: x[plane][C][HW] -> xp[plane][HW][Cp] (blocked == 0) or blocks of 8 U channels with the block
+// index outermost, xp[comp * nblk + block][img][HW][8 U] -- a batched transposition without padding (the tensor maps supply it as
+// zero fill). A CTA takes 1024 / U consecutive pixels (across planes) of one block of 8 U channels: a thread loads V pixels of
+// 8 channels (coalesced along the pixels; V divides HW, so the pixels lie in one plane and the address is aligned), turns them in
+// registers into V 16-byte units of 8 channels, and the units leave through shared memory, 16 U contiguous bytes per
+// pixel. The units' places are permuted inside 128 bytes so that neither side has bank conflicts. Bound by memory: 51 MB of
+// 14 x 14 planes 38 -> 18 us, 28 x 28 planes of 128 channels (103 MB) 56 -> 36 us against a thread per pixel group and 8 channels that
+// wrote its units itself.
+constexpr int STAGE_THREADS = 256, STAGE_UNITS = 1024;
+template <int V, int U>
+__device__ __forceinline__ int stage_unit(int px, int g) {
+    constexpr int LINE = 8 / U > V ? 8 / U : V;                    // pixels that share a permutation
+    return (px * U + g) ^ ((px / LINE) & 7);
+}
+template <int V, int U>
+__global__ void __launch_bounds__(STAGE_THREADS)
+stage_compact_kernel(const uint16_t* __restrict__ x, uint4* __restrict__ xp, unsigned total_px /*planes * HW*/, unsigned HW, int C, int nblk, unsigned Nb, int blocked) {
+    constexpr int TPX = STAGE_UNITS / U;
+    __shared__ uint4 tile[STAGE_UNITS];
+    const unsigned px0 = blockIdx.x * TPX;
+    const int c0 = blockIdx.y * 8 * U;
+#pragma unroll
+    for (int it = 0; it < STAGE_UNITS / V / STAGE_THREADS; ++it) {
+        const int item = threadIdx.x + it * STAGE_THREADS, l = item % (TPX / V), g = item / (TPX / V);
+        const unsigned P = px0 + l * V;
+        uint32_t raw[8][V == 4 ? 2 : 1];
+        const unsigned plane = P / HW;
+        const uint16_t* src = x + ((size_t)plane * C + c0 + 8 * g) * HW + (P - plane * HW);
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const bool ok = P < total_px && c0 + 8 * g + e < C;
+            if (V == 4) {
+                uint2 w = make_uint2(0u, 0u);
+                if (ok) w = __ldg(reinterpret_cast<const uint2*>(src + (size_t)e * HW));
+                raw[e][0] = w.x; raw[e][V == 4 ? 1 : 0] = w.y;
+            } else if (V == 2) {
+                raw[e][0] = ok ? __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)e * HW)) : 0u;
+            } else {
+                raw[e][0] = ok ? (uint32_t)__ldg(src + (size_t)e * HW) : 0u;
+            }
+        }
+#pragma unroll
+        for (int j = 0; j < V; ++j) {
+            uint32_t w[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) w[i] = __byte_perm(raw[2 * i][j / 2], raw[2 * i + 1][j / 2], (j & 1) ? 0x7632 : 0x5410);
+            tile[stage_unit<V, U>(l * V + j, g)] = make_uint4(w[0], w[1], w[2], w[3]);
+        }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < STAGE_UNITS / STAGE_THREADS; ++it) {
+        const int i = threadIdx.x + it * STAGE_THREADS, px = i / U, g = i % U;
+        const unsigned P = px0 + px;
+        if (P >= total_px) continue;
+        size_t unit;
+        if (blocked) {
+            const unsigned plane = P / HW, comp = plane / Nb;        // pixel of plane (comp * nblk + block) * Nb + img
+            unit = ((size_t)P + (size_t)(comp * (unsigned)(nblk - 1) + blockIdx.y) * Nb * HW) * U + g;
+        } else {
+            unit = ((size_t)P * nblk + blockIdx.y) * U + g;
+        }
+        xp[unit] = tile[stage_unit<V, U>(px, g)];
+    }
+}
+template <int U>
+void launch_stage_compact(const void* src, void* dst, int planes, int C, int HW, int nblk, int Nb, int blocked, cudaStream_t stream) {
+    const uintptr_t at = reinterpret_cast<uintptr_t>(src);
+    const unsigned total = (unsigned)planes * (unsigned)HW, TPX = STAGE_UNITS / U;
+    const dim3 grid((total + TPX - 1) / TPX, (unsigned)nblk);
+    const uint16_t* x = static_cast<const uint16_t*>(src);
+    uint4* xp = static_cast<uint4*>(dst);
+    if (HW % 4 == 0 && at % 8 == 0) stage_compact_kernel<4, U><<<grid, STAGE_THREADS, 0, stream>>>(x, xp, total, HW, C, nblk, Nb, blocked);
+    else if (HW % 2 == 0 && at % 4 == 0) stage_compact_kernel<2, U><<<grid, STAGE_THREADS, 0, stream>>>(x, xp, total, HW, C, nblk, Nb, blocked);
+    else stage_compact_kernel<1, U><<<grid, STAGE_THREADS, 0, stream>>>(x, xp, total, HW, C, nblk, Nb, blocked);
+}
+int channel_block(int cp) { return cp % 64 == 0 ? 64 : (cp % 32 == 0 ? 32 : 16); }
+
+// Host dispatch of the activation staging. cb > 0 selects the channel-block layout of the filter-gradient kernels (Nb images per
+// component). `ss` = nullptr: a dense NCHW source (the fast forms apply); otherwise its element strides.
 void stage_activations(int fmt, const void* src, void* dst, int planes, int C, int H, int W, int Hp, int Wp, int Cp, int pad_top, int pad_left,
                        int ins_h, int ins_w, cudaStream_t stream, int cb = 0, int Nb = 1, const SrcStrides* ss = nullptr) {
     const size_t total = (size_t)planes * Hp * Wp * (Cp / 8);
-    const int px = ss ? 0 : pack_rows_px(src, W, Wp, pad_left, ins_h, ins_w);
     const SrcStrides dense = {(long long)C * H * W, (long long)H * W, (long long)W, 1};
     const SrcStrides st = ss ? *ss : dense;
-    if (px == 4) {
-        const int blocks = grid_cap(total / 4 + 1, 256, 16);
-        if (fmt == 0) pack_rows_kernel<__half, 4><<<blocks, 256, 0, stream>>>((const __half*)src, (__half*)dst, planes, C, H, W, Hp, Wp, Cp / 8, pad_top, pad_left, 0, cb, Nb);
-        else pack_rows_kernel<__nv_bfloat16, 4><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)src, (__nv_bfloat16*)dst, planes, C, H, W, Hp, Wp, Cp / 8, pad_top, pad_left, 0, cb, Nb);
-    } else if (px == 2) {
-        const int blocks = grid_cap(total / 2 + 1, 256, 16);
-        if (fmt == 0) pack_rows_kernel<__half, 2><<<blocks, 256, 0, stream>>>((const __half*)src, (__half*)dst, planes, C, H, W, Hp, Wp, Cp / 8, pad_top, pad_left, 0, cb, Nb);
-        else pack_rows_kernel<__nv_bfloat16, 2><<<blocks, 256, 0, stream>>>((const __nv_bfloat16*)src, (__nv_bfloat16*)dst, planes, C, H, W, Hp, Wp, Cp / 8, pad_top, pad_left, 0, cb, Nb);
+    const bool compact = Hp == H && Wp == W && pad_top == 0 && pad_left == 0 && ins_h == 1 && ins_w == 1;
+    if (!ss && compact && H * W >= 16) {                            // (tiny planes: consecutive pixels are C elements apart)
+        const int block = channel_block(Cp);
+        if (block == 64) launch_stage_compact<8>(src, dst, planes, C, H * W, Cp / block, Nb, cb > 0, stream);
+        else if (block == 32) launch_stage_compact<4>(src, dst, planes, C, H * W, Cp / block, Nb, cb > 0, stream);
+        else launch_stage_compact<2>(src, dst, planes, C, H * W, Cp / block, Nb, cb > 0, stream);
     } else if (!ss && (size_t)C * H * W * 2 <= PACK_SMEM_MAX_BYTES && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
         const size_t smem = ((size_t)C * H * W * 2 + 15) / 16 * 16;
         const int scatter = (ins_h > 1 || ins_w > 1) ? 1 : 0;
@@ -800,8 +874,7 @@ struct FGParams {
     int TPG;                      // x-major variant: taps stacked along M per work item
     int nc, ga;                   // algebra: components, GA(3,0,0) component order
     unsigned long long neg;       // negative entries of the block, bit (8*l + d)
-    int off_w, off_h;             // added to the pixel coordinates of every x box: 0 for the staged (padded) copy, minus the padding
-                                  // when the caller's channels-last x is read in place
+    int off_w, off_h;             // added to the pixel coordinates of every x box: minus the padding (out-of-range coordinates read zeros)
 };
 
 __device__ __forceinline__ uint64_t make_desc_mn_blocks(uint32_t smem_addr, int cb, uint32_t block_bytes) {
@@ -1100,7 +1173,7 @@ __global__ void unpack_filter_grad_kernel(const float* __restrict__ src, T* __re
 struct Plan {
     int Cin, Cout;                 // channels per component of the convolved / produced tensor
     int Hin, Win, Hout, Wout;
-    int pad_top, pad_left;         // zero padding materialised in the staged copy
+    int pad_top, pad_left;         // zero padding: materialised in a zero-inserted copy, the tensor map's zero fill otherwise
     int SH, SW;
     int ins_h, ins_w;              // zero-insertion factors of the staged copy (strided backward-data)
     int Cp, Hp, Wp, Mp, Kp;
@@ -1127,13 +1200,13 @@ Plan make_plan(Pass pass, const Geom& g) {
         pl.ins_h = g.SH; pl.ins_w = g.SW;
     }
     pl.dual = dual_classes(pass, g) ? 1 : 0;
-    if (pl.dual) { pl.ins_h = pl.ins_w = 1; pl.pad_top = pl.pad_left = 0; }   // dy as it is: taps past its edges read zeros
+    if (pl.dual) { pl.ins_h = pl.ins_w = 1; pl.pad_top = pl.pad_left = 0; }   // (the kernel places the taps itself)
     pl.LK = (pass == PASS_FWD && g.real_in) ? 1 : g.nc;
     pl.Cp = round_up(pl.Cin, 16);
     pl.KS = (pl.Cp % 64 == 0) ? 64 : ((pl.Cp % 32 == 0) ? 32 : 16);   // the widest slice: a TMA copy costs about the same whatever its size
     pl.Hp = (pl.Hout - 1) * pl.SH + (g.KH - 1) * g.DH + 1;
     pl.Wp = (pl.Wout - 1) * pl.SW + (g.KW - 1) * g.DW + 1;
-    if (pl.dual) { pl.Hp = pl.Hin; pl.Wp = pl.Win; }
+    if (pl.ins_h == 1 && pl.ins_w == 1) { pl.Hp = pl.Hin; pl.Wp = pl.Win; }   // the copy is not padded: the tensor map's zero fill is the padding
     pl.Mp = round_up(g.nc * pl.Cout, GM);
     pl.Kp = pl.LK * pl.Cp;
     pl.xp_bytes = ((size_t)pl.LK * g.Nb * pl.Hp * pl.Wp * pl.Cp * 2 + 1023) / 1024 * 1024;
@@ -1156,7 +1229,7 @@ bool conv_tc_supported(Pass pass, int dtype, int variant, const Geom& g) {
         if ((g.KH - 1) * g.DH < g.PT || (g.KW - 1) * g.DW < g.PL) return false;
     }
     const Plan pl = make_plan(pass, g);
-    if (pl.Hp > 65535 || pl.Wp > 65535) return false;
+    if ((long long)(pl.Hout - 1) * pl.SH + (long long)(g.KH - 1) * g.DH > 65534 || (long long)(pl.Wout - 1) * pl.SW + (long long)(g.KW - 1) * g.DW > 65534) return false;
     if ((long long)pl.Wp * pl.Cp * 2 > (1ll << 31) || pl.xp_bytes > (size_t)8 << 30) return false;
     return true;
 }
@@ -1184,18 +1257,17 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     bool direct = !g.plain && sa.c == 1 && sa.w == pl.Cin && sa.h == (long long)pl.Win * pl.Cin && sa.p == (long long)pl.Hin * pl.Win * pl.Cin &&
                   pl.Cin % 16 == 0 && pl.ins_h == 1 && pl.ins_w == 1 && (reinterpret_cast<uintptr_t>(act) & 15u) == 0;
 
+    const bool inserted = pl.ins_h != 1 || pl.ins_w != 1;
+
     // stage the operands
     {
-        const size_t total = (size_t)pl.LK * g.Nb * pl.Hp * pl.Wp * (pl.Cp / 8);
-        const int blocks = (int)((total + 255) / 256 < (size_t)sm_count() * 16 ? (total + 255) / 256 : (size_t)sm_count() * 16);
-        (void)blocks;
         // the filter matrix is packed beside the staging pass, on the side stream (neither reads what the other writes): the
         // side stream is forked off before the staging kernel is enqueued and joined before the convolution kernel
         SideStream& ss = side_stream();
         const cudaStream_t wstream = direct ? stream : ss.fork(stream);
         if (!direct)
-            stage_activations(fmt, act, xp, pl.LK * g.Nb, pl.Cin, pl.Hin, pl.Win, pl.Hp, pl.Wp, pl.Cp, pl.pad_top, pl.pad_left, pl.ins_h, pl.ins_w, stream,
-                              0, 1, g.plain ? nullptr : &sa);
+            stage_activations(fmt, act, xp, pl.LK * g.Nb, pl.Cin, pl.Hin, pl.Win, pl.Hp, pl.Wp, pl.Cp, inserted ? pl.pad_top : 0, inserted ? pl.pad_left : 0,
+                              pl.ins_h, pl.ins_w, stream, 0, 1, g.plain ? nullptr : &sa);
         const FilterStrides fs = {g.wr, g.wo, g.wi, g.wh, g.ww, g.KW};
         if (fmt == 0) {
             pack_filters<__half>((const __half*)w, (__half*)wexp, g.Co, g.Ci, taps, pl.Mp, pl.Kp, pl.Cp, pass == PASS_BWD_DATA ? 1 : 0, g.nc, g.ga, g.neg, fs,
@@ -1275,7 +1347,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     p.o_cl32 = (cl32 && p.o_generic && p.lw >= 0) ? 1 : 0;
     p.o_p = (int)so.p; p.o_c = (int)so.c; p.o_h = (int)so.h; p.o_w = (int)so.w;
     p.bias_ld = g.bias_ld;
-    p.off_w = direct ? -pl.pad_left : 0; p.off_h = direct ? -pl.pad_top : 0;
+    p.off_w = inserted ? 0 : -pl.pad_left; p.off_h = inserted ? 0 : -pl.pad_top;
     p.plane_mode = (!p.o_generic && !halo && !pl.dual && p.PW >= pl.Wout && p.PH >= pl.Hout && pl.Cout % GM == 0 && p.lh >= 0 && (p.lw == 3 || p.lw == 4) &&
                     (reinterpret_cast<uintptr_t>(out) & 15u) == 0) ? 1 : 0;
     // Planes of at most 256 pixels: the box is exactly PN whole planes (7 x 7 x 5 = 245 of 256 columns instead of 8 x 8 x 4 with
@@ -1329,8 +1401,8 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (filters) failed with code %d", (int)r); return PCB_ERR_CUDA; }
     }
     {
-        // staged copy [comp][img][Hp][Wp][Cp], or the caller's channels-last tensor [comp][img][Hin][Win][Cin] read in place
-        const int Wd = direct ? pl.Win : pl.Wp, Hd = direct ? pl.Hin : pl.Hp;
+        // staged copy [comp][img][Hp][Wp][Cp], or the caller's channels-last tensor (the same without padding) read in place
+        const int Wd = pl.Wp, Hd = pl.Hp;
         const cuuint64_t dims[5] = {(cuuint64_t)pl.Cp, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
         const cuuint64_t strides[4] = {(cuuint64_t)pl.Cp * 2, (cuuint64_t)Wd * pl.Cp * 2, (cuuint64_t)Hd * Wd * pl.Cp * 2,
                                        (cuuint64_t)g.Nb * Hd * Wd * pl.Cp * 2};
@@ -1361,10 +1433,8 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
 }
 
 namespace {
-int channel_block(int cp) { return cp % 64 == 0 ? 64 : (cp % 32 == 0 ? 32 : 16); }
-
 struct FilterPlan {
-    int Cop, Cip, Hp, Wp;
+    int Cop, Cip;
     size_t xp_bytes, dyp_bytes, acc_bytes;
 };
 
@@ -1372,9 +1442,7 @@ FilterPlan make_filter_plan(const Geom& g) {
     FilterPlan f;
     f.Cop = round_up(g.Co, 16);
     f.Cip = round_up(g.Ci, 16);
-    f.Hp = (g.HO - 1) * g.SH + (g.KH - 1) * g.DH + 1;
-    f.Wp = (g.WO - 1) * g.SW + (g.KW - 1) * g.DW + 1;
-    f.xp_bytes = ((size_t)(g.real_in ? 1 : g.nc) * g.Nb * f.Hp * f.Wp * f.Cip * 2 + 1023) / 1024 * 1024;
+    f.xp_bytes = ((size_t)(g.real_in ? 1 : g.nc) * g.Nb * g.H * g.W * f.Cip * 2 + 1023) / 1024 * 1024;
     f.dyp_bytes = ((size_t)g.nc * g.Nb * g.HO * g.WO * f.Cop * 2 + 1023) / 1024 * 1024;
     f.acc_bytes = ((size_t)g.nc * g.Co * g.Ci * g.KH * g.KW * sizeof(float) + 1023) / 1024 * 1024;
     return f;
@@ -1397,7 +1465,8 @@ bool conv_filter_tc_supported(int dtype, int variant, const Geom& g) {
     if (g.real_in && !filter_xmajor(g, make_filter_plan(g))) return false;
     if (g.SH > 2 || g.SW > 2) return false;
     const FilterPlan f = make_filter_plan(g);
-    if (f.Hp > 65535 || f.Wp > 65535 || f.xp_bytes + f.dyp_bytes > (size_t)12 << 30) return false;
+    if ((long long)(g.HO - 1) * g.SH + (long long)(g.KH - 1) * g.DH > 65534 || (long long)(g.WO - 1) * g.SW + (long long)(g.KW - 1) * g.DW > 65534 ||
+        f.xp_bytes + f.dyp_bytes > (size_t)12 << 30) return false;
     return true;
 }
 
@@ -1416,8 +1485,8 @@ bool conv_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes) {
     if (!g.plain || pl.ins_h != 1 || pl.ins_w != 1) return false;   // backward-data reads a zero-inserted copy
     const FilterPlan f = make_filter_plan(g);
     if (channel_block(f.Cop) != f.Cop) return false;            // the filter gradient would block the channels
-    if (pl.Cp != f.Cop || pl.pad_top < 0 || pl.pad_left < 0) return false;
-    view->Hp = pl.Hp; view->Wp = pl.Wp; view->pad_top = pl.pad_top; view->pad_left = pl.pad_left;
+    if (pl.Cp != f.Cop) return false;
+    view->Hp = pl.Hp; view->Wp = pl.Wp; view->pad_top = view->pad_left = 0;
     *bytes = pl.xp_bytes;
     return true;
 }
@@ -1442,13 +1511,9 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
                            channel_block(f.Cop) == g.Co && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
     {   // stage both activations channels-last
         const int lk = g.real_in ? 1 : g.nc;
-        const size_t tx = (size_t)lk * g.Nb * f.Hp * f.Wp * (f.Cip / 8), ty = (size_t)g.nc * g.Nb * g.HO * g.WO * (f.Cop / 8);
-        const size_t cap = (size_t)sm_count() * 16;
-        const int bx = (int)((tx + 255) / 256 < cap ? (tx + 255) / 256 : cap), by = (int)((ty + 255) / 256 < cap ? (ty + 255) / 256 : cap);
-        (void)bx; (void)by;
         const SrcStrides sx = {g.xp, g.xc, g.xh, g.xw}, sy = {g.yp, g.yc, g.yh, g.yw};
         if (!direct_x && !kept_x)
-            stage_activations(fmt, x, xp, lk * g.Nb, g.Ci, g.H, g.W, f.Hp, f.Wp, f.Cip, g.PT, g.PL, 1, 1, stream, channel_block(f.Cip), g.Nb, g.plain ? nullptr : &sx);
+            stage_activations(fmt, x, xp, lk * g.Nb, g.Ci, g.H, g.W, g.H, g.W, f.Cip, 0, 0, 1, 1, stream, channel_block(f.Cip), g.Nb, g.plain ? nullptr : &sx);
         if (!direct_dy && !kept_dy)
             stage_activations(fmt, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, stream, channel_block(f.Cop), g.Nb, g.plain ? nullptr : &sy);
         PCB_CUDA_TRY(cudaGetLastError());
@@ -1475,7 +1540,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     p.n_tiles = (n_cols + GN - 1) / GN;
     p.n_tile_cols = n_cols < GN ? n_cols : GN;           // 4*Cip is a multiple of 64; tiles of a multi-tile problem are full or padded by zero blocks
     p.LK = g.real_in ? 1 : g.nc;
-    p.off_w = direct_x ? -g.PL : 0; p.off_h = direct_x ? -g.PT : 0;
+    p.off_w = -g.PL; p.off_h = -g.PT;
     const bool xmajor = filter_xmajor(g, f);
     p.TPG = xmajor ? GM / (p.LK * p.cbB) : 1;
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
@@ -1510,7 +1575,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
         if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (dy) failed with code %d", (int)r); return PCB_ERR_CUDA; }
     }
     {
-        const int Wd = direct_x ? g.W : f.Wp, Hd = direct_x ? g.H : f.Hp;
+        const int Wd = g.W, Hd = g.H;
         const cuuint64_t dims[5] = {(cuuint64_t)p.cbB, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)(p.LK * (f.Cip / p.cbB))};
         const cuuint64_t strides[4] = {(cuuint64_t)p.cbB * 2, (cuuint64_t)Wd * p.cbB * 2, (cuuint64_t)Hd * Wd * p.cbB * 2,
                                        (cuuint64_t)g.Nb * Hd * Wd * p.cbB * 2};
