@@ -12,8 +12,7 @@
 // The rows m are contiguous in the output of every pass, so the 32 lanes of an epilogue warp store 32 consecutive elements.
 // (replaces the 16 GEMM calls and accumulate passes of the reference, src/dense.hpp:21-379, src/backend/cudnn/dense.hpp:20-218.)
 //
-// Three groups of four warps load (plain loads of the widest type that the rows' alignment allows: feature counts need no
-// alignment, which a tensor map would ask for), expand and store the operands in the tcgen05 layouts, each group its own stages;
+// Three groups of four warps load (plain loads: feature counts need no alignment, which a tensor map would ask for), expand and store the operands in the tcgen05 layouts, each group its own stages;
 // one thread of a thirteenth warp issues the MMAs. fp32 operands are split into hi + lo TF32 numbers on their way
 // (three MMAs per product, as in conv_tf32.cu). The reduced dimension of a tile is cut over the CTAs of a cluster, which add
 // their partial tiles through distributed shared memory in a fixed order (results do not depend on timing, nothing is zeroed or
@@ -44,7 +43,7 @@ struct QOperand {
     const void* p;
     int cs, ld;
     int nu, nv;          // extents of u and v
-    int chunk;           // bytes per load: the largest of 16, 8, 4, 2 that divides every row start
+    int chunk;           // bytes per load: the largest of 16, 8, 4 that divides every row start; 2: unaligned chunks of 16
 };
 struct QProblem {
     QOperand a, b;
@@ -86,7 +85,7 @@ __device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t
 }
 
 // ---- operand tiles ----------------------------------------------------------------------------------------------------------
-// ROWS (m or n) x 128 bytes of K (64 16-bit or 32 fp32 elements), moved by the 128 threads of a loader group in chunks of CB bytes.
+// ROWS (m or n) x 128 bytes of K (64 16-bit or 32 fp32 elements), moved by the 128 threads of a loader group in chunks of CB = 16, 8 or 4 bytes.
 //   KMAJ: u = k. Chunk i of thread t: row t / PER + i * STEP, byte (t % PER) * CB of that row's 128.
 //   else: u = m or n, v = k. Chunk i: k row t / PER + i * STEP, byte (t % PER) * CB of the ROWS elements.
 template <bool F32, bool KMAJ, int ROWS, int CB>
@@ -115,11 +114,8 @@ __device__ __forceinline__ void load_chunks(uint32_t (&r)[ROWS / 4], const QOper
             uint2 w = make_uint2(0u, 0u);
             if (ok) w = __ldg(reinterpret_cast<const uint2*>(q));
             r[2 * i] = w.x; r[2 * i + 1] = w.y;
-        } else if (CB == 4) {
-            r[i] = ok ? __ldg(reinterpret_cast<const uint32_t*>(q)) : 0u;
         } else {
-            const uint32_t w = ok ? (uint32_t)__ldg(reinterpret_cast<const uint16_t*>(q)) : 0u;
-            if (i & 1) r[i / 2] |= w << 16; else r[i / 2] = w;
+            r[i] = ok ? __ldg(reinterpret_cast<const uint32_t*>(q)) : 0u;
         }
     }
 }
@@ -146,16 +142,46 @@ __device__ __forceinline__ void store_chunks(const uint32_t (&r)[ROWS / 4], uint
                   (F32 ? (uint32_t)(((in >> 5) ^ (v & 3)) << 5) + (uint32_t)(in & 31) : (uint32_t)(((in >> 4) ^ (v & 7)) << 4) + (uint32_t)(in & 15));
         }
         uint32_t w[4], lo[4];
-        constexpr int W = CB >= 4 ? CB / 4 : 1;
+        constexpr int W = CB / 4;
 #pragma unroll
         for (int j = 0; j < W; ++j) {
-            w[j] = (CB >= 4 ? r[W * i + j] : ((i & 1) ? r[i / 2] >> 16 : r[i / 2])) ^ flip;
+            w[j] = r[W * i + j] ^ flip;
             if (F32) { lo[j] = tf32_lo(w[j]); w[j] = tf32_hi(w[j]); }
         }
         if (CB == 16) { st_shared_v4(dst, w[0], w[1], w[2], w[3]); if (F32) st_shared_v4(dst + lo_ofs, lo[0], lo[1], lo[2], lo[3]); }
         else if (CB == 8) { st_shared_v2(dst, w[0], w[1]); if (F32) st_shared_v2(dst + lo_ofs, lo[0], lo[1]); }
-        else if (CB == 4) { st_shared_u32(dst, w[0]); if (F32) st_shared_u32(dst + lo_ofs, lo[0]); }
-        else st_shared_u16(dst, (uint16_t)(w[0] & 0xffffu));
+        else { st_shared_u32(dst, w[0]); if (F32) st_shared_u32(dst + lo_ofs, lo[0]); }
+    }
+}
+// 16-bit rows that start at any element, in 16-byte chunks: the aligned 8-byte vectors that hold a chunk are loaded and shifted into
+// place, elements past the row end are cleared. The tensor, four components, is a whole number of such vectors, so one that holds
+// an element never reaches past its end. Against element loads (eight load and eight store instructions per chunk instead of
+// three and one): 974 x 608 -> 431, fp16, forward + backward 231 -> 174 us. (With 4-byte aligned rows the plain 4-byte form is
+// faster, 31 against 37 us for 128 -> 250 at batch 128, and so it is for fp32.)
+template <bool KMAJ, int ROWS>
+__device__ __forceinline__ void load_unaligned(uint32_t (&r)[ROWS / 4], const QOperand& o, int comp, int row0, int k0, int t) {
+    typedef QChunks<false, KMAJ, ROWS, 16> C;
+    const int u = (KMAJ ? k0 : row0) + (t % C::PER) * 8, v0 = (KMAJ ? row0 : k0) + t / C::PER;
+    const int left = o.nu - u, total = 4 * o.cs;                       // valid elements of the chunk; elements of the tensor
+    uint32_t mask[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) mask[j] = (2 * j < left ? 0xffffu : 0u) | (2 * j + 1 < left ? 0xffff0000u : 0u);
+    const int at0 = comp * o.cs + v0 * o.ld + u;
+#pragma unroll
+    for (int i = 0; i < C::COUNT; ++i) {
+        const bool ok = left > 0 && v0 + i * C::STEP < o.nv;
+        const int at = at0 + i * C::STEP * o.ld, al = at & ~3, sh = at & 3;
+        const uint2* q = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(o.p) + al);
+        uint2 a = make_uint2(0u, 0u), b = a, c = a;
+        if (ok) a = __ldg(q);
+        if (ok && al + 4 < total) b = __ldg(q + 1);
+        if (ok && sh && al + 8 < total) c = __ldg(q + 2);
+        uint32_t w[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
+#pragma unroll
+        for (int j = 0; j < 5; ++j) w[j] = (sh & 2) ? w[j + 1] : w[j];
+        const uint32_t sel = (sh & 1) ? 0x5432u : 0x3210u;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) r[4 * i + j] = __byte_perm(w[j], w[j + 1], sel) & mask[j];
     }
 }
 template <bool F32, bool KMAJ, int ROWS>
@@ -163,14 +189,13 @@ __device__ __forceinline__ void load_tile(uint32_t (&r)[ROWS / 4], const QOperan
     if (o.chunk == 16) load_chunks<F32, KMAJ, ROWS, 16>(r, o, comp, row0, k0, t);
     else if (o.chunk == 8) load_chunks<F32, KMAJ, ROWS, 8>(r, o, comp, row0, k0, t);
     else if (F32 || o.chunk == 4) load_chunks<F32, KMAJ, ROWS, 4>(r, o, comp, row0, k0, t);
-    else load_chunks<false, KMAJ, ROWS, 2>(r, o, comp, row0, k0, t);
+    else load_unaligned<KMAJ, ROWS>(r, o, comp, row0, k0, t);
 }
 template <bool F32, bool KMAJ, int ROWS>
 __device__ __forceinline__ void store_tile(const uint32_t (&r)[ROWS / 4], const QOperand& o, uint32_t tile, uint32_t lo_ofs, int row_base, uint32_t flip, int t) {
-    if (o.chunk == 16) store_chunks<F32, KMAJ, ROWS, 16>(r, tile, lo_ofs, row_base, flip, t);
-    else if (o.chunk == 8) store_chunks<F32, KMAJ, ROWS, 8>(r, tile, lo_ofs, row_base, flip, t);
-    else if (F32 || o.chunk == 4) store_chunks<F32, KMAJ, ROWS, 4>(r, tile, lo_ofs, row_base, flip, t);
-    else store_chunks<false, KMAJ, ROWS, 2>(r, tile, lo_ofs, row_base, flip, t);
+    if (o.chunk == 8) store_chunks<F32, KMAJ, ROWS, 8>(r, tile, lo_ofs, row_base, flip, t);
+    else if (o.chunk == 4) store_chunks<F32, KMAJ, ROWS, 4>(r, tile, lo_ofs, row_base, flip, t);
+    else store_chunks<F32, KMAJ, ROWS, 16>(r, tile, lo_ofs, row_base, flip, t);
 }
 // fp32 operand with its rows contiguous along m or n: blocks of 32 rows `block_bytes` apart, groups of 4 K rows 512 bytes apart.
 __device__ __forceinline__ uint64_t make_desc_mn_f32(uint32_t addr, uint32_t block_bytes) {
