@@ -689,7 +689,31 @@ void launch_stage_compact(const void* src, void* dst, int planes, int C, int HW,
     else if (HW % 2 == 0 && at % 4 == 0) stage_compact_kernel<2, U><<<grid, STAGE_THREADS, 0, stream>>>(x, xp, total, HW, C, nblk, Nb, blocked);
     else stage_compact_kernel<1, U><<<grid, STAGE_THREADS, 0, stream>>>(x, xp, total, HW, C, nblk, Nb, blocked);
 }
-int channel_block(int cp) { return cp % 64 == 0 ? 64 : (cp % 32 == 0 ? 32 : 16); }
+// Channels are taken in slices of 64, 32 or 16, and their number is padded to whole slices (zeros in the filter matrix, and in the
+// staged copy or by the zero fill of the tensor map). A TMA copy costs about the same whatever its size and moves rows of one slice,
+// so 16-channel slices are kept for layers of at most 16 channels: 48 channels as one slice of 64 instead of three of 16 take a
+// 3x3 forward pass (44 images of 39 x 47, 40 output channels) from 164 to 105 us although a quarter of the products are zeros.
+int channel_slice(int c) { return c <= 16 ? 16 : (round_up(c, 32) % 64 == 0 ? 64 : 32); }
+int padded_channels(int c) { return round_up(c, channel_slice(c)); }
+
+// Channels-last sources that have to be copied (padded to slices, or cut into blocks of 8 U channels for the filter gradient): 16-byte
+// units, C a multiple of 8. Destination as for stage_compact_kernel.
+__global__ void repack_channels_last_kernel(const uint4* __restrict__ x, uint4* __restrict__ xp, unsigned total_px, unsigned HW, int src_units, int U, int nblk,
+                                            unsigned Nb, int blocked) {
+    const unsigned per_px = (unsigned)(nblk * U);
+    const size_t total = (size_t)total_px * per_px;
+    for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (size_t)gridDim.x * blockDim.x) {
+        const unsigned P = (unsigned)(i / per_px), u = (unsigned)(i - (size_t)P * per_px);
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if ((int)u < src_units) v = __ldg(x + (size_t)P * src_units + u);
+        size_t dst = i;
+        if (blocked) {
+            const unsigned comp = P / HW / Nb, b = u / U;
+            dst = ((size_t)P + (size_t)(comp * (unsigned)(nblk - 1) + b) * Nb * HW) * U + (u - b * U);
+        }
+        xp[dst] = v;
+    }
+}
 
 // Host dispatch of the activation staging. cb > 0 selects the channel-block layout of the filter-gradient kernels (Nb images per
 // component). `ss` = nullptr: a dense NCHW source (the fast forms apply); otherwise its element strides.
@@ -699,8 +723,12 @@ void stage_activations(int fmt, const void* src, void* dst, int planes, int C, i
     const SrcStrides dense = {(long long)C * H * W, (long long)H * W, (long long)W, 1};
     const SrcStrides st = ss ? *ss : dense;
     const bool compact = Hp == H && Wp == W && pad_top == 0 && pad_left == 0 && ins_h == 1 && ins_w == 1;
-    if (!ss && compact && H * W >= 16) {                            // (tiny planes: consecutive pixels are C elements apart)
-        const int block = channel_block(Cp);
+    const int block = channel_slice(C);
+    if (ss && compact && ss->c == 1 && ss->w == C && ss->h == (long long)W * C && ss->p == (long long)H * W * C && C % 8 == 0 &&
+        (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
+        repack_channels_last_kernel<<<grid_cap(total, 256, 16), 256, 0, stream>>>((const uint4*)src, (uint4*)dst, (unsigned)planes * H * W, H * W, C / 8,
+                                                                                  block / 8, Cp / block, Nb, cb > 0);
+    } else if (!ss && compact && H * W >= 16) {                     // (tiny planes: consecutive pixels are C elements apart)
         if (block == 64) launch_stage_compact<8>(src, dst, planes, C, H * W, Cp / block, Nb, cb > 0, stream);
         else if (block == 32) launch_stage_compact<4>(src, dst, planes, C, H * W, Cp / block, Nb, cb > 0, stream);
         else launch_stage_compact<2>(src, dst, planes, C, H * W, Cp / block, Nb, cb > 0, stream);
@@ -1202,8 +1230,8 @@ Plan make_plan(Pass pass, const Geom& g) {
     pl.dual = dual_classes(pass, g) ? 1 : 0;
     if (pl.dual) { pl.ins_h = pl.ins_w = 1; pl.pad_top = pl.pad_left = 0; }   // (the kernel places the taps itself)
     pl.LK = (pass == PASS_FWD && g.real_in) ? 1 : g.nc;
-    pl.Cp = round_up(pl.Cin, 16);
-    pl.KS = (pl.Cp % 64 == 0) ? 64 : ((pl.Cp % 32 == 0) ? 32 : 16);   // the widest slice: a TMA copy costs about the same whatever its size
+    pl.KS = channel_slice(pl.Cin);
+    pl.Cp = padded_channels(pl.Cin);
     pl.Hp = (pl.Hout - 1) * pl.SH + (g.KH - 1) * g.DH + 1;
     pl.Wp = (pl.Wout - 1) * pl.SW + (g.KW - 1) * g.DW + 1;
     if (pl.ins_h == 1 && pl.ins_w == 1) { pl.Hp = pl.Hin; pl.Wp = pl.Win; }   // the copy is not padded: the tensor map's zero fill is the padding
@@ -1252,7 +1280,9 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     const SrcStrides sa = pass == PASS_FWD ? SrcStrides{g.xp, g.xc, g.xh, g.xw} : SrcStrides{g.yp, g.yc, g.yh, g.yw};
     const SrcStrides so = pass == PASS_FWD ? SrcStrides{g.yp, g.yc, g.yh, g.yw} : SrcStrides{g.xp, g.xc, g.xh, g.xw};
     // A channels-last tensor whose channel count is a multiple of 16 already IS the staged layout: it is read in place, the
-    // padding comes from the zero fill of out-of-range TMA coordinates, and no copy of the activations is made at all.
+    // padding (of the image and of the last channel slice) comes from the zero fill of out-of-range TMA coordinates, and no copy of
+    // the activations is made at all. (Other multiples of 8 are copied to padded pixels: a 5x5 layer of 56 channels, 45 x 45, batch 105, takes
+    // 1506 us forward + backward with its 112-byte pixels read in place and 1309 us from a copy with 128-byte pixels.)
     // (Not for zero-inserted gradients, channel slices of grouped layers, or images smaller than a tile box.)
     bool direct = !g.plain && sa.c == 1 && sa.w == pl.Cin && sa.h == (long long)pl.Win * pl.Cin && sa.p == (long long)pl.Hin * pl.Win * pl.Cin &&
                   pl.Cin % 16 == 0 && pl.ins_h == 1 && pl.ins_w == 1 && (reinterpret_cast<uintptr_t>(act) & 15u) == 0;
@@ -1402,10 +1432,9 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     }
     {
         // staged copy [comp][img][Hp][Wp][Cp], or the caller's channels-last tensor (the same without padding) read in place
-        const int Wd = pl.Wp, Hd = pl.Hp;
-        const cuuint64_t dims[5] = {(cuuint64_t)pl.Cp, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
-        const cuuint64_t strides[4] = {(cuuint64_t)pl.Cp * 2, (cuuint64_t)Wd * pl.Cp * 2, (cuuint64_t)Hd * Wd * pl.Cp * 2,
-                                       (cuuint64_t)g.Nb * Hd * Wd * pl.Cp * 2};
+        const int Wd = pl.Wp, Hd = pl.Hp, Cd = direct ? pl.Cin : pl.Cp;
+        const cuuint64_t dims[5] = {(cuuint64_t)Cd, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
+        const cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)Wd * Cd * 2, (cuuint64_t)Hd * Wd * Cd * 2, (cuuint64_t)g.Nb * Hd * Wd * Cd * 2};
         // with an element stride s the box extent is given in input elements: s * (pixels - 1) + 1 of them hold the pixels loaded
         const cuuint32_t box[5] = {(cuuint32_t)ks, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : (p.PH - 1) * pl.SH + 1),
                                    (cuuint32_t)p.PN, 1};
@@ -1440,8 +1469,8 @@ struct FilterPlan {
 
 FilterPlan make_filter_plan(const Geom& g) {
     FilterPlan f;
-    f.Cop = round_up(g.Co, 16);
-    f.Cip = round_up(g.Ci, 16);
+    f.Cop = padded_channels(g.Co);
+    f.Cip = padded_channels(g.Ci);
     f.xp_bytes = ((size_t)(g.real_in ? 1 : g.nc) * g.Nb * g.H * g.W * f.Cip * 2 + 1023) / 1024 * 1024;
     f.dyp_bytes = ((size_t)g.nc * g.Nb * g.HO * g.WO * f.Cop * 2 + 1023) / 1024 * 1024;
     f.acc_bytes = ((size_t)g.nc * g.Co * g.Ci * g.KH * g.KW * sizeof(float) + 1023) / 1024 * 1024;
@@ -1453,16 +1482,21 @@ namespace {
 // x-major variant: one x box per tap must tile M = 128 exactly and dy's (d, co) columns must fit one MMA.
 bool filter_xmajor(const Geom& g, const FilterPlan& f) {
     const int lk = g.real_in ? 1 : g.nc;
-    const int cbx = channel_block(f.Cip), cby = channel_block(f.Cop);
+    const int cbx = channel_slice(g.Ci), cby = channel_slice(g.Co);
     return f.Cip == cbx && f.Cop == cby && lk * cbx <= 64 && g.nc * cby <= 256;
 }
+}  // namespace
+
+namespace {
+// At most 64 channels that fill a block of 16, 32 or 64 to its last 16 (not 33 .. 48, which are padded by more).
+bool one_block(int c) { const int p16 = round_up(c, 16); return p16 == 16 || p16 == 32 || p16 == 64; }
 }  // namespace
 
 bool conv_filter_tc_supported(int dtype, int variant, const Geom& g) {
     if (dtype != PCB_F16 && dtype != PCB_BF16) return false;
     if (variant != PCB_VARIANT_16_PRODUCT) return false;
     if (g.dw_io && g.KH * g.KW != 1) return false;                      // input-major gradient: dense layers
-    if (g.real_in && !filter_xmajor(g, make_filter_plan(g))) return false;
+    if (g.real_in && !(one_block(g.Ci) && one_block(g.Co) && filter_xmajor(g, make_filter_plan(g)))) return false;
     if (g.SH > 2 || g.SW > 2) return false;
     const FilterPlan f = make_filter_plan(g);
     if ((long long)(g.HO - 1) * g.SH + (long long)(g.KH - 1) * g.DH > 65534 || (long long)(g.WO - 1) * g.SW + (long long)(g.KW - 1) * g.DW > 65534 ||
@@ -1477,14 +1511,14 @@ size_t conv_filter_tc_scratch_bytes(const Geom& g) {
 
 bool conv_filter_tc_stages_like_forward(const Geom& g) {
     const FilterPlan f = make_filter_plan(g);
-    return g.plain && channel_block(f.Cip) == f.Cip && f.xp_bytes == make_plan(PASS_FWD, g).xp_bytes;
+    return g.plain && one_block(g.Ci) && f.xp_bytes == make_plan(PASS_FWD, g).xp_bytes;
 }
 
 bool conv_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes) {
     const Plan pl = make_plan(PASS_BWD_DATA, g);
     if (!g.plain || pl.ins_h != 1 || pl.ins_w != 1) return false;   // backward-data reads a zero-inserted copy
     const FilterPlan f = make_filter_plan(g);
-    if (channel_block(f.Cop) != f.Cop) return false;            // the filter gradient would block the channels
+    if (channel_slice(g.Co) != f.Cop) return false;             // the filter gradient would block the channels
     if (pl.Cp != f.Cop) return false;
     view->Hp = pl.Hp; view->Wp = pl.Wp; view->pad_top = view->pad_left = 0;
     *bytes = pl.xp_bytes;
@@ -1503,19 +1537,19 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     uint8_t* dyp = static_cast<uint8_t*>(scratch) + f.xp_bytes;
     float* acc = reinterpret_cast<float*>(dyp + f.dyp_bytes);
 
-    // A channels-last tensor with one channel block per component (16, 32 or 64 channels) already is the staged layout
-    // [component][image][h][w][channels]: it is read in place, x with its padding supplied by out-of-range TMA coordinates.
+    // A channels-last tensor with one channel block per component (at most 64 channels, a multiple of 16) already is the staged layout
+    // [component][image][h][w][channels]: it is read in place, its padding supplied by out-of-range TMA coordinates.
     const bool direct_x = !g.plain && g.xc == 1 && g.xw == g.Ci && g.xh == g.W * g.Ci && (long long)g.xp == (long long)g.H * g.W * g.Ci &&
-                          channel_block(f.Cip) == g.Ci && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+                          channel_slice(g.Ci) == f.Cip && g.Ci % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     const bool direct_dy = !g.plain && g.yc == 1 && g.yw == g.Co && g.yh == g.WO * g.Co && (long long)g.yp == (long long)g.HO * g.WO * g.Co &&
-                           channel_block(f.Cop) == g.Co && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
+                           channel_slice(g.Co) == f.Cop && g.Co % 16 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
     {   // stage both activations channels-last
         const int lk = g.real_in ? 1 : g.nc;
         const SrcStrides sx = {g.xp, g.xc, g.xh, g.xw}, sy = {g.yp, g.yc, g.yh, g.yw};
         if (!direct_x && !kept_x)
-            stage_activations(fmt, x, xp, lk * g.Nb, g.Ci, g.H, g.W, g.H, g.W, f.Cip, 0, 0, 1, 1, stream, channel_block(f.Cip), g.Nb, g.plain ? nullptr : &sx);
+            stage_activations(fmt, x, xp, lk * g.Nb, g.Ci, g.H, g.W, g.H, g.W, f.Cip, 0, 0, 1, 1, stream, channel_slice(g.Ci), g.Nb, g.plain ? nullptr : &sx);
         if (!direct_dy && !kept_dy)
-            stage_activations(fmt, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, stream, channel_block(f.Cop), g.Nb, g.plain ? nullptr : &sy);
+            stage_activations(fmt, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, stream, channel_slice(g.Co), g.Nb, g.plain ? nullptr : &sy);
         PCB_CUDA_TRY(cudaGetLastError());
         PCB_CUDA_TRY(cudaMemsetAsync(acc, 0, (size_t)g.nc * g.Co * g.Ci * taps * sizeof(float), stream));
     }
@@ -1523,7 +1557,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     FGParams p;
     p.nc = g.nc; p.ga = g.ga; p.neg = g.neg;
     p.Nb = g.Nb; p.Co = g.Co; p.Ci = g.Ci; p.HO = g.HO; p.WO = g.WO; p.Cop = f.Cop; p.Cip = f.Cip;
-    p.cbA = channel_block(f.Cop); p.cbB = channel_block(f.Cip);
+    p.cbA = channel_slice(g.Co); p.cbB = channel_slice(g.Ci);
     p.KH = g.KH; p.KW = g.KW; p.SH = g.SH; p.SW = g.SW; p.DH = g.DH; p.DW = g.DW; p.fmt = fmt;
     {   // pixel box of FK pixels wasting the fewest K rows
         long long best = -1;
@@ -1557,9 +1591,10 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     // staged tensors: [component * blocks per component + channel block][image][h][w][cb channels]; the last box extent is
     // the number of channel blocks one tile takes (blocks past the end read as zeros)
     {
-        const cuuint64_t dims[5] = {(cuuint64_t)p.cbA, (cuuint64_t)g.WO, (cuuint64_t)g.HO, (cuuint64_t)g.Nb, (cuuint64_t)(g.nc * (f.Cop / p.cbA))};
-        cuuint64_t strides[4] = {(cuuint64_t)p.cbA * 2, (cuuint64_t)g.WO * p.cbA * 2, (cuuint64_t)g.HO * g.WO * p.cbA * 2,
-                                 (cuuint64_t)g.Nb * g.HO * g.WO * p.cbA * 2};
+        const int Cd = direct_dy ? g.Co : p.cbA;
+        const cuuint64_t dims[5] = {(cuuint64_t)Cd, (cuuint64_t)g.WO, (cuuint64_t)g.HO, (cuuint64_t)g.Nb, (cuuint64_t)(g.nc * (f.Cop / p.cbA))};
+        cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)g.WO * Cd * 2, (cuuint64_t)g.HO * g.WO * Cd * 2,
+                                 (cuuint64_t)g.Nb * g.HO * g.WO * Cd * 2};
         void* dy_base = direct_dy ? const_cast<void*>(dy) : static_cast<void*>(dyp);
         if (kept_dy) {
             // the copy backward-data staged: [d][img][Hp][Wp][Cop] with pixel (0, 0) at (pad_top, pad_left); the map covers the
@@ -1575,10 +1610,10 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
         if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (dy) failed with code %d", (int)r); return PCB_ERR_CUDA; }
     }
     {
-        const int Wd = g.W, Hd = g.H;
-        const cuuint64_t dims[5] = {(cuuint64_t)p.cbB, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)(p.LK * (f.Cip / p.cbB))};
-        const cuuint64_t strides[4] = {(cuuint64_t)p.cbB * 2, (cuuint64_t)Wd * p.cbB * 2, (cuuint64_t)Hd * Wd * p.cbB * 2,
-                                       (cuuint64_t)g.Nb * Hd * Wd * p.cbB * 2};
+        const int Wd = g.W, Hd = g.H, Cd = direct_x ? g.Ci : p.cbB;
+        const cuuint64_t dims[5] = {(cuuint64_t)Cd, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)(p.LK * (f.Cip / p.cbB))};
+        const cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)Wd * Cd * 2, (cuuint64_t)Hd * Wd * Cd * 2,
+                                       (cuuint64_t)g.Nb * Hd * Wd * Cd * 2};
         const cuuint32_t box[5] = {(cuuint32_t)p.cbB, (cuuint32_t)((p.PW - 1) * g.SW + 1), (cuuint32_t)((p.PH - 1) * g.SH + 1), (cuuint32_t)p.PN,
                                    (cuuint32_t)(xmajor ? p.LK : p.n_tile_cols / p.cbB)};
         const cuuint32_t es[5] = {1, (cuuint32_t)g.SW, (cuuint32_t)g.SH, 1, 1};
