@@ -24,8 +24,21 @@ struct PassExtras {
     StagedView dy;
     size_t scratch_offset = 0;
 };
+// The reset of the device status word that an API call owes its workspace before its first kernel. Launches that have a kernel in
+// front of the waiting ones let that kernel do it; everything else calls now() first.
+struct StatusClear {
+    int* word = nullptr;
+    bool pending = false;
+    int now(cudaStream_t stream) {
+        if (!pending) return PCB_OK;
+        pending = false;
+        PCB_CUDA_TRY(cudaMemsetAsync(word, 0, sizeof(int), stream));
+        return PCB_OK;
+    }
+};
+// `sc` (may be null: nothing is owed) is settled before any kernel of the pass can wait.
 int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* a, const void* b, const void* bias,
-                  void* out, float* scratch, int* status, cudaStream_t stream, const PassExtras* extras = nullptr);
+                  void* out, float* scratch, int* status, cudaStream_t stream, const PassExtras* extras = nullptr, StatusClear* sc = nullptr);
 // True when the backward-data pass of this layer stages dy (at the start of its scratch, `bytes` long) in a layout its
 // filter gradient can read through a tensor map: stride-1 layers on the narrow pair of kernels, or on the general pair with
 // one channel block per component. `view` receives the padded geometry (its base is left null).
@@ -62,12 +75,12 @@ size_t conv_tc_scratch_bytes(Pass pass, const Geom& g);
 // Backward-data of a layer with strides 2 x 2 whose pixel classes the kernel takes in one launch (no zero insertion).
 bool conv_tc_dual_classes(Pass pass, const Geom& g);
 int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const void* act, const void* bias, void* out,
-                   void* scratch, int* status, cudaStream_t stream);
+                   void* scratch, int* status, cudaStream_t stream, StatusClear* sc = nullptr);
 
 bool conv_filter_tc_supported(int dtype, int variant, const Geom& g);
 size_t conv_filter_tc_scratch_bytes(const Geom& g);
 int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* x, void* dw, void* scratch, int* status,
-                          cudaStream_t stream, const void* kept_x = nullptr, const StagedView* kept_dy = nullptr);
+                          cudaStream_t stream, const void* kept_x = nullptr, const StagedView* kept_dy = nullptr, StatusClear* sc = nullptr);
 // Geometry of the copy of dy that the general backward-data kernel stages; false when it inserts zeros (strided layers) or
 // the filter gradient would block its channels.
 bool conv_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes);
