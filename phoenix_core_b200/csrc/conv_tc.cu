@@ -618,15 +618,9 @@ pack_activations_smem_kernel(const T* __restrict__ x, T* __restrict__ xp, int C,
 // zero fill). A CTA takes 1024 / U consecutive pixels (across planes) of one block of 8 U channels: a thread loads V pixels of
 // 8 channels (coalesced along the pixels; V divides HW, so the pixels lie in one plane and the address is aligned), turns them in
 // registers into V 16-byte units of 8 channels, and the units leave through shared memory, 16 U contiguous bytes per
-// pixel. The units' places are permuted inside 128 bytes so that neither side has bank conflicts. Bound by memory: 51 MB of
+// pixel. Bound by memory: 51 MB of
 // 14 x 14 planes 38 -> 18 us, 28 x 28 planes of 128 channels (103 MB) 56 -> 36 us against a thread per pixel group and 8 channels that
 // wrote its units itself.
-constexpr int STAGE_THREADS = 256, STAGE_UNITS = 1024;
-template <int V, int U>
-__device__ __forceinline__ int stage_unit(int px, int g) {
-    constexpr int LINE = 8 / U > V ? 8 / U : V;                    // pixels that share a permutation
-    return (px * U + g) ^ ((px / LINE) & 7);
-}
 struct StageJob {
     const void* x;
     void* xp;

@@ -36,6 +36,8 @@ struct TParams {
     int tiles_w, tiles_h, tiles_n, tiles_m;
     int has_bias, LK, store_vec;
     int n_chunks, chunk_len;          // a work item's K range runs in n_chunks pieces of at most chunk_len stages
+    int off_w, off_h;                 // added to the pixel coordinates of every activation box: minus the padding; 0 for a zero-inserted copy
+    int rows_epi;                     // image rows not a multiple of 8 pixels: stored through shared memory (store_rows_f32)
     int splits, k_per_split;          // the K loop of a tile is cut into `splits` work items of k_per_split stages; with more than one
                                       // the partial results meet in the (zeroed) output by fp32 reductions
 };
@@ -97,7 +99,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                 int cs = k0 % c_steps, l = (k0 / c_steps) % p.LK, tap = k0 / (c_steps * p.LK);
                 for (int k = k0; k < k1; ++k, ++it) {
                     const int kh = tap / p.KW, kw = tap - kh * p.KW;
-                    const int wp0 = ow0 * p.SW + kw * p.DW, hp0 = oh0 * p.SH + kh * p.DH;
+                    const int wp0 = ow0 * p.SW + kw * p.DW + p.off_w, hp0 = oh0 * p.SH + kh * p.DH + p.off_h;
                     const int s = it % T_STAGES;
                     ok = mbar_wait_bounded(empty_bar + 8 * s, ((it / T_STAGES) & 1) ^ 1, status, ST_T_PRODUCER);
                     if (!ok) break;
@@ -204,10 +206,22 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                 const int col0 = chalf * 128 + cb * 32;
                 tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * TN + col0, v);
                 tmem_ld_wait();
-                if (!row_ok) continue;
+                if (!row_ok && !p.rows_epi) continue;
 #pragma unroll
                 for (int e = 0; e < 32; ++e)
                     v[e] = __float_as_uint(__uint_as_float(v[e]) + (CHUNKED ? part[cb][e] : 0.f) + badd);
+                if (p.rows_epi) {
+                    const uint32_t rbuf = smem_u32(base) + T_STAGES * T_STAGE + 512 + (uint32_t)(warp - 2) * EPI_ROWS_F32_BYTES;
+                    const int HWo = p.HO * p.WO, je = col0 + (sv == 1 ? lane : (sv == 2 ? (lane & 15) * 2 : (lane & 7) * 4));
+                    const int wl = je % p.PW, hl = (je / p.PW) % p.PH, nl = je / (p.PW * p.PH);
+                    const int ow = ow0 + wl, oh = oh0 + hl, img = n0 + nl;
+                    const int pix_off = (ow < p.WO && oh < p.HO && img < p.Nb) ? (img * p.Cout * p.HO + oh) * p.WO + ow : -1;
+                    const int row_off = row_ok ? (d * p.Nb * p.Cout + co) * HWo : -1;
+                    if (sv == 1) store_rows_f32<1>(rbuf, v, out, row_off, pix_off, lane, reduce);
+                    else if (sv == 2) store_rows_f32<2>(rbuf, v, out, row_off, pix_off, lane, reduce);
+                    else store_rows_f32<4>(rbuf, v, out, row_off, pix_off, lane, reduce);
+                    continue;
+                }
 #pragma unroll
                 for (int g8 = 0; g8 < 4; ++g8) {
                     const int j = col0 + g8 * 8;
@@ -216,32 +230,13 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                     if (p.PW >= 8) {
                         if (ow >= p.WO || oh >= p.HO || img >= p.Nb) continue;
                         float* dst = out + (((size_t)(d * p.Nb + img) * p.Cout + co) * p.HO + oh) * p.WO + ow;
-                        if (reduce) {
-                            if (sv >= 4) {
-#pragma unroll
-                                for (int h = 0; h < 2; ++h)
-                                    if (ow + 4 * h < p.WO)
-                                        red_add_f32x4(dst + 4 * h, __uint_as_float(v[8 * g8 + 4 * h]), __uint_as_float(v[8 * g8 + 4 * h + 1]),
-                                                      __uint_as_float(v[8 * g8 + 4 * h + 2]), __uint_as_float(v[8 * g8 + 4 * h + 3]));
-                            } else {
-#pragma unroll
-                                for (int e = 0; e < 8; ++e)
-                                    if (ow + e < p.WO) atomicAdd(dst + e, __uint_as_float(v[8 * g8 + e]));
-                            }
-                        } else if (sv >= 8) {
-                            st_global_v8(dst, &v[8 * g8]);
-                        } else if (sv == 4) {
+                        if (reduce) {                      // rows of whole 8-pixel runs (all others: store_rows_f32)
 #pragma unroll
                             for (int h = 0; h < 2; ++h)
-                                if (ow + 4 * h < p.WO) *reinterpret_cast<uint4*>(dst + 4 * h) = make_uint4(v[8 * g8 + 4 * h], v[8 * g8 + 4 * h + 1], v[8 * g8 + 4 * h + 2], v[8 * g8 + 4 * h + 3]);
-                        } else if (sv == 2) {
-#pragma unroll
-                            for (int h = 0; h < 4; ++h)
-                                if (ow + 2 * h < p.WO) *reinterpret_cast<uint2*>(dst + 2 * h) = make_uint2(v[8 * g8 + 2 * h], v[8 * g8 + 2 * h + 1]);
+                                red_add_f32x4(dst + 4 * h, __uint_as_float(v[8 * g8 + 4 * h]), __uint_as_float(v[8 * g8 + 4 * h + 1]),
+                                              __uint_as_float(v[8 * g8 + 4 * h + 2]), __uint_as_float(v[8 * g8 + 4 * h + 3]));
                         } else {
-#pragma unroll
-                            for (int e = 0; e < 8; ++e)
-                                if (ow + e < p.WO) dst[e] = __uint_as_float(v[8 * g8 + e]);
+                            st_global_v8(dst, &v[8 * g8]);
                         }
                     } else {
                         // narrow boxes (dense layers: one pixel per image): every column is its own (image, row, pixel)
@@ -363,33 +358,89 @@ __global__ void pack_activations_f32_small_kernel(const float* __restrict__ x, f
     }
 }
 
-void stage_activations_f32(const float* x, float* hi, float* lo, int planes, int C, int H, int W, int Hp, int Wp, int Cp, int pad_top, int pad_left,
-                           int ins_h, int ins_w, int cb, int Nb, cudaStream_t stream) {
-    if (Hp * Wp < 32) {
-        pack_activations_f32_small_kernel<<<grid_cap((size_t)planes * Hp * Wp * (Cp / 4), 256, 16), 256, 0, stream>>>(
-            x, hi, lo, planes, C, H, W, Hp, Wp, Cp, pad_top, pad_left, ins_h, ins_w, cb, Nb);
-    } else {
-        const size_t tiles = (size_t)planes * ((Hp * Wp + 31) / 32);
-        pack_activations_f32_kernel<<<grid_cap(tiles, 1, 16), 256, 0, stream>>>(x, hi, lo, planes, C, H, W, Hp, Wp, Cp, pad_top, pad_left, ins_h,
-                                                                                 ins_w, cb, Nb);
+// ---- everything a call needs before its main kernel, in one launch (as in conv_tc.cu): status word, filters, copies, zeroed output ----
+// Staging of dense NCHW tensors without padding, x[plane][C][HW] -> hi, lo [plane][HW][Cp] (blocked == 0) or blocks of 4 U channels
+// with the block index outermost: the transposition of conv_tc.cu's stage_compact with units of four channels, split into hi and lo
+// where the units leave shared memory.
+struct StageJob32 {
+    const float* x;
+    float *hi, *lo;
+    unsigned total_px, HW, Nb;
+    int C, nblk, U, V, blocked;
+    unsigned bx, blocks;
+};
+template <int V, int U>
+__device__ __forceinline__ void stage_compact_f32(const StageJob32& p, unsigned block, float4* tile /*[STAGE_UNITS]*/) {
+    constexpr int TPX = STAGE_UNITS / U;
+    const unsigned by = block / p.bx, px0 = (block - by * p.bx) * TPX, HW = p.HW;
+    const int c0 = by * 4 * U;
+#pragma unroll
+    for (int it = 0; it < STAGE_UNITS / V / STAGE_THREADS; ++it) {
+        const int item = threadIdx.x + it * STAGE_THREADS, l = item % (TPX / V), g = item / (TPX / V);
+        const unsigned P = px0 + l * V, plane = P / HW;
+        const float* src = p.x + ((size_t)plane * p.C + c0 + 4 * g) * HW + (P - plane * HW);
+        float raw[4][V];
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const bool ok = P < p.total_px && c0 + 4 * g + e < p.C;
+#pragma unroll
+            for (int j = 0; j < V; ++j) raw[e][j] = 0.f;
+            if (!ok) continue;
+            const float* q = src + (size_t)e * HW;
+            if (V == 4) { const float4 f = __ldg(reinterpret_cast<const float4*>(q)); raw[e][0] = f.x; raw[e][V > 1 ? 1 : 0] = f.y; raw[e][V > 2 ? 2 : 0] = f.z; raw[e][V > 3 ? 3 : 0] = f.w; }
+            else if (V == 2) { const float2 f = __ldg(reinterpret_cast<const float2*>(q)); raw[e][0] = f.x; raw[e][V > 1 ? 1 : 0] = f.y; }
+            else raw[e][0] = __ldg(q);
+        }
+#pragma unroll
+        for (int j = 0; j < V; ++j) tile[stage_unit<V, U>(l * V + j, g)] = make_float4(raw[0][j], raw[1][j], raw[2][j], raw[3][j]);
+    }
+    __syncthreads();
+#pragma unroll
+    for (int it = 0; it < STAGE_UNITS / STAGE_THREADS; ++it) {
+        const int i = threadIdx.x + it * STAGE_THREADS, px = i / U, g = i % U;
+        const unsigned P = px0 + px;
+        if (P >= p.total_px) continue;
+        size_t unit;
+        if (p.blocked) unit = ((size_t)P + (size_t)((P / HW / p.Nb) * (unsigned)(p.nblk - 1) + by) * p.Nb * HW) * U + g;
+        else unit = ((size_t)P * p.nblk + by) * U + g;
+        const float4 f = tile[stage_unit<V, U>(px, g)];
+        float4 h, lo;
+        split_tf32(f.x, h.x, lo.x); split_tf32(f.y, h.y, lo.y); split_tf32(f.z, h.z, lo.z); split_tf32(f.w, h.w, lo.w);
+        reinterpret_cast<float4*>(p.hi)[unit] = h;
+        reinterpret_cast<float4*>(p.lo)[unit] = lo;
     }
 }
-
+template <int U>
+__device__ __forceinline__ void stage_compact_f32(const StageJob32& p, unsigned block, float4* tile) {
+    if (p.V == 4) stage_compact_f32<4, U>(p, block, tile);
+    else if (p.V == 2) stage_compact_f32<2, U>(p, block, tile);
+    else stage_compact_f32<1, U>(p, block, tile);
+}
+struct FilterJob32 {
+    const float* w;
+    float *hi, *lo;
+    int Co, Ci, taps, Mp, Kp, Cp, transposed, w_io, nc, ga;
+    unsigned long long neg;
+};
 // Forward:       Wexp[tap][m = d*Co + co][k = l*Cp + ci]  = s(l,d) * w[l^d](co, ci, tap)
 // Backward-data: Wexp[tap][m = l*Ci + ci][k = d*Cop + co] = s(l,d) * w[l^d](co, ci, taps-1-tap)
 // w_io: the filters are stored [r][ci][co] (dense input-major layout, one tap).
-__global__ void pack_filters_f32_kernel(const float* __restrict__ w, float* __restrict__ hi, float* __restrict__ lo, int Co, int Ci, int taps,
-                                        int Mp, int Kp, int Cp, int transposed, int w_io, int nc, int ga, unsigned long long neg) {
+__device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned block, unsigned blocks) {
     // one row (tap, m) of the expanded matrix per block iteration; the row is decoded once and the threads walk k
+    const float* __restrict__ w = p.w;
+    float* __restrict__ hi = p.hi;
+    float* __restrict__ lo = p.lo;
+    const int Co = p.Co, Ci = p.Ci, taps = p.taps, Mp = p.Mp, Kp = p.Kp, Cp = p.Cp, transposed = p.transposed, w_io = p.w_io, nc = p.nc, ga = p.ga;
+    const unsigned long long neg = p.neg;
     const int Cm = transposed ? Ci : Co, Ck = transposed ? Co : Ci;
     const int rows = taps * Mp;
-    for (int row = blockIdx.x; row < rows; row += gridDim.x) {
+    for (int row = block; row < rows; row += blocks) {
         const int tap = row / Mp, m = row - tap * Mp;
         const int cm_comp = m / Cm, cm = m - cm_comp * Cm;
         const int src_tap = transposed ? taps - 1 - tap : tap;
         float* hrow = hi + (size_t)row * Kp;
         float* lrow = lo + (size_t)row * Kp;
-        for (int k = threadIdx.x; k < Kp; k += blockDim.x) {
+        for (int k = threadIdx.x; k < Kp; k += STAGE_THREADS) {
             const int ck_comp = k / Cp, ck = k - ck_comp * Cp;
             float v = 0.f;
             if (cm_comp < nc && ck_comp < nc && ck < Ck) {
@@ -408,6 +459,71 @@ __global__ void pack_filters_f32_kernel(const float* __restrict__ w, float* __re
     }
 }
 
+struct Prologue32 {
+    int* status = nullptr;
+    FilterJob32 filter;
+    StageJob32 stage[2];
+    float4* zero = nullptr;
+    unsigned zero_units = 0, filter_blocks = 0, stage_blocks[2] = {0, 0}, zero_blocks = 0;
+    int n_stages = 0;
+};
+__global__ void __launch_bounds__(STAGE_THREADS) prologue_f32_kernel(const __grid_constant__ Prologue32 p) {
+    __shared__ float4 tile[STAGE_UNITS];
+    unsigned block = blockIdx.x;
+    if (block == 0 && threadIdx.x == 0 && p.status) *p.status = 0;
+    if (block < p.filter_blocks) { pack_filters_f32(p.filter, block, p.filter_blocks); return; }
+    block -= p.filter_blocks;
+    if (block < p.zero_blocks) {
+        for (unsigned i = block * STAGE_THREADS + threadIdx.x; i < p.zero_units; i += p.zero_blocks * STAGE_THREADS) p.zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+        return;
+    }
+    block -= p.zero_blocks;
+    const bool second = block >= p.stage_blocks[0];
+    const StageJob32& job = second ? p.stage[1] : p.stage[0];
+    if (second) block -= p.stage_blocks[0];
+    if (job.U == 8) stage_compact_f32<8>(job, block, tile);
+    else stage_compact_f32<4>(job, block, tile);
+}
+// 16-byte aligned, a multiple of 16 bytes; false otherwise (the caller clears it).
+bool add_zero_job(Prologue32& pro, void* p, size_t bytes) {
+    if ((bytes | reinterpret_cast<uintptr_t>(p)) % 16 != 0 || bytes / 16 > 0x7fffffffull) return false;
+    pro.zero = static_cast<float4*>(p);
+    pro.zero_units = (unsigned)(bytes / 16);
+    pro.zero_blocks = grid_cap(pro.zero_units, 4 * STAGE_THREADS, 4);
+    return true;
+}
+int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream) {
+    const unsigned blocks = pro.filter_blocks + pro.zero_blocks + pro.stage_blocks[0] + pro.stage_blocks[1];
+    if (blocks == 0) return PCB_OK;
+    if (sc && sc->pending) { pro.status = sc->word; sc->pending = false; }
+    prologue_f32_kernel<<<blocks, STAGE_THREADS, 0, stream>>>(pro);
+    PCB_CUDA_TRY(cudaGetLastError());
+    return PCB_OK;
+}
+
+// A job of the prologue launch for unpadded copies, a kernel of its own otherwise (zero-inserted gradients, planes of a few pixels).
+void stage_activations_f32(Prologue32& pro, const float* x, float* hi, float* lo, int planes, int C, int H, int W, int Hp, int Wp, int Cp, int pad_top,
+                           int pad_left, int ins_h, int ins_w, int cb, int Nb, cudaStream_t stream) {
+    if (Hp == H && Wp == W && pad_top == 0 && pad_left == 0 && ins_h == 1 && ins_w == 1 && H * W >= 16) {
+        const int block = Cp % 32 == 0 ? 32 : 16;                  // (cb is 0 or 32, and then Cp a multiple of 32)
+        const uintptr_t at = reinterpret_cast<uintptr_t>(x);
+        StageJob32& j = pro.stage[pro.n_stages];
+        j.x = x; j.hi = hi; j.lo = lo; j.total_px = (unsigned)planes * H * W; j.HW = H * W; j.Nb = Nb;
+        j.C = C; j.U = block / 4; j.nblk = Cp / block; j.blocked = cb > 0;
+        j.V = j.HW % 4 == 0 && at % 16 == 0 ? 4 : (j.HW % 2 == 0 && at % 8 == 0 ? 2 : 1);
+        j.bx = (j.total_px + STAGE_UNITS / j.U - 1) / (STAGE_UNITS / j.U);
+        j.blocks = j.bx * j.nblk;
+        pro.stage_blocks[pro.n_stages++] = j.blocks;
+    } else if (Hp * Wp < 32) {
+        pack_activations_f32_small_kernel<<<grid_cap((size_t)planes * Hp * Wp * (Cp / 4), 256, 16), 256, 0, stream>>>(
+            x, hi, lo, planes, C, H, W, Hp, Wp, Cp, pad_top, pad_left, ins_h, ins_w, cb, Nb);
+    } else {
+        const size_t tiles = (size_t)planes * ((Hp * Wp + 31) / 32);
+        pack_activations_f32_kernel<<<grid_cap(tiles, 1, 16), 256, 0, stream>>>(x, hi, lo, planes, C, H, W, Hp, Wp, Cp, pad_top, pad_left, ins_h,
+                                                                                 ins_w, cb, Nb);
+    }
+}
+
 // ---- backward-filter ------------------------------------------------------------------------------------
 // Both staged tensors MN-major (K = pixels, 16 per stage), M = (d, co), N = (l, ci); per K step of 8 pixels three
 // TF32 MMAs; the epilogue folds G[(d,co),(l,ci)] through the quaternion table into fp32 scratch [tap][r][co][ci].
@@ -419,6 +535,7 @@ struct TFParams {
     int Nb, Co, Ci, HO, WO, Cop, Cip, cbA, cbB;             // channel-block width in fp32 elements: 32
     int KH, KW, SH, SW, DH, DW, PW, PH, PN, tiles_w, tiles_h, tiles_n;
     int m_tiles, n_tiles, n_tile_cols, splits, steps_per_split;
+    int off_w, off_h;             // added to the pixel coordinates of every x box: minus the padding (out-of-range coordinates read zeros)
     int nc, ga;                                              // algebra: components, GA(3,0,0) component order
     unsigned long long neg;                                  // negative entries of the block, bit (8*l + d)
 };
@@ -491,7 +608,7 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
                 mbar_arrive_expect_tx(bar, 2 * (a_bytes + b_bytes));
                 tma_load_5d(a_hi, &map_dy_hi, 0, ow0, oh0, n0, blockA0, bar);
                 tma_load_5d(a_lo, &map_dy_lo, 0, ow0, oh0, n0, blockA0, bar);
-                const int wp0 = ow0 * p.SW + kw * p.DW, hp0 = oh0 * p.SH + kh * p.DH;
+                const int wp0 = ow0 * p.SW + kw * p.DW + p.off_w, hp0 = oh0 * p.SH + kh * p.DH + p.off_h;
                 tma_load_5d(b_hi, &map_x_hi, 0, wp0, hp0, n0, blockB0, bar);
                 tma_load_5d(b_lo, &map_x_lo, 0, wp0, hp0, n0, blockB0, bar);
             }
@@ -643,6 +760,7 @@ Plan32 make_plan32(Pass pass, const Geom& g) {
     pl.Cp = round_up(pl.Cin, 16);
     pl.Hp = (pl.Hout - 1) * pl.SH + (g.KH - 1) * g.DH + 1;
     pl.Wp = (pl.Wout - 1) * pl.SW + (g.KW - 1) * g.DW + 1;
+    if (pl.ins_h == 1 && pl.ins_w == 1) { pl.Hp = pl.Hin; pl.Wp = pl.Win; }   // the copy is not padded: the tensor map's zero fill is the padding
     pl.Mp = round_up(g.nc * pl.Cout, TM);
     pl.Kp = pl.LK * pl.Cp;
     pl.xp_bytes = ((size_t)pl.LK * g.Nb * pl.Hp * pl.Wp * pl.Cp * 4 + 1023) / 1024 * 1024;
@@ -651,7 +769,7 @@ Plan32 make_plan32(Pass pass, const Geom& g) {
 }
 
 struct FilterPlan32 {
-    int Cop, Cip, Hp, Wp;
+    int Cop, Cip;
     size_t xp_bytes, dyp_bytes, acc_bytes;
 };
 
@@ -659,12 +777,15 @@ FilterPlan32 make_filter_plan32(const Geom& g) {
     FilterPlan32 f;
     f.Cop = round_up(g.Co, 32);
     f.Cip = round_up(g.Ci, 32);
-    f.Hp = (g.HO - 1) * g.SH + (g.KH - 1) * g.DH + 1;
-    f.Wp = (g.WO - 1) * g.SW + (g.KW - 1) * g.DW + 1;
-    f.xp_bytes = ((size_t)g.nc * g.Nb * f.Hp * f.Wp * f.Cip * 4 + 1023) / 1024 * 1024;
+    f.xp_bytes = ((size_t)g.nc * g.Nb * g.H * g.W * f.Cip * 4 + 1023) / 1024 * 1024;
     f.dyp_bytes = ((size_t)g.nc * g.Nb * g.HO * g.WO * f.Cop * 4 + 1023) / 1024 * 1024;
     f.acc_bytes = ((size_t)g.nc * g.Co * g.Ci * g.KH * g.KW * 4 + 1023) / 1024 * 1024;
     return f;
+}
+
+// Extents of the padded image, which the tensor-map coordinates span.
+bool extents_ok(const Geom& g, int Hout, int Wout, int SH, int SW) {
+    return (long long)(Hout - 1) * SH + (long long)(g.KH - 1) * g.DH <= 65534 && (long long)(Wout - 1) * SW + (long long)(g.KW - 1) * g.DW <= 65534;
 }
 
 bool common_ok(int dtype, int variant, const Geom& g) {
@@ -681,12 +802,12 @@ bool conv_tf32_supported(Pass pass, int dtype, int variant, const Geom& g) {
     if (pass == PASS_BWD_FILTER) {
         if (g.real_in) return false;
         const FilterPlan32 f = make_filter_plan32(g);
-        return f.Hp <= 65535 && f.Wp <= 65535 && 2 * (f.xp_bytes + f.dyp_bytes) <= ((size_t)16 << 30);
+        return extents_ok(g, g.HO, g.WO, g.SH, g.SW) && 2 * (f.xp_bytes + f.dyp_bytes) <= ((size_t)16 << 30);
     }
     if (g.real_in && pass != PASS_FWD) return false;
     if (pass == PASS_BWD_DATA && ((g.KH - 1) * g.DH < g.PT || (g.KW - 1) * g.DW < g.PL)) return false;
     const Plan32 pl = make_plan32(pass, g);
-    return pl.Hp <= 65535 && pl.Wp <= 65535 && 2 * pl.xp_bytes <= ((size_t)16 << 30);
+    return extents_ok(g, pl.Hout, pl.Wout, pl.SH, pl.SW) && 2 * pl.xp_bytes <= ((size_t)16 << 30);
 }
 
 size_t conv_tf32_scratch_bytes(Pass pass, const Geom& g) {
@@ -698,7 +819,7 @@ size_t conv_tf32_scratch_bytes(Pass pass, const Geom& g) {
     return 2 * (pl.xp_bytes + pl.w_bytes);
 }
 
-static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* x, float* dw, void* scratch, int* status, cudaStream_t stream) {
+static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* x, float* dw, void* scratch, int* status, cudaStream_t stream, StatusClear* sc) {
     const FilterPlan32 f = make_filter_plan32(g);
     const int taps = g.KH * g.KW;
     uint8_t* s8 = static_cast<uint8_t*>(scratch);
@@ -707,16 +828,22 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     float* y_hi = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes);
     float* y_lo = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes + f.dyp_bytes);
     float* acc = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes + 2 * f.dyp_bytes);
-    stage_activations_f32(x, x_hi, x_lo, g.nc * g.Nb, g.Ci, g.H, g.W, f.Hp, f.Wp, f.Cip, g.PT, g.PL, 1, 1, 32, g.Nb, stream);
-    stage_activations_f32(dy, y_hi, y_lo, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, 32, g.Nb, stream);
+    Prologue32 pro;
+    stage_activations_f32(pro, x, x_hi, x_lo, g.nc * g.Nb, g.Ci, g.H, g.W, g.H, g.W, f.Cip, 0, 0, 1, 1, 32, g.Nb, stream);
+    stage_activations_f32(pro, dy, y_hi, y_lo, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, 32, g.Nb, stream);
     PCB_CUDA_TRY(cudaGetLastError());
-    PCB_CUDA_TRY(cudaMemsetAsync(acc, 0, (size_t)g.nc * g.Co * g.Ci * taps * sizeof(float), stream));
+    add_zero_job(pro, acc, f.acc_bytes);                             // (rounded up to 1 KB: always whole units)
+    {
+        const int rc = launch_prologue(pro, sc, stream);
+        if (rc != PCB_OK) return rc;
+    }
 
     TFParams p;
     p.nc = g.nc; p.ga = g.ga; p.neg = g.neg;
     p.Nb = g.Nb; p.Co = g.Co; p.Ci = g.Ci; p.HO = g.HO; p.WO = g.WO; p.Cop = f.Cop; p.Cip = f.Cip;
     p.cbA = 32; p.cbB = 32;
     p.KH = g.KH; p.KW = g.KW; p.SH = g.SH; p.SW = g.SW; p.DH = g.DH; p.DW = g.DW;
+    p.off_w = -g.PL; p.off_h = -g.PT;
     {
         long long best = -1;
         for (int pw = 1; pw <= TFK; pw *= 2)
@@ -753,9 +880,9 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
         if (rc != PCB_OK) return rc;
     }
     {
-        const cuuint64_t dims[5] = {(cuuint64_t)p.cbB, (cuuint64_t)f.Wp, (cuuint64_t)f.Hp, (cuuint64_t)g.Nb, (cuuint64_t)(g.nc * (f.Cip / p.cbB))};
-        const cuuint64_t strides[4] = {(cuuint64_t)p.cbB * 4, (cuuint64_t)f.Wp * p.cbB * 4, (cuuint64_t)f.Hp * f.Wp * p.cbB * 4,
-                                       (cuuint64_t)g.Nb * f.Hp * f.Wp * p.cbB * 4};
+        const cuuint64_t dims[5] = {(cuuint64_t)p.cbB, (cuuint64_t)g.W, (cuuint64_t)g.H, (cuuint64_t)g.Nb, (cuuint64_t)(g.nc * (f.Cip / p.cbB))};
+        const cuuint64_t strides[4] = {(cuuint64_t)p.cbB * 4, (cuuint64_t)g.W * p.cbB * 4, (cuuint64_t)g.H * g.W * p.cbB * 4,
+                                       (cuuint64_t)g.Nb * g.H * g.W * p.cbB * 4};
         const cuuint32_t box[5] = {(cuuint32_t)p.cbB, (cuuint32_t)((p.PW - 1) * g.SW + 1), (cuuint32_t)((p.PH - 1) * g.SH + 1), (cuuint32_t)p.PN,
                                    (cuuint32_t)(p.n_tile_cols / p.cbB)};
         const cuuint32_t es[5] = {1, (cuuint32_t)g.SW, (cuuint32_t)g.SH, 1, 1};
@@ -773,9 +900,9 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
 }
 
 int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, const void* bias, void* out, void* scratch, int* status,
-                     cudaStream_t stream) {
+                     cudaStream_t stream, StatusClear* sc) {
     // operand roles as for the other launchers: forward/backward-data a = filters, b = activations; backward-filter a = dy, b = x
-    if (pass == PASS_BWD_FILTER) return conv_tf32_filter_launch(g, (const float*)a, (const float*)b, (float*)out, scratch, status, stream);
+    if (pass == PASS_BWD_FILTER) return conv_tf32_filter_launch(g, (const float*)a, (const float*)b, (float*)out, scratch, status, stream, sc);
     const Plan32 pl = make_plan32(pass, g);
     const int taps = g.KH * g.KW;
     uint8_t* s8 = static_cast<uint8_t*>(scratch);
@@ -783,11 +910,13 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     float* x_lo = reinterpret_cast<float*>(s8 + pl.xp_bytes);
     float* w_hi = reinterpret_cast<float*>(s8 + 2 * pl.xp_bytes);
     float* w_lo = reinterpret_cast<float*>(s8 + 2 * pl.xp_bytes + pl.w_bytes);
-    stage_activations_f32((const float*)b, x_hi, x_lo, pl.LK * g.Nb, pl.Cin, pl.Hin, pl.Win, pl.Hp, pl.Wp, pl.Cp, pl.pad_top, pl.pad_left, pl.ins_h,
-                          pl.ins_w, 0, 1, stream);
-    pack_filters_f32_kernel<<<grid_cap((size_t)taps * pl.Mp, 1, 8), pl.Kp >= 256 ? 256 : 128, 0, stream>>>(
-        (const float*)a, w_hi, w_lo, g.Co, g.Ci, taps, pl.Mp, pl.Kp, pl.Cp, pass == PASS_BWD_DATA ? 1 : 0, g.w_io, g.nc, g.ga, g.neg);
+    const bool inserted = pl.ins_h != 1 || pl.ins_w != 1;
+    Prologue32 pro;
+    stage_activations_f32(pro, (const float*)b, x_hi, x_lo, pl.LK * g.Nb, pl.Cin, pl.Hin, pl.Win, pl.Hp, pl.Wp, pl.Cp, inserted ? pl.pad_top : 0,
+                          inserted ? pl.pad_left : 0, pl.ins_h, pl.ins_w, 0, 1, stream);
     PCB_CUDA_TRY(cudaGetLastError());
+    pro.filter = FilterJob32{(const float*)a, w_hi, w_lo, g.Co, g.Ci, taps, pl.Mp, pl.Kp, pl.Cp, pass == PASS_BWD_DATA ? 1 : 0, g.w_io, g.nc, g.ga, g.neg};
+    pro.filter_blocks = grid_cap((size_t)taps * pl.Mp, 1, 8);
 
     TParams p;
     {
@@ -809,6 +938,8 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     p.LK = pl.LK;
     p.store_vec = 1;
     while (p.store_vec < 8 && pl.Wout % (p.store_vec * 2) == 0 && (reinterpret_cast<uintptr_t>(out) % (size_t)(p.store_vec * 8)) == 0) p.store_vec *= 2;
+    p.rows_epi = (p.PW >= 8 && p.store_vec < 8) ? 1 : 0;
+    p.off_w = inserted ? 0 : -pl.pad_left; p.off_h = inserted ? 0 : -pl.pad_top;
 
     alignas(64) CUtensorMap m_w_hi, m_w_lo, m_x_hi, m_x_lo;
     {
@@ -840,17 +971,23 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         while (n_k % p.splits != 0) --p.splits;                      // equal work items: every chunk of every item holds stages
     }
     p.k_per_split = n_k / p.splits;
-    if (p.splits > 1) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, (size_t)g.nc * g.Nb * pl.Cout * pl.Hout * pl.Wout * sizeof(float), stream));
+    {
+        const size_t out_bytes = (size_t)g.nc * g.Nb * pl.Cout * pl.Hout * pl.Wout * sizeof(float);
+        if (p.splits > 1 && !add_zero_job(pro, out, out_bytes)) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
+        const int rc = launch_prologue(pro, sc, stream);
+        if (rc != PCB_OK) return rc;
+    }
     const int n_items = n_tiles * p.splits;
     const int grid = n_items < sm_count() ? n_items : sm_count();
     p.n_chunks = (p.k_per_split + T_CHUNK - 1) / T_CHUNK;
     p.chunk_len = (p.k_per_split + p.n_chunks - 1) / p.n_chunks;
+    const size_t smem = T_SMEM + (p.rows_epi ? 8 * EPI_ROWS_F32_BYTES : 0);
     if (p.n_chunks > 1) {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T_SMEM));
-        qconv_general_tf32_kernel<true><<<grid, T_THREADS, T_SMEM, stream>>>(m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status);
+        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        qconv_general_tf32_kernel<true><<<grid, T_THREADS, smem, stream>>>(m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status);
     } else {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)T_SMEM));
-        qconv_general_tf32_kernel<false><<<grid, T_THREADS, T_SMEM, stream>>>(m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status);
+        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        qconv_general_tf32_kernel<false><<<grid, T_THREADS, smem, stream>>>(m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status);
     }
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;

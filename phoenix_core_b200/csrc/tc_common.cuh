@@ -101,6 +101,47 @@ __device__ __forceinline__ void store_rows(uint32_t buf, const uint32_t (&packed
     }
 }
 
+// The same for fp32 results: 32 columns of floats per lane; `reduce`: added to the output instead of stored.
+constexpr int EPI_ROWS_F32_PITCH = 33;
+constexpr int EPI_ROWS_F32_BYTES = 32 * EPI_ROWS_F32_PITCH * 4;
+template <int V>
+__device__ __forceinline__ void store_rows_f32(uint32_t buf, const uint32_t (&v)[32], float* out, int row_off, int pix_off, int lane, bool reduce) {
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 32; ++e) asm volatile("st.shared.u32 [%0], %1;" ::"r"(buf + (uint32_t)(lane * EPI_ROWS_F32_PITCH + e) * 4u), "r"(v[e]) : "memory");
+    __syncwarp();
+    constexpr int LANES = 32 / V;
+    const int sub = lane / LANES, col = (lane % LANES) * V;
+    const uint32_t src = buf + (uint32_t)(sub * EPI_ROWS_F32_PITCH + col) * 4u;
+#pragma unroll 8
+    for (int r = 0; r < 32; r += V) {
+        const int ro = __shfl_sync(0xffffffffu, row_off, r + sub);
+        float w[V];
+#pragma unroll
+        for (int e = 0; e < V; ++e) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(w[e]) : "r"(src + (uint32_t)(r * EPI_ROWS_F32_PITCH + e) * 4u) : "memory");
+        if (ro < 0 || pix_off < 0) continue;
+        float* dst = out + (size_t)ro + pix_off;
+        if (reduce) {
+            if (V == 4) red_add_f32x4(dst, w[0], w[V > 1 ? 1 : 0], w[V > 2 ? 2 : 0], w[V > 3 ? 3 : 0]);
+            else {
+#pragma unroll
+                for (int e = 0; e < V; ++e) atomicAdd(dst + e, w[e]);
+            }
+        } else if (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(w[0], w[V > 1 ? 1 : 0], w[V > 2 ? 2 : 0], w[V > 3 ? 3 : 0]);
+        else if (V == 2) *reinterpret_cast<float2*>(dst) = make_float2(w[0], w[V > 1 ? 1 : 0]);
+        else *dst = w[0];
+    }
+}
+
+// A tile of 16-byte units on its way from pixel-major rows of channels to channel-major rows of pixels (the staging kernels): U units
+// per pixel, V pixels per load of a thread. The units' places are permuted inside 128 bytes so that neither side has bank conflicts.
+constexpr int STAGE_THREADS = 256, STAGE_UNITS = 1024;
+template <int V, int U>
+__device__ __forceinline__ int stage_unit(int px, int g) {
+    constexpr int LINE = 8 / U > V ? 8 / U : V;                    // pixels that share a permutation
+    return (px * U + g) ^ ((px / LINE) & 7);
+}
+
 // Staging copy of NCHW activations for the TMA-fed kernels, fast form (no zero insertion, W a multiple of PX = 4 or 2,
 // rows aligned to PX elements): one thread moves 8 channels x PX pixels -- eight loads of 2 PX bytes and PX 16-byte stores. Destination: channels-last xp[plane][hp][wp][Cp] (planar == 0),
 // planar xp[plane][c / 8][hp][wp][8] (planar == 1), or -- cb > 0 -- blocks of cb channels with the block index outermost,

@@ -706,11 +706,12 @@ bool backward_shares_staged_dy(int dtype, int variant, const Geom& g, StagedView
 }
 
 namespace {
-// Whether tensor_launch goes straight to the general 16-bit kernels (conv_tc.cu): the same order of preference.
+// Whether tensor_launch goes straight to the general kernels (conv_tc.cu, conv_tf32.cu): the same order of preference.
 bool general_route(Pass pass, int dtype, int variant, const Geom& g) {
     if (!g.plain) return true;
     if (strided_pointwise(g) && tensor_path_supported(pass, dtype, variant, compact_geom(g))) return false;
     if (pass == PASS_BWD_DATA && strided_classes_supported(dtype, variant, g)) return false;
+    if (dtype == PCB_F32) return true;
     if (pointwise_pair_tc_supported(pass, dtype, variant, g) || pointwise_tc_supported(pass, dtype, variant, g)) return false;
     if (pass == PASS_BWD_FILTER)
         return !pointwise_filter_tc_supported(dtype, variant, g) && !narrow_filter_tc_supported(dtype, variant, g) && conv_filter_tc_supported(dtype, variant, g);
@@ -721,7 +722,7 @@ bool general_route(Pass pass, int dtype, int variant, const Geom& g) {
 int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* a, const void* b, const void* bias,
                   void* out, float* scratch, int* status, cudaStream_t stream, const PassExtras* extras, StatusClear* sc) {
     // the general kernels' prologue launch resets the status word; every other route does it here
-    const bool own_launch = variant == PCB_VARIANT_16_PRODUCT && dtype != PCB_F32 && general_route(pass, dtype, variant, g);
+    const bool own_launch = variant == PCB_VARIANT_16_PRODUCT && general_route(pass, dtype, variant, g);
     if (sc && !own_launch) { const int rc = sc->now(stream); if (rc != PCB_OK) return rc; }
     const void* kept_x = extras ? extras->kept_x : nullptr;
     const StagedView* kept_dy = (extras && extras->dy.base) ? &extras->dy : nullptr;
@@ -792,7 +793,7 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
         return PCB_OK;
     }
     // the status word is cleared once per API call by the caller of this function; the kernels only OR into it
-    if (dtype == PCB_F32) return conv_tf32_launch(pass, g, a, b, bias, out, scratch, status, stream);
+    if (dtype == PCB_F32) return conv_tf32_launch(pass, g, a, b, bias, out, scratch, status, stream, sc);
     TcParams p;
     p.g = g;
     p.pass = pass;

@@ -103,7 +103,7 @@ bool narrow_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes);
 bool conv_tf32_supported(Pass pass, int dtype, int variant, const Geom& g);
 size_t conv_tf32_scratch_bytes(Pass pass, const Geom& g);
 int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, const void* bias, void* out, void* scratch, int* status,
-                     cudaStream_t stream);
+                     cudaStream_t stream, StatusClear* sc = nullptr);
 
 // Dense layers of quaternions without staging, both gradients in one launch; see qgemm_tc.cu. Any feature counts; every
 // tensor 16-byte aligned. Nothing but the status word of the workspace is used.
