@@ -30,7 +30,11 @@ using namespace umma;
 using namespace tc;
 
 constexpr int NM = 128;                  // MMA M: (d, co) rows, padded
-constexpr int N_THREADS = 320;           // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
+constexpr int N_THREADS = 320;           // filter gradient: warp 0 TMA, warp 1 MMA, warps 2..9 epilogue
+// Forward / backward-data: warps 2..17 epilogue, four per TMEM lane quadrant. Layers of this file have few rows (16 quaternion channels:
+// 64 of the 128 lanes), so half of the epilogue warps have none, and with two warps per quadrant the drain of a tile took twice as
+// long as its MMAs.
+constexpr int N_EPI_WARPS = 16, NW_THREADS = 64 + 32 * N_EPI_WARPS;
 constexpr int NB_STAGES = 4;             // halo tiles in flight (one per input component)
 constexpr uint32_t NA_BYTES = NM * 16 * 2;   // one (tap, component) slice of the filter matrix: [2 planes][128 rows][8]
 constexpr int ST_N_PRODUCER = 0x10000, ST_N_MMA = 0x20000, ST_N_EPILOGUE = 0x40000;
@@ -43,6 +47,7 @@ struct NParams {
     int tiles_w, tiles_h;
     int LK, taps;
     int fmt, has_bias, store_vec;
+    int rows_epi;                        // image rows that are not 16-byte aligned leave through shared memory (store_rows)
     uint32_t stage_bytes;                // shared-memory pitch of one halo stage
     uint32_t plane_bytes;                // Ht * Wt * 16
 };
@@ -58,7 +63,7 @@ __device__ __forceinline__ uint64_t desc_plain(uint32_t smem_addr, uint32_t lead
 // ===================================================================================================
 // Forward / backward-data: D[(d,co), pixel] = sum over (tap, l, ci) of Wexp * x, tile 128 x (8 x PH pixels).
 // ===================================================================================================
-__global__ void __launch_bounds__(N_THREADS, 1)
+__global__ void __launch_bounds__(NW_THREADS, 1)
 qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, NParams p,
                        const uint16_t* __restrict__ bias, uint16_t* __restrict__ out, int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
@@ -78,7 +83,7 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 
     if (t == 0) {
         for (int s = 0; s < NB_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, 8); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, N_EPI_WARPS); }
         mbar_init(a_full, 1);
         fence_barrier_init();
     }
@@ -144,9 +149,11 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             }
         }
     } else {
-        // ---------------------------------------------------------------- epilogue (warps 2..9)
+        // ---------------------------------------------------------------- epilogue (warps 2..17)
         const int q = warp & 3;                    // TMEM lane quadrant
-        const int chalf = (warp - 2) >> 2;         // which 128 of the 256 columns
+        const int part = (warp - 2) >> 2;          // takes the 32-column blocks part, part + 4
+        const bool some_rows = q * 32 < p.Mvalid;  // warp-uniform
+        const uint32_t rbuf = smem_u32(bars) + 256 + (uint32_t)(warp - 2) * EPI_ROWS_BYTES;
         const int sv = p.store_vec;                // output pixels per store: 8, 4, 2 or 1
         int local_tile = 0;
         bool ok = true;
@@ -164,23 +171,31 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             const int th = r / p.tiles_w, tw = r - th * p.tiles_w;
             const int ow0 = tw * 8, oh0 = th * p.PH;
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_N_EPILOGUE);
-            ok = __all_sync(0xffffffffu, ok && (*reinterpret_cast<volatile int*>(status) == 0));
+            ok = __all_sync(0xffffffffu, ok);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll 1
-            for (int cb = 0; cb < 4; ++cb) {
-                const int col0 = chalf * 128 + cb * 32;
-                if (col0 >= n_cols) break;                               // warp-uniform
+            for (int col0 = part * 32; col0 < n_cols && some_rows; col0 += 128) {
                 uint32_t v[32];
                 tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256 + col0, v);
                 tmem_ld_wait();
-                if (!row_ok) continue;
+                if (!row_ok && !p.rows_epi) continue;
                 uint32_t packed[16];
 #pragma unroll
                 for (int e = 0; e < 16; ++e) {
                     const float f0 = __uint_as_float(v[2 * e]) + badd, f1 = __uint_as_float(v[2 * e + 1]) + badd;
                     if (p.fmt == 0) { const __half2 h = __floats2half2_rn(f0, f1); packed[e] = *reinterpret_cast<const uint32_t*>(&h); }
                     else { const __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1); packed[e] = *reinterpret_cast<const uint32_t*>(&h); }
+                }
+                if (p.rows_epi) {
+                    const int je = col0 + (sv == 1 ? lane : (sv == 2 ? (lane & 15) * 2 : (lane & 7) * 4));
+                    const int ow = ow0 + (je & 7), oh = oh0 + (je >> 3);
+                    const int pix_off = (je < n_cols && ow < p.WO && oh < p.HO) ? (img * p.Cout * p.HO + oh) * p.WO + ow : -1;
+                    const int row_off = row_ok ? (d * p.Nb * p.Cout + co) * p.HO * p.WO : -1;
+                    if (sv == 1) store_rows<1>(rbuf, packed, out, row_off, pix_off, lane);
+                    else if (sv == 2) store_rows<2>(rbuf, packed, out, row_off, pix_off, lane);
+                    else store_rows<4>(rbuf, packed, out, row_off, pix_off, lane);
+                    continue;
                 }
 #pragma unroll
                 for (int g8 = 0; g8 < 4; ++g8) {                         // 8 columns = one row of the tile
@@ -352,7 +367,8 @@ __global__ void pack_filters_planar_kernel(const T* __restrict__ w, T* __restric
 // (16 bytes) over the same staged copy -- overlapping views -- so that one box brings the tile shifted by every kw:
 // [kw][l][plane][Ht][8 px][8], planes at one uniform pitch, N = KW * LK * 16 columns, one MMA per filter row and 16 pixels.
 // A real-valued x (one component) leaves a map dimension free for the filter rows as well (stride: one staged row): the
-// box is then [kw][kh][plane][PH][8 px][8] without halo rows and ONE MMA of N = KH * KW * 16 columns serves every tap.
+// box is then [kw][kh][plane][Ht][8 px][8] and one MMA of N = fold_h * KW * 16 columns serves fold_h filter rows: all of them (no halo
+// rows), or half of them from four rows up.
 // ===================================================================================================
 constexpr int NF_STAGES = 2;
 constexpr int NF_MAX_GROUPS = 16;        // tap groups that can be given CTA shares of their own
@@ -455,7 +471,7 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
     } else {
         const int q = warp & 3, tsel = (warp - 2) >> 2;                // two warps per lane quadrant share the taps
         bool ok = mbar_wait_bounded(tmem_full, 0, status, ST_N_EPILOGUE);
-        ok = __all_sync(0xffffffffu, ok && (*reinterpret_cast<volatile int*>(status) == 0));
+        ok = __all_sync(0xffffffffu, ok);
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
             const int m = q * 32 + lane;                                // row -> (d, plane, channel within the plane)
@@ -469,7 +485,7 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
                     tmem_ld_wait();
                     if (!row_ok) continue;
                     int kwf, l, tap;
-                    if (p.fold_h > 1) { kwf = (c0 >> 4) / p.fold_h; l = 0; tap = ((c0 >> 4) - kwf * p.fold_h) * p.fold + kwf; }
+                    if (p.fold_h > 1) { kwf = (c0 >> 4) / p.fold_h; l = 0; tap = ((tap0 + tl) * p.fold_h + (c0 >> 4) - kwf * p.fold_h) * p.fold + kwf; }
                     else { kwf = (c0 >> 4) / p.LKr; l = (c0 >> 4) - kwf * p.LKr; tap = (tap0 + tl) * p.fold + kwf; }
                     float* tap_base = dw32 + (size_t)tap * p.nc * comp_stride;
                     const float sgn = alg_negative(p.neg, l, d) ? -1.f : 1.f;
@@ -653,8 +669,11 @@ int narrow_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const v
     }
     const int n_tiles = pl.tiles_w * pl.tiles_h * g.Nb;
     const int grid = n_tiles < sm_count() ? n_tiles : sm_count();
-    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)pl.smem));
-    qconv_narrow_tc_kernel<<<grid, N_THREADS, pl.smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
+    // (the largest filter matrices leave no room for the row buffers: those layers store from the registers)
+    p.rows_epi = p.store_vec < 8 && pl.smem + N_EPI_WARPS * EPI_ROWS_BYTES <= 227 * 1024;
+    const size_t smem = pl.smem + (p.rows_epi ? N_EPI_WARPS * EPI_ROWS_BYTES : 0);
+    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    qconv_narrow_tc_kernel<<<grid, NW_THREADS, smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
@@ -687,8 +706,12 @@ NFPlan make_nfplan(const Geom& g) {
     f.fold = (f.KWe > 1 && f.KWe * f.LK * 16 <= 256) ? f.KWe : 1;
     // ... and the filter rows too for a one-component x (the tensor map has a dimension to spare)
     f.fold_h = (f.fold > 1 && f.LK == 1 && f.KHe > 1 && f.KHe * f.KWe * 16 <= 256) ? f.KHe : 1;
+    // From four filter rows up only half of them: the box holds every folded row and column once more, 80 KB per 8 x 16 pixels at
+    // 4 x 4 taps, and the kernel is bound by that traffic from L2 (117 us for the 7x7/2 stem at batch 128). Two of the four rows in the
+    // columns of an MMA and the other two as a shifted start address move half of it.
+    if (f.fold_h >= 4 && f.fold_h % 2 == 0) f.fold_h /= 2;
     f.LKe = f.LK * f.fold * f.fold_h;
-    f.taps = f.fold_h > 1 ? 1 : (f.fold > 1 ? f.KHe : f.KHe * f.KWe);
+    f.taps = f.fold_h > 1 ? f.KHe / f.fold_h : (f.fold > 1 ? f.KHe : f.KHe * f.KWe);
     f.Wt = f.fold > 1 ? 8 : 8 + (f.KWe - 1) * f.DWe;
     const int ncols = f.LKe * 16;
     f.n_groups = (f.taps * ncols + 511) / 512;
@@ -699,7 +722,7 @@ NFPlan make_nfplan(const Geom& g) {
     for (int r = rows;; ++r) {
         f.PH = (((g.HO + r - 1) / r) + 1) & ~1;
         f.tiles_h = (g.HO + f.PH - 1) / f.PH;
-        f.Ht = f.fold_h > 1 ? f.PH : f.PH + (f.KHe - 1) * f.DHe;
+        f.Ht = f.PH + (f.KHe - f.fold_h) * f.DHe;                   // (all rows folded: no halo)
         f.y_bytes = (uint32_t)g.nc * f.y_planes * f.PH * 128;
         f.x_bytes = (uint32_t)f.LKe * 2 * f.Ht * f.Wt * 16;
         f.stage_bytes = (f.y_bytes + f.x_bytes + 1023) / 1024 * 1024;
@@ -774,7 +797,7 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
     }
     NFParams p;
     p.Nb = g.Nb; p.Co = g.Co; p.Ci = f.Cie; p.nc = g.nc; p.ga = g.ga; p.neg = g.neg;
-    p.KH = f.KHe; p.KW = f.fold > 1 ? 1 : f.KWe; p.DH = f.DHe; p.DW = f.DWe;
+    p.KH = f.KHe; p.KW = f.fold > 1 ? 1 : f.KWe; p.DH = f.DHe * f.fold_h; p.DW = f.DWe;
     p.PH = f.PH; p.Wt = f.Wt; p.Ht = f.Ht; p.tiles_w = f.tiles_w; p.tiles_h = f.tiles_h;
     p.LK = f.LKe; p.LKr = f.LK; p.fold = f.fold; p.fold_h = f.fold_h;
     p.taps = f.taps; p.taps_per_group = f.taps_per_group; p.n_groups = f.n_groups; p.y_planes = f.y_planes;
@@ -836,7 +859,7 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
         // the second extent stops short of the halo rows for the same reason.
         const size_t plane = (size_t)f.Hp * f.Wp * 16;
         const bool fh = f.fold_h > 1;
-        const cuuint64_t dims[5] = {(cuuint64_t)f.WOp * 8, (cuuint64_t)(fh ? f.HOp : f.Hp), (cuuint64_t)2 * g.Nb, (cuuint64_t)(fh ? f.fold_h : f.LK),
+        const cuuint64_t dims[5] = {(cuuint64_t)f.WOp * 8, (cuuint64_t)(f.Hp - (f.fold_h - 1) * f.DHe), (cuuint64_t)2 * g.Nb, (cuuint64_t)(fh ? f.fold_h : f.LK),
                                     (cuuint64_t)f.fold};
         const cuuint64_t strides[4] = {(cuuint64_t)f.Wp * 16, plane, fh ? (cuuint64_t)f.DHe * f.Wp * 16 : (cuuint64_t)g.Nb * 2 * plane,
                                        (cuuint64_t)f.DWe * 16};

@@ -85,3 +85,29 @@ def test_stride_two_classes_channels_last_and_groups(gpu, oracle):
         ic, oc = slice(g * ci // 2, (g + 1) * ci // 2), slice(g * co // 2, (g + 1) * co // 2)
         rdw, rdx = oracle.conv2d_bwd(np.ascontiguousarray(x[:, ic]), np.ascontiguousarray(fg[:, oc]), np.ascontiguousarray(dy[:, oc]), (2, 2), (1, 1), pad)
         assert rel_err(dxg[:, ic], rdx) <= TOL["f16"] and rel_err(dwg[:, oc], rdw) <= TOL["f16"]
+
+
+# layers of at most 16 channels have kernels of their own: the same row alignments, 17 to 64 output rows, several tiles per image
+@pytest.mark.parametrize("shape", [(2, 16, 16, 21, 19), (1, 12, 8, 70, 26), (3, 8, 16, 16, 20), (1, 16, 5, 33, 40)])
+def test_unaligned_rows_narrow(gpu, oracle, shape):
+    n, ci, co, h, w = shape
+    _case(gpu, oracle, n, ci, co, h, w, 3, 3, (1, 1), (1, 1, 1, 1), "f16")
+
+
+# real-valued stems: 3 and 4 staged filter rows (all rows in one matrix instruction, or half of them)
+@pytest.mark.parametrize("k", [5, 7, 8])
+def test_real_valued_stem_filter_gradient(gpu, oracle, k):
+    import phoenix_core_b200 as pcb
+    x = gpu.rounded(uniform(61, (3, 3, 44, 36)), "f16")
+    f = gpu.rounded(normal(62, (4, 16, 3, k, k), std=0.1), "f16")
+    pad = (k // 2, k // 2, k // 2, k // 2)
+    y = gpu.run_conv_fwd(x, f, None, (2, 2), pad, "f16", "16p", "tensor", True)
+    x4 = np.concatenate([x, np.zeros((9, 3, 44, 36), np.float32)])             # the quaternions with zero imaginary parts
+    ref = oracle.conv2d_fwd(x4, f, None, (2, 2), (1, 1), pad)
+    assert rel_err(y, ref) <= TOL["f16"]
+    dy = gpu.rounded(normal(63, ref.shape), "f16")
+    rdw, _ = oracle.conv2d_bwd(x4, f, dy, (2, 2), (1, 1), pad)
+    _, bwd = gpu.conv_descriptors(x.shape, f.shape, (2, 2), pad, False, False, True)
+    dw = torch.full(f.shape, float("nan"), dtype=torch.float16, device="cuda")
+    pcb.conv2DBwd(gpu.dev(x, "f16"), gpu.dev(f, "f16"), gpu.dev(dy, "f16"), dw, None, bwd, gpu.context("16p"), gpu.ENGINES["tensor"])
+    assert rel_err(dw.float().cpu().numpy(), rdw) <= TOL["f16"]
