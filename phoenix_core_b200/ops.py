@@ -43,6 +43,9 @@ class Device:
     @classmethod
     def get(cls, torch_device):
         idx = torch_device.index if torch_device.index is not None else torch.cuda.current_device()
+        dev = cls._devices.get(idx)                    # entries are made once, under the lock, and never replaced
+        if dev is not None:
+            return dev
         with cls._registry_lock:
             dev = cls._devices.get(idx)
             if dev is None:
@@ -99,7 +102,8 @@ def getSmMargin():
 
 
 def _ptr(t):
-    return None if t is None else ctypes.c_void_p(t.data_ptr())
+    """A tensor's address as the C ABI's pointer arguments take it (a plain integer; None is a null pointer)."""
+    return None if t is None else t.data_ptr()
 
 
 def _check_tensor(t, name, dtype=None, shape=None):
@@ -109,8 +113,11 @@ def _check_tensor(t, name, dtype=None, shape=None):
         raise ValueError("%s must be contiguous" % name)
     if dtype is not None and t.dtype != dtype:
         raise ValueError("%s dtype mismatch: %s vs %s" % (name, t.dtype, dtype))
-    if shape is not None and tuple(t.shape) != tuple(shape):
+    if shape is not None and t.shape != shape:           # (torch.Size compares as a tuple)
         raise ValueError("%s shape mismatch: %s vs expected %s" % (name, tuple(t.shape), tuple(shape)))
+
+
+_get_raw_stream = getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def _raw_stream(index=None):
@@ -118,14 +125,13 @@ def _raw_stream(index=None):
     builds a Python stream object on every call)."""
     if index is None:
         index = torch.cuda.current_device()
-    getter = getattr(torch._C, "_cuda_getCurrentRawStream", None)
-    if getter is not None:
-        return getter(index)
+    if _get_raw_stream is not None:
+        return _get_raw_stream(index)
     return torch.cuda.current_stream(index).cuda_stream
 
 
 def _stream(index=None):
-    return ctypes.c_void_p(_raw_stream(index))
+    return _raw_stream(index)
 
 
 class _OnDevice:
@@ -286,6 +292,16 @@ def conv2DBwd(inputTensor, filterTensor, gradTensor, filterGradTensor, inputGrad
 
 
 def _dense_desc(descriptor, dtype, context, engine, has_bias=False, require_input_grad=False):
+    """As ``_conv_desc``."""
+    key = (dtype, context.variant(), engine, bool(has_bias), bool(require_input_grad))
+    cache = descriptor.__dict__.setdefault("_pcb_dense_desc", {})
+    d = cache.get(key)
+    if d is None:
+        d = cache[key] = _build_dense_desc(descriptor, dtype, context, engine, has_bias, require_input_grad)
+    return d
+
+
+def _build_dense_desc(descriptor, dtype, context, engine, has_bias, require_input_grad):
     algebra = descriptor.getAlgebra()
     dim = MULTIVECTOR_DIM[algebra]
     ishape = descriptor.getInputShape()
@@ -323,7 +339,9 @@ def denseFwd(inputTensor, filterTensor, biasTensor, outputTensor, descriptor, co
     d = _dense_desc(descriptor, inputTensor.dtype, context, engine, has_bias=biasTensor is not None)
     L = _lib.lib()
     with dev.accessControl, _OnDevice(dev.index):
-        need = L.pcb_qdense_fwd_workspace_size(ctypes.byref(d))
+        need = getattr(d, "_fwd_need", None)
+        if need is None:
+            need = d._fwd_need = L.pcb_qdense_fwd_workspace_size(ctypes.byref(d))
         ws = dev.requestWorkspace(need)
         _lib.check(L.pcb_qdense_fwd(ctypes.byref(d), _ptr(inputTensor), _ptr(filterTensor), _ptr(biasTensor),
                                     _ptr(outputTensor), _ptr(ws), ws.numel(), _stream()))
@@ -351,7 +369,9 @@ def denseBwd(inputTensor, filterTensor, gradTensor, filterGradTensor, inputGradT
     d = _dense_desc(descriptor, inputTensor.dtype, context, engine, require_input_grad=need_dx)
     L = _lib.lib()
     with dev.accessControl, _OnDevice(dev.index):
-        need = L.pcb_qdense_bwd_workspace_size(ctypes.byref(d))
+        need = getattr(d, "_bwd_need", None)
+        if need is None:
+            need = d._bwd_need = L.pcb_qdense_bwd_workspace_size(ctypes.byref(d))
         ws = dev.requestWorkspace(need)
         _lib.check(L.pcb_qdense_bwd(ctypes.byref(d), _ptr(inputTensor), _ptr(filterTensor), _ptr(gradTensor),
                                     _ptr(filterGradTensor), _ptr(inputGradTensor) if need_dx else None,
