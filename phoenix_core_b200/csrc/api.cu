@@ -7,10 +7,23 @@
 #include <unordered_map>
 
 #include "common.cuh"
+#include "tc_common.cuh"
 #include "tensor_path.cuh"
 #include "umma.cuh"
 
 namespace pcb {
+// (a kernel and not a memset, so that the kernel behind it can be chained to it)
+static __global__ void clear_status_kernel(int* word) {
+    tc::chain_next();
+    tc::chain_wait();
+    if (threadIdx.x == 0) *word = 0;
+}
+int clear_status_word(int* word, cudaStream_t stream) {
+    if (reinterpret_cast<uintptr_t>(word) % sizeof(int) != 0) PCB_CUDA_TRY(cudaMemsetAsync(word, 0, sizeof(int), stream));   // any workspace address is taken
+    else PCB_CUDA_TRY(tc::launch_chained(clear_status_kernel, 1, 32, 0, stream, word));
+    return PCB_OK;
+}
+
 int g_sm_margin = 0;         // SMs the persistent kernels leave free (pcb_set_sm_margin)
 
 static thread_local char g_error[512] = {0};
@@ -114,8 +127,7 @@ constexpr size_t WS_HEADER = 256;
 // A call that hands the reset to its first launch (StatusClear) settles it with finish_status: a call that launched nothing
 // resets the word all the same.
 int reset_status(void* workspace, size_t ws_bytes, cudaStream_t stream) {
-    if (workspace && ws_bytes >= sizeof(int)) PCB_CUDA_TRY(cudaMemsetAsync(workspace, 0, sizeof(int), stream));
-    return PCB_OK;
+    return workspace && ws_bytes >= sizeof(int) ? clear_status_word(static_cast<int*>(workspace), stream) : (int)PCB_OK;
 }
 
 StatusClear owe_status(void* workspace, size_t ws_bytes) {

@@ -181,6 +181,8 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
+    chain_wait();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -837,6 +839,8 @@ struct Prologue {
 __global__ void __launch_bounds__(STAGE_THREADS) prologue_kernel(const __grid_constant__ Prologue p) {
     extern __shared__ __align__(16) uint8_t pack_smem[];
     unsigned block = blockIdx.x;
+    chain_next();
+    chain_wait();
     if (block == 0 && threadIdx.x == 0 && p.status) *p.status = 0;
     if (block < p.filter_blocks) {
         if (p.filter.tiled) pack_filters_tile(p.filter, block, reinterpret_cast<uint16_t*>(pack_smem));
@@ -890,7 +894,7 @@ int launch_prologue(Prologue& pro, StatusClear* sc, cudaStream_t stream) {
     size_t smem = pro.n_stages ? STAGE_UNITS * sizeof(uint4) : 0;
     const size_t tile = pro.filter_blocks && f.tiled ? (size_t)(f.transposed ? PACK_TK * (PACK_TM * f.taps + 2) : PACK_TM * (PACK_TK * f.taps + 2)) * 2 : 0;
     if (tile > smem) smem = tile;
-    prologue_kernel<<<blocks, STAGE_THREADS, smem, stream>>>(pro);
+    PCB_CUDA_TRY(launch_chained(prologue_kernel, blocks, STAGE_THREADS, smem, stream, pro));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
@@ -1012,6 +1016,8 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
+    chain_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1145,6 +1151,8 @@ qconv_filter_xmajor_tc_kernel(const __grid_constant__ CUtensorMap map_x, const _
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
+    chain_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1239,6 +1247,8 @@ template <typename T>
 __global__ void unpack_filter_grad_kernel(const float* __restrict__ src, T* __restrict__ dw, int taps, size_t per_tap, int dense_oihw,
                                           int Co, int Ci, FilterStrides ds) {
     const size_t total = per_tap * taps;
+    chain_next();
+    chain_wait();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
         if (dense_oihw) {
             const int tap = (int)(idx % taps);
@@ -1501,7 +1511,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     const size_t smem = 1024 + (size_t)p.n_stages * p.stage_bytes + 512 + tail_bytes;
     auto run = [&](auto* kernel) -> int {
         PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kernel<<<grid, G_THREADS, smem, stream>>>(map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status);
+        PCB_CUDA_TRY(launch_chained(kernel, grid, G_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
         return PCB_OK;
     };
     int rc;
@@ -1678,18 +1688,18 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     }
     if (xmajor) {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_xmajor_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG_SMEM));
-        qconv_filter_xmajor_tc_kernel<<<items * p.splits, G_THREADS, FG_SMEM, stream>>>(map_x, map_dy, p, acc, status);
+        PCB_CUDA_TRY(launch_chained(qconv_filter_xmajor_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_x, map_dy, p, acc, status));
     } else {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_general_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG_SMEM));
-        qconv_filter_general_tc_kernel<<<items * p.splits, G_THREADS, FG_SMEM, stream>>>(map_dy, map_x, p, acc, status);
+        PCB_CUDA_TRY(launch_chained(qconv_filter_general_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_dy, map_x, p, acc, status));
     }
     PCB_CUDA_TRY(cudaGetLastError());
     const size_t per_tap = (size_t)g.nc * g.Co * g.Ci, total = per_tap * taps;
     const int blocks = (int)((total + 255) / 256 < 2368 ? (total + 255) / 256 : 2368);
     const FilterStrides ds = {g.dr, g.dco, g.dci, g.dkh, g.dkw, g.KW};
     const int dense_oihw = (g.dci == taps && g.dco == g.Ci * taps && (long long)g.dr == (long long)g.Co * g.Ci * taps && g.dkh == g.KW && g.dkw == 1) ? 1 : 0;
-    if (fmt == 0) unpack_filter_grad_kernel<__half><<<blocks, 256, 0, stream>>>(acc, (__half*)dw, taps, per_tap, dense_oihw, g.Co, g.Ci, ds);
-    else unpack_filter_grad_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(acc, (__nv_bfloat16*)dw, taps, per_tap, dense_oihw, g.Co, g.Ci, ds);
+    if (fmt == 0) PCB_CUDA_TRY(launch_chained(unpack_filter_grad_kernel<__half>, blocks, 256, 0, stream, acc, (__half*)dw, taps, per_tap, dense_oihw, g.Co, g.Ci, ds));
+    else PCB_CUDA_TRY(launch_chained(unpack_filter_grad_kernel<__nv_bfloat16>, blocks, 256, 0, stream, acc, (__nv_bfloat16*)dw, taps, per_tap, dense_oihw, g.Co, g.Ci, ds));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }

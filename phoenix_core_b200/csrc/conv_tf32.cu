@@ -81,6 +81,8 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
+    chain_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -470,6 +472,8 @@ struct Prologue32 {
 __global__ void __launch_bounds__(STAGE_THREADS) prologue_f32_kernel(const __grid_constant__ Prologue32 p) {
     __shared__ float4 tile[STAGE_UNITS];
     unsigned block = blockIdx.x;
+    chain_next();
+    chain_wait();
     if (block == 0 && threadIdx.x == 0 && p.status) *p.status = 0;
     if (block < p.filter_blocks) { pack_filters_f32(p.filter, block, p.filter_blocks); return; }
     block -= p.filter_blocks;
@@ -496,7 +500,7 @@ int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream) {
     const unsigned blocks = pro.filter_blocks + pro.zero_blocks + pro.stage_blocks[0] + pro.stage_blocks[1];
     if (blocks == 0) return PCB_OK;
     if (sc && sc->pending) { pro.status = sc->word; sc->pending = false; }
-    prologue_f32_kernel<<<blocks, STAGE_THREADS, 0, stream>>>(pro);
+    PCB_CUDA_TRY(launch_chained(prologue_f32_kernel, blocks, STAGE_THREADS, 0, stream, pro));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
@@ -588,6 +592,8 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
+    chain_wait();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -728,6 +734,8 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
 // scratch [tap][r][co][ci] -> dw [r][co][ci][tap], or [r][ci][co] for dense layers (input-major, one tap)
 __global__ void unpack_filter_grad_f32_kernel(const float* __restrict__ src, float* __restrict__ dw, int taps, int Co, int Ci, int dw_io, int nc) {
     const size_t per_tap = (size_t)nc * Co * Ci, total = per_tap * taps;
+    chain_next();
+    chain_wait();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
         if (dw_io) {
             const int co = (int)(idx % Co);
@@ -892,9 +900,9 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     }
     constexpr size_t smem = 1024 + T_STAGES * TF_STAGE + 512;
     PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    qconv_filter_tf32_kernel<<<items * p.splits, T_THREADS, smem, stream>>>(m_dy_hi, m_dy_lo, m_x_hi, m_x_lo, p, acc, status);
+    PCB_CUDA_TRY(launch_chained(qconv_filter_tf32_kernel, items * p.splits, T_THREADS, smem, stream, m_dy_hi, m_dy_lo, m_x_hi, m_x_lo, p, acc, status));
     PCB_CUDA_TRY(cudaGetLastError());
-    unpack_filter_grad_f32_kernel<<<grid_cap((size_t)g.nc * g.Co * g.Ci * taps, 256, 16), 256, 0, stream>>>(acc, dw, taps, g.Co, g.Ci, g.dw_io, g.nc);
+    PCB_CUDA_TRY(launch_chained(unpack_filter_grad_f32_kernel, grid_cap((size_t)g.nc * g.Co * g.Ci * taps, 256, 16), 256, 0, stream, acc, dw, taps, g.Co, g.Ci, g.dw_io, g.nc));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
@@ -984,10 +992,10 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     const size_t smem = T_SMEM + (p.rows_epi ? 8 * EPI_ROWS_F32_BYTES : 0);
     if (p.n_chunks > 1) {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        qconv_general_tf32_kernel<true><<<grid, T_THREADS, smem, stream>>>(m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status);
+        PCB_CUDA_TRY(launch_chained(qconv_general_tf32_kernel<true>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
     } else {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        qconv_general_tf32_kernel<false><<<grid, T_THREADS, smem, stream>>>(m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status);
+        PCB_CUDA_TRY(launch_chained(qconv_general_tf32_kernel<false>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
     }
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;

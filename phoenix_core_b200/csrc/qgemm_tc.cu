@@ -402,6 +402,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) qgemm_tc_kernel(const __grid_con
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
+    chain_next();
+    chain_wait();
     const int block = blockIdx.x;
     if (!PAIR || block < p.first_blocks)
         q_tile<F32, NT, AK, BK>(p.prob[0], block, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, status);
@@ -422,11 +424,13 @@ int q_launch(const QParams& p, int blocks, int* status, cudaStream_t stream) {
     cfg.blockDim = dim3(Q_THREADS);
     cfg.dynamicSmemBytes = L::SMEM;
     cfg.stream = stream;
-    cudaLaunchAttribute attr[1];
+    cudaLaunchAttribute attr[2];
+    attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;    // as launch_chained
+    attr[1].val.programmaticStreamSerializationAllowed = 1;
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)p.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = 2;
     PCB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, status));
     return PCB_OK;
 }

@@ -28,6 +28,28 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
         ::"r"(dst), "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(c4), "r"(bar) : "memory");
 }
 
+// Programmatic dependent launch. A kernel launched with launch_chained may start while the kernel in front of it in the stream is
+// still running, once every CTA of that one has called chain_next() (or ended); every thread calls chain_wait() before its first access
+// to global memory, which returns when the kernel in front has completed and its writes are visible. What comes before that call
+// (barriers, tensor memory, the launch itself) then overlaps the tail of the kernel in front: about 1.5 us per launch of a chain of small
+// kernels. A kernel calls chain_next() first thing: its dependents only take what it leaves free, and wait.
+__device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(grid);
+    cfg.blockDim = dim3(block);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+
 // TMA store of one shared-memory box (written by ordinary stores, then fence_proxy_async) to global memory; elements of
 // the box that fall outside the tensor are not written. Completion is tracked per thread in bulk groups.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {

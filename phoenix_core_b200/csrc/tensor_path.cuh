@@ -26,14 +26,14 @@ struct PassExtras {
 };
 // The reset of the device status word that an API call owes its workspace before its first kernel. Launches that have a kernel in
 // front of the waiting ones let that kernel do it; everything else calls now() first.
+int clear_status_word(int* word, cudaStream_t stream);    // defined in api.cu
 struct StatusClear {
     int* word = nullptr;
     bool pending = false;
     int now(cudaStream_t stream) {
         if (!pending) return PCB_OK;
         pending = false;
-        PCB_CUDA_TRY(cudaMemsetAsync(word, 0, sizeof(int), stream));
-        return PCB_OK;
+        return clear_status_word(word, stream);
     }
 };
 // `sc` (may be null: nothing is owed) is settled before any kernel of the pass can wait.
