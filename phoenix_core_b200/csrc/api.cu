@@ -14,8 +14,8 @@
 namespace pcb {
 // (a kernel and not a memset, so that the kernel behind it can be chained to it)
 static __global__ void clear_status_kernel(int* word) {
-    tc::chain_next();
     tc::chain_wait();
+    tc::chain_next();
     if (threadIdx.x == 0) *word = 0;
 }
 int clear_status_word(int* word, cudaStream_t stream) {

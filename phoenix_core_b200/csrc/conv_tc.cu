@@ -181,8 +181,8 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -839,8 +839,8 @@ struct Prologue {
 __global__ void __launch_bounds__(STAGE_THREADS) prologue_kernel(const __grid_constant__ Prologue p) {
     extern __shared__ __align__(16) uint8_t pack_smem[];
     unsigned block = blockIdx.x;
-    chain_next();
     chain_wait();
+    chain_next();
     if (block == 0 && threadIdx.x == 0 && p.status) *p.status = 0;
     if (block < p.filter_blocks) {
         if (p.filter.tiled) pack_filters_tile(p.filter, block, reinterpret_cast<uint16_t*>(pack_smem));
@@ -886,8 +886,10 @@ void add_zero_job(Prologue& pro, void* p, size_t bytes) {          // a multiple
     pro.zero_blocks = grid_cap(pro.zero_units, 4 * STAGE_THREADS, 1);
 }
 // `sc`: the pending reset of the status word, done by this launch.
-int launch_prologue(Prologue& pro, StatusClear* sc, cudaStream_t stream) {
+// `chain`: whether the main kernel may be chained to this launch.
+int launch_prologue(Prologue& pro, StatusClear* sc, cudaStream_t stream, bool* chain) {
     const unsigned blocks = pro.filter_blocks + pro.zero_blocks + pro.stage_blocks[0] + pro.stage_blocks[1];
+    *chain = chain_behind(blocks, 8);
     if (blocks == 0) return PCB_OK;                                // (nothing to prepare: the caller's status reset stays pending)
     if (sc && sc->pending) { pro.status = sc->word; sc->pending = false; }
     const FilterJob& f = pro.filter;
@@ -1016,8 +1018,8 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1151,8 +1153,8 @@ qconv_filter_xmajor_tc_kernel(const __grid_constant__ CUtensorMap map_x, const _
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -1247,8 +1249,8 @@ template <typename T>
 __global__ void unpack_filter_grad_kernel(const float* __restrict__ src, T* __restrict__ dw, int taps, size_t per_tap, int dense_oihw,
                                           int Co, int Ci, FilterStrides ds) {
     const size_t total = per_tap * taps;
-    chain_next();
     chain_wait();
+    chain_next();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
         if (dense_oihw) {
             const int tap = (int)(idx % taps);
@@ -1358,6 +1360,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
                   pl.Cin % 16 == 0 && pl.ins_h == 1 && pl.ins_w == 1 && (reinterpret_cast<uintptr_t>(act) & 15u) == 0;
 
     const bool inserted = pl.ins_h != 1 || pl.ins_w != 1;
+    bool chain = false;
 
     // stage the operands
     {
@@ -1367,7 +1370,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
                               pl.ins_h, pl.ins_w, stream, 0, 1, g.plain ? nullptr : &sa);
         const FilterStrides fs = {g.wr, g.wo, g.wi, g.wh, g.ww, g.KW};
         add_filter_job(pro, w, wexp, g.Co, g.Ci, taps, pl.Mp, pl.Kp, pl.Cp, pass == PASS_BWD_DATA ? 1 : 0, g.nc, g.ga, g.neg, fs);
-        const int rc = launch_prologue(pro, sc, stream);
+        const int rc = launch_prologue(pro, sc, stream, &chain);
         if (rc != PCB_OK) return rc;
         PCB_CUDA_TRY(cudaGetLastError());
     }
@@ -1508,10 +1511,11 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
 
     const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * (pl.dual ? 2 : 1);
     const int grid = n_tiles < sm_count() ? n_tiles : sm_count();
-    const size_t smem = 1024 + (size_t)p.n_stages * p.stage_bytes + 512 + tail_bytes;
+    size_t smem = 1024 + (size_t)p.n_stages * p.stage_bytes + 512 + tail_bytes;
+    if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
     auto run = [&](auto* kernel) -> int {
         PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        PCB_CUDA_TRY(launch_chained(kernel, grid, G_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
+        PCB_CUDA_TRY(launch_chained_if(chain, kernel, grid, G_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
         return PCB_OK;
     };
     int rc;
@@ -1605,6 +1609,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
                           channel_slice(g.Ci) == f.Cip && g.Ci % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     const bool direct_dy = !g.plain && g.yc == 1 && g.yw == g.Co && g.yh == g.WO * g.Co && (long long)g.yp == (long long)g.HO * g.WO * g.Co &&
                            channel_slice(g.Co) == f.Cop && g.Co % 16 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
+    bool chain = false;
     {   // stage both activations channels-last, clear the accumulator
         Prologue pro;
         const int lk = g.real_in ? 1 : g.nc;
@@ -1615,7 +1620,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
             stage_activations(pro, fmt, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, stream, channel_slice(g.Co), g.Nb, g.plain ? nullptr : &sy);
         PCB_CUDA_TRY(cudaGetLastError());
         add_zero_job(pro, acc, f.acc_bytes);
-        const int rc = launch_prologue(pro, sc, stream);
+        const int rc = launch_prologue(pro, sc, stream, &chain);
         if (rc != PCB_OK) return rc;
     }
 
@@ -1688,10 +1693,10 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     }
     if (xmajor) {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_xmajor_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG_SMEM));
-        PCB_CUDA_TRY(launch_chained(qconv_filter_xmajor_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_x, map_dy, p, acc, status));
+        PCB_CUDA_TRY(launch_chained_if(chain, qconv_filter_xmajor_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_x, map_dy, p, acc, status));
     } else {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_general_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG_SMEM));
-        PCB_CUDA_TRY(launch_chained(qconv_filter_general_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_dy, map_x, p, acc, status));
+        PCB_CUDA_TRY(launch_chained_if(chain, qconv_filter_general_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_dy, map_x, p, acc, status));
     }
     PCB_CUDA_TRY(cudaGetLastError());
     const size_t per_tap = (size_t)g.nc * g.Co * g.Ci, total = per_tap * taps;

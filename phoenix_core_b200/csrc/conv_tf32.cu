@@ -81,8 +81,8 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -472,8 +472,8 @@ struct Prologue32 {
 __global__ void __launch_bounds__(STAGE_THREADS) prologue_f32_kernel(const __grid_constant__ Prologue32 p) {
     __shared__ float4 tile[STAGE_UNITS];
     unsigned block = blockIdx.x;
-    chain_next();
     chain_wait();
+    chain_next();
     if (block == 0 && threadIdx.x == 0 && p.status) *p.status = 0;
     if (block < p.filter_blocks) { pack_filters_f32(p.filter, block, p.filter_blocks); return; }
     block -= p.filter_blocks;
@@ -496,8 +496,10 @@ bool add_zero_job(Prologue32& pro, void* p, size_t bytes) {
     pro.zero_blocks = grid_cap(pro.zero_units, 4 * STAGE_THREADS, 4);
     return true;
 }
-int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream) {
+// `chain`: whether the main kernel may be chained to this launch.
+int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream, bool* chain) {
     const unsigned blocks = pro.filter_blocks + pro.zero_blocks + pro.stage_blocks[0] + pro.stage_blocks[1];
+    *chain = chain_behind(blocks, 8);
     if (blocks == 0) return PCB_OK;
     if (sc && sc->pending) { pro.status = sc->word; sc->pending = false; }
     PCB_CUDA_TRY(launch_chained(prologue_f32_kernel, blocks, STAGE_THREADS, 0, stream, pro));
@@ -592,8 +594,8 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -734,8 +736,8 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
 // scratch [tap][r][co][ci] -> dw [r][co][ci][tap], or [r][ci][co] for dense layers (input-major, one tap)
 __global__ void unpack_filter_grad_f32_kernel(const float* __restrict__ src, float* __restrict__ dw, int taps, int Co, int Ci, int dw_io, int nc) {
     const size_t per_tap = (size_t)nc * Co * Ci, total = per_tap * taps;
-    chain_next();
     chain_wait();
+    chain_next();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
         if (dw_io) {
             const int co = (int)(idx % Co);
@@ -836,13 +838,14 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     float* y_hi = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes);
     float* y_lo = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes + f.dyp_bytes);
     float* acc = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes + 2 * f.dyp_bytes);
+    bool chain = false;
     Prologue32 pro;
     stage_activations_f32(pro, x, x_hi, x_lo, g.nc * g.Nb, g.Ci, g.H, g.W, g.H, g.W, f.Cip, 0, 0, 1, 1, 32, g.Nb, stream);
     stage_activations_f32(pro, dy, y_hi, y_lo, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, 32, g.Nb, stream);
     PCB_CUDA_TRY(cudaGetLastError());
     add_zero_job(pro, acc, f.acc_bytes);                             // (rounded up to 1 KB: always whole units)
     {
-        const int rc = launch_prologue(pro, sc, stream);
+        const int rc = launch_prologue(pro, sc, stream, &chain);
         if (rc != PCB_OK) return rc;
     }
 
@@ -900,7 +903,7 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     }
     constexpr size_t smem = 1024 + T_STAGES * TF_STAGE + 512;
     PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PCB_CUDA_TRY(launch_chained(qconv_filter_tf32_kernel, items * p.splits, T_THREADS, smem, stream, m_dy_hi, m_dy_lo, m_x_hi, m_x_lo, p, acc, status));
+    PCB_CUDA_TRY(launch_chained_if(chain, qconv_filter_tf32_kernel, items * p.splits, T_THREADS, smem, stream, m_dy_hi, m_dy_lo, m_x_hi, m_x_lo, p, acc, status));
     PCB_CUDA_TRY(cudaGetLastError());
     PCB_CUDA_TRY(launch_chained(unpack_filter_grad_f32_kernel, grid_cap((size_t)g.nc * g.Co * g.Ci * taps, 256, 16), 256, 0, stream, acc, dw, taps, g.Co, g.Ci, g.dw_io, g.nc));
     PCB_CUDA_TRY(cudaGetLastError());
@@ -919,6 +922,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     float* w_hi = reinterpret_cast<float*>(s8 + 2 * pl.xp_bytes);
     float* w_lo = reinterpret_cast<float*>(s8 + 2 * pl.xp_bytes + pl.w_bytes);
     const bool inserted = pl.ins_h != 1 || pl.ins_w != 1;
+    bool chain = false;
     Prologue32 pro;
     stage_activations_f32(pro, (const float*)b, x_hi, x_lo, pl.LK * g.Nb, pl.Cin, pl.Hin, pl.Win, pl.Hp, pl.Wp, pl.Cp, inserted ? pl.pad_top : 0,
                           inserted ? pl.pad_left : 0, pl.ins_h, pl.ins_w, 0, 1, stream);
@@ -982,7 +986,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     {
         const size_t out_bytes = (size_t)g.nc * g.Nb * pl.Cout * pl.Hout * pl.Wout * sizeof(float);
         if (p.splits > 1 && !add_zero_job(pro, out, out_bytes)) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
-        const int rc = launch_prologue(pro, sc, stream);
+        const int rc = launch_prologue(pro, sc, stream, &chain);
         if (rc != PCB_OK) return rc;
     }
     const int n_items = n_tiles * p.splits;
@@ -992,10 +996,10 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     const size_t smem = T_SMEM + (p.rows_epi ? 8 * EPI_ROWS_F32_BYTES : 0);
     if (p.n_chunks > 1) {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        PCB_CUDA_TRY(launch_chained(qconv_general_tf32_kernel<true>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
+        PCB_CUDA_TRY(launch_chained_if(chain, qconv_general_tf32_kernel<true>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
     } else {
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        PCB_CUDA_TRY(launch_chained(qconv_general_tf32_kernel<false>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
+        PCB_CUDA_TRY(launch_chained_if(chain, qconv_general_tf32_kernel<false>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
     }
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;

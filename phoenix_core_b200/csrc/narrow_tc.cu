@@ -92,8 +92,8 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
@@ -427,8 +427,8 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -519,8 +519,8 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
 template <typename T>
 __global__ void unpack_narrow_filter_grad_kernel(const float* __restrict__ src, T* __restrict__ dw, int taps, size_t per_tap) {
     const size_t total = per_tap * taps;
-    chain_next();
     chain_wait();
+    chain_next();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
         const int tap = (int)(idx % taps);
         DType<T>::store(dw + idx, src[(size_t)tap * per_tap + idx / taps]);
@@ -531,8 +531,8 @@ template <typename T>
 __global__ void unpack_narrow_filter_grad_s2d_kernel(const float* __restrict__ src, T* __restrict__ dw, int rows /*nc*Co*/, int Ci, int KH, int KW,
                                                      int KWe, int taps_e) {
     const size_t total = (size_t)rows * Ci * KH * KW;
-    chain_next();
     chain_wait();
+    chain_next();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
         const int kw = (int)(idx % KW);
         size_t rest = idx / KW;
@@ -681,7 +681,7 @@ int narrow_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const v
     p.rows_epi = p.store_vec < 8 && pl.smem + N_EPI_WARPS * EPI_ROWS_BYTES <= 227 * 1024;
     const size_t smem = pl.smem + (p.rows_epi ? N_EPI_WARPS * EPI_ROWS_BYTES : 0);
     PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PCB_CUDA_TRY(launch_chained(qconv_narrow_tc_kernel, grid, NW_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
+    PCB_CUDA_TRY(launch_chained_if(false, qconv_narrow_tc_kernel, grid, NW_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
@@ -883,7 +883,7 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
         if (rc != PCB_OK) return rc;
     }
     PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_filter_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)f.smem));
-    PCB_CUDA_TRY(launch_chained(qconv_narrow_filter_tc_kernel, grid, N_THREADS, f.smem, stream, map_dy, map_x, p, acc, status));
+    PCB_CUDA_TRY(launch_chained_if(false, qconv_narrow_filter_tc_kernel, grid, N_THREADS, f.smem, stream, map_dy, map_x, p, acc, status));
     PCB_CUDA_TRY(cudaGetLastError());
     const size_t per_tap = (size_t)g.nc * g.Co * g.Ci;
     const int blocks = grid_cap(per_tap * g.KH * g.KW, 256, 16);

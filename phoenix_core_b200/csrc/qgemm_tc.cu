@@ -402,8 +402,8 @@ __global__ void __launch_bounds__(Q_THREADS, 1) qgemm_tc_kernel(const __grid_con
     __syncthreads();
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
-    chain_next();
     chain_wait();
+    chain_next();
     const int block = blockIdx.x;
     if (!PAIR || block < p.first_blocks)
         q_tile<F32, NT, AK, BK>(p.prob[0], block, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, status);

@@ -32,11 +32,15 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
 // still running, once every CTA of that one has called chain_next() (or ended); every thread calls chain_wait() before its first access
 // to global memory, which returns when the kernel in front has completed and its writes are visible. What comes before that call
 // (barriers, tensor memory, the launch itself) then overlaps the tail of the kernel in front: about 1.5 us per launch of a chain of small
-// kernels. A kernel calls chain_next() first thing: its dependents only take what it leaves free, and wait.
+// kernels. A kernel calls chain_next() once its own wait is over, so that only its direct successor sits beside it. A persistent kernel
+// that takes the whole tensor memory must also ask for more than half of the shared memory (ONE_CTA_SMEM): beside the tail of another
+// kernel the SMs become free one by one, and an SM that could hold two of its CTAs could be given two, the second one waiting for the
+// first one's tensor memory.
+constexpr size_t ONE_CTA_SMEM = 116 * 1024;
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 template <typename... Params, typename... Args>
-cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
+cudaError_t launch_chained_if(bool chained, void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(block);
@@ -46,8 +50,12 @@ cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, unsigned bl
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = 1;
+    cfg.numAttrs = chained ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kernel, static_cast<Params>(args)...);
+}
+template <typename... Params, typename... Args>
+cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
+    return launch_chained_if(true, kernel, grid, block, smem, stream, args...);
 }
 
 // TMA store of one shared-memory box (written by ordinary stores, then fence_proxy_async) to global memory; elements of
@@ -311,6 +319,12 @@ inline int sm_count() {
     const int left = sms - pcb::g_sm_margin;
     return left < 2 ? 2 : left;
 }
+
+// Whether a main kernel is chained to a prologue of that many CTAs: only behind a short one. Behind a longer prologue the gap does not
+// matter, and the main kernel, started CTA by CTA beside the last wave, runs 2 to 3 % slower for its whole length (fp32 3x3, 128
+// channels, 28 x 28, batch 128, forward + backward: 6825 us chained, 6790 not; 3x3/2 128 channels 616 / 609; the 7x7/2 stem 442 / 357). At 5
+// to 20 MB of copies it is worth 3 to 7 % (3x3 16 -> 16, 45 x 37, batch 32: 96 us chained, 102 not).
+inline bool chain_behind(unsigned prologue_blocks, unsigned per_sm) { return prologue_blocks <= per_sm * (unsigned)sm_count(); }
 
 inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 // Number of slices to cut each of `items` work items into when every CTA occupies a whole SM: the CTAs must fill
