@@ -172,113 +172,6 @@ __device__ __forceinline__ int stage_unit(int px, int g) {
     return (px * U + g) ^ ((px / LINE) & 7);
 }
 
-// Staging copy of NCHW activations for the TMA-fed kernels, fast form (no zero insertion, W a multiple of PX = 4 or 2,
-// rows aligned to PX elements): one thread moves 8 channels x PX pixels -- eight loads of 2 PX bytes and PX 16-byte stores. Destination: channels-last xp[plane][hp][wp][Cp] (planar == 0),
-// planar xp[plane][c / 8][hp][wp][8] (planar == 1), or -- cb > 0 -- blocks of cb channels with the block index outermost,
-// xp[comp * (Cp / cb) + c / cb][img][hp][wp][cb] where plane = comp * Nb + img (one TMA box can then span the channel
-// blocks of several components). Zero outside the image and for c >= C. The threads at the ends of a row also write
-// the padding columns.
-template <typename T, int PX>
-__global__ void pack_rows_kernel(const T* __restrict__ x, T* __restrict__ xp, int planes, int C, int H, int W, int Hp, int Wp, int groups,
-                                 int pad_top, int pad_left, int planar, int cb = 0, int Nb = 1) {
-    const int Wq = W / PX;
-    const unsigned total = (unsigned)planes * groups * Hp * Wq;         // 32-bit indices: staged copies stay below 2^32 / 8 threads
-    const int Cp = groups * 8;
-    for (unsigned idx = blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += gridDim.x * blockDim.x) {
-        // The channel group runs fastest across threads: the lanes of a warp that share a pixel group then write the channel
-        // groups of a pixel side by side (whole 32- to 128-byte runs per pixel instead of one 16-byte piece per lane and
-        // 32 half-filled sectors per store), while every load instruction still fetches full 32-byte sectors (PX * 2 bytes
-        // from each of the neighbouring pixel groups of one channel row).
-        const int grp = (int)(idx % groups);
-        unsigned rest = idx / groups;
-        const int q = (int)(rest % Wq); rest /= Wq;
-        const int hp = (int)(rest % Hp);
-        const int plane = (int)(rest / Hp);
-        const int ih = hp - pad_top;
-        const bool row_in = ih >= 0 && ih < H;
-        alignas(8) T v[8][PX];
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const int c = grp * 8 + e;
-            if (PX == 4) {
-                uint2 raw = make_uint2(0u, 0u);
-                if (row_in && c < C) raw = __ldg(reinterpret_cast<const uint2*>(x + (((size_t)plane * C + c) * H + ih) * W + 4 * q));
-                *reinterpret_cast<uint2*>(v[e]) = raw;
-            } else {
-                uint32_t raw = 0u;
-                if (row_in && c < C) raw = __ldg(reinterpret_cast<const uint32_t*>(x + (((size_t)plane * C + c) * H + ih) * W + 2 * q));
-                *reinterpret_cast<uint32_t*>(v[e]) = raw;
-            }
-        }
-        size_t blk_plane = 0;                       // (block, image) index and channel offset inside the block
-        int c_lo = 0;
-        if (cb > 0) {
-            const int comp = plane / Nb, img = plane - comp * Nb, b = (grp * 8) / cb;
-            c_lo = grp * 8 - b * cb;
-            blk_plane = ((size_t)comp * (Cp / cb) + b) * Nb + img;
-        }
-        auto dst = [&](int wp) {
-            if (cb > 0) return xp + ((blk_plane * Hp + hp) * Wp + wp) * cb + c_lo;
-            return planar ? xp + ((((size_t)plane * groups + grp) * Hp + hp) * Wp + wp) * 8 : xp + (((size_t)plane * Hp + hp) * Wp + wp) * Cp + grp * 8;
-        };
-#pragma unroll
-        for (int j = 0; j < PX; ++j) {
-            alignas(16) T o[8];
-#pragma unroll
-            for (int e = 0; e < 8; ++e) o[e] = v[e][j];
-            *reinterpret_cast<uint4*>(dst(pad_left + PX * q + j)) = *reinterpret_cast<const uint4*>(o);
-        }
-        const uint4 zero = make_uint4(0u, 0u, 0u, 0u);
-        if (q == 0)
-            for (int wp = 0; wp < pad_left && wp < Wp; ++wp) *reinterpret_cast<uint4*>(dst(wp)) = zero;
-        if (q == Wq - 1)
-            for (int wp = pad_left + W; wp < Wp; ++wp) *reinterpret_cast<uint4*>(dst(wp)) = zero;
-    }
-}
-// A side stream per host thread and device, for a prologue kernel that is independent of its neighbour: the filter matrix
-// is packed beside the staging of the activations instead of after it (both are short, one bound by memory, the other by
-// latency). fork() orders the side stream after everything enqueued so far on the caller's stream and returns it; join()
-// makes the caller's stream wait for it. Where the side stream cannot be made the caller's stream is returned and join()
-// does nothing. The fork / join pattern is also what stream capture expects.
-struct SideStream {
-    cudaStream_t side = nullptr;
-    cudaEvent_t forked = nullptr, joined = nullptr;
-    bool tried = false;
-    cudaStream_t fork(cudaStream_t main) {
-        if (!tried) {
-            tried = true;
-            const char* off = getenv("PCB_NO_SIDE_STREAM");      // escape hatch: everything on the caller's stream
-            if (off && off[0] && off[0] != '0') return main;
-            if (cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking) != cudaSuccess) side = nullptr;
-            if (side && (cudaEventCreateWithFlags(&forked, cudaEventDisableTiming) != cudaSuccess ||
-                         cudaEventCreateWithFlags(&joined, cudaEventDisableTiming) != cudaSuccess)) side = nullptr;
-            if (!side) (void)cudaGetLastError();
-        }
-        if (!side) return main;
-        if (cudaEventRecord(forked, main) != cudaSuccess || cudaStreamWaitEvent(side, forked, 0) != cudaSuccess) { (void)cudaGetLastError(); return main; }
-        return side;
-    }
-    void join(cudaStream_t main, cudaStream_t used) {
-        if (used == main) return;
-        cudaEventRecord(joined, used);
-        cudaStreamWaitEvent(main, joined, 0);
-    }
-};
-inline SideStream& side_stream() {
-    static thread_local SideStream per_device[16];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 16) dev = 0;
-    return per_device[dev];
-}
-
-// Pixels per thread pack_rows_kernel can take for this tensor: 4, 2, or 0 (the general staging kernel must run).
-inline int pack_rows_px(const void* x, int W, int Wp, int pad_left, int ins_h, int ins_w) {
-    if (ins_h != 1 || ins_w != 1 || pad_left < 0 || pad_left + W > Wp) return 0;
-    if (W % 4 == 0 && W >= 4 && reinterpret_cast<uintptr_t>(x) % 8 == 0) return 4;
-    if (W % 2 == 0 && W >= 2 && reinterpret_cast<uintptr_t>(x) % 4 == 0) return 2;
-    return 0;
-}
-
 typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                   const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                   CUtensorMapL2promotion, CUtensorMapFloatOOBfill);

@@ -706,23 +706,23 @@ bool backward_shares_staged_dy(int dtype, int variant, const Geom& g, StagedView
 }
 
 namespace {
-// Whether tensor_launch goes straight to the general kernels (conv_tc.cu, conv_tf32.cu): the same order of preference.
-bool general_route(Pass pass, int dtype, int variant, const Geom& g) {
+// Whether tensor_launch goes straight to kernels with a prologue launch (conv_tc.cu, conv_tf32.cu, narrow_tc.cu): the same order of preference.
+bool prologue_route(Pass pass, int dtype, int variant, const Geom& g) {
     if (!g.plain) return true;
     if (strided_pointwise(g) && tensor_path_supported(pass, dtype, variant, compact_geom(g))) return false;
     if (pass == PASS_BWD_DATA && strided_classes_supported(dtype, variant, g)) return false;
     if (dtype == PCB_F32) return true;
     if (pointwise_pair_tc_supported(pass, dtype, variant, g) || pointwise_tc_supported(pass, dtype, variant, g)) return false;
     if (pass == PASS_BWD_FILTER)
-        return !pointwise_filter_tc_supported(dtype, variant, g) && !narrow_filter_tc_supported(dtype, variant, g) && conv_filter_tc_supported(dtype, variant, g);
-    return !narrow_tc_supported(pass, dtype, variant, g) && conv_tc_supported(pass, dtype, variant, g);
+        return !pointwise_filter_tc_supported(dtype, variant, g) && (narrow_filter_tc_supported(dtype, variant, g) || conv_filter_tc_supported(dtype, variant, g));
+    return narrow_tc_supported(pass, dtype, variant, g) || conv_tc_supported(pass, dtype, variant, g);
 }
 }  // namespace
 
 int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* a, const void* b, const void* bias,
                   void* out, float* scratch, int* status, cudaStream_t stream, const PassExtras* extras, StatusClear* sc) {
-    // the general kernels' prologue launch resets the status word; every other route does it here
-    const bool own_launch = variant == PCB_VARIANT_16_PRODUCT && general_route(pass, dtype, variant, g);
+    // a prologue launch resets the status word; every other route does it here
+    const bool own_launch = variant == PCB_VARIANT_16_PRODUCT && prologue_route(pass, dtype, variant, g);
     if (sc && !own_launch) { const int rc = sc->now(stream); if (rc != PCB_OK) return rc; }
     const void* kept_x = extras ? extras->kept_x : nullptr;
     const StagedView* kept_dy = (extras && extras->dy.base) ? &extras->dy : nullptr;
@@ -807,7 +807,7 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
     if (pointwise_pair_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g)) return pointwise_pair_tc_launch(dtype, g, a, b, bias, out, status, stream);
     if (pointwise_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g)) return pointwise_tc_launch(pass, dtype, g, a, b, bias, out, status, stream);
     if (pass != PASS_BWD_FILTER && narrow_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g))
-        return narrow_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream);
+        return narrow_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream, sc);
     if (pass != PASS_BWD_FILTER && conv_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g))
         return conv_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream, sc);
     if (pass == PASS_FWD) return launch_tc<PASS_FWD>(p, 1, a, b, bias, out, nullptr, status, stream);
@@ -817,7 +817,7 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
     // accumulate in fp32 scratch, then cast once.
     if (scratch == nullptr) { set_error("backward-filter needs fp32 scratch"); return PCB_ERR_WORKSPACE; }
     if (pointwise_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return pointwise_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream);
-    if (narrow_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return narrow_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream, kept_x, kept_dy);
+    if (narrow_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return narrow_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream, kept_x, kept_dy, sc);
     if (conv_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return conv_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream, kept_x, kept_dy, sc);
     const int tiles = ((p.M + TBM - 1) / TBM) * ((p.N + TBN - 1) / TBN);
     int splits = (2 * sm_count() + tiles - 1) / tiles;

@@ -91,12 +91,12 @@ bool conv_filter_tc_stages_like_forward(const Geom& g);
 bool narrow_tc_supported(Pass pass, int dtype, int variant, const Geom& g);
 size_t narrow_tc_scratch_bytes(Pass pass, const Geom& g);
 int narrow_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const void* act, const void* bias, void* out, void* scratch,
-                     int* status, cudaStream_t stream);
+                     int* status, cudaStream_t stream, StatusClear* sc = nullptr);
 
 bool narrow_filter_tc_supported(int dtype, int variant, const Geom& g);
 size_t narrow_filter_tc_scratch_bytes(const Geom& g);
 int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* x, void* dw, void* scratch, int* status, cudaStream_t stream,
-                            const void* kept_x = nullptr, const StagedView* kept_dy = nullptr);
+                            const void* kept_x = nullptr, const StagedView* kept_dy = nullptr, StatusClear* sc = nullptr);
 bool narrow_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes);
 
 // fp32 tensors on the tensor cores with error-compensated TF32 (convolution and dense); see conv_tf32.cu.
