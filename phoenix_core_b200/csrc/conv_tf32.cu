@@ -35,6 +35,7 @@ struct TParams {
     int PW, PH, PN;
     int tiles_w, tiles_h, tiles_n, tiles_m;
     int has_bias, LK, store_vec;
+    int n_cols;                       // pixels of a tile: 256, or 128 where few tiles leave most SMs idle
     int n_chunks, chunk_len;          // a work item's K range runs in n_chunks pieces of at most chunk_len stages
     int off_w, off_h;                 // added to the pixel coordinates of every activation box: minus the padding; 0 for a zero-inserted copy
     int rows_epi;                     // image rows not a multiple of 8 pixels: stored through shared memory (store_rows_f32)
@@ -106,7 +107,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                     ok = mbar_wait_bounded(empty_bar + 8 * s, ((it / T_STAGES) & 1) ^ 1, status, ST_T_PRODUCER);
                     if (!ok) break;
                     const uint32_t dst = tiles_addr + s * T_STAGE, bar = full_bar + 8 * s;
-                    mbar_arrive_expect_tx(bar, T_STAGE);
+                    mbar_arrive_expect_tx(bar, 2 * (TA_BYTES + (uint32_t)p.n_cols * TKS * 4));
                     tma_load_3d(dst, &map_w_hi, l * p.Cp + cs * TKS, m0, tap, bar);
                     tma_load_3d(dst + TA_BYTES, &map_w_lo, l * p.Cp + cs * TKS, m0, tap, bar);
                     tma_load_5d(dst + 2 * TA_BYTES, &map_x_hi, cs * TKS, wp0, hp0, n0, l, bar);
@@ -117,7 +118,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
         }
         __syncwarp();
     } else if (warp == 1) {
-        const uint32_t idesc = make_idesc_f16(2, TM, TN, false, false);
+        const uint32_t idesc = make_idesc_f16(2, TM, p.n_cols, false, false);
         int it = 0, unit = 0;                       // unit = one accumulator's worth of work: a chunk of a tile
         bool ok = true;
         for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
@@ -184,8 +185,9 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                     tc_fence_after_sync();
 #pragma unroll
                     for (int cb = 0; cb < 4; ++cb) {
+                        if (cb * 64 >= p.n_cols) break;
                         uint32_t v[32];
-                        tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * TN + chalf * 128 + cb * 32, v);
+                        tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * TN + chalf * (p.n_cols / 2) + cb * 32, v);
                         tmem_ld_wait();
 #pragma unroll
                         for (int e = 0; e < 32; ++e) part[cb][e] += __uint_as_float(v[e]);
@@ -205,7 +207,8 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
 #pragma unroll(CHUNKED ? 4 : 1)
             for (int cb = 0; cb < 4; ++cb) {
                 uint32_t v[32];
-                const int col0 = chalf * 128 + cb * 32;
+                if (cb * 64 >= p.n_cols) break;
+                const int col0 = chalf * (p.n_cols / 2) + cb * 32;
                 tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * TN + col0, v);
                 tmem_ld_wait();
                 if (!row_ok && !p.rows_epi) continue;
@@ -931,21 +934,40 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     pro.filter_blocks = grid_cap((size_t)taps * pl.Mp, 1, 8);
 
     TParams p;
-    {
+    const int n_k = taps * pl.LK * (pl.Cp / TKS);
+    // Box of `cols` pixels that wastes the fewest columns, and the cut of its K loop. Too few tiles for the SMs (dense layers, small
+    // planes): the K loop of every tile is cut into work items of at least one chunk each; their partial sums meet in the output, zeroed
+    // first, by fp32 reductions (the order of which is not fixed).
+    auto plan_tiles = [&](int cols) -> long long {
         long long best = -1;
+        p.n_cols = cols;
         for (int pw = 1; pw <= 128; pw *= 2)
-            for (int ph = 1; ph * pw <= 256; ph *= 2) {
-                const int pn = 256 / (pw * ph);
+            for (int ph = 1; ph * pw <= cols; ph *= 2) {
+                const int pn = cols / (pw * ph);
                 if (pn > 256 || (pw - 1) * pl.SW + 1 > 256 || (ph - 1) * pl.SH + 1 > 256) continue;
                 if (pw < 8 && pl.Wout >= 8) continue;                      // narrow boxes only for narrow planes
                 const long long vol = (long long)round_up(pl.Wout, pw) * round_up(pl.Hout, ph) * round_up(g.Nb, pn);
                 if (best < 0 || vol < best || (vol == best && pw > p.PW)) { best = vol; p.PW = pw; p.PH = ph; p.PN = pn; }
             }
-    }
+        p.tiles_w = (pl.Wout + p.PW - 1) / p.PW; p.tiles_h = (pl.Hout + p.PH - 1) / p.PH; p.tiles_n = (g.Nb + p.PN - 1) / p.PN;
+        p.tiles_m = pl.Mp / TM;
+        const long long tiles = (long long)p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m;
+        p.splits = 1;
+        if (2 * tiles <= sm_count() && n_k >= 2 * T_CHUNK) {
+            p.splits = sm_count() / (int)tiles;
+            if (p.splits > n_k / T_CHUNK) p.splits = n_k / T_CHUNK;
+            while (n_k % p.splits != 0) --p.splits;                  // equal work items: every chunk of every item holds stages
+        }
+        p.k_per_split = n_k / p.splits;
+        const long long rounds = (tiles * p.splits + sm_count() - 1) / sm_count();
+        return rounds * p.k_per_split * (cols == 256 ? 128 : 80);        // clocks of an MMA
+    };
+    // 128-pixel tiles where the longest CTA has less to do with them (an MMA of 128 columns takes 80 clocks, of 256 columns 128): only
+    // layers that leave SMs idle. Forward: 3x3, 16 channels, 32 x 32, batch 8: 25.0 -> 22.5 us; 1x1, 32 channels, 79 x 79, batch 6: 47 -> 40 us.
+    const long long narrow_cost = plan_tiles(128);
+    if (10 * plan_tiles(256) > 11 * narrow_cost) plan_tiles(128);
     p.Nb = g.Nb; p.Cout = pl.Cout; p.Mvalid = g.nc * pl.Cout; p.HO = pl.Hout; p.WO = pl.Wout; p.Cp = pl.Cp;
     p.KH = g.KH; p.KW = g.KW; p.SH = pl.SH; p.SW = pl.SW; p.DH = g.DH; p.DW = g.DW;
-    p.tiles_w = (pl.Wout + p.PW - 1) / p.PW; p.tiles_h = (pl.Hout + p.PH - 1) / p.PH; p.tiles_n = (g.Nb + p.PN - 1) / p.PN;
-    p.tiles_m = pl.Mp / TM;
     p.has_bias = (pass == PASS_FWD && g.has_bias) ? 1 : 0;
     p.LK = pl.LK;
     p.store_vec = 1;
@@ -973,16 +995,6 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         if (rc != PCB_OK) return rc;
     }
     const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m;
-    const int n_k = taps * pl.LK * (pl.Cp / TKS);
-    // Too few tiles for the SMs (dense layers, small planes): cut the K loop of every tile into work items of at least one chunk
-    // each; their partial sums meet in the output, zeroed first, by fp32 reductions (the order of which is not fixed).
-    p.splits = 1;
-    if (2 * n_tiles <= sm_count() && n_k >= 2 * T_CHUNK) {
-        p.splits = sm_count() / n_tiles;
-        if (p.splits > n_k / T_CHUNK) p.splits = n_k / T_CHUNK;
-        while (n_k % p.splits != 0) --p.splits;                      // equal work items: every chunk of every item holds stages
-    }
-    p.k_per_split = n_k / p.splits;
     {
         const size_t out_bytes = (size_t)g.nc * g.Nb * pl.Cout * pl.Hout * pl.Wout * sizeof(float);
         if (p.splits > 1 && !add_zero_job(pro, out, out_bytes)) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
