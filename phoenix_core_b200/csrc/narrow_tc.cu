@@ -820,7 +820,10 @@ NFPlan make_nfplan(const Geom& g) {
     f.taps = f.fold_h > 1 ? f.KHe / f.fold_h : (f.fold > 1 ? f.KHe : f.KHe * f.KWe);
     f.Wt = f.fold > 1 ? 8 : 8 + (f.KWe - 1) * f.DWe;
     const int ncols = f.LKe * 16;
-    f.n_groups = (f.taps * ncols + 511) / 512;
+    // as many taps per group as the 512 accumulator columns hold whole (ncols <= 256), spread evenly over the fewest groups; three taps
+    // of 192 columns -- five or seven rows of a 3-wide filter -- would need 576 columns
+    const int fit = 512 / ncols;
+    f.n_groups = (f.taps + fit - 1) / fit;
     f.taps_per_group = (f.taps + f.n_groups - 1) / f.n_groups;
     f.n_groups = (f.taps + f.taps_per_group - 1) / f.taps_per_group;
     // the kernel's own tile height: the standard one, lowered until two stages fit the shared memory (rows past the staged
