@@ -810,6 +810,7 @@ __device__ __forceinline__ void pack_filters_tile(const FilterJob& p, unsigned b
         for (int dd = 0; dd < nc; ++dd)
             if (alg_pair(ga, l, dd) == r) d = dd;
         if (d < 0) continue;
+        if ((transposed ? d : l) * Cp >= Kp) continue;      // a real-valued input has one component along K
         const uint32_t flip = alg_negative(neg, l, d) ? 0x80008000u : 0u;
         const int m_comp = transposed ? l : d, k_comp = transposed ? d : l;
         uint16_t* dst = wexp + ((size_t)m_comp * Cm + cm0 + cm) * Kp + (size_t)k_comp * Cp + ck;
