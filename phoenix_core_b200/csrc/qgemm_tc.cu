@@ -21,6 +21,7 @@
 // All mbarrier waits are bounded.
 #include "tc_common.cuh"
 #include "tensor_path.cuh"
+#include "unaligned_chunk.h"
 
 namespace pcb {
 namespace {
@@ -166,16 +167,17 @@ __device__ __forceinline__ void load_unaligned(uint32_t (&r)[ROWS / 4], const QO
     uint32_t mask[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) mask[j] = (2 * j < left ? 0xffffu : 0u) | (2 * j + 1 < left ? 0xffff0000u : 0u);
-    const int at0 = comp * o.cs + v0 * o.ld + u;
+    const unsigned at0 = (unsigned)comp * o.cs + (unsigned)v0 * o.ld + u;  // (unsigned: rows past the last one may leave the 32-bit range)
 #pragma unroll
     for (int i = 0; i < C::COUNT; ++i) {
         const bool ok = left > 0 && v0 + i * C::STEP < o.nv;
-        const int at = at0 + i * C::STEP * o.ld, al = at & ~3, sh = at & 3;
+        const int at = (int)(at0 + (unsigned)(i * C::STEP) * o.ld), al = at & ~3, sh = at & 3;
+        const int vectors = ok ? chunk_vectors(at, total) : 0;
         const uint2* q = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(o.p) + al);
         uint2 a = make_uint2(0u, 0u), b = a, c = a;
-        if (ok) a = __ldg(q);
-        if (ok && al + 4 < total) b = __ldg(q + 1);
-        if (ok && sh && al + 8 < total) c = __ldg(q + 2);
+        if (vectors > 0) a = __ldg(q);
+        if (vectors > 1) b = __ldg(q + 1);
+        if (vectors > 2) c = __ldg(q + 2);
         uint32_t w[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
 #pragma unroll
         for (int j = 0; j < 5; ++j) w[j] = (sh & 2) ? w[j + 1] : w[j];
