@@ -15,6 +15,8 @@
  *       dense input   [4*B, I];  dense filters [4, I, O] (IO) or [4, O, I] (OI);  dense bias [4, O]
  *     (reference: src/backend/tensor.hpp:501-545 TensorSplit, src/backend/conv2d_descriptor.hpp:39-42,
  *      :333-345, src/backend/dense_descriptor.hpp:28-52)
+ *   - Results must not share memory with operands of the same call. (Dense layers and NCHW fp32 convolutions on the tensor cores
+ *     copy their operands first where they do, so that there y may replace x, and dx may replace x or dy.)
  *   - Work is enqueued on the given CUDA stream and the call returns without synchronising.
  *   - The library never allocates device memory in these entry points: scratch comes from the caller
  *     (`workspace`, sized by the *_workspace_size query), as the reference's operators obtain theirs from

@@ -126,6 +126,13 @@ inline bool algebra_setup(int algebra, Geom& g) {
 
 inline size_t dtype_size(int dtype) { return dtype == PCB_F32 ? 4 : 2; }
 
+// Whether two tensors share memory. A kernel that reads a caller's tensor while other CTAs write the result (or a launch that clears the
+// result beside the staging of an operand) may only run where they do not.
+inline bool overlaps(const void* a, size_t a_bytes, const void* b, size_t b_bytes) {
+    const uintptr_t pa = reinterpret_cast<uintptr_t>(a), pb = reinterpret_cast<uintptr_t>(b);
+    return a && b && pa < pb + b_bytes && pb < pa + a_bytes;
+}
+
 // Error plumbing (host side). The message of the last failure is kept per host thread.
 void set_error(const char* fmt, ...);
 #define PCB_CUDA_TRY(expr)                                                                      \
