@@ -996,10 +996,14 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     }
     const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m;
     {
+        // the output is cleared beside the staging of the operands, unless it shares memory with one of them
         const size_t out_bytes = (size_t)g.nc * g.Nb * pl.Cout * pl.Hout * pl.Wout * sizeof(float);
-        if (p.splits > 1 && !add_zero_job(pro, out, out_bytes)) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
+        const bool apart = !overlaps(out, out_bytes, b, (size_t)pl.LK * g.Nb * pl.Cin * pl.Hin * pl.Win * sizeof(float)) &&
+                           !overlaps(out, out_bytes, a, (size_t)g.nc * g.Co * g.Ci * taps * sizeof(float));
+        const bool cleared = p.splits > 1 && apart && add_zero_job(pro, out, out_bytes);
         const int rc = launch_prologue(pro, sc, stream, &chain);
         if (rc != PCB_OK) return rc;
+        if (p.splits > 1 && !cleared) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
     }
     const int n_items = n_tiles * p.splits;
     const int grid = n_items < sm_count() ? n_items : sm_count();

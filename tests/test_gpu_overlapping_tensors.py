@@ -65,3 +65,25 @@ def test_dense(pcb, dtype, batch, ci, co):
         pcb.denseBwd(x, w, dy2, dw2, dx2, bwd)
         _close(dx2, dx, tol)
         _close(dw2, dw, tol)
+
+
+# few tiles and a long reduction: the fp32 kernel cuts it and adds into a cleared output
+@pytest.mark.parametrize("n,c,h,w", [(2, 64, 8, 8), (1, 48, 14, 9), (3, 96, 7, 7)])
+def test_fp32_convolution(pcb, n, c, h, w):
+    t, tol = TYPES["f32"]
+    xs, ws = (4 * n, c, h, w), (4, c, c, 3, 3)
+    args = (xs, ws, 1, 1, pcb.Padding.SAME, (), 1, pcb.Algebra.QUATERNION, pcb.DataFormat.NCHW, pcb.FilterLayout.OIHW)
+    fwd, bwd = pcb.Conv2DFwdDescriptor(*args, False), pcb.Conv2DBwdDescriptor(*args, True)
+    x, f, dy = _normal(1, xs, t), _normal(2, ws, t, 0.04), _normal(3, xs, t)
+    y, dw, dx = torch.empty_like(x), torch.empty_like(f), torch.empty_like(x)
+    pcb.conv2DFwd(x, f, None, y, fwd)
+    pcb.conv2DBwd(x, f, dy, dw, dx, bwd)
+    for _ in range(3):
+        x2 = x.clone()
+        pcb.conv2DFwd(x2, f, None, x2, fwd)
+        _close(x2, y, tol)
+        for target in ("x", "dy"):
+            a, b, dw2 = x.clone(), dy.clone(), torch.empty_like(f)
+            pcb.conv2DBwd(a, f, b, dw2, a if target == "x" else b, bwd)
+            _close(a if target == "x" else b, dx, tol)
+            _close(dw2, dw, tol)
