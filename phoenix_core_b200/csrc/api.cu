@@ -348,7 +348,9 @@ int conv_bwd_both(const pcb_conv2d_desc* desc, const void* x, const void* w, con
     size_t offset = 0;
     const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(dy) |
                           reinterpret_cast<uintptr_t>(dw) | reinterpret_cast<uintptr_t>(dx) | reinterpret_cast<uintptr_t>(workspace);
-    if (x && w && dy && dw && dx && workspace && (all & 15u) == 0 && bwd_shares_dy(desc, g, &view, &offset) &&
+    // (not where dx replaces x: the filter gradient, run second, reads x)
+    const size_t x_bytes = (size_t)g.nc * g.Nb * g.Ci * g.groups * g.H * g.W * dtype_size(desc->dtype);
+    if (x && w && dy && dw && dx && workspace && (all & 15u) == 0 && !overlaps(dx, x_bytes, x, x_bytes) && bwd_shares_dy(desc, g, &view, &offset) &&
         workspace_bytes_ >= conv_workspace_bytes(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g) + offset) {
         // backward-data first: it leaves the padded dy in [WS_HEADER, WS_HEADER + offset)
         rc = conv_bwd_data(desc, w, dy, dx, workspace, workspace_bytes_, stream, sc);

@@ -1359,6 +1359,9 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     // (Not for zero-inserted gradients, channel slices of grouped layers, or images smaller than a tile box.)
     bool direct = !g.plain && sa.c == 1 && sa.w == pl.Cin && sa.h == (long long)pl.Win * pl.Cin && sa.p == (long long)pl.Hin * pl.Win * pl.Cin &&
                   pl.Cin % 16 == 0 && pl.ins_h == 1 && pl.ins_w == 1 && (reinterpret_cast<uintptr_t>(act) & 15u) == 0;
+    // The strided backward-data pass reads a copy of dy where dx shares its memory.
+    if (pl.dual && direct)
+        direct = !overlaps(out, (size_t)g.nc * g.Nb * pl.Cout * pl.Hout * pl.Wout * 2, act, (size_t)pl.LK * g.Nb * pl.Cin * pl.Hin * pl.Win * 2);
 
     const bool inserted = pl.ins_h != 1 || pl.ins_w != 1;
     bool chain = false;

@@ -87,3 +87,28 @@ def test_fp32_convolution(pcb, n, c, h, w):
             pcb.conv2DBwd(a, f, b, dw2, a if target == "x" else b, bwd)
             _close(a if target == "x" else b, dx, tol)
             _close(dw2, dw, tol)
+
+
+@pytest.mark.parametrize("layout", ["nchw", "nhwc"])
+def test_strided_backward(pcb, layout):
+    t, tol = TYPES["f16"]
+    nhwc = layout == "nhwc"
+    n, c, h, w = 6, 32, 40, 36
+    xs, ys = ((4 * n, h, w, c), (4 * n, h // 2, w // 2, c)) if nhwc else ((4 * n, c, h, w), (4 * n, c, h // 2, w // 2))
+    ws = (4, c, 3, 3, c) if nhwc else (4, c, c, 3, 3)
+    bwd = pcb.Conv2DBwdDescriptor(xs, ws, 2, 1, pcb.Padding.SAME, (), 1, pcb.Algebra.QUATERNION, pcb.DataFormat.NHWC if nhwc else pcb.DataFormat.NCHW,
+                                  pcb.FilterLayout.OHWI if nhwc else pcb.FilterLayout.OIHW, True)
+    x, f, dy = _normal(1, xs, t), _normal(2, ws, t, 0.05), _normal(3, ys, t)
+    dw, dx = torch.empty_like(f), torch.empty_like(x)
+    pcb.conv2DBwd(x, f, dy, dw, dx, bwd)
+    for _ in range(3):
+        x2, dw2 = x.clone(), torch.empty_like(f)                            # dx over x
+        pcb.conv2DBwd(x2, f, dy, dw2, x2, bwd)
+        _close(x2, dx, tol)
+        _close(dw2, dw, tol)
+        buf = torch.zeros(x.numel(), dtype=t, device="cuda")                # dx over dy
+        dy2 = buf[:dy.numel()].view(ys)
+        dy2.copy_(dy)
+        dx2, dw2 = buf.view(xs), torch.empty_like(f)
+        pcb.conv2DBwd(x, f, dy2, dw2, dx2, bwd)
+        _close(dx2, dx, tol)
