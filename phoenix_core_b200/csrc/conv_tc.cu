@@ -146,7 +146,7 @@ template <int KS, bool DUAL> constexpr int G_MAX_STAGES = KS == 64 ? (DUAL ? 6 :
 template <int KS, bool HALO, bool DUAL>
 __global__ void __launch_bounds__(G_THREADS, 1)
 qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GParams p,
-                        const uint16_t* __restrict__ bias, uint16_t* __restrict__ out, int* __restrict__ status) {
+                        const uint16_t* bias, uint16_t* __restrict__ out, int* __restrict__ status) {
     constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = (DUAL ? GN / 2 : GN) * KS * 2;
     constexpr int MAX_STAGES = G_MAX_STAGES<KS, DUAL>;
     const uint32_t STAGE = HALO ? p.stage_bytes : A_BYTES + B_BYTES;
@@ -358,7 +358,7 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             const int d = row_ok ? m / p.Cout : 0, co = m - d * p.Cout;
             float badd = 0.f;
             if (row_ok && p.has_bias) {
-                const uint16_t raw = bias[d * p.bias_ld + co];
+                const uint16_t raw = ld_chained(bias + d * p.bias_ld + co);
                 badd = p.fmt == 0 ? __half2float(__ushort_as_half(raw)) : __bfloat162float(__ushort_as_bfloat16(raw));
             }
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_G_EPILOGUE);
@@ -634,7 +634,7 @@ struct StageJob {
 template <int V, int U>
 __device__ __forceinline__ void stage_compact(const StageJob& p, unsigned block, uint4* tile /*[STAGE_UNITS]*/) {
     constexpr int TPX = STAGE_UNITS / U;
-    const uint16_t* __restrict__ x = static_cast<const uint16_t*>(p.x);
+    const uint16_t* x = static_cast<const uint16_t*>(p.x);
     uint4* __restrict__ xp = static_cast<uint4*>(p.xp);
     const unsigned total_px = p.total_px, HW = p.HW, by = block / p.bx;
     const int C = p.C, nblk = p.nblk;
@@ -651,13 +651,12 @@ __device__ __forceinline__ void stage_compact(const StageJob& p, unsigned block,
         for (int e = 0; e < 8; ++e) {
             const bool ok = P < total_px && c0 + 8 * g + e < C;
             if (V == 4) {
-                uint2 w = make_uint2(0u, 0u);
-                if (ok) w = __ldg(reinterpret_cast<const uint2*>(src + (size_t)e * HW));
+                const uint2 w = ld_chained(reinterpret_cast<const uint2*>(src + (size_t)e * HW), ok);
                 raw[e][0] = w.x; raw[e][V == 4 ? 1 : 0] = w.y;
             } else if (V == 2) {
-                raw[e][0] = ok ? __ldg(reinterpret_cast<const uint32_t*>(src + (size_t)e * HW)) : 0u;
+                raw[e][0] = ld_chained(reinterpret_cast<const uint32_t*>(src + (size_t)e * HW), ok);
             } else {
-                raw[e][0] = ok ? (uint32_t)__ldg(src + (size_t)e * HW) : 0u;
+                raw[e][0] = ld_chained(src + (size_t)e * HW, ok);
             }
         }
 #pragma unroll
@@ -700,14 +699,13 @@ int padded_channels(int c) { return round_up(c, channel_slice(c)); }
 // Channels-last sources that have to be copied (padded to slices, or cut into blocks of 8 U channels for the filter gradient): 16-byte
 // units, C a multiple of 8. Destination as for stage_compact_kernel.
 __device__ __forceinline__ void repack_channels_last(const StageJob& p, unsigned block) {
-    const uint4* __restrict__ x = static_cast<const uint4*>(p.x);
+    const uint4* x = static_cast<const uint4*>(p.x);
     uint4* __restrict__ xp = static_cast<uint4*>(p.xp);
     const unsigned per_px = (unsigned)(p.nblk * p.U), src_units = (unsigned)p.C / 8;
     const size_t total = (size_t)p.total_px * per_px;
     for (size_t i = (size_t)block * STAGE_THREADS + threadIdx.x; i < total; i += (size_t)p.blocks * STAGE_THREADS) {
         const unsigned P = (unsigned)(i / per_px), u = (unsigned)(i - (size_t)P * per_px);
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (u < src_units) v = __ldg(x + (size_t)P * src_units + u);
+        const uint4 v = ld_chained(x + (size_t)P * src_units + u, u < src_units);
         size_t dst = i;
         if (p.blocked) {
             const unsigned comp = P / p.HW / p.Nb, b = u / p.U;
@@ -754,7 +752,7 @@ __device__ __forceinline__ void pack_filters_rows(const FilterJob& p, unsigned b
                 const int kh = src_tap / p.fs.KW, kw = src_tap - kh * p.fs.KW;
                 src = p.w + (long long)alg_pair(p.ga, l, d) * p.fs.r + (long long)kh * p.fs.h + (long long)kw * p.fs.w + (long long)cm * (p.transposed ? p.fs.i : p.fs.o);
             }
-            for (int ck = tx; ck < p.Cp; ck += wx) dst[k0 + ck] = (comp_ok && ck < Ck) ? (uint16_t)(__ldg(src + ck * ck_stride) ^ flip) : (uint16_t)0;
+            for (int ck = tx; ck < p.Cp; ck += wx) dst[k0 + ck] = (comp_ok && ck < Ck) ? (uint16_t)(ld_chained(src + ck * ck_stride) ^ flip) : (uint16_t)0;
         }
     }
 }
@@ -768,7 +766,7 @@ constexpr int PACK_TM = 32, PACK_TK = 64;   // rows (M-side channels) and K colu
 constexpr int PACK_TILE_MAX_TAPS = 9;     // 37 KB of shared memory at 9 taps
 // (every thread writes 8 consecutive K columns with one 16-byte store)
 __device__ __forceinline__ void pack_filters_tile(const FilterJob& p, unsigned block, uint16_t* tile) {
-    const uint16_t* __restrict__ w = p.w;
+    const uint16_t* w = p.w;
     uint16_t* __restrict__ wexp = p.wexp;
     const int Co = p.Co, Ci = p.Ci, taps = p.taps, Mp = p.Mp, Kp = p.Kp, Cp = p.Cp, transposed = p.transposed, nc = p.nc, ga = p.ga, tap_split = p.tap_split;
     const unsigned long long neg = p.neg;
@@ -792,7 +790,7 @@ __device__ __forceinline__ void pack_filters_tile(const FilterJob& p, unsigned b
             const int limit = co0 + co < Co ? e_limit : 0;
             uint16_t* trow = tile + co * pitch;
 #pragma unroll 9
-            for (int e = lane; e < run; e += 32) trow[e] = e < limit ? __ldg(row + e) : (uint16_t)0;
+            for (int e = lane; e < run; e += 32) trow[e] = ld_chained(row + e, e < limit);
         }
     }
     __syncthreads();
@@ -1247,7 +1245,7 @@ qconv_filter_xmajor_tc_kernel(const __grid_constant__ CUtensorMap map_x, const _
 // destination (coalesced stores); otherwise the destination is addressed through the filter-gradient strides (OHWI, HWIO,
 // the input-major dense gradient, the slice of one group) and the threads walk the source.
 template <typename T>
-__global__ void unpack_filter_grad_kernel(const float* __restrict__ src, T* __restrict__ dw, int taps, size_t per_tap, int dense_oihw,
+__global__ void unpack_filter_grad_kernel(const float* src, T* __restrict__ dw, int taps, size_t per_tap, int dense_oihw,
                                           int Co, int Ci, FilterStrides ds) {
     const size_t total = per_tap * taps;
     chain_wait();
@@ -1256,7 +1254,7 @@ __global__ void unpack_filter_grad_kernel(const float* __restrict__ src, T* __re
         if (dense_oihw) {
             const int tap = (int)(idx % taps);
             const size_t e = idx / taps;
-            DType<T>::store(dw + idx, src[(size_t)tap * per_tap + e]);
+            DType<T>::store(dw + idx, ld_chained(src + (size_t)tap * per_tap + e));
             continue;
         }
         const int ci = (int)(idx % Ci);
@@ -1265,7 +1263,7 @@ __global__ void unpack_filter_grad_kernel(const float* __restrict__ src, T* __re
         const size_t comps = per_tap / ((size_t)Co * Ci);
         const int r = (int)(rest % comps), tap = (int)(rest / comps);
         const int kh = tap / ds.KW, kw = tap - kh * ds.KW;
-        DType<T>::store(dw + (long long)r * ds.r + (long long)co * ds.o + (long long)ci * ds.i + (long long)kh * ds.h + (long long)kw * ds.w, src[idx]);
+        DType<T>::store(dw + (long long)r * ds.r + (long long)co * ds.o + (long long)ci * ds.i + (long long)kh * ds.h + (long long)kw * ds.w, ld_chained(src + idx));
     }
 }
 

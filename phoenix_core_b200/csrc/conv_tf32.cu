@@ -58,7 +58,7 @@ template <bool CHUNKED>
 __global__ void __launch_bounds__(T_THREADS, 1)
 qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __grid_constant__ CUtensorMap map_w_lo,
                           const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo, TParams p,
-                          const float* __restrict__ bias, float* __restrict__ out, int* __restrict__ status) {
+                          const float* bias, float* __restrict__ out, int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -170,7 +170,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
             const int m = tm * TM + q * 32 + lane;
             const bool row_ok = m < p.Mvalid;
             const int d = row_ok ? m / p.Cout : 0, co = m - d * p.Cout;
-            const float badd = (row_ok && p.has_bias && split == 0) ? bias[d * p.Cout + co] : 0.f;
+            const float badd = (row_ok && p.has_bias && split == 0) ? ld_chained(bias + d * p.Cout + co) : 0.f;
             float part[CHUNKED ? 4 : 1][CHUNKED ? 32 : 1];          // this thread's 128 columns, summed over the chunks so far
             if (CHUNKED) {
 #pragma unroll
@@ -388,13 +388,10 @@ __device__ __forceinline__ void stage_compact_f32(const StageJob32& p, unsigned 
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const bool ok = P < p.total_px && c0 + 4 * g + e < p.C;
-#pragma unroll
-            for (int j = 0; j < V; ++j) raw[e][j] = 0.f;
-            if (!ok) continue;
             const float* q = src + (size_t)e * HW;
-            if (V == 4) { const float4 f = __ldg(reinterpret_cast<const float4*>(q)); raw[e][0] = f.x; raw[e][V > 1 ? 1 : 0] = f.y; raw[e][V > 2 ? 2 : 0] = f.z; raw[e][V > 3 ? 3 : 0] = f.w; }
-            else if (V == 2) { const float2 f = __ldg(reinterpret_cast<const float2*>(q)); raw[e][0] = f.x; raw[e][V > 1 ? 1 : 0] = f.y; }
-            else raw[e][0] = __ldg(q);
+            if (V == 4) { const float4 f = ld_chained(reinterpret_cast<const float4*>(q), ok); raw[e][0] = f.x; raw[e][V > 1 ? 1 : 0] = f.y; raw[e][V > 2 ? 2 : 0] = f.z; raw[e][V > 3 ? 3 : 0] = f.w; }
+            else if (V == 2) { const float2 f = ld_chained(reinterpret_cast<const float2*>(q), ok); raw[e][0] = f.x; raw[e][V > 1 ? 1 : 0] = f.y; }
+            else raw[e][0] = ld_chained(q, ok);
         }
 #pragma unroll
         for (int j = 0; j < V; ++j) tile[stage_unit<V, U>(l * V + j, g)] = make_float4(raw[0][j], raw[1][j], raw[2][j], raw[3][j]);
@@ -432,7 +429,7 @@ struct FilterJob32 {
 // w_io: the filters are stored [r][ci][co] (dense input-major layout, one tap).
 __device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned block, unsigned blocks) {
     // one row (tap, m) of the expanded matrix per block iteration; the row is decoded once and the threads walk k
-    const float* __restrict__ w = p.w;
+    const float* w = p.w;
     float* __restrict__ hi = p.hi;
     float* __restrict__ lo = p.lo;
     const int Co = p.Co, Ci = p.Ci, taps = p.taps, Mp = p.Mp, Kp = p.Kp, Cp = p.Cp, transposed = p.transposed, w_io = p.w_io, nc = p.nc, ga = p.ga;
@@ -453,7 +450,7 @@ __device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned 
                 const int co = transposed ? ck : cm, ci = transposed ? cm : ck;
                 const int r = alg_pair(ga, l, d);
                 const size_t src = w_io ? ((size_t)r * Ci + ci) * Co + co : ((size_t)(r * Co + co) * Ci + ci) * taps + src_tap;
-                v = __ldg(w + src);
+                v = ld_chained(w + src);
                 if (alg_negative(neg, l, d)) v = -v;
             }
             float h, lw;
@@ -737,7 +734,7 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
 }
 
 // scratch [tap][r][co][ci] -> dw [r][co][ci][tap], or [r][ci][co] for dense layers (input-major, one tap)
-__global__ void unpack_filter_grad_f32_kernel(const float* __restrict__ src, float* __restrict__ dw, int taps, int Co, int Ci, int dw_io, int nc) {
+__global__ void unpack_filter_grad_f32_kernel(const float* src, float* __restrict__ dw, int taps, int Co, int Ci, int dw_io, int nc) {
     const size_t per_tap = (size_t)nc * Co * Ci, total = per_tap * taps;
     chain_wait();
     chain_next();
@@ -746,10 +743,10 @@ __global__ void unpack_filter_grad_f32_kernel(const float* __restrict__ src, flo
             const int co = (int)(idx % Co);
             const int ci = (int)((idx / Co) % Ci);
             const int r = (int)(idx / ((size_t)Co * Ci));
-            dw[idx] = src[((size_t)r * Co + co) * Ci + ci];
+            dw[idx] = ld_chained(src + ((size_t)r * Co + co) * Ci + ci);
         } else {
             const int tap = (int)(idx % taps);
-            dw[idx] = src[(size_t)tap * per_tap + idx / taps];
+            dw[idx] = ld_chained(src + (size_t)tap * per_tap + idx / taps);
         }
     }
 }

@@ -65,7 +65,7 @@ __device__ __forceinline__ uint64_t desc_plain(uint32_t smem_addr, uint32_t lead
 // ===================================================================================================
 __global__ void __launch_bounds__(NW_THREADS, 1)
 qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, NParams p,
-                       const uint16_t* __restrict__ bias, uint16_t* __restrict__ out, int* __restrict__ status) {
+                       const uint16_t* bias, uint16_t* __restrict__ out, int* __restrict__ status) {
     extern __shared__ uint8_t smem_raw[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -164,7 +164,7 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         const int d = row_ok ? m / p.Cout : 0, co = m - d * p.Cout;
         float badd = 0.f;
         if (row_ok && p.has_bias) {
-            const uint16_t raw = bias[d * p.Cout + co];
+            const uint16_t raw = ld_chained(bias + d * p.Cout + co);
             badd = p.fmt == 0 ? __half2float(__ushort_as_half(raw)) : __bfloat162float(__ushort_as_bfloat16(raw));
         }
         for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local_tile) {
@@ -271,9 +271,9 @@ __device__ __forceinline__ void pack_planar_any(const PlanarJob& p, unsigned blo
             if (p.s2d) {
                 const int sub = c / p.C, cs = c - sub * p.C;             // sub = dy * 2 + dx
                 const int sh = 2 * hp + (sub >> 1) - p.pad_top, sw = 2 * wp + (sub & 1) - p.pad_left;
-                if (sub < 4 && sh >= 0 && sw >= 0 && sh < p.H && sw < p.W) v = p.x[(((size_t)plane * p.C + cs) * p.H + sh) * p.W + sw];
+                if (sub < 4 && sh >= 0 && sw >= 0 && sh < p.H && sw < p.W) v = ld_chained(p.x + (((size_t)plane * p.C + cs) * p.H + sh) * p.W + sw);
             } else if (c < p.C && inside) {
-                v = p.x[(((size_t)plane * p.C + c) * p.H + ih) * p.W + iw];
+                v = ld_chained(p.x + (((size_t)plane * p.C + c) * p.H + ih) * p.W + iw);
             }
             vals[e] = v;
         }
@@ -298,8 +298,7 @@ __device__ __forceinline__ void pack_planar_rows(const PlanarJob& p, unsigned bl
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const int c = grp * 8 + e;
-            uint2 raw = make_uint2(0u, 0u);
-            if (row_in && c < p.C) raw = __ldg(reinterpret_cast<const uint2*>(p.x + (((size_t)plane * p.C + c) * p.H + ih) * p.W + 4 * q));
+            const uint2 raw = ld_chained(reinterpret_cast<const uint2*>(p.x + (((size_t)plane * p.C + c) * p.H + ih) * p.W + 4 * q), row_in && c < p.C);
             *reinterpret_cast<uint2*>(v[e]) = raw;
         }
         uint16_t* row = p.xp + (((size_t)plane * p.groups + grp) * p.Hp + hp) * (size_t)p.Wp * 8;
@@ -340,7 +339,7 @@ __device__ __forceinline__ void pack_planar_s2d_pairs(const PlanarJob& p, unsign
             if (sh < 0 || sh >= p.H || sw < 0 || sw >= p.W) continue;   // W is even, so sw + 1 < W as well
 #pragma unroll
             for (int cs = 0; cs < C; ++cs) {
-                const uint32_t pair = __ldg(reinterpret_cast<const uint32_t*>(p.x + (((size_t)plane * C + cs) * p.H + sh) * p.W + sw));
+                const uint32_t pair = ld_chained(reinterpret_cast<const uint32_t*>(p.x + (((size_t)plane * C + cs) * p.H + sh) * p.W + sw));
                 vals[(dy * 2 + 0) * C + cs] = (uint16_t)(pair & 0xffffu);             // staged channel (dy, dx, c)
                 vals[(dy * 2 + 1) * C + cs] = (uint16_t)(pair >> 16);
             }
@@ -375,14 +374,14 @@ __device__ __forceinline__ void pack_filters_planar(const PlanarFilterJob& p, un
             const int sub = ck / p.Ci, ci = ck - sub * p.Ci;
             const int kh = 2 * (tap / p.KWe) + (sub >> 1), kw = 2 * (tap % p.KWe) + (sub & 1);
             if (cm_comp < p.nc && ck_comp < p.nc && sub < 4 && kh < p.KH && kw < p.KW) {
-                v = __ldg(p.w + ((size_t)(alg_pair(p.ga, ck_comp, cm_comp) * p.Co + cm) * p.Ci + ci) * (p.KH * p.KW) + kh * p.KW + kw);
+                v = ld_chained(p.w + ((size_t)(alg_pair(p.ga, ck_comp, cm_comp) * p.Co + cm) * p.Ci + ci) * (p.KH * p.KW) + kh * p.KW + kw);
                 if (alg_negative(p.neg, ck_comp, cm_comp)) v ^= 0x8000u;
             }
         } else if (cm_comp < p.nc && ck_comp < p.nc && ck < Ck) {
             const int d = p.transposed ? ck_comp : cm_comp, l = p.transposed ? cm_comp : ck_comp;
             const int co = p.transposed ? ck : cm, ci = p.transposed ? cm : ck;
             const int src_tap = p.transposed ? p.taps - 1 - tap : tap;
-            v = __ldg(p.w + ((size_t)(alg_pair(p.ga, l, d) * p.Co + co) * p.Ci + ci) * p.taps + src_tap);
+            v = ld_chained(p.w + ((size_t)(alg_pair(p.ga, l, d) * p.Co + co) * p.Ci + ci) * p.taps + src_tap);
             if (alg_negative(p.neg, l, d)) v ^= 0x8000u;
         }
         p.wexp[(((size_t)tap * (p.Kp / 8) + k / 8) * NM + m) * 8 + (k & 7)] = v;
@@ -636,18 +635,18 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
 
 // scratch [tap][r][co][ci] fp32 -> dw [r][co][ci][tap] in the tensor type
 template <typename T>
-__global__ void unpack_narrow_filter_grad_kernel(const float* __restrict__ src, T* __restrict__ dw, int taps, size_t per_tap) {
+__global__ void unpack_narrow_filter_grad_kernel(const float* src, T* __restrict__ dw, int taps, size_t per_tap) {
     const size_t total = per_tap * taps;
     chain_wait();
     chain_next();
     for (size_t idx = (size_t)blockIdx.x * blockDim.x + threadIdx.x; idx < total; idx += (size_t)gridDim.x * blockDim.x) {
         const int tap = (int)(idx % taps);
-        DType<T>::store(dw + idx, src[(size_t)tap * per_tap + idx / taps]);
+        DType<T>::store(dw + idx, ld_chained(src + (size_t)tap * per_tap + idx / taps));
     }
 }
 // s2d: scratch [staged tap][r][co][c' = (dy, dx, ci)] -> dw [r][co][ci][kh][kw]
 template <typename T>
-__global__ void unpack_narrow_filter_grad_s2d_kernel(const float* __restrict__ src, T* __restrict__ dw, int rows /*nc*Co*/, int Ci, int KH, int KW,
+__global__ void unpack_narrow_filter_grad_s2d_kernel(const float* src, T* __restrict__ dw, int rows /*nc*Co*/, int Ci, int KH, int KW,
                                                      int KWe, int taps_e) {
     const size_t total = (size_t)rows * Ci * KH * KW;
     chain_wait();
@@ -659,7 +658,7 @@ __global__ void unpack_narrow_filter_grad_s2d_kernel(const float* __restrict__ s
         const int ci = (int)(rest % Ci);
         const size_t row = rest / Ci;
         const int tap = (kh >> 1) * KWe + (kw >> 1), cp = ((kh & 1) * 2 + (kw & 1)) * Ci + ci;
-        DType<T>::store(dw + idx, src[((size_t)tap * rows + row) * (4 * Ci) + cp]);
+        DType<T>::store(dw + idx, ld_chained(src + ((size_t)tap * rows + row) * (4 * Ci) + cp));
     }
 }
 

@@ -108,15 +108,13 @@ __device__ __forceinline__ void load_chunks(uint32_t (&r)[ROWS / 4], const QOper
         const bool ok = u_ok && v0 + i * C::STEP < o.nv;
         const char* q = src + i * step;
         if (CB == 16) {
-            uint4 w = make_uint4(0u, 0u, 0u, 0u);
-            if (ok) w = __ldg(reinterpret_cast<const uint4*>(q));
+            const uint4 w = ld_chained(reinterpret_cast<const uint4*>(q), ok);
             r[4 * i] = w.x; r[4 * i + 1] = w.y; r[4 * i + 2] = w.z; r[4 * i + 3] = w.w;
         } else if (CB == 8) {
-            uint2 w = make_uint2(0u, 0u);
-            if (ok) w = __ldg(reinterpret_cast<const uint2*>(q));
+            const uint2 w = ld_chained(reinterpret_cast<const uint2*>(q), ok);
             r[2 * i] = w.x; r[2 * i + 1] = w.y;
         } else {
-            r[i] = ok ? __ldg(reinterpret_cast<const uint32_t*>(q)) : 0u;
+            r[i] = ld_chained(reinterpret_cast<const uint32_t*>(q), ok);
         }
     }
 }
@@ -174,10 +172,7 @@ __device__ __forceinline__ void load_unaligned(uint32_t (&r)[ROWS / 4], const QO
         const int at = (int)(at0 + (unsigned)(i * C::STEP) * o.ld), al = at & ~3, sh = at & 3;
         const int vectors = ok ? chunk_vectors(at, total) : 0;
         const uint2* q = reinterpret_cast<const uint2*>(static_cast<const uint16_t*>(o.p) + al);
-        uint2 a = make_uint2(0u, 0u), b = a, c = a;
-        if (vectors > 0) a = __ldg(q);
-        if (vectors > 1) b = __ldg(q + 1);
-        if (vectors > 2) c = __ldg(q + 2);
+        const uint2 a = ld_chained(q, vectors > 0), b = ld_chained(q + 1, vectors > 1), c = ld_chained(q + 2, vectors > 2);
         uint32_t w[6] = {a.x, a.y, b.x, b.y, c.x, c.y};
 #pragma unroll
         for (int j = 0; j < 5; ++j) w[j] = (sh & 2) ? w[j + 1] : w[j];
@@ -225,9 +220,9 @@ __device__ __forceinline__ void q_store(void* out, size_t at, float v, int fmt) 
     else static_cast<__nv_bfloat16*>(out)[at] = __float2bfloat16_rn(v);
 }
 __device__ __forceinline__ float q_bias(const void* bias, size_t at, int fmt) {
-    if (fmt == 2) return static_cast<const float*>(bias)[at];
-    if (fmt == 0) return __half2float(static_cast<const __half*>(bias)[at]);
-    return __bfloat162float(static_cast<const __nv_bfloat16*>(bias)[at]);
+    if (fmt == 2) return ld_chained(static_cast<const float*>(bias) + at);
+    const uint16_t raw = ld_chained(static_cast<const uint16_t*>(bias) + at);
+    return fmt == 0 ? __half2float(__ushort_as_half(raw)) : __bfloat162float(__ushort_as_bfloat16(raw));
 }
 
 template <bool F32, int NT, bool AK, bool BK>

@@ -39,6 +39,41 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
 constexpr size_t ONE_CTA_SMEM = 116 * 1024;
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Loads of a chained kernel behind chain_wait(): the grid is resident while the kernel in front still writes, so data may not go through the
+// non-coherent path (__ldg, or const __restrict__ parameters), which is for data that nobody writes during the life of the grid.
+// Not loaded, and zero, where `ok` is false.
+__device__ __forceinline__ uint16_t ld_chained(const uint16_t* p, bool ok = true) {
+    uint16_t v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u16 %0, 0;\n\t@q ld.global.u16 %0, [%1];\n\t}" : "=h"(v) : "l"(p), "r"((uint32_t)ok));
+    return v;
+}
+__device__ __forceinline__ uint32_t ld_chained(const uint32_t* p, bool ok = true) {
+    uint32_t v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %2, 0;\n\tmov.u32 %0, 0;\n\t@q ld.global.u32 %0, [%1];\n\t}" : "=r"(v) : "l"(p), "r"((uint32_t)ok));
+    return v;
+}
+__device__ __forceinline__ uint2 ld_chained(const uint2* p, bool ok = true) {
+    uint2 v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %3, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\t@q ld.global.v2.u32 {%0, %1}, [%2];\n\t}"
+                 : "=r"(v.x), "=r"(v.y) : "l"(p), "r"((uint32_t)ok));
+    return v;
+}
+__device__ __forceinline__ uint4 ld_chained(const uint4* p, bool ok = true) {
+    uint4 v;
+    asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.u32 q, %5, 0;\n\tmov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+                 "@q ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+                 : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p), "r"((uint32_t)ok));
+    return v;
+}
+__device__ __forceinline__ float ld_chained(const float* p, bool ok = true) { return __uint_as_float(ld_chained(reinterpret_cast<const uint32_t*>(p), ok)); }
+__device__ __forceinline__ float2 ld_chained(const float2* p, bool ok = true) {
+    const uint2 v = ld_chained(reinterpret_cast<const uint2*>(p), ok);
+    return make_float2(__uint_as_float(v.x), __uint_as_float(v.y));
+}
+__device__ __forceinline__ float4 ld_chained(const float4* p, bool ok = true) {
+    const uint4 v = ld_chained(reinterpret_cast<const uint4*>(p), ok);
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
 template <typename... Params, typename... Args>
 cudaError_t launch_chained_if(bool chained, void (*kernel)(Params...), unsigned grid, unsigned block, size_t smem, cudaStream_t stream, Args... args) {
     cudaLaunchConfig_t cfg = {};
