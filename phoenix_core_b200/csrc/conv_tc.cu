@@ -362,7 +362,7 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 badd = p.fmt == 0 ? __half2float(__ushort_as_half(raw)) : __bfloat162float(__ushort_as_bfloat16(raw));
             }
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_G_EPILOGUE);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_may_store(ok, status);
             if (!ok) break;
             tc_fence_after_sync();
             if (p.plane_mode) {
@@ -1067,7 +1067,7 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
         bool ok = mbar_wait_bounded(tmem_full, 0, status, ST_G_EPILOGUE);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = warp_may_store(ok, status);
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
             // row of the tile -> (output component d, channel co)
@@ -1206,7 +1206,7 @@ qconv_filter_xmajor_tc_kernel(const __grid_constant__ CUtensorMap map_x, const _
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
         bool ok = mbar_wait_bounded(tmem_full, 0, status, ST_G_EPILOGUE);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = warp_may_store(ok, status);
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
             const int row = q * 32 + lane;                       // row -> (tap, input component l, channel ci)

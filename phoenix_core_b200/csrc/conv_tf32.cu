@@ -180,7 +180,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                 for (int c = 0; c + 1 < p.n_chunks && ok; ++c, ++unit) {
                     const int buf = unit & 1, use = unit >> 1;
                     ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
-                    ok = __all_sync(0xffffffffu, ok);
+                    ok = warp_may_store(ok, status);
                     if (!ok) break;
                     tc_fence_after_sync();
 #pragma unroll
@@ -201,7 +201,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
             const int buf = unit & 1, use = unit >> 1;
             ++unit;
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_may_store(ok, status);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll(CHUNKED ? 4 : 1)
@@ -667,7 +667,7 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
         for (int c = 0; c + 1 < n_chunks && ok; ++c) {
             const int buf = c & 1, use = c >> 1;
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_may_store(ok, status);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll
@@ -687,7 +687,7 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
         const int last = n_chunks > 0 ? n_chunks - 1 : 0, lbuf = last & 1;
         if (ok) {
             ok = mbar_wait_bounded(tmem_full + 8 * lbuf, (last >> 1) & 1, status, ST_T_EPILOGUE);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_may_store(ok, status);
         }
         tc_fence_after_sync();
         if (ok && n_steps > 0) {

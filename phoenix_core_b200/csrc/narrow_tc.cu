@@ -173,7 +173,7 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             const int th = r / p.tiles_w, tw = r - th * p.tiles_w;
             const int ow0 = tw * 8, oh0 = th * p.PH;
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_N_EPILOGUE);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_may_store(ok, status);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll 1
@@ -593,7 +593,7 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
     } else {
         const int q = warp & 3, tsel = (warp - 2) >> 2;                // two warps per lane quadrant share the taps
         bool ok = mbar_wait_bounded(tmem_full, 0, status, ST_N_EPILOGUE);
-        ok = __all_sync(0xffffffffu, ok);
+        ok = warp_may_store(ok, status);
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
             const int m = q * 32 + lane;                                // row -> (d, plane, channel within the plane)

@@ -340,7 +340,7 @@ qconv_pointwise8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
 
             // ------------------------------------------------------------ epilogue of the job
             ok = mbar_wait_bounded(tmem_full, job & 1, status, ST_E_WORKER);
-            ok = __all_sync(0xffffffffu, ok);
+            ok = warp_may_store(ok, status);
             if (!ok) break;
             tc_fence_after_sync();
             const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + chalf * 32;

@@ -93,6 +93,12 @@ cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, unsigned bl
     return launch_chained_if(true, kernel, grid, block, smem, stream, args...);
 }
 
+// Whether a warp may store what the barrier it waited for announced: its own wait succeeded in every lane, and no wait of the call has
+// expired -- a completed barrier does not say that the stages in front of it were all filled.
+__device__ __forceinline__ bool warp_may_store(bool ok, const int* status) {
+    return __all_sync(0xffffffffu, ok && *reinterpret_cast<const volatile int*>(status) == 0);
+}
+
 // TMA store of one shared-memory box (written by ordinary stores, then fence_proxy_async) to global memory; elements of
 // the box that fall outside the tensor are not written. Completion is tracked per thread in bulk groups.
 __device__ __forceinline__ void tma_store_4d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2, int c3) {

@@ -1,0 +1,21 @@
+"""What an expired wait must not lead to: a stored tile. Every epilogue asks the status word of the call before it stores, and a loader whose
+wait ran out does not announce its stage. No test can make a wait of these kernels run out (nothing may be taken out of them), so this
+reads the sources."""
+import os
+import re
+
+import pytest
+
+from conftest import ROOT
+
+CSRC = os.path.join(ROOT, "phoenix_core_b200", "csrc")
+KERNELS = ["conv_tc.cu", "conv_tf32.cu", "narrow_tc.cu", "pointwise_tc.cu", "pointwise2_tc.cu"]
+
+
+@pytest.mark.parametrize("name", KERNELS)
+def test_epilogues_read_the_status_word(name):
+    lines = open(os.path.join(CSRC, name)).read().split("\n")
+    waits = [i for i, line in enumerate(lines) if re.search(r"mbar_wait_bounded\(.*_EPILOGUE\)", line) and "epi_bar" not in line and "if (!" not in line]
+    assert waits
+    for i in waits:
+        assert any("warp_may_store(ok, status)" in line for line in lines[i:i + 3]), "%s:%d" % (name, i + 1)
