@@ -9,7 +9,7 @@ import pytest
 from conftest import ROOT
 
 CSRC = os.path.join(ROOT, "phoenix_core_b200", "csrc")
-KERNELS = ["conv_tc.cu", "conv_tf32.cu", "narrow_tc.cu", "pointwise_tc.cu", "pointwise2_tc.cu"]
+KERNELS = ["conv_tc.cu", "conv_tf32.cu", "narrow_tc.cu", "pointwise_tc.cu", "pointwise2_tc.cu", "qgemm_tc.cu"]
 
 
 @pytest.mark.parametrize("name", KERNELS)
@@ -19,3 +19,9 @@ def test_epilogues_read_the_status_word(name):
     assert waits
     for i in waits:
         assert any("warp_may_store(ok, status)" in line for line in lines[i:i + 3]), "%s:%d" % (name, i + 1)
+
+
+def test_a_loader_does_not_announce_an_unfilled_stage():
+    text = open(os.path.join(CSRC, "qgemm_tc.cu")).read()
+    arrivals = re.findall(r"^.*mbar_arrive\(full_bar.*$", text, re.M)
+    assert arrivals and all("if (ok && lane == 0)" in line for line in arrivals)
