@@ -361,8 +361,9 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 const uint16_t raw = ld_chained(bias + d * p.bias_ld + co);
                 badd = p.fmt == 0 ? __half2float(__ushort_as_half(raw)) : __bfloat162float(__ushort_as_bfloat16(raw));
             }
+            const int seen = read_status(status);
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_G_EPILOGUE);
-            ok = warp_may_store(ok, status);
+            ok = warp_may_store(ok, seen);
             if (!ok) break;
             tc_fence_after_sync();
             if (p.plane_mode) {
@@ -1066,8 +1067,9 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
         __syncwarp();
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
+        const int seen = read_status(status);
         bool ok = mbar_wait_bounded(tmem_full, 0, status, ST_G_EPILOGUE);
-        ok = warp_may_store(ok, status);
+        ok = warp_may_store(ok, seen);
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
             // row of the tile -> (output component d, channel co)
@@ -1205,8 +1207,9 @@ qconv_filter_xmajor_tc_kernel(const __grid_constant__ CUtensorMap map_x, const _
         __syncwarp();
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
+        const int seen = read_status(status);
         bool ok = mbar_wait_bounded(tmem_full, 0, status, ST_G_EPILOGUE);
-        ok = warp_may_store(ok, status);
+        ok = warp_may_store(ok, seen);
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
             const int row = q * 32 + lane;                       // row -> (tap, input component l, channel ci)

@@ -179,8 +179,9 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                     for (int e = 0; e < 32; ++e) part[cb][e] = 0.f;
                 for (int c = 0; c + 1 < p.n_chunks && ok; ++c, ++unit) {
                     const int buf = unit & 1, use = unit >> 1;
+                    const int seen = read_status(status);
                     ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
-                    ok = warp_may_store(ok, status);
+                    ok = warp_may_store(ok, seen);
                     if (!ok) break;
                     tc_fence_after_sync();
 #pragma unroll
@@ -200,8 +201,9 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
             }
             const int buf = unit & 1, use = unit >> 1;
             ++unit;
+            const int seen = read_status(status);
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
-            ok = warp_may_store(ok, status);
+            ok = warp_may_store(ok, seen);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll(CHUNKED ? 4 : 1)
@@ -666,8 +668,9 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
         bool ok = true;
         for (int c = 0; c + 1 < n_chunks && ok; ++c) {
             const int buf = c & 1, use = c >> 1;
+            const int seen = read_status(status);
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
-            ok = warp_may_store(ok, status);
+            ok = warp_may_store(ok, seen);
             if (!ok) break;
             tc_fence_after_sync();
 #pragma unroll
@@ -686,8 +689,9 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
         }
         const int last = n_chunks > 0 ? n_chunks - 1 : 0, lbuf = last & 1;
         if (ok) {
+            const int seen = read_status(status);
             ok = mbar_wait_bounded(tmem_full + 8 * lbuf, (last >> 1) & 1, status, ST_T_EPILOGUE);
-            ok = warp_may_store(ok, status);
+            ok = warp_may_store(ok, seen);
         }
         tc_fence_after_sync();
         if (ok && n_steps > 0) {

@@ -339,8 +339,9 @@ qconv_pointwise8_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __gr
             if (!ok) break;
 
             // ------------------------------------------------------------ epilogue of the job
+            const int seen = read_status(status);
             ok = mbar_wait_bounded(tmem_full, job & 1, status, ST_E_WORKER);
-            ok = warp_may_store(ok, status);
+            ok = warp_may_store(ok, seen);
             if (!ok) break;
             tc_fence_after_sync();
             const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + chalf * 32;

@@ -239,6 +239,7 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
     const int n_stages = tile < p.tiles_m * p.tiles_n ? (c_end - c_beg) * 4 : 0;
 
     bool ok = true;
+    const int seen = read_status(status);                              // asked before the first stage, needed behind the last
     if (t < Q_LOADERS) {
         // ------------------------------------------------------------------------------------------ loaders
         // group g fills stages g, g + Q_GROUPS, ...: while one group waits for its loads the others write theirs
@@ -250,7 +251,7 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
             load_tile<F32, AK, QM>(ra, p.a, kc, m0, k0, tg);
 #pragma unroll
             for (int c = 0; c < HALF; ++c) load_tile<F32, BK, NT>(rb[c], p.b, c ^ kc, n0, k0, tg);
-            ok = __all_sync(0xffffffffu, mbar_wait_bounded(empty_bar + 8 * s, (st / L::STAGES + 1) & 1, status, ST_Q_LOADER));
+            ok = mbar_wait_bounded(empty_bar + 8 * s, (st / L::STAGES + 1) & 1, status, ST_Q_LOADER);
             if (ok) {
                 const uint32_t a_tile = tiles + s * L::STAGE, b_tile = a_tile + L::A_TILE * (F32 ? 2 : 1);
                 constexpr uint32_t SIGN = F32 ? 0x80000000u : 0x80008000u;
@@ -268,7 +269,7 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
                 }
                 fence_proxy_async_smem();
             }
-            __syncwarp();
+            ok = __all_sync(0xffffffffu, ok);
             if (ok && lane == 0) mbar_arrive(full_bar + 8 * s);    // (not after an expired wait: the MMA thread's own wait then runs out)
         }
     } else if (lane == 0 && n_stages > 0) {
@@ -311,7 +312,7 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
     const int q = warp & 3, half = warp >> 2;                          // TMEM lane quadrant, half of the columns (warps 0 .. 7)
     if (warp < 8) {
         if (n_stages > 0) ok = mbar_wait_bounded(done_bar, 0, status, ST_Q_EPILOGUE) && ok;
-        ok = warp_may_store(ok, status);
+        ok = warp_may_store(ok, seen);
         tc_fence_after_sync();
         const int row = q * 32 + lane, m = m0 + row;
 #pragma unroll 1

@@ -93,11 +93,11 @@ cudaError_t launch_chained(void (*kernel)(Params...), unsigned grid, unsigned bl
     return launch_chained_if(true, kernel, grid, block, smem, stream, args...);
 }
 
-// Whether a warp may store what the barrier it waited for announced: its own wait succeeded in every lane, and no wait of the call has
-// expired -- a completed barrier does not say that the stages in front of it were all filled.
-__device__ __forceinline__ bool warp_may_store(bool ok, const int* status) {
-    return __all_sync(0xffffffffu, ok && *reinterpret_cast<const volatile int*>(status) == 0);
-}
+// Whether a warp may store what the barrier it waits for announces: its own wait succeeds in every lane, and no wait of the call had
+// expired when the status word was read, which is done in front of the wait to hide the read. (A wait that expires meanwhile leaves the
+// barrier open: whoever gives up no longer signals.)
+__device__ __forceinline__ int read_status(const int* status) { return *reinterpret_cast<const volatile int*>(status); }
+__device__ __forceinline__ bool warp_may_store(bool ok, int status_before) { return __all_sync(0xffffffffu, ok && status_before == 0); }
 
 // TMA store of one shared-memory box (written by ordinary stores, then fence_proxy_async) to global memory; elements of
 // the box that fall outside the tensor are not written. Completion is tracked per thread in bulk groups.
