@@ -198,6 +198,8 @@ int run_pass(Pass pass, int dtype, int variant, int engine, const Geom& g, const
     const bool aligned = ((tensors | reinterpret_cast<uintptr_t>(workspace)) & 15u) == 0;
     if (engine != PCB_ENGINE_SIMT && aligned && tensor_path_supported(pass, dtype, tv, g)) {
         const int rc = tensor_launch(pass, dtype, tv, g, a, b, bias, out, scratch, status, stream, extras, sc);
+        // (a reset behind the kernels would hide what they reported, and they would have waited against an old word)
+        if (rc == PCB_OK && sc && sc->pending) { set_error("status word not reset in front of the kernels"); return PCB_ERR_CUDA; }
         if (rc == PCB_OK && pass == PASS_FWD && forward_keeps_staged_input(dtype, tv, g)) remember_kept(workspace, b, problem_signature(dtype, g));
         return rc;
     }

@@ -705,25 +705,11 @@ bool backward_shares_staged_dy(int dtype, int variant, const Geom& g, StagedView
     return conv_tc_supported(PASS_BWD_DATA, dtype, variant, g) && conv_filter_tc_supported(dtype, variant, g) && conv_tc_staged_dy_view(g, view, bytes);
 }
 
-namespace {
-// Whether tensor_launch goes straight to kernels with a prologue launch (conv_tc.cu, conv_tf32.cu, narrow_tc.cu): the same order of preference.
-bool prologue_route(Pass pass, int dtype, int variant, const Geom& g) {
-    if (!g.plain) return true;
-    if (strided_pointwise(g) && tensor_path_supported(pass, dtype, variant, compact_geom(g))) return false;
-    if (pass == PASS_BWD_DATA && strided_classes_supported(dtype, variant, g)) return false;
-    if (dtype == PCB_F32) return true;
-    if (pointwise_pair_tc_supported(pass, dtype, variant, g) || pointwise_tc_supported(pass, dtype, variant, g)) return false;
-    if (pass == PASS_BWD_FILTER)
-        return !pointwise_filter_tc_supported(dtype, variant, g) && (narrow_filter_tc_supported(dtype, variant, g) || conv_filter_tc_supported(dtype, variant, g));
-    return narrow_tc_supported(pass, dtype, variant, g) || conv_tc_supported(pass, dtype, variant, g);
-}
-}  // namespace
-
 int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* a, const void* b, const void* bias,
                   void* out, float* scratch, int* status, cudaStream_t stream, const PassExtras* extras, StatusClear* sc) {
-    // a prologue launch resets the status word; every other route does it here
-    const bool own_launch = variant == PCB_VARIANT_16_PRODUCT && prologue_route(pass, dtype, variant, g);
-    if (sc && !own_launch) { const int rc = sc->now(stream); if (rc != PCB_OK) return rc; }
+    // launchers that take `sc` reset the status word in their prologue launch; in front of all others it is done here
+    auto settle = [&]() -> int { return sc ? sc->now(stream) : (int)PCB_OK; };
+#define PCB_SETTLED(launch) (settle() != PCB_OK ? (int)PCB_ERR_CUDA : (launch))
     const void* kept_x = extras ? extras->kept_x : nullptr;
     const StagedView* kept_dy = (extras && extras->dy.base) ? &extras->dy : nullptr;
     if (kept_x && !(pass == PASS_BWD_FILTER && forward_keeps_staged_input(dtype, variant, g))) kept_x = nullptr;
@@ -732,12 +718,13 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
         size_t bytes;
         if (!(pass == PASS_BWD_FILTER && backward_shares_staged_dy(dtype, variant, g, &v, &bytes))) kept_dy = nullptr;
     }
-    if (variant == PCB_VARIANT_8_PRODUCT) return pointwise8_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream);
+    if (variant == PCB_VARIANT_8_PRODUCT) return PCB_SETTLED(pointwise8_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream));
     if (!g.plain) {
         if (pass == PASS_BWD_FILTER) return conv_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream, nullptr, nullptr, sc);
         return conv_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream, sc);
     }
     if (strided_pointwise(g) && tensor_path_supported(pass, dtype, variant, compact_geom(g))) {
+        if (settle() != PCB_OK) return PCB_ERR_CUDA;
         const Geom s = compact_geom(g);
         void* compact = scratch;
         float* rest = reinterpret_cast<float*>(reinterpret_cast<char*>(scratch) + compact_bytes(pass, dtype, g));
@@ -752,6 +739,7 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
         return tensor_launch(pass, dtype, variant, s, a, compact, bias, out, rest, status, stream);
     }
     if (pass == PASS_BWD_DATA && strided_classes_supported(dtype, variant, g)) {
+        if (settle() != PCB_OK) return PCB_ERR_CUDA;
         StrideClass cls[4];
         size_t bytes;
         const int n = stride_classes(g, dtype, cls, &bytes);
@@ -792,7 +780,6 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
         PCB_CUDA_TRY(cudaGetLastError());
         return PCB_OK;
     }
-    // the status word is cleared once per API call by the caller of this function; the kernels only OR into it
     if (dtype == PCB_F32) return conv_tf32_launch(pass, g, a, b, bias, out, scratch, status, stream, sc);
     TcParams p;
     p.g = g;
@@ -804,21 +791,22 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
     else                            { p.M = 4 * g.Co; p.N = g.Ci;      p.K = 4 * g.Nb * HW; }
     p.k_per_split = (p.K + TBK - 1) / TBK * TBK;
     p.atomic_out = 0;
-    if (pointwise_pair_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g)) return pointwise_pair_tc_launch(dtype, g, a, b, bias, out, status, stream);
-    if (pointwise_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g)) return pointwise_tc_launch(pass, dtype, g, a, b, bias, out, status, stream);
+    if (pointwise_pair_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g)) return PCB_SETTLED(pointwise_pair_tc_launch(dtype, g, a, b, bias, out, status, stream));
+    if (pointwise_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g)) return PCB_SETTLED(pointwise_tc_launch(pass, dtype, g, a, b, bias, out, status, stream));
     if (pass != PASS_BWD_FILTER && narrow_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g))
         return narrow_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream, sc);
     if (pass != PASS_BWD_FILTER && conv_tc_supported(pass, dtype, PCB_VARIANT_16_PRODUCT, g))
         return conv_tc_launch(pass, dtype, g, a, b, bias, out, scratch, status, stream, sc);
-    if (pass == PASS_FWD) return launch_tc<PASS_FWD>(p, 1, a, b, bias, out, nullptr, status, stream);
-    if (pass == PASS_BWD_DATA) return launch_tc<PASS_BWD_DATA>(p, 1, a, b, bias, out, nullptr, status, stream);
+    if (pass == PASS_FWD) return PCB_SETTLED(launch_tc<PASS_FWD>(p, 1, a, b, bias, out, nullptr, status, stream));
+    if (pass == PASS_BWD_DATA) return PCB_SETTLED(launch_tc<PASS_BWD_DATA>(p, 1, a, b, bias, out, nullptr, status, stream));
 
     // backward-filter: the output is tiny and K is the whole batch of pixels -> split K across the grid,
     // accumulate in fp32 scratch, then cast once.
     if (scratch == nullptr) { set_error("backward-filter needs fp32 scratch"); return PCB_ERR_WORKSPACE; }
-    if (pointwise_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return pointwise_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream);
+    if (pointwise_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return PCB_SETTLED(pointwise_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream));
     if (narrow_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return narrow_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream, kept_x, kept_dy, sc);
     if (conv_filter_tc_supported(dtype, PCB_VARIANT_16_PRODUCT, g)) return conv_filter_tc_launch(dtype, g, a, b, out, scratch, status, stream, kept_x, kept_dy, sc);
+    if (settle() != PCB_OK) return PCB_ERR_CUDA;
     const int tiles = ((p.M + TBM - 1) / TBM) * ((p.N + TBN - 1) / TBN);
     int splits = (2 * sm_count() + tiles - 1) / tiles;
     const int max_splits = (p.K + 4 * TBK - 1) / (4 * TBK);
@@ -838,6 +826,7 @@ int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* 
     else cast_f32_to_16_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(scratch, (__nv_bfloat16*)out, numel);
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
+#undef PCB_SETTLED
 }
 
 }  // namespace pcb
