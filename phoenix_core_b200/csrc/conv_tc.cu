@@ -1519,7 +1519,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     size_t smem = 1024 + (size_t)p.n_stages * p.stage_bytes + 512 + tail_bytes;
     if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
     auto run = [&](auto* kernel) -> int {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
         PCB_CUDA_TRY(launch_chained_if(chain, kernel, grid, G_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
         return PCB_OK;
     };

@@ -1012,10 +1012,10 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     p.chunk_len = (p.k_per_split + p.n_chunks - 1) / p.n_chunks;
     const size_t smem = T_SMEM + (p.rows_epi ? 8 * EPI_ROWS_F32_BYTES : 0);
     if (p.n_chunks > 1) {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
         PCB_CUDA_TRY(launch_chained_if(chain, qconv_general_tf32_kernel<true>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
     } else {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
         PCB_CUDA_TRY(launch_chained_if(chain, qconv_general_tf32_kernel<false>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
     }
     PCB_CUDA_TRY(cudaGetLastError());

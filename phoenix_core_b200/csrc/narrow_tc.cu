@@ -780,7 +780,7 @@ int narrow_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const v
     p.rows_epi = p.store_vec < 8 && pl.smem + N_EPI_WARPS * EPI_ROWS_BYTES <= 227 * 1024;
     size_t smem = pl.smem + (p.rows_epi ? N_EPI_WARPS * EPI_ROWS_BYTES : 0);
     if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
-    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
     PCB_CUDA_TRY(launch_chained_if(chain, qconv_narrow_tc_kernel, grid, NW_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
@@ -976,7 +976,7 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
         if (rc != PCB_OK) return rc;
     }
     const size_t fsmem = f.smem < ONE_CTA_SMEM ? ONE_CTA_SMEM : f.smem;
-    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_filter_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)fsmem));
+    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_filter_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
     PCB_CUDA_TRY(launch_chained_if(chain, qconv_narrow_filter_tc_kernel, grid, N_THREADS, fsmem, stream, map_dy, map_x, p, acc, status));
     PCB_CUDA_TRY(cudaGetLastError());
     const size_t per_tap = (size_t)g.nc * g.Co * g.Ci;

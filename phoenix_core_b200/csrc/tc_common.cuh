@@ -37,6 +37,9 @@ __device__ __forceinline__ void tma_load_5d(uint32_t dst, const CUtensorMap* map
 // kernel the SMs become free one by one, and an SM that could hold two of its CTAs could be given two, the second one waiting for the
 // first one's tensor memory.
 constexpr size_t ONE_CTA_SMEM = 116 * 1024;
+// Dynamic shared memory a CTA may have. Kernels whose need varies from call to call are given this limit whatever the call needs: the
+// limit is state of the function, and another host thread could lower it between a thread's own setting and its launch.
+constexpr int MAX_CTA_SMEM = 227 * 1024;
 __device__ __forceinline__ void chain_next() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 __device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 // Loads of a chained kernel behind chain_wait(): the grid is resident while the kernel in front still writes, so data may not go through the
