@@ -215,10 +215,10 @@ int run_pass(Pass pass, int dtype, int variant, int engine, const Geom& g, const
 // tensor addresses of the call; `apart`: no result shares memory with an operand, which these kernels read while they write (the
 // staged kernels copy their operands first, so a gradient may replace the tensor it belongs to). The workspace must be what the
 // size query asks for, as for every other path.
-bool dense_direct(const pcb_dense_desc* desc, const Geom& g, uintptr_t tensors, bool apart, void* workspace, size_t ws_bytes, size_t need) {
+bool dense_direct(const pcb_dense_desc* desc, const Geom& g, uintptr_t tensors, bool apart, bool backward, void* workspace, size_t ws_bytes, size_t need) {
     const int tv = tensor_variant(variant_for(g, desc->variant), desc->engine);
     return desc->engine != PCB_ENGINE_SIMT && apart && workspace && ws_bytes >= need && ((tensors | reinterpret_cast<uintptr_t>(workspace)) & 15u) == 0 &&
-           dense_tc_supported(desc->dtype, tv, g);
+           dense_tc_supported(desc->dtype, tv, g) && dense_tc_fits(desc->dtype, g, backward, backward && desc->require_input_grad);
 }
 // Bytes of a dense layer's tensors.
 struct DenseBytes { size_t x, y, w; };
@@ -513,7 +513,7 @@ int pcb_qdense_fwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
     const DenseBytes n = dense_bytes(desc->dtype, g);
     const bool apart = !overlaps(y, n.y, x, n.x) && !overlaps(y, n.y, w, n.w);
-    if (dense_direct(desc, g, all, apart, workspace, workspace_bytes_, pcb_qdense_fwd_workspace_size(desc))) {
+    if (dense_direct(desc, g, all, apart, false, workspace, workspace_bytes_, pcb_qdense_fwd_workspace_size(desc))) {
         forget_kept(workspace);
         return dense_tc_fwd(desc->dtype, g, x, w, bias, y, static_cast<int*>(workspace), (cudaStream_t)stream);
     }
@@ -539,7 +539,7 @@ int pcb_qdense_bwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     const DenseBytes n = dense_bytes(desc->dtype, g);
     auto free_of_operands = [&](const void* out, size_t bytes) { return !overlaps(out, bytes, x, n.x) && !overlaps(out, bytes, w, n.w) && !overlaps(out, bytes, dy, n.y); };
     const bool apart = free_of_operands(dw, n.w) && free_of_operands(gx, n.x) && !overlaps(dw, n.w, gx, n.x);
-    if (dense_direct(desc, g, all, apart, workspace, workspace_bytes_, pcb_qdense_bwd_workspace_size(desc))) {
+    if (dense_direct(desc, g, all, apart, true, workspace, workspace_bytes_, pcb_qdense_bwd_workspace_size(desc))) {
         forget_kept(workspace);
         return dense_tc_bwd(desc->dtype, g, x, w, dy, dw, gx, static_cast<int*>(workspace), (cudaStream_t)stream);
     }

@@ -527,50 +527,72 @@ bool dense_tc_supported(int dtype, int variant, const Geom& g) {
     return true;
 }
 
-int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream) {
-    const int f32 = dtype == PCB_F32;
+namespace {
+// What a call launches; blocks == 0: no cut of the reduced dimensions fits the machine.
+struct DensePlan {
     QParams p;
-    p.fmt = f32 ? 2 : (dtype == PCB_F16 ? 0 : 1);
-    p.prob[0] = dense_problem(PASS_FWD, g, x, w, nullptr, bias, y, 32, f32);
-    const bool wide = !f32 && q_tiles(p.prob[0]) > sm_count();
-    if (wide) p.prob[0] = dense_problem(PASS_FWD, g, x, w, nullptr, bias, y, 64, f32);
-    p.prob[1] = p.prob[0];
-    const int blocks = q_plan(p, false, f32);
-    if (blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
-    if (f32) return g.w_io ? q_launch<true, 32, false, true, false, false, false>(p, blocks, status, stream)
-                           : q_launch<true, 32, true, true, false, false, false>(p, blocks, status, stream);
-    if (wide) return g.w_io ? q_launch<false, 64, false, true, false, false, false>(p, blocks, status, stream)
-                            : q_launch<false, 64, true, true, false, false, false>(p, blocks, status, stream);
-    return g.w_io ? q_launch<false, 32, false, true, false, false, false>(p, blocks, status, stream)
-                  : q_launch<false, 32, true, true, false, false, false>(p, blocks, status, stream);
+    int blocks, wide;
+};
+DensePlan plan_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y) {
+    const int f32 = dtype == PCB_F32;
+    DensePlan d;
+    d.p.fmt = f32 ? 2 : (dtype == PCB_F16 ? 0 : 1);
+    d.p.prob[0] = dense_problem(PASS_FWD, g, x, w, nullptr, bias, y, 32, f32);
+    d.wide = !f32 && q_tiles(d.p.prob[0]) > sm_count();
+    if (d.wide) d.p.prob[0] = dense_problem(PASS_FWD, g, x, w, nullptr, bias, y, 64, f32);
+    d.p.prob[1] = d.p.prob[0];
+    d.blocks = q_plan(d.p, false, f32);
+    return d;
+}
+DensePlan plan_bwd(int dtype, const Geom& g, const void* x, const void* w, const void* dy, void* dw, void* dx, bool both) {
+    const int f32 = dtype == PCB_F32;
+    DensePlan d;
+    d.p.fmt = f32 ? 2 : (dtype == PCB_F16 ? 0 : 1);
+    auto build = [&](int NT) {
+        d.p.prob[0] = dense_problem(PASS_BWD_FILTER, g, x, w, dy, nullptr, dw, NT, f32);
+        d.p.prob[1] = both ? dense_problem(PASS_BWD_DATA, g, x, w, dy, nullptr, dx, NT, f32) : d.p.prob[0];
+        return q_tiles(d.p.prob[0]) + (both ? q_tiles(d.p.prob[1]) : 0);
+    };
+    d.wide = !f32 && build(32) > sm_count();
+    build(d.wide ? 64 : 32);
+    d.blocks = q_plan(d.p, both, f32);
+    return d;
+}
+// These grids are not persistent: with an SM margin they are taken only where all their CTAs fit beside it at once.
+bool plan_fits(const DensePlan& d) { return d.blocks > 0 && (g_sm_margin == 0 || d.blocks <= sm_count()); }
+}  // namespace
+
+bool dense_tc_fits(int dtype, const Geom& g, bool backward, bool need_dx) {
+    return plan_fits(backward ? plan_bwd(dtype, g, nullptr, nullptr, nullptr, nullptr, nullptr, need_dx) : plan_fwd(dtype, g, nullptr, nullptr, nullptr, nullptr));
+}
+
+int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream) {
+    const DensePlan d = plan_fwd(dtype, g, x, w, bias, y);
+    if (d.blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
+    if (d.p.fmt == 2) return g.w_io ? q_launch<true, 32, false, true, false, false, false>(d.p, d.blocks, status, stream)
+                                    : q_launch<true, 32, true, true, false, false, false>(d.p, d.blocks, status, stream);
+    if (d.wide) return g.w_io ? q_launch<false, 64, false, true, false, false, false>(d.p, d.blocks, status, stream)
+                              : q_launch<false, 64, true, true, false, false, false>(d.p, d.blocks, status, stream);
+    return g.w_io ? q_launch<false, 32, false, true, false, false, false>(d.p, d.blocks, status, stream)
+                  : q_launch<false, 32, true, true, false, false, false>(d.p, d.blocks, status, stream);
 }
 
 // dw, and dx unless it is null, in one launch.
 int dense_tc_bwd(int dtype, const Geom& g, const void* x, const void* w, const void* dy, void* dw, void* dx, int* status, cudaStream_t stream) {
-    const int f32 = dtype == PCB_F32;
-    QParams p;
-    p.fmt = f32 ? 2 : (dtype == PCB_F16 ? 0 : 1);
-    auto build = [&](int NT) {
-        p.prob[0] = dense_problem(PASS_BWD_FILTER, g, x, w, dy, nullptr, dw, NT, f32);
-        p.prob[1] = dx ? dense_problem(PASS_BWD_DATA, g, x, w, dy, nullptr, dx, NT, f32) : p.prob[0];
-        return q_tiles(p.prob[0]) + (dx ? q_tiles(p.prob[1]) : 0);
-    };
-    int tiles = build(32);
-    const bool wide = !f32 && tiles > sm_count();
-    if (wide) tiles = build(64);
-    const int blocks = q_plan(p, dx != nullptr, f32);
-    if (blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
+    const DensePlan d = plan_bwd(dtype, g, x, w, dy, dw, dx, dx != nullptr);
+    if (d.blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
+    const bool f32 = d.p.fmt == 2;
     if (!dx) {
-        if (f32) return q_launch<true, 32, false, false, false, false, false>(p, blocks, status, stream);
-        return wide ? q_launch<false, 64, false, false, false, false, false>(p, blocks, status, stream)
-                    : q_launch<false, 32, false, false, false, false, false>(p, blocks, status, stream);
+        if (f32) return q_launch<true, 32, false, false, false, false, false>(d.p, d.blocks, status, stream);
+        return d.wide ? q_launch<false, 64, false, false, false, false, false>(d.p, d.blocks, status, stream)
+                      : q_launch<false, 32, false, false, false, false, false>(d.p, d.blocks, status, stream);
     }
-    if (f32) return g.w_io ? q_launch<true, 32, false, false, true, true, true>(p, blocks, status, stream)
-                           : q_launch<true, 32, false, false, true, false, true>(p, blocks, status, stream);
-    if (wide) return g.w_io ? q_launch<false, 64, false, false, true, true, true>(p, blocks, status, stream)
-                            : q_launch<false, 64, false, false, true, false, true>(p, blocks, status, stream);
-    return g.w_io ? q_launch<false, 32, false, false, true, true, true>(p, blocks, status, stream)
-                  : q_launch<false, 32, false, false, true, false, true>(p, blocks, status, stream);
+    if (f32) return g.w_io ? q_launch<true, 32, false, false, true, true, true>(d.p, d.blocks, status, stream)
+                           : q_launch<true, 32, false, false, true, false, true>(d.p, d.blocks, status, stream);
+    if (d.wide) return g.w_io ? q_launch<false, 64, false, false, true, true, true>(d.p, d.blocks, status, stream)
+                              : q_launch<false, 64, false, false, true, false, true>(d.p, d.blocks, status, stream);
+    return g.w_io ? q_launch<false, 32, false, false, true, true, true>(d.p, d.blocks, status, stream)
+                  : q_launch<false, 32, false, false, true, false, true>(d.p, d.blocks, status, stream);
 }
 
 }  // namespace pcb
