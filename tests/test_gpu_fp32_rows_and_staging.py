@@ -38,3 +38,20 @@ def test_fp32_tile_edges(gpu, oracle, shape):
     for got, want, what in ((y, ref, "y"), (dx, rdx, "dx"), (dw, rdw, "dw")):
         assert np.all(np.isfinite(got)), what
         assert rel_err(got, want) <= 1e-5, (what, rel_err(got, want))
+
+
+# planes of 1 to 15 pixels: staged thread by thread beside the filters, 1 to 40 channels in blocks of 16 and 32, several images
+@pytest.mark.parametrize("shape", [(5, 33, 17, 1, 1, 1, 0), (3, 6, 40, 3, 5, 3, 1), (7, 1, 3, 2, 2, 2, 0), (2, 64, 31, 1, 15, 3, 1), (130, 20, 24, 3, 3, 3, 1)])
+def test_fp32_tiny_planes(gpu, oracle, shape):
+    n, ci, co, h, w, k, p = shape
+    pad = (p, p, p, p)
+    x = uniform(95, (4 * n, ci, h, w))
+    f = normal(96, (4, co, ci, k, k), std=(2.0 / (4 * ci * k * k)) ** 0.5)
+    ref = oracle.conv2d_fwd(x, f, None, (1, 1), (1, 1), pad)
+    y = gpu.run_conv_fwd(x, f, None, (1, 1), pad, "f32", "16p", "tensor")
+    dy = normal(98, ref.shape)
+    rdw, rdx = oracle.conv2d_bwd(x, f, dy, (1, 1), (1, 1), pad)
+    dw, dx = gpu.run_conv_bwd(x, f, dy, (1, 1), pad, "f32", "16p", "tensor", True)
+    for got, want, what in ((y, ref, "y"), (dx, rdx, "dx"), (dw, rdw, "dw")):
+        assert np.all(np.isfinite(got)), what
+        assert rel_err(got, want) <= 1e-5, (what, rel_err(got, want))
