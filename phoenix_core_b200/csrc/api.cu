@@ -211,14 +211,15 @@ int run_pass(Pass pass, int dtype, int variant, int engine, const Geom& g, const
     return simt_launch(pass, dtype, variant, g, a, b, bias, out, scratch, stream);
 }
 
-// Whether a dense call runs on the kernels that take the caller's tensors as they are (qgemm_tc.cu). `tensors`: the OR of all
+// How far a dense call runs on the kernels that take the caller's tensors as they are (qgemm_tc.cu). `tensors`: the OR of all
 // tensor addresses of the call; `apart`: no result shares memory with an operand, which these kernels read while they write (the
 // staged kernels copy their operands first, so a gradient may replace the tensor it belongs to). The workspace must be what the
 // size query asks for, as for every other path.
-bool dense_direct(const pcb_dense_desc* desc, const Geom& g, uintptr_t tensors, bool apart, bool backward, void* workspace, size_t ws_bytes, size_t need) {
+DenseRoute dense_route(const pcb_dense_desc* desc, const Geom& g, uintptr_t tensors, bool apart, bool backward, void* workspace, size_t ws_bytes, size_t need) {
     const int tv = tensor_variant(variant_for(g, desc->variant), desc->engine);
-    return desc->engine != PCB_ENGINE_SIMT && apart && workspace && ws_bytes >= need && ((tensors | reinterpret_cast<uintptr_t>(workspace)) & 15u) == 0 &&
-           dense_tc_supported(desc->dtype, tv, g) && dense_tc_fits(desc->dtype, g, backward, backward && desc->require_input_grad);
+    const bool direct = desc->engine != PCB_ENGINE_SIMT && apart && workspace && ws_bytes >= need &&
+                        ((tensors | reinterpret_cast<uintptr_t>(workspace)) & 15u) == 0 && dense_tc_supported(desc->dtype, tv, g);
+    return direct ? dense_tc_route(desc->dtype, g, backward, backward && desc->require_input_grad) : DENSE_STAGED;
 }
 // Bytes of a dense layer's tensors.
 struct DenseBytes { size_t x, y, w; };
@@ -513,7 +514,7 @@ int pcb_qdense_fwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
     const DenseBytes n = dense_bytes(desc->dtype, g);
     const bool apart = !overlaps(y, n.y, x, n.x) && !overlaps(y, n.y, w, n.w);
-    if (dense_direct(desc, g, all, apart, false, workspace, workspace_bytes_, pcb_qdense_fwd_workspace_size(desc))) {
+    if (dense_route(desc, g, all, apart, false, workspace, workspace_bytes_, pcb_qdense_fwd_workspace_size(desc)) == DENSE_DIRECT) {
         forget_kept(workspace);
         return dense_tc_fwd(desc->dtype, g, x, w, bias, y, static_cast<int*>(workspace), (cudaStream_t)stream);
     }
@@ -539,12 +540,14 @@ int pcb_qdense_bwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     const DenseBytes n = dense_bytes(desc->dtype, g);
     auto free_of_operands = [&](const void* out, size_t bytes) { return !overlaps(out, bytes, x, n.x) && !overlaps(out, bytes, w, n.w) && !overlaps(out, bytes, dy, n.y); };
     const bool apart = free_of_operands(dw, n.w) && free_of_operands(gx, n.x) && !overlaps(dw, n.w, gx, n.x);
-    if (dense_direct(desc, g, all, apart, true, workspace, workspace_bytes_, pcb_qdense_bwd_workspace_size(desc))) {
+    const DenseRoute route = dense_route(desc, g, all, apart, true, workspace, workspace_bytes_, pcb_qdense_bwd_workspace_size(desc));
+    if (route != DENSE_STAGED) {
         forget_kept(workspace);
-        return dense_tc_bwd(desc->dtype, g, x, w, dy, dw, gx, static_cast<int*>(workspace), (cudaStream_t)stream);
+        rc = dense_tc_bwd(desc->dtype, g, x, w, dy, dw, route == DENSE_DIRECT ? gx : nullptr, static_cast<int*>(workspace), (cudaStream_t)stream);
+    } else {
+        rc = run_pass(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g, dy, x, nullptr, dw, workspace, workspace_bytes_, (cudaStream_t)stream);
     }
-    rc = run_pass(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g, dy, x, nullptr, dw, workspace, workspace_bytes_, (cudaStream_t)stream);
-    if (rc != PCB_OK) return rc;
+    if (rc != PCB_OK || route == DENSE_DIRECT) return rc;
     if (desc->require_input_grad)
         rc = run_pass(PASS_BWD_DATA, desc->dtype, variant_for(g, desc->variant), desc->engine, g, w, dy, nullptr, dx, workspace, workspace_bytes_, (cudaStream_t)stream);
     return rc;

@@ -562,8 +562,51 @@ DensePlan plan_bwd(int dtype, const Geom& g, const void* x, const void* w, const
 bool plan_fits(const DensePlan& d) { return d.blocks > 0 && (g_sm_margin == 0 || d.blocks <= sm_count()); }
 }  // namespace
 
-bool dense_tc_fits(int dtype, const Geom& g, bool backward, bool need_dx) {
-    return plan_fits(backward ? plan_bwd(dtype, g, nullptr, nullptr, nullptr, nullptr, nullptr, need_dx) : plan_fwd(dtype, g, nullptr, nullptr, nullptr, nullptr));
+// Where the staged kernels are the faster ones. They pay once for the copies and for the expanded filter matrix (16 products of I x O,
+// whatever the batch) and then read their operands by TMA; here every tile loads, splits (fp32) or shifts (odd rows) its operands
+// again. So they win for large batches of wide layers, earlier in fp32 and for rows that are not a whole number of load units, and
+// for the filter gradient, whose reduction is the batch, where its few tiles leave it on as many CTAs. Batch x I x O, this kernel / staged,
+// us:
+//   forward        fp16  4096 x 2048 x 2048   641 /  772    8192 x 1536 x 1024   629 /  577    16384 x 512 x 512   219 /  261
+//                  fp16  1024 x  511 x  333    42 /   48    4096 x  511 x  333   112 /   82     2048 x 1001 x 999   216 /  139
+//                  fp32  1536 x 2048 x  512   398 /  449    2048 x 2048 x  512   543 /  521     1536 x 611 x 703   242 /  207
+//   both gradients fp16  2048 x 2048 x 2048   657 /  959    4096 x 3072 x  768   981 /  927    16384 x 511 x 333   766 /  692
+//                  fp32  1024 x 1024 x 1024   472 /  515    1536 x  768 x  768   478 /  397     2048 x 1024 x 1024 1029 /  845
+//   dw alone       fp16  8192 x 2048 x 2048  1421 / 1496   16384 x  768 x  768   589 /  552     8192 x 511 x 333   327 /  260
+//                  fp32  1024 x  256 x  256    38 /   56    1280 x  512 x  512   108 /   77     2048 x 1024 x 1024  526 /  370
+// Both gradients of a large 16-bit layer are faster apart, dw here and dx staged: 4096 x 2048 x 1024 866 -> 710, 8192 x 1024 x 1024
+// 926 -> 640 (both staged: 780).
+DenseRoute preferred_route(int dtype, const Geom& g, bool backward, bool need_dx) {
+    const long long B = g.Nb, I = g.Ci, O = g.Co, IO = I * O, P = B * IO;
+    if (dtype == PCB_F32) {
+        bool staged;                               // (rows of O alone that are not a whole number of 16-byte units: 1000 x 768 x 1001 forward 217 / 250)
+        if (backward && !need_dx) staged = (B >= 1280 && P >= 180000000) || (B >= 768 && P >= 400000000);
+        else if (I % 4 != 0 && (!backward || O % 4 != 0)) staged = P >= 500000000;
+        else if (backward) staged = (B >= 1280 && P >= 720000000) || P >= 2000000000;
+        else staged = B >= 1792 && I >= 2 * O && P >= 1500000000;
+        return staged ? DENSE_STAGED : DENSE_DIRECT;
+    }
+    if (I % 2 != 0 || O % 2 != 0) {
+        const bool both = I % 2 != 0 && O % 2 != 0, wide = IO >= 1 << 17;
+        bool staged;
+        if (backward && !need_dx) staged = (B >= 4096 && wide) || (B >= 65536 && IO >= 1 << 15);
+        else if (backward) staged = (B >= 8192 && wide && (both || P >= 3000000000)) || (IO >= 500000 && B >= (both ? 2048 : 4096));
+        else staged = (B >= 4096 && wide) || (B >= 1024 && I % 2 != 0 && IO >= 900000);
+        return staged ? DENSE_STAGED : DENSE_DIRECT;
+    }
+    if (IO < 1 << 19) return DENSE_DIRECT;
+    if (!backward) return B >= 6144 && P >= 6000000000 ? DENSE_STAGED : DENSE_DIRECT;
+    // (dw of up to one tile per SM at a long reduction: 128 CTAs with a thousand stages each)
+    if (B >= 16384 && IO <= 148ll * 128 * 32) return DENSE_STAGED;
+    return need_dx && (B >= 6144 || (B >= 3072 && I >= 2 * O)) ? DENSE_FILTER_DIRECT : DENSE_DIRECT;
+}
+
+DenseRoute dense_tc_route(int dtype, const Geom& g, bool backward, bool need_dx) {
+    const DenseRoute route = preferred_route(dtype, g, backward, need_dx);
+    if (route == DENSE_STAGED) return route;
+    const bool both = need_dx && route == DENSE_DIRECT;
+    const bool fits = plan_fits(backward ? plan_bwd(dtype, g, nullptr, nullptr, nullptr, nullptr, nullptr, both) : plan_fwd(dtype, g, nullptr, nullptr, nullptr, nullptr));
+    return fits ? route : DENSE_STAGED;
 }
 
 int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream) {

@@ -58,3 +58,40 @@ def test_sm_margin(lib, dtype, backward, batch, ci, co, fits):
     assert staged == (not fits)
     for a, b in zip(got, want):
         assert ((a.double() - b.double()).abs().max() / b.double().abs().max()).item() <= TYPES[dtype][2]
+
+
+# sizes on both sides of the lines between the two kernel families: dtype, batch, ci, co, and whether (y, dw and dx, dw alone) are staged
+@pytest.mark.parametrize("dtype,batch,ci,co,staged", [
+    ("f16", 1024, 511, 333, (False, False, False)), ("f16", 4096, 511, 333, (True, False, True)), ("f16", 2048, 1001, 999, (True, True, False)),
+    ("f16", 4096, 1024, 511, (True, True, True)), ("f16", 8192, 768, 1024, (True, True, False)), ("f16", 4096, 2048, 1024, (False, True, False)),
+    ("f16", 16384, 512, 1024, (True, True, True)), ("f16", 16384, 256, 256, (False, False, False)),
+    ("f32", 1024, 512, 512, (False, False, False)), ("f32", 1536, 768, 768, (False, True, True)), ("f32", 1024, 611, 900, (True, False, True)), ("f32", 1024, 768, 701, (False, False, True)),
+    ("f32", 768, 512, 512, (False, False, False)), ("f32", 2048, 2048, 512, (True, True, True))])
+def test_large_layers(lib, dtype, batch, ci, co, staged):
+    t, tol = TYPES[dtype][1:]
+    gen = torch.Generator(device="cuda").manual_seed(3)                      # the tensors that _run makes
+    x, w, dy = ((torch.randn(shape, generator=gen, device="cuda") * std).to(t)
+                for shape, std in (((4 * batch, ci), 1.0), ((4, ci, co), (1.0 / (4 * ci)) ** 0.5), ((4 * batch, co), 1.0)))
+    # y = x (Hamilton product) w: component l of x times component l ^ d of w goes into component d of y, with these negative
+    negative = {(1, 0), (1, 2), (2, 0), (2, 3), (3, 0), (3, 1)}
+    block = torch.cat([torch.cat([(-1.0 if (l, d) in negative else 1.0) * w[l ^ d].double() for d in range(4)], dim=1) for l in range(4)], dim=0)
+
+    def join(v):
+        return v.view(4, batch, -1).transpose(0, 1).reshape(batch, -1).double()
+
+    def split(v, c):
+        return v.view(batch, 4, c).transpose(0, 1).reshape(4 * batch, c)
+
+    want_y = split(join(x) @ block, co)
+    want_dx = split(join(dy) @ block.t(), ci)
+    g = join(x).t() @ join(dy)
+    want_dw = torch.zeros(4, ci, co, dtype=torch.float64, device="cuda")
+    for l in range(4):
+        for d in range(4):
+            want_dw[l ^ d] += (-1.0 if (l, d) in negative else 1.0) * g[l * ci:(l + 1) * ci, d * co:(d + 1) * co]
+    calls = ((False, True, (want_y,)), (True, True, (want_dw, want_dx)), (True, False, (want_dw,)))
+    for (backward, need_dx, want), expected in zip(calls, staged):
+        got, was_staged = _run(lib, dtype, batch, ci, co, backward, need_dx)
+        assert was_staged == expected, (backward, need_dx)
+        for a, b in zip(got, want):
+            assert ((a.double() - b).abs().max() / b.abs().max()).item() <= tol
