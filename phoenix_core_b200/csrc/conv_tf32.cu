@@ -494,6 +494,9 @@ struct Prologue32 {
     unsigned zero_units = 0, filter_blocks = 0, stage_blocks[2] = {0, 0}, zero_blocks = 0;
     int n_stages = 0;
 };
+__device__ __forceinline__ void zero_f32(const Prologue32& p, unsigned block) {
+    for (unsigned i = block * STAGE_THREADS + threadIdx.x; i < p.zero_units; i += p.zero_blocks * STAGE_THREADS) p.zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+}
 __global__ void __launch_bounds__(STAGE_THREADS) prologue_f32_kernel(const __grid_constant__ Prologue32 p) {
     __shared__ float4 tile[STAGE_UNITS];
     unsigned block = blockIdx.x;
@@ -502,10 +505,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) prologue_f32_kernel(const __gri
     if (block == 0 && threadIdx.x == 0 && p.status) *p.status = 0;
     if (block < p.filter_blocks) { pack_filters_f32(p.filter, block, p.filter_blocks); return; }
     block -= p.filter_blocks;
-    if (block < p.zero_blocks) {
-        for (unsigned i = block * STAGE_THREADS + threadIdx.x; i < p.zero_units; i += p.zero_blocks * STAGE_THREADS) p.zero[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-        return;
-    }
+    if (block < p.zero_blocks) { zero_f32(p, block); return; }
     block -= p.zero_blocks;
     const bool second = block >= p.stage_blocks[0];
     const StageJob32& job = second ? p.stage[1] : p.stage[0];
@@ -513,6 +513,15 @@ __global__ void __launch_bounds__(STAGE_THREADS) prologue_f32_kernel(const __gri
     if (job.V == 0) stage_tiny_f32(job, block);
     else if (job.U == 8) stage_compact_f32<8>(job, block, tile);
     else stage_compact_f32<4>(job, block, tile);
+}
+// Without the copies: fewer registers and no shared memory, eight CTAs per SM instead of five.
+__global__ void __launch_bounds__(STAGE_THREADS) filter_prologue_f32_kernel(const __grid_constant__ Prologue32 p) {
+    const unsigned block = blockIdx.x;
+    chain_wait();
+    chain_next();
+    if (block == 0 && threadIdx.x == 0 && p.status) *p.status = 0;
+    if (block < p.filter_blocks) pack_filters_f32(p.filter, block, p.filter_blocks);
+    else zero_f32(p, block - p.filter_blocks);
 }
 // 16-byte aligned, a multiple of 16 bytes; false otherwise (the caller clears it).
 bool add_zero_job(Prologue32& pro, void* p, size_t bytes) {
@@ -524,10 +533,24 @@ bool add_zero_job(Prologue32& pro, void* p, size_t bytes) {
 }
 // `chain`: whether the main kernel may be chained to this launch.
 int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream, bool* chain) {
-    const unsigned blocks = pro.filter_blocks + pro.zero_blocks + pro.stage_blocks[0] + pro.stage_blocks[1];
+    unsigned blocks = pro.filter_blocks + pro.zero_blocks + pro.stage_blocks[0] + pro.stage_blocks[1];
     *chain = chain_behind(blocks, 8);
     if (blocks == 0) return PCB_OK;
     if (sc && sc->pending) { pro.status = sc->word; sc->pending = false; }
+    // A large filter matrix that is gathered across its storage order (backward-data of OIHW filters, forward of input-major ones), one
+    // sector per element, is bound by the loads in flight, and by rows that lie side by side being packed at the same time, when they share
+    // what they fetch. It is packed by a launch of its own, which is not chained: CTAs that start on a few SMs beside the tail of the kernel
+    // in front fall out of step with the rest. Backward-data, one chained launch / this: 7 x 7, batch 4, 512 channels (302 MB)
+    // 551 / 306 us; 14 x 14, batch 4, 256 channels (75 MB) 180 / 154; batch 8, 128 channels (19 MB) 68 / 72; dense 1024 x 2048 x 2048
+    // forward (537 MB) 1206 / 1036.
+    const FilterJob32& f = pro.filter;
+    if (pro.filter_blocks > 0 && f.transposed != f.w_io && (size_t)f.taps * f.Mp * f.Kp * 8 > (size_t)64 << 20) {
+        PCB_CUDA_TRY(launch_chained_if(false, filter_prologue_f32_kernel, pro.filter_blocks + pro.zero_blocks, STAGE_THREADS, 0, stream, pro));
+        blocks -= pro.filter_blocks + pro.zero_blocks;
+        if (blocks == 0) return PCB_OK;
+        pro.status = nullptr;
+        pro.filter_blocks = pro.zero_blocks = 0;
+    }
     PCB_CUDA_TRY(launch_chained(prologue_f32_kernel, blocks, STAGE_THREADS, 0, stream, pro));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;

@@ -55,3 +55,18 @@ def test_fp32_tiny_planes(gpu, oracle, shape):
     for got, want, what in ((y, ref, "y"), (dx, rdx, "dx"), (dw, rdw, "dw")):
         assert np.all(np.isfinite(got)), what
         assert rel_err(got, want) <= 1e-5, (what, rel_err(got, want))
+
+
+# filter matrices of more than 64 MB, gathered across their storage order by a launch of their own: backward-data of a wide 3x3 layer on
+# planes of 16 and more and of fewer pixels, with and without a cut reduction
+@pytest.mark.parametrize("n,c,h,w", [(1, 256, 5, 6), (3, 264, 3, 4)])
+def test_fp32_large_filter_matrix(gpu, oracle, n, c, h, w):
+    pad = (1, 1, 1, 1)
+    x = uniform(95, (4 * n, c, h, w))
+    f = normal(96, (4, c, c, 3, 3), std=(2.0 / (36 * c)) ** 0.5)
+    dy = normal(98, (4 * n, c, h, w))
+    rdw, rdx = oracle.conv2d_bwd(x, f, dy, (1, 1), (1, 1), pad)
+    dw, dx = gpu.run_conv_bwd(x, f, dy, (1, 1), pad, "f32", "16p", "tensor", True)
+    for got, want, what in ((dx, rdx, "dx"), (dw, rdw, "dw")):
+        assert np.all(np.isfinite(got)), what
+        assert rel_err(got, want) <= 1e-5, (what, rel_err(got, want))
