@@ -896,7 +896,10 @@ int launch_prologue(Prologue& pro, StatusClear* sc, cudaStream_t stream, bool* c
     size_t smem = pro.n_stages ? STAGE_UNITS * sizeof(uint4) : 0;
     const size_t tile = pro.filter_blocks && f.tiled ? (size_t)(f.transposed ? PACK_TK * (PACK_TM * f.taps + 2) : PACK_TM * (PACK_TK * f.taps + 2)) * 2 : 0;
     if (tile > smem) smem = tile;
-    PCB_CUDA_TRY(launch_chained(prologue_kernel, blocks, STAGE_THREADS, smem, stream, pro));
+    // Not chained where a large filter matrix is gathered element by element (conv_tf32.cu): 14 x 14, batch 16, 256 channels, 5 x 5, fp16,
+    // backward-data 333 us chained, 285 not; channels-last 7 x 7, 512 channels, 3 x 3 278 / 258; 256 channels, 3 x 3 (19 MB) 98.5 / 98.5.
+    const bool gathers = pro.filter_blocks && !f.tiled && (f.transposed ? f.fs.o : f.fs.i) != 1 && (size_t)f.taps * f.Mp * f.Kp * 2 > (size_t)32 << 20;
+    PCB_CUDA_TRY(launch_chained_if(!gathers, prologue_kernel, blocks, STAGE_THREADS, smem, stream, pro));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
