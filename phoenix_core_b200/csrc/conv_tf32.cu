@@ -368,12 +368,15 @@ __global__ void pack_activations_f32_small_kernel(const float* __restrict__ x, f
 // ---- everything a call needs before its main kernel, in one launch (as in conv_tc.cu): status word, filters, copies, zeroed output ----
 // Staging of dense NCHW tensors without padding, x[plane][C][HW] -> hi, lo [plane][HW][Cp] (blocked == 0) or blocks of 4 U channels
 // with the block index outermost: the transposition of conv_tc.cu's stage_compact with units of four channels, split into hi and lo
-// where the units leave shared memory.
+// where the units leave shared memory. Blocks of 64 channels wherever there are more than 32 (the last one may hold fewer): a CTA writes
+// 256 bytes per pixel. 112 channels of 67 x 67, batch 125, 2 x 1 taps, forward 691 us, with blocks of 16 channels 811; 48 channels of
+// 56 x 56, batch 32, 1 x 1, 99 / 120.
 struct StageJob32 {
     const float* x;
     float *hi, *lo;
     unsigned total_px, HW, Nb;
     int C, nblk, U, V, blocked;
+    unsigned units;                   // units of a pixel (all blocks)
     unsigned bx, blocks;
 };
 template <int V, int U>
@@ -403,10 +406,10 @@ __device__ __forceinline__ void stage_compact_f32(const StageJob32& p, unsigned 
     for (int it = 0; it < STAGE_UNITS / STAGE_THREADS; ++it) {
         const int i = threadIdx.x + it * STAGE_THREADS, px = i / U, g = i % U;
         const unsigned P = px0 + px;
-        if (P >= p.total_px) continue;
+        if (P >= p.total_px || by * U + g >= p.units) continue;
         size_t unit;
         if (p.blocked) unit = ((size_t)P + (size_t)((P / HW / p.Nb) * (unsigned)(p.nblk - 1) + by) * p.Nb * HW) * U + g;
-        else unit = ((size_t)P * p.nblk + by) * U + g;
+        else unit = (size_t)P * p.units + by * U + g;
         const float4 f = tile[stage_unit<V, U>(px, g)];
         float4 h, lo;
         split_tf32(f.x, h.x, lo.x); split_tf32(f.y, h.y, lo.y); split_tf32(f.z, h.z, lo.z); split_tf32(f.w, h.w, lo.w);
@@ -423,7 +426,7 @@ __device__ __forceinline__ void stage_compact_f32(const StageJob32& p, unsigned 
 // The same copy for planes of fewer than 16 pixels (dense layers are 1 x 1 images), where consecutive pixels of a channel are few: one
 // thread per pixel and 4 channels, consecutive threads along the pixels of a plane and then its channel groups.
 __device__ __forceinline__ void stage_tiny_f32(const StageJob32& p, unsigned block) {
-    const unsigned groups = p.nblk * p.U, HW = p.HW;
+    const unsigned groups = p.units, HW = p.HW;
     const size_t total = (size_t)p.total_px * groups;
     for (size_t i = (size_t)block * STAGE_THREADS + threadIdx.x; i < total; i += (size_t)p.blocks * STAGE_THREADS) {
         const unsigned px = (unsigned)(i % HW), grp = (unsigned)(i / HW % groups), plane = (unsigned)(i / HW / groups);
@@ -511,6 +514,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) prologue_f32_kernel(const __gri
     const StageJob32& job = second ? p.stage[1] : p.stage[0];
     if (second) block -= p.stage_blocks[0];
     if (job.V == 0) stage_tiny_f32(job, block);
+    else if (job.U == 16) stage_compact_f32<16>(job, block, tile);
     else if (job.U == 8) stage_compact_f32<8>(job, block, tile);
     else stage_compact_f32<4>(job, block, tile);
 }
@@ -562,11 +566,11 @@ int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream, bool*
 void stage_activations_f32(Prologue32& pro, const float* x, float* hi, float* lo, int planes, int C, int H, int W, int Hp, int Wp, int Cp, int pad_top,
                            int pad_left, int ins_h, int ins_w, int cb, int Nb, cudaStream_t stream) {
     if (Hp == H && Wp == W && pad_top == 0 && pad_left == 0 && ins_h == 1 && ins_w == 1) {
-        const int block = Cp % 32 == 0 ? 32 : 16;                  // (cb is 0 or 32, and then Cp a multiple of 32)
+        const int block = cb > 0 ? cb : (Cp > 32 ? 64 : (Cp > 16 ? 32 : 16));       // (cb is 0 or 32, and then Cp a multiple of 32)
         const uintptr_t at = reinterpret_cast<uintptr_t>(x);
         StageJob32& j = pro.stage[pro.n_stages];
         j.x = x; j.hi = hi; j.lo = lo; j.total_px = (unsigned)planes * H * W; j.HW = H * W; j.Nb = Nb;
-        j.C = C; j.U = block / 4; j.nblk = Cp / block; j.blocked = cb > 0;
+        j.C = C; j.U = block / 4; j.nblk = (Cp + block - 1) / block; j.units = Cp / 4; j.blocked = cb > 0;
         j.V = H * W < 16 ? 0 : (j.HW % 4 == 0 && at % 16 == 0 ? 4 : (j.HW % 2 == 0 && at % 8 == 0 ? 2 : 1));
         j.bx = (j.total_px + STAGE_UNITS / j.U - 1) / (STAGE_UNITS / j.U);
         j.blocks = j.V ? j.bx * j.nblk : (unsigned)grid_cap((size_t)j.total_px * (Cp / 4), STAGE_THREADS, 16);
