@@ -207,6 +207,47 @@ __device__ __forceinline__ void store_rows_f32(uint32_t buf, const uint32_t (&v)
     }
 }
 
+// The same for tiles of at most 64 rows, where two to four of the eight epilogue warps have any: each of them is bound by the latency of its
+// chain of shuffles, reads and stores, not by the stores. (Real-valued 8 -> 8 channels, 70 x 75, batch 105, 1 x 1: 139 us, as above
+// 221. With all rows in use the bursts are slower: 8 -> 112 channels, 67 x 67, batch 125, two components, 578 / 453.)
+template <int V>
+__device__ __forceinline__ void store_rows_f32_few(uint32_t buf, const uint32_t (&v)[32], float* out, int row_off, int pix_off, int lane, bool reduce) {
+    __syncwarp();
+#pragma unroll
+    for (int e = 0; e < 32; ++e) asm volatile("st.shared.u32 [%0], %1;" ::"r"(buf + (uint32_t)(lane * EPI_ROWS_F32_PITCH + e) * 4u), "r"(v[e]) : "memory");
+    __syncwarp();
+    constexpr int LANES = 32 / V;
+    const int sub = lane / LANES, col = (lane % LANES) * V;
+    const uint32_t src = buf + (uint32_t)(sub * EPI_ROWS_F32_PITCH + col) * 4u;
+    // eight instructions' reads in flight before the first of their stores
+#pragma unroll 1
+    for (int r0 = 0; r0 < 32; r0 += 8 * V) {
+        float w[8][V];
+        int ro[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            const int r = r0 + i * V;
+            ro[i] = __shfl_sync(0xffffffffu, row_off, r + sub);
+#pragma unroll
+            for (int e = 0; e < V; ++e) asm volatile("ld.shared.f32 %0, [%1];" : "=f"(w[i][e]) : "r"(src + (uint32_t)(r * EPI_ROWS_F32_PITCH + e) * 4u));
+        }
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+            if (ro[i] < 0 || pix_off < 0) continue;
+            float* dst = out + (size_t)ro[i] + pix_off;
+            if (reduce) {
+                if (V == 4) red_add_f32x4(dst, w[i][0], w[i][V > 1 ? 1 : 0], w[i][V > 2 ? 2 : 0], w[i][V > 3 ? 3 : 0]);
+                else {
+#pragma unroll
+                    for (int e = 0; e < V; ++e) atomicAdd(dst + e, w[i][e]);
+                }
+            } else if (V == 4) *reinterpret_cast<float4*>(dst) = make_float4(w[i][0], w[i][V > 1 ? 1 : 0], w[i][V > 2 ? 2 : 0], w[i][V > 3 ? 3 : 0]);
+            else if (V == 2) *reinterpret_cast<float2*>(dst) = make_float2(w[i][0], w[i][V > 1 ? 1 : 0]);
+            else *dst = w[i][0];
+        }
+    }
+}
+
 // A tile of 16-byte units on its way from pixel-major rows of channels to channel-major rows of pixels (the staging kernels): U units
 // per pixel, V pixels per load of a thread. The units' places are permuted inside 128 bytes so that neither side has bank conflicts.
 constexpr int STAGE_THREADS = 256, STAGE_UNITS = 1024;
