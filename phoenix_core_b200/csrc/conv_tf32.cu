@@ -460,8 +460,10 @@ struct FilterJob32 {
 // Forward:       Wexp[tap][m = d*Co + co][k = l*Cp + ci]  = s(l,d) * w[l^d](co, ci, tap)
 // Backward-data: Wexp[tap][m = l*Ci + ci][k = d*Cop + co] = s(l,d) * w[l^d](co, ci, taps-1-tap)
 // w_io: the filters are stored [r][ci][co] (dense input-major layout, one tap).
+// Threads per row: short rows share a CTA (8 -> 275 channels, 6 x 7, batch 16, 5 x 5, forward 43 us, 62 with a CTA per row).
+__host__ __device__ __forceinline__ int pack_threads_f32(int Kp) { return Kp > 128 ? 256 : (Kp > 64 ? 128 : 64); }
 __device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned block, unsigned blocks) {
-    // one row (tap, m) of the expanded matrix per block iteration; the row is decoded once and the threads walk k
+    // one row (tap, m) of the expanded matrix per `wx` threads; the row is decoded once and its threads walk k
     const float* w = p.w;
     float* __restrict__ hi = p.hi;
     float* __restrict__ lo = p.lo;
@@ -469,13 +471,14 @@ __device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned 
     const unsigned long long neg = p.neg;
     const int Cm = transposed ? Ci : Co, Ck = transposed ? Co : Ci;
     const int rows = taps * Mp;
-    for (int row = block; row < rows; row += blocks) {
+    const int wx = pack_threads_f32(Kp), tx = threadIdx.x % wx, per = STAGE_THREADS / wx;
+    for (int row = block * per + threadIdx.x / wx; row < rows; row += blocks * per) {
         const int tap = row / Mp, m = row - tap * Mp;
         const int cm_comp = m / Cm, cm = m - cm_comp * Cm;
         const int src_tap = transposed ? taps - 1 - tap : tap;
         float* hrow = hi + (size_t)row * Kp;
         float* lrow = lo + (size_t)row * Kp;
-        for (int k = threadIdx.x; k < Kp; k += STAGE_THREADS) {
+        for (int k = tx; k < Kp; k += wx) {
             const int ck_comp = k / Cp, ck = k - ck_comp * Cp;
             float v = 0.f;
             if (cm_comp < nc && ck_comp < nc && ck < Ck) {
@@ -546,14 +549,15 @@ int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream, bool*
     *chain = chain_behind(blocks, 8);
     if (blocks == 0) return PCB_OK;
     if (sc && sc->pending) { pro.status = sc->word; sc->pending = false; }
-    // A large filter matrix that is gathered across its storage order (backward-data of OIHW filters, forward of input-major ones), one
-    // sector per element, is bound by the loads in flight, and by rows that lie side by side being packed at the same time, when they share
+    // A large filter matrix that is gathered across its storage order (backward-data of OIHW filters, forward of input-major ones or of many
+    // taps), one sector per element, is bound by the loads in flight, and by rows that lie side by side being packed at the same time, when they share
     // what they fetch. It is packed by a launch of its own, which is not chained: CTAs that start on a few SMs beside the tail of the kernel
     // in front fall out of step with the rest. Backward-data, one chained launch / this: 7 x 7, batch 4, 512 channels (302 MB)
     // 551 / 306 us; 14 x 14, batch 4, 256 channels (75 MB) 180 / 154; batch 8, 128 channels (19 MB) 68 / 72; dense 1024 x 2048 x 2048
     // forward (537 MB) 1206 / 1036.
     const FilterJob32& f = pro.filter;
-    if (pro.filter_blocks > 0 && f.transposed != f.w_io && (size_t)f.taps * f.Mp * f.Kp * 8 > (size_t)64 << 20) {
+    const bool gathers = f.transposed != f.w_io || f.taps >= 16;        // (elements 64 and more bytes apart)
+    if (pro.filter_blocks > 0 && gathers && (size_t)f.taps * f.Mp * f.Kp * 8 > (size_t)64 << 20) {
         PCB_CUDA_TRY(launch_chained_if(false, filter_prologue_f32_kernel, pro.filter_blocks + pro.zero_blocks, STAGE_THREADS, 0, stream, pro));
         blocks -= pro.filter_blocks + pro.zero_blocks;
         if (blocks == 0) return PCB_OK;
@@ -990,7 +994,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
                           inserted ? pl.pad_left : 0, pl.ins_h, pl.ins_w, 0, 1, stream);
     PCB_CUDA_TRY(cudaGetLastError());
     pro.filter = FilterJob32{(const float*)a, w_hi, w_lo, g.Co, g.Ci, taps, pl.Mp, pl.Kp, pl.Cp, pass == PASS_BWD_DATA ? 1 : 0, g.w_io, g.nc, g.ga, g.neg};
-    pro.filter_blocks = grid_cap((size_t)taps * pl.Mp, 1, 8);
+    pro.filter_blocks = grid_cap((size_t)taps * pl.Mp, STAGE_THREADS / pack_threads_f32(pl.Kp), 8);
 
     TParams p;
     const int n_k = taps * pl.LK * (pl.Cp / TKS);
