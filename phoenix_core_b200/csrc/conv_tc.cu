@@ -628,7 +628,8 @@ struct StageJob {
     const void* x;
     void* xp;
     unsigned total_px, HW, Nb;      // pixels of all planes, of one plane; images per component
-    int C, nblk, U, V;              // channels, blocks of 8 U channels, pixels per load (0: a channels-last source)
+    size_t plane;                   // elements between the planes of x (more than C * HW: a channel slice of a wider tensor)
+    int C, nblk, U, V;              // channels, blocks of 8 U channels, pixels per load (0: a channels-last source, -1: tiny planes)
     int blocked;
     unsigned bx, blocks;            // CTAs along the pixels; all CTAs
 };
@@ -647,7 +648,7 @@ __device__ __forceinline__ void stage_compact(const StageJob& p, unsigned block,
         const unsigned P = px0 + l * V;
         uint32_t raw[8][V == 4 ? 2 : 1];
         const unsigned plane = P / HW;
-        const uint16_t* src = x + ((size_t)plane * C + c0 + 8 * g) * HW + (P - plane * HW);
+        const uint16_t* src = x + plane * p.plane + (size_t)(c0 + 8 * g) * HW + (P - plane * HW);
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const bool ok = P < total_px && c0 + 8 * g + e < C;
@@ -713,6 +714,31 @@ __device__ __forceinline__ void repack_channels_last(const StageJob& p, unsigned
             dst = ((size_t)P + (size_t)(comp * (unsigned)(p.nblk - 1) + b) * p.Nb * p.HW) * p.U + (u - b * p.U);
         }
         xp[dst] = v;
+    }
+}
+
+// NCHW planes of fewer than 16 pixels: a thread per pixel and 8 channels, consecutive threads along the pixels of a plane and then its
+// channel groups. (The batched transposition loads along the pixels, of which there are too few.)
+__device__ __forceinline__ void stage_tiny(const StageJob& p, unsigned block) {
+    const uint16_t* x = static_cast<const uint16_t*>(p.x);
+    uint4* __restrict__ xp = static_cast<uint4*>(p.xp);
+    const unsigned groups = (unsigned)(p.nblk * p.U), HW = p.HW;
+    const size_t total = (size_t)p.total_px * groups;
+    for (size_t i = (size_t)block * STAGE_THREADS + threadIdx.x; i < total; i += (size_t)p.blocks * STAGE_THREADS) {
+        const unsigned px = (unsigned)(i % HW), grp = (unsigned)(i / HW % groups), plane = (unsigned)(i / HW / groups);
+        const uint16_t* src = x + plane * p.plane + (size_t)(8 * grp) * HW + px;
+        uint32_t w[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            w[e] = (uint32_t)ld_chained(src + (size_t)(2 * e) * HW, (int)(8 * grp) + 2 * e < p.C) |
+                   (uint32_t)ld_chained(src + (size_t)(2 * e + 1) * HW, (int)(8 * grp) + 2 * e + 1 < p.C) << 16;
+        const size_t P = (size_t)plane * HW + px;
+        size_t dst = P * groups + grp;
+        if (p.blocked) {
+            const unsigned comp = plane / p.Nb, b = grp / p.U;
+            dst = (P + (size_t)(comp * (unsigned)(p.nblk - 1) + b) * p.Nb * HW) * p.U + (grp - b * p.U);
+        }
+        xp[dst] = make_uint4(w[0], w[1], w[2], w[3]);
     }
 }
 
@@ -858,6 +884,7 @@ __global__ void __launch_bounds__(STAGE_THREADS) prologue_kernel(const __grid_co
     if (second) block -= p.stage_blocks[0];
     uint4* tile = reinterpret_cast<uint4*>(pack_smem);
     if (job.V == 0) repack_channels_last(job, block);
+    else if (job.V < 0) stage_tiny(job, block);
     else if (job.U == 8) stage_compact<8>(job, block, tile);
     else if (job.U == 4) stage_compact<4>(job, block, tile);
     else stage_compact<2>(job, block, tile);
@@ -914,14 +941,18 @@ void stage_activations(Prologue& pro, int fmt, const void* src, void* dst, int p
     const bool compact = Hp == H && Wp == W && pad_top == 0 && pad_left == 0 && ins_h == 1 && ins_w == 1;
     const int block = channel_slice(C);
     const uintptr_t at = reinterpret_cast<uintptr_t>(src);
-    const bool last = ss && ss->c == 1 && ss->w == C && ss->h == (long long)W * C && ss->p == (long long)H * W * C && C % 8 == 0 && at % 16 == 0;
-    if (compact && (last || (!ss && H * W >= 16))) {               // (tiny NCHW planes: consecutive pixels are C elements apart)
+    const bool last = (ss ? ss->c == 1 && ss->w == C && ss->h == (long long)W * C && ss->p == (long long)H * W * C : H * W == 1) && C % 8 == 0 && at % 16 == 0;
+    // NCHW planes: the whole tensor, or the channel slice of a group (as a thread per pixel and 8 channels, bf16 72 -> 6 channels of two groups,
+    // 105 x 105, batch 7, 1 x 1, forward took 198 us instead of 156). Tiny planes up to 16 MB; larger ones are copied faster through
+    // shared memory, by a kernel of their own (2 -> 40 channels, 1 x 5, batch 69, filter gradient 31 us with two of those, 21 without).
+    const bool nchw = st.w == 1 && st.h == W && st.c == (long long)H * W;
+    if (compact && (last || (nchw && (H * W >= 16 || total <= (size_t)1 << 20)))) {
         StageJob& j = pro.stage[pro.n_stages];
-        j.x = src; j.xp = dst; j.total_px = (unsigned)planes * H * W; j.HW = H * W; j.Nb = Nb;
+        j.x = src; j.xp = dst; j.total_px = (unsigned)planes * H * W; j.HW = H * W; j.Nb = Nb; j.plane = (size_t)st.p;
         j.C = C; j.U = block / 8; j.nblk = Cp / block; j.blocked = cb > 0;
-        j.V = last ? 0 : (j.HW % 4 == 0 && at % 8 == 0 ? 4 : (j.HW % 2 == 0 && at % 4 == 0 ? 2 : 1));
+        j.V = last ? 0 : (H * W < 16 ? -1 : (j.HW % 4 == 0 && at % 8 == 0 ? 4 : (j.HW % 2 == 0 && at % 4 == 0 ? 2 : 1)));
         j.bx = (j.total_px + STAGE_UNITS / j.U - 1) / (STAGE_UNITS / j.U);
-        j.blocks = last ? (unsigned)grid_cap(total, STAGE_THREADS, 16) : j.bx * j.nblk;
+        j.blocks = j.V <= 0 ? (unsigned)grid_cap(total, STAGE_THREADS, 16) : j.bx * j.nblk;
         pro.stage_blocks[pro.n_stages++] = j.blocks;
     } else if (!ss && (size_t)C * H * W * 2 <= PACK_SMEM_MAX_BYTES && (reinterpret_cast<uintptr_t>(src) & 15u) == 0) {
         const size_t smem = ((size_t)C * H * W * 2 + 15) / 16 * 16;

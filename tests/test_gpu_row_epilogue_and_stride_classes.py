@@ -111,3 +111,28 @@ def test_real_valued_stem_filter_gradient(gpu, oracle, k):
     dw = torch.full(f.shape, float("nan"), dtype=torch.float16, device="cuda")
     pcb.conv2DBwd(gpu.dev(x, "f16"), gpu.dev(f, "f16"), gpu.dev(dy, "f16"), dw, None, bwd, gpu.context("16p"), gpu.ENGINES["tensor"])
     assert rel_err(dw.float().cpu().numpy(), rdw) <= TOL["f16"]
+
+
+# planes of 1 to 15 pixels, staged thread by thread beside the filters; 1 x 1 planes of whole 16-byte units, copied unit by unit
+@pytest.mark.parametrize("shape", [(5, 33, 17, 1, 1, 1), (3, 6, 40, 3, 5, 3), (69, 2, 40, 1, 5, 1), (2, 64, 31, 1, 15, 3), (40, 72, 24, 3, 3, 3), (9, 96, 40, 1, 1, 1)])
+def test_tiny_planes(gpu, oracle, shape):
+    n, ci, co, h, w, k = shape
+    _case(gpu, oracle, n, ci, co, h, w, k, k, (1, 1), (k // 2,) * 4, "f16")
+
+
+# two and three groups: channel slices of every alignment, odd and even planes, staged as slices of the tensors
+@pytest.mark.parametrize("groups,ci,co,h,w,k", [(2, 24, 48, 14, 14, 3), (3, 7, 33, 9, 11, 1), (2, 33, 10, 12, 10, 3), (2, 16, 32, 3, 4, 1)])
+def test_groups_stage_slices(gpu, oracle, groups, ci, co, h, w, k):
+    n, pad = 3, (k // 2,) * 4
+    x = gpu.rounded(uniform(81, (4 * n, ci * groups, h, w)), "f16")
+    f = gpu.rounded(normal(82, (4, co - co % groups, ci, k, k), std=(2.0 / (4 * ci * k * k)) ** 0.5), "f16")
+    per = f.shape[1] // groups
+    y = gpu.run_conv_fwd(x, f, None, (1, 1), pad, "f16", "16p", "tensor", groups=groups)
+    dy = gpu.rounded(normal(84, y.shape), "f16")
+    dw, dx = gpu.run_conv_bwd(x, f, dy, (1, 1), pad, "f16", "16p", "tensor", True, groups=groups)
+    for g in range(groups):
+        ic, oc = slice(g * ci, (g + 1) * ci), slice(g * per, (g + 1) * per)
+        xg, fg, gg = (np.ascontiguousarray(v) for v in (x[:, ic], f[:, oc], dy[:, oc]))
+        rdw, rdx = oracle.conv2d_bwd(xg, fg, gg, (1, 1), (1, 1), pad)
+        ref = oracle.conv2d_fwd(xg, fg, None, (1, 1), (1, 1), pad)
+        assert rel_err(y[:, oc], ref) <= TOL["f16"] and rel_err(dx[:, ic], rdx) <= TOL["f16"] and rel_err(dw[:, oc], rdw) <= TOL["f16"]
