@@ -500,8 +500,13 @@ int stride_classes(const Geom& g, int dtype, StrideClass* cls, size_t* bytes) {
 
 bool strided_classes_supported(int dtype, int variant, const Geom& g) {
     if (!strided_taps(g)) return false;
-    // 16-bit layers with strides 2 x 2: one launch over all classes (the general kernel's DUAL form)
-    if (dtype != PCB_F32 && conv_tc_dual_classes(PASS_BWD_DATA, g) && conv_tc_supported(PASS_BWD_DATA, dtype, variant, g)) return false;
+    // 16-bit layers with strides 2 x 2: one launch over all classes (the general kernel's DUAL form). Not for wide filters of more than nine
+    // taps: their matrix is packed element by element there and run by run for each class (at most nine of 5 x 5 taps), and the stride-1
+    // kernel does more per operand byte. 5 x 5, 14 x 14, DUAL form / classes: 512 channels, batch 64 1524 / 1002 us; 384, batch 32 621 / 438;
+    // 320, batch 32 368 / 465; 256, batch 128 674 / 578, batch 32 270 / 333; 128 channels, 28 x 28, batch 128 617 / 632.
+    const int rows = g.nc * g.Ci;
+    const bool many_taps = g.KH * g.KW > 9 && (rows >= 1536 || (rows >= 1024 && (long long)g.Nb * g.H * g.W >= 20000));
+    if (dtype != PCB_F32 && !many_taps && conv_tc_dual_classes(PASS_BWD_DATA, g) && conv_tc_supported(PASS_BWD_DATA, dtype, variant, g)) return false;
     StrideClass cls[4];
     size_t bytes;
     const int n = stride_classes(g, dtype, cls, &bytes);
@@ -697,7 +702,7 @@ bool forward_keeps_staged_input(int dtype, int variant, const Geom& g) {
 bool backward_shares_staged_dy(int dtype, int variant, const Geom& g, StagedView* view, size_t* bytes) {
     if ((dtype != PCB_F16 && dtype != PCB_BF16) || variant != PCB_VARIANT_16_PRODUCT || !g.plain || g.groups != 1 || g.real_in) return false;
     if (g.KH * g.KW == 1) return false;
-    if ((g.SH != 1 || g.SW != 1) && !conv_tc_dual_classes(PASS_BWD_DATA, g)) return false;
+    if ((g.SH != 1 || g.SW != 1) && (!conv_tc_dual_classes(PASS_BWD_DATA, g) || strided_classes_supported(dtype, variant, g))) return false;
     // the same order of preference as tensor_launch, for both passes
     if (pointwise_filter_tc_supported(dtype, variant, g)) return false;
     const bool narrow_dat = narrow_tc_supported(PASS_BWD_DATA, dtype, variant, g), narrow_flt = narrow_filter_tc_supported(dtype, variant, g);

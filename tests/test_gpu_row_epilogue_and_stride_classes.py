@@ -136,3 +136,10 @@ def test_groups_stage_slices(gpu, oracle, groups, ci, co, h, w, k):
         rdw, rdx = oracle.conv2d_bwd(xg, fg, gg, (1, 1), (1, 1), pad)
         ref = oracle.conv2d_fwd(xg, fg, None, (1, 1), (1, 1), pad)
         assert rel_err(y[:, oc], ref) <= TOL["f16"] and rel_err(dx[:, ic], rdx) <= TOL["f16"] and rel_err(dw[:, oc], rdw) <= TOL["f16"]
+
+
+# wide filters of more than nine taps at strides 2 x 2 take the classes one by one, as one-row filters do at any width
+@pytest.mark.parametrize("n,ci,co,h,w,taps,pad", [(1, 384, 24, 9, 10, (5, 5), (2, 2, 2, 2)), (2, 384, 16, 8, 8, (4, 4), (1, 1, 1, 1)),
+                                                  (1, 136, 24, 9, 14, (1, 3), (0, 1, 0, 1)), (1, 136, 20, 12, 9, (3, 1), (1, 0, 1, 0))])
+def test_stride_classes_one_by_one(gpu, oracle, n, ci, co, h, w, taps, pad):
+    _case(gpu, oracle, n, ci, co, h, w, taps[0], taps[1], (2, 2), pad, "f16")
