@@ -125,7 +125,8 @@ const char* pcb_last_error_message(void);
  * (replaces upstride::computeWindowedOutputSizeAndPadding, src/utils.cc:41-50). */
 int pcb_conv2d_output_size(const pcb_conv2d_desc* desc, int32_t* out_h, int32_t* out_w);
 
-/* Bytes of caller-provided scratch needed by the corresponding call (may be 0).
+/* Bytes of caller-provided scratch needed by the corresponding call (may be 0). Some layers also run, slower, with less: the call
+ * then takes its smallest layout, and answers PCB_ERR_WORKSPACE where the workspace is too small for that one as well.
  * (replaces the MemoryRequest protocol of src/backend/memory_request.hpp:73-114.) */
 size_t pcb_qconv2d_fwd_workspace_size(const pcb_conv2d_desc* desc);
 size_t pcb_qconv2d_bwd_workspace_size(const pcb_conv2d_desc* desc);

@@ -178,11 +178,18 @@ size_t workspace_bytes(Pass pass, int dtype, int variant, int engine, const Geom
     return WS_HEADER + ((s + 255) / 256) * 256;
 }
 
-int run_pass(Pass pass, int dtype, int variant, int engine, const Geom& g, const void* a, const void* b, const void* bias,
+// `full`: the problem as described; where the workspace is too small for it the kernels take the tight layout (Geom), so that a workspace
+// of a size that once was enough still is.
+int run_pass(Pass pass, int dtype, int variant, int engine, const Geom& full, const void* a, const void* b, const void* bias,
              void* out, void* workspace, size_t ws_bytes, cudaStream_t stream, const PassExtras* extras = nullptr, StatusClear* sc = nullptr) {
     forget_kept(workspace);
+    Geom g = full;
     const size_t offset = extras ? extras->scratch_offset : 0;       // scratch another pass of the same call still needs
-    const size_t need = workspace_bytes(pass, dtype, variant, engine, g) + offset;
+    size_t need = workspace_bytes(pass, dtype, variant, engine, g) + offset;
+    if (workspace && ws_bytes < need) {
+        g.tight = 1;
+        need = workspace_bytes(pass, dtype, variant, engine, g) + offset;
+    }
     const int tv = tensor_variant(variant, engine);
     const bool needs_ws = need > WS_HEADER || tensor_path_supported(pass, dtype, tv, g);
     if (needs_ws && (workspace == nullptr || ws_bytes < need)) {
@@ -213,10 +220,17 @@ int run_pass(Pass pass, int dtype, int variant, int engine, const Geom& g, const
 
 // How far a dense call runs on the kernels that take the caller's tensors as they are (qgemm_tc.cu). `tensors`: the OR of all
 // tensor addresses of the call; `apart`: no result shares memory with an operand, which these kernels read while they write (the
-// staged kernels copy their operands first, so a gradient may replace the tensor it belongs to). The workspace must be what the
-// size query asks for, as for every other path.
-DenseRoute dense_route(const pcb_dense_desc* desc, const Geom& g, uintptr_t tensors, bool apart, bool backward, void* workspace, size_t ws_bytes, size_t need) {
-    const int tv = tensor_variant(variant_for(g, desc->variant), desc->engine);
+// staged kernels copy their operands first, so a gradient may replace the tensor it belongs to). The workspace must be large enough for
+// the staged kernels (in their tight layout), which take the call where these do not.
+DenseRoute dense_route(const pcb_dense_desc* desc, const Geom& g, uintptr_t tensors, bool apart, bool backward, void* workspace, size_t ws_bytes) {
+    const int v = variant_for(g, desc->variant), tv = tensor_variant(v, desc->engine);
+    Geom tight = g;
+    tight.tight = 1;
+    size_t need = workspace_bytes(backward ? PASS_BWD_FILTER : PASS_FWD, desc->dtype, v, desc->engine, tight);
+    if (backward) {
+        const size_t data = workspace_bytes(PASS_BWD_DATA, desc->dtype, v, desc->engine, tight);
+        if (data > need) need = data;
+    }
     const bool direct = desc->engine != PCB_ENGINE_SIMT && apart && workspace && ws_bytes >= need &&
                         ((tensors | reinterpret_cast<uintptr_t>(workspace)) & 15u) == 0 && dense_tc_supported(desc->dtype, tv, g);
     return direct ? dense_tc_route(desc->dtype, g, backward, backward && desc->require_input_grad) : DENSE_STAGED;
@@ -241,11 +255,16 @@ size_t conv_workspace_bytes(Pass pass, int dtype, int variant, int engine, const
     return workspace_bytes(pass, dtype, variant, engine, g) + (pass == PASS_BWD_FILTER ? group_slice_bytes(dtype, g) : 0);
 }
 
-int run_conv_pass(Pass pass, int dtype, int variant, int engine, const Geom& g, const void* a, const void* b, const void* bias,
+int run_conv_pass(Pass pass, int dtype, int variant, int engine, const Geom& full, const void* a, const void* b, const void* bias,
                   void* out, void* workspace, size_t ws_bytes, cudaStream_t stream, const PassExtras* extras = nullptr, StatusClear* sc = nullptr) {
-    if (g.groups == 1) return run_pass(pass, dtype, variant, engine, g, a, b, bias, out, workspace, ws_bytes, stream, extras, sc);
+    if (full.groups == 1) return run_pass(pass, dtype, variant, engine, full, a, b, bias, out, workspace, ws_bytes, stream, extras, sc);
     const size_t es = dtype_size(dtype);
-    const size_t need = conv_workspace_bytes(pass, dtype, variant, engine, g);
+    Geom g = full;
+    size_t need = conv_workspace_bytes(pass, dtype, variant, engine, g);
+    if (workspace && ws_bytes < need) {
+        g.tight = 1;
+        need = conv_workspace_bytes(pass, dtype, variant, engine, g);
+    }
     if (need > WS_HEADER && (workspace == nullptr || ws_bytes < need)) {
         set_error("workspace of %zu bytes required, %zu given", need, workspace ? ws_bytes : (size_t)0);
         return PCB_ERR_WORKSPACE;
@@ -328,9 +347,10 @@ int conv_bwd_filter(const pcb_conv2d_desc* desc, const void* x, const void* dy, 
     return run_conv_pass(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g, dy, x, nullptr, dw, workspace, workspace_bytes_, stream, extras, sc);
 }
 
-// Staged dy shared by the two gradients of one call: the padded copy that backward-data makes at the start of the scratch
-// stays where it is, and the filter gradient -- run second, its own scratch placed behind that copy -- reads it through a
-// tensor map instead of staging dy again. Applies to 16-bit stride-1 tapped layers whose two kernels agree on the layout.
+// Staged dy shared by the two gradients of one call: the copy that backward-data makes at the start of the scratch stays where it
+// is, and the filter gradient -- run second, its own scratch placed behind that copy -- reads it through a tensor map instead of
+// staging dy again. Applies to 16-bit layers whose backward-data pass reads an uninserted copy (stride 1, or 2 x 2 by pixel
+// classes) and whose two kernels agree on the layout.
 bool bwd_shares_dy(const pcb_conv2d_desc* desc, const Geom& g, StagedView* view, size_t* offset) {
     if (desc->engine == PCB_ENGINE_SIMT || !desc->require_input_grad || g.Nb == 0 || g.groups != 1) return false;
     size_t bytes = 0;
@@ -354,8 +374,9 @@ int conv_bwd_both(const pcb_conv2d_desc* desc, const void* x, const void* w, con
     // (not where dx replaces x: the filter gradient, run second, reads x)
     const size_t x_bytes = (size_t)g.nc * g.Nb * g.Ci * g.groups * g.H * g.W * dtype_size(desc->dtype);
     if (x && w && dy && dw && dx && workspace && (all & 15u) == 0 && !overlaps(dx, x_bytes, x, x_bytes) && bwd_shares_dy(desc, g, &view, &offset) &&
+        workspace_bytes_ >= conv_workspace_bytes(PASS_BWD_DATA, desc->dtype, variant_for(g, desc->variant), desc->engine, g) &&
         workspace_bytes_ >= conv_workspace_bytes(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g) + offset) {
-        // backward-data first: it leaves the padded dy in [WS_HEADER, WS_HEADER + offset)
+        // backward-data first: it leaves dy in [WS_HEADER, WS_HEADER + offset), in the layout of a workspace that is large enough
         rc = conv_bwd_data(desc, w, dy, dx, workspace, workspace_bytes_, stream, sc);
         if (rc != PCB_OK) return rc;
         view.base = static_cast<const char*>(workspace) + WS_HEADER;
@@ -514,7 +535,7 @@ int pcb_qdense_fwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
     const DenseBytes n = dense_bytes(desc->dtype, g);
     const bool apart = !overlaps(y, n.y, x, n.x) && !overlaps(y, n.y, w, n.w);
-    if (dense_route(desc, g, all, apart, false, workspace, workspace_bytes_, pcb_qdense_fwd_workspace_size(desc)) == DENSE_DIRECT) {
+    if (dense_route(desc, g, all, apart, false, workspace, workspace_bytes_) == DENSE_DIRECT) {
         forget_kept(workspace);
         return dense_tc_fwd(desc->dtype, g, x, w, bias, y, static_cast<int*>(workspace), (cudaStream_t)stream);
     }
@@ -540,7 +561,7 @@ int pcb_qdense_bwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     const DenseBytes n = dense_bytes(desc->dtype, g);
     auto free_of_operands = [&](const void* out, size_t bytes) { return !overlaps(out, bytes, x, n.x) && !overlaps(out, bytes, w, n.w) && !overlaps(out, bytes, dy, n.y); };
     const bool apart = free_of_operands(dw, n.w) && free_of_operands(gx, n.x) && !overlaps(dw, n.w, gx, n.x);
-    const DenseRoute route = dense_route(desc, g, all, apart, true, workspace, workspace_bytes_, pcb_qdense_bwd_workspace_size(desc));
+    const DenseRoute route = dense_route(desc, g, all, apart, true, workspace, workspace_bytes_);
     if (route != DENSE_STAGED) {
         forget_kept(workspace);
         rc = dense_tc_bwd(desc->dtype, g, x, w, dy, dw, route == DENSE_DIRECT ? gx : nullptr, static_cast<int*>(workspace), (cudaStream_t)stream);

@@ -59,6 +59,8 @@ struct Geom {
     int bias_ld;         // bias is [components][bias_ld]
     int plain;           // NCHW activations, OIHW (or dense) filters, one group: the layouts the tensor-core kernels read
     int groups;          // host side only: groups of the convolution; Ci / Co above are the channels of ONE group
+    int tight = 0;       // host side only: the smallest scratch the kernels run with (channels in slices of 16, copies that end at the last
+                         // pixel a tap reads) -- for workspaces too small for the faster layout, and tensors close to the scratch limits
 };
 
 enum { LAYOUT_NCHW = 0, LAYOUT_NHWC = 1 };
@@ -125,6 +127,12 @@ inline bool algebra_setup(int algebra, Geom& g) {
 }
 
 inline size_t dtype_size(int dtype) { return dtype == PCB_F32 ? 4 : 2; }
+
+// Rows (or columns) of an image of `size` that the taps of `out` output rows read.
+inline int reached(int size, int out, int stride, int k, int dilation, int pad) {
+    const int r = (out - 1) * stride + (k - 1) * dilation + 1 - pad;
+    return r < 1 ? 1 : (r < size ? r : size);
+}
 
 // Whether two tensors share memory. A kernel that reads a caller's tensor while other CTAs write the result (or a launch that clears the
 // result beside the staging of an operand) may only run where they do not.

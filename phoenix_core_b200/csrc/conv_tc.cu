@@ -695,8 +695,9 @@ __device__ __forceinline__ void stage_compact(const StageJob& p, unsigned block,
 // staged copy or by the zero fill of the tensor map). A TMA copy costs about the same whatever its size and moves rows of one slice,
 // so 16-channel slices are kept for layers of at most 16 channels: 48 channels as one slice of 64 instead of three of 16 take a
 // 3x3 forward pass (44 images of 39 x 47, 40 output channels) from 164 to 105 us although a quarter of the products are zeros.
-int channel_slice(int c) { return c <= 16 ? 16 : (round_up(c, 32) % 64 == 0 ? 64 : 32); }
-int padded_channels(int c) { return round_up(c, channel_slice(c)); }
+// `tight` (see Geom): the fewest channels, a multiple of 16.
+int padded_channels(int c, bool tight) { return round_up(c, c <= 16 || tight ? 16 : (round_up(c, 32) % 64 == 0 ? 64 : 32)); }
+int channel_slice(int c, bool tight) { const int p = padded_channels(c, tight); return p % 64 == 0 ? 64 : (p % 32 == 0 ? 32 : 16); }
 
 // Channels-last sources that have to be copied (padded to slices, or cut into blocks of 8 U channels for the filter gradient): 16-byte
 // units, C a multiple of 8. Destination as for stage_compact_kernel.
@@ -934,12 +935,11 @@ int launch_prologue(Prologue& pro, StatusClear* sc, cudaStream_t stream, bool* c
 // Host dispatch of the activation staging: a job of the prologue launch where that form applies, a kernel of its own otherwise. cb > 0 selects the channel-block layout of the filter-gradient kernels (Nb images per
 // component). `ss` = nullptr: a dense NCHW source (the fast forms apply); otherwise its element strides.
 void stage_activations(Prologue& pro, int fmt, const void* src, void* dst, int planes, int C, int H, int W, int Hp, int Wp, int Cp, int pad_top, int pad_left,
-                       int ins_h, int ins_w, cudaStream_t stream, int cb = 0, int Nb = 1, const SrcStrides* ss = nullptr) {
+                       int ins_h, int ins_w, int block, cudaStream_t stream, int cb = 0, int Nb = 1, const SrcStrides* ss = nullptr) {
     const size_t total = (size_t)planes * Hp * Wp * (Cp / 8);
     const SrcStrides dense = {(long long)C * H * W, (long long)H * W, (long long)W, 1};
     const SrcStrides st = ss ? *ss : dense;
     const bool compact = Hp == H && Wp == W && pad_top == 0 && pad_left == 0 && ins_h == 1 && ins_w == 1;
-    const int block = channel_slice(C);
     const uintptr_t at = reinterpret_cast<uintptr_t>(src);
     const bool last = (ss ? ss->c == 1 && ss->w == C && ss->h == (long long)W * C && ss->p == (long long)H * W * C : H * W == 1) && C % 8 == 0 && at % 16 == 0;
     // NCHW planes: the whole tensor, or the channel slice of a group (as a thread per pixel and 8 channels, bf16 72 -> 6 channels of two groups,
@@ -1316,6 +1316,7 @@ struct Plan {
     int LK;                        // components of the convolved tensor (1 for a real-valued input)
     int KS;
     int dual;                      // backward-data with strides 2 x 2 by pixel classes (the kernel's DUAL form)
+    bool tight;                    // see Geom
     size_t xp_bytes, w_bytes;
 };
 
@@ -1324,8 +1325,9 @@ bool dual_classes(Pass pass, const Geom& g) {
     return pass == PASS_BWD_DATA && g.SH == 2 && g.SW == 2 && g.DH == 1 && g.DW == 1 && g.KH >= 2 && g.KW >= 2;
 }
 
-Plan make_plan(Pass pass, const Geom& g) {
+Plan make_plan(Pass pass, const Geom& g, bool tight) {
     Plan pl;
+    pl.tight = tight;
     if (pass == PASS_FWD) {
         pl.Cin = g.Ci; pl.Cout = g.Co; pl.Hin = g.H; pl.Win = g.W; pl.Hout = g.HO; pl.Wout = g.WO;
         pl.pad_top = g.PT; pl.pad_left = g.PL; pl.SH = g.SH; pl.SW = g.SW; pl.ins_h = pl.ins_w = 1;
@@ -1338,16 +1340,25 @@ Plan make_plan(Pass pass, const Geom& g) {
     pl.dual = dual_classes(pass, g) ? 1 : 0;
     if (pl.dual) { pl.ins_h = pl.ins_w = 1; pl.pad_top = pl.pad_left = 0; }   // (the kernel places the taps itself)
     pl.LK = (pass == PASS_FWD && g.real_in) ? 1 : g.nc;
-    pl.KS = channel_slice(pl.Cin);
-    pl.Cp = padded_channels(pl.Cin);
+    pl.KS = channel_slice(pl.Cin, tight);
+    pl.Cp = padded_channels(pl.Cin, tight);
     pl.Hp = (pl.Hout - 1) * pl.SH + (g.KH - 1) * g.DH + 1;
     pl.Wp = (pl.Wout - 1) * pl.SW + (g.KW - 1) * g.DW + 1;
-    if (pl.ins_h == 1 && pl.ins_w == 1) { pl.Hp = pl.Hin; pl.Wp = pl.Win; }   // the copy is not padded: the tensor map's zero fill is the padding
+    if (pl.ins_h == 1 && pl.ins_w == 1) {                              // the copy is not padded: the tensor map's zero fill is the padding
+        pl.Hp = tight && !pl.dual ? reached(pl.Hin, pl.Hout, pl.SH, g.KH, g.DH, pl.pad_top) : pl.Hin;
+        pl.Wp = tight && !pl.dual ? reached(pl.Win, pl.Wout, pl.SW, g.KW, g.DW, pl.pad_left) : pl.Win;
+    }
     pl.Mp = round_up(g.nc * pl.Cout, GM);
     pl.Kp = pl.LK * pl.Cp;
     pl.xp_bytes = ((size_t)pl.LK * g.Nb * pl.Hp * pl.Wp * pl.Cp * 2 + 1023) / 1024 * 1024;
     pl.w_bytes = ((size_t)g.KH * g.KW * pl.Mp * pl.Kp * 2 + 1023) / 1024 * 1024;
     return pl;
+}
+
+constexpr size_t MAX_COPY = (size_t)8 << 30;
+Plan make_plan(Pass pass, const Geom& g) {
+    const Plan pl = make_plan(pass, g, g.tight != 0);
+    return pl.xp_bytes <= MAX_COPY ? pl : make_plan(pass, g, true);
 }
 
 }  // namespace
@@ -1366,7 +1377,7 @@ bool conv_tc_supported(Pass pass, int dtype, int variant, const Geom& g) {
     }
     const Plan pl = make_plan(pass, g);
     if ((long long)(pl.Hout - 1) * pl.SH + (long long)(g.KH - 1) * g.DH > 65534 || (long long)(pl.Wout - 1) * pl.SW + (long long)(g.KW - 1) * g.DW > 65534) return false;
-    if ((long long)pl.Wp * pl.Cp * 2 > (1ll << 31) || pl.xp_bytes > (size_t)8 << 30) return false;
+    if ((long long)pl.Wp * pl.Cp * 2 > (1ll << 31) || pl.xp_bytes > MAX_COPY) return false;
     return true;
 }
 
@@ -1406,7 +1417,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         Prologue pro;
         if (!direct)
             stage_activations(pro, fmt, act, xp, pl.LK * g.Nb, pl.Cin, pl.Hin, pl.Win, pl.Hp, pl.Wp, pl.Cp, inserted ? pl.pad_top : 0, inserted ? pl.pad_left : 0,
-                              pl.ins_h, pl.ins_w, stream, 0, 1, g.plain ? nullptr : &sa);
+                              pl.ins_h, pl.ins_w, pl.KS, stream, 0, 1, g.plain ? nullptr : &sa);
         const FilterStrides fs = {g.wr, g.wo, g.wi, g.wh, g.ww, g.KW};
         add_filter_job(pro, w, wexp, g.Co, g.Ci, taps, pl.Mp, pl.Kp, pl.Cp, pass == PASS_BWD_DATA ? 1 : 0, g.nc, g.ga, g.neg, fs);
         const int rc = launch_prologue(pro, sc, stream, &chain);
@@ -1536,7 +1547,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     }
     {
         // staged copy [comp][img][Hp][Wp][Cp], or the caller's channels-last tensor (the same without padding) read in place
-        const int Wd = pl.Wp, Hd = pl.Hp, Cd = direct ? pl.Cin : pl.Cp;
+        const int Wd = direct ? pl.Win : pl.Wp, Hd = direct ? pl.Hin : pl.Hp, Cd = direct ? pl.Cin : pl.Cp;
         const cuuint64_t dims[5] = {(cuuint64_t)Cd, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
         const cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)Wd * Cd * 2, (cuuint64_t)Hd * Wd * Cd * 2, (cuuint64_t)g.Nb * Hd * Wd * Cd * 2};
         // with an element stride s the box extent is given in input elements: s * (pixels - 1) + 1 of them hold the pixels loaded
@@ -1568,18 +1579,28 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
 
 namespace {
 struct FilterPlan {
-    int Cop, Cip;
+    int Cop, Cip, cbx, cby;        // padded channels and the width of their blocks
+    int H, W;                      // extents of the copy of x
+    bool tight;                    // see Geom
     size_t xp_bytes, dyp_bytes, acc_bytes;
 };
 
-FilterPlan make_filter_plan(const Geom& g) {
+FilterPlan make_filter_plan(const Geom& g, bool tight) {
     FilterPlan f;
-    f.Cop = padded_channels(g.Co);
-    f.Cip = padded_channels(g.Ci);
-    f.xp_bytes = ((size_t)(g.real_in ? 1 : g.nc) * g.Nb * g.H * g.W * f.Cip * 2 + 1023) / 1024 * 1024;
+    f.tight = tight;
+    f.Cop = padded_channels(g.Co, tight); f.cby = channel_slice(g.Co, tight);
+    f.Cip = padded_channels(g.Ci, tight); f.cbx = channel_slice(g.Ci, tight);
+    f.H = tight ? reached(g.H, g.HO, g.SH, g.KH, g.DH, g.PT) : g.H;
+    f.W = tight ? reached(g.W, g.WO, g.SW, g.KW, g.DW, g.PL) : g.W;
+    f.xp_bytes = ((size_t)(g.real_in ? 1 : g.nc) * g.Nb * f.H * f.W * f.Cip * 2 + 1023) / 1024 * 1024;
     f.dyp_bytes = ((size_t)g.nc * g.Nb * g.HO * g.WO * f.Cop * 2 + 1023) / 1024 * 1024;
     f.acc_bytes = ((size_t)g.nc * g.Co * g.Ci * g.KH * g.KW * sizeof(float) + 1023) / 1024 * 1024;
     return f;
+}
+constexpr size_t MAX_COPIES = (size_t)12 << 30;
+FilterPlan make_filter_plan(const Geom& g) {
+    const FilterPlan f = make_filter_plan(g, g.tight != 0);
+    return f.xp_bytes + f.dyp_bytes <= MAX_COPIES ? f : make_filter_plan(g, true);
 }
 }  // namespace
 
@@ -1587,8 +1608,7 @@ namespace {
 // x-major variant: one x box per tap must tile M = 128 exactly and dy's (d, co) columns must fit one MMA.
 bool filter_xmajor(const Geom& g, const FilterPlan& f) {
     const int lk = g.real_in ? 1 : g.nc;
-    const int cbx = channel_slice(g.Ci), cby = channel_slice(g.Co);
-    return f.Cip == cbx && f.Cop == cby && lk * cbx <= 64 && g.nc * cby <= 256;
+    return f.Cip == f.cbx && f.Cop == f.cby && lk * f.cbx <= 64 && g.nc * f.cby <= 256;
 }
 }  // namespace
 
@@ -1605,7 +1625,7 @@ bool conv_filter_tc_supported(int dtype, int variant, const Geom& g) {
     if (g.SH > 2 || g.SW > 2) return false;
     const FilterPlan f = make_filter_plan(g);
     if ((long long)(g.HO - 1) * g.SH + (long long)(g.KH - 1) * g.DH > 65534 || (long long)(g.WO - 1) * g.SW + (long long)(g.KW - 1) * g.DW > 65534 ||
-        f.xp_bytes + f.dyp_bytes > (size_t)12 << 30) return false;
+        f.xp_bytes + f.dyp_bytes > MAX_COPIES) return false;
     return true;
 }
 
@@ -1616,15 +1636,16 @@ size_t conv_filter_tc_scratch_bytes(const Geom& g) {
 
 bool conv_filter_tc_stages_like_forward(const Geom& g) {
     const FilterPlan f = make_filter_plan(g);
-    return g.plain && one_block(g.Ci) && f.xp_bytes == make_plan(PASS_FWD, g).xp_bytes;
+    const Plan pl = make_plan(PASS_FWD, g);
+    return g.plain && one_block(g.Ci) && !f.tight && !pl.tight && f.xp_bytes == pl.xp_bytes;
 }
 
 bool conv_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes) {
     const Plan pl = make_plan(PASS_BWD_DATA, g);
     if (!g.plain || pl.ins_h != 1 || pl.ins_w != 1) return false;   // backward-data reads a zero-inserted copy
     const FilterPlan f = make_filter_plan(g);
-    if (channel_slice(g.Co) != f.Cop) return false;             // the filter gradient would block the channels
-    if (pl.Cp != f.Cop) return false;
+    if (f.cby != f.Cop) return false;                           // the filter gradient would block the channels
+    if (pl.Cp != f.Cop || pl.tight || f.tight) return false;
     view->Hp = pl.Hp; view->Wp = pl.Wp; view->pad_top = view->pad_left = 0;
     *bytes = pl.xp_bytes;
     return true;
@@ -1645,18 +1666,18 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     // A channels-last tensor with one channel block per component (at most 64 channels, a multiple of 16) already is the staged layout
     // [component][image][h][w][channels]: it is read in place, its padding supplied by out-of-range TMA coordinates.
     const bool direct_x = !g.plain && g.xc == 1 && g.xw == g.Ci && g.xh == g.W * g.Ci && (long long)g.xp == (long long)g.H * g.W * g.Ci &&
-                          channel_slice(g.Ci) == f.Cip && g.Ci % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
+                          f.cbx == f.Cip && g.Ci % 16 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;
     const bool direct_dy = !g.plain && g.yc == 1 && g.yw == g.Co && g.yh == g.WO * g.Co && (long long)g.yp == (long long)g.HO * g.WO * g.Co &&
-                           channel_slice(g.Co) == f.Cop && g.Co % 16 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
+                           f.cby == f.Cop && g.Co % 16 == 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
     bool chain = false;
     {   // stage both activations channels-last, clear the accumulator
         Prologue pro;
         const int lk = g.real_in ? 1 : g.nc;
         const SrcStrides sx = {g.xp, g.xc, g.xh, g.xw}, sy = {g.yp, g.yc, g.yh, g.yw};
         if (!direct_x && !kept_x)
-            stage_activations(pro, fmt, x, xp, lk * g.Nb, g.Ci, g.H, g.W, g.H, g.W, f.Cip, 0, 0, 1, 1, stream, channel_slice(g.Ci), g.Nb, g.plain ? nullptr : &sx);
+            stage_activations(pro, fmt, x, xp, lk * g.Nb, g.Ci, g.H, g.W, f.H, f.W, f.Cip, 0, 0, 1, 1, f.cbx, stream, f.cbx, g.Nb, g.plain ? nullptr : &sx);
         if (!direct_dy && !kept_dy)
-            stage_activations(pro, fmt, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, stream, channel_slice(g.Co), g.Nb, g.plain ? nullptr : &sy);
+            stage_activations(pro, fmt, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, g.HO, g.WO, f.Cop, 0, 0, 1, 1, f.cby, stream, f.cby, g.Nb, g.plain ? nullptr : &sy);
         PCB_CUDA_TRY(cudaGetLastError());
         add_zero_job(pro, acc, f.acc_bytes);
         const int rc = launch_prologue(pro, sc, stream, &chain);
@@ -1666,7 +1687,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     FGParams p;
     p.nc = g.nc; p.ga = g.ga; p.neg = g.neg;
     p.Nb = g.Nb; p.Co = g.Co; p.Ci = g.Ci; p.HO = g.HO; p.WO = g.WO; p.Cop = f.Cop; p.Cip = f.Cip;
-    p.cbA = channel_slice(g.Co); p.cbB = channel_slice(g.Ci);
+    p.cbA = f.cby; p.cbB = f.cbx;
     p.KH = g.KH; p.KW = g.KW; p.SH = g.SH; p.SW = g.SW; p.DH = g.DH; p.DW = g.DW; p.fmt = fmt;
     {   // pixel box of FK pixels wasting the fewest K rows
         long long best = -1;
@@ -1719,7 +1740,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
         if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (dy) failed with code %d", (int)r); return PCB_ERR_CUDA; }
     }
     {
-        const int Wd = g.W, Hd = g.H, Cd = direct_x ? g.Ci : p.cbB;
+        const int Wd = direct_x ? g.W : f.W, Hd = direct_x ? g.H : f.H, Cd = direct_x ? g.Ci : p.cbB;
         const cuuint64_t dims[5] = {(cuuint64_t)Cd, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)(p.LK * (f.Cip / p.cbB))};
         const cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)Wd * Cd * 2, (cuuint64_t)Hd * Wd * Cd * 2,
                                        (cuuint64_t)g.Nb * Hd * Wd * Cd * 2};

@@ -690,7 +690,7 @@ size_t tensor_scratch_bytes(Pass pass, int dtype, int variant, int engine, const
 
 bool forward_keeps_staged_input(int dtype, int variant, const Geom& g) {
     if ((dtype != PCB_F16 && dtype != PCB_BF16) || variant != PCB_VARIANT_16_PRODUCT || !g.plain || g.groups != 1) return false;
-    if (g.KH * g.KW == 1) return false;             // pointwise layers read x in place (or a compacted copy of their own)
+    if (g.KH * g.KW == 1 || g.tight) return false;  // pointwise layers read x in place (or a compacted copy of their own)
     // the same order of preference as tensor_launch
     if (pointwise_pair_tc_supported(PASS_FWD, dtype, variant, g) || pointwise_tc_supported(PASS_FWD, dtype, variant, g)) return false;
     if (pointwise_filter_tc_supported(dtype, variant, g)) return false;
