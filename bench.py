@@ -9,7 +9,8 @@ Work per step and GPU: 3 passes x 32*N*H*W*Co*Ci = 631.4 GFLOP. Under torchrun e
 batch (weak scaling) and the filter gradient is summed across ranks with one NCCL all-reduce per step, started on
 a side stream as soon as the filter gradient is enqueued so that it runs beside backward-data.
 
-Prints one JSON line:
+Prints one JSON line of a few kilobytes (readers of a log's tail see all of it) and writes the full record, with every table and note,
+to `--detail` (bench_detail.json beside this file). The record:
   value          device-timed throughput with inputs resident in HBM
   parity         relative errors of the timed tensors themselves (batch 64) against the CPU checker
   roofline       the slowest of the three kernels, timed alone for >= 2 s of back-to-back launches against the measured
@@ -148,6 +149,50 @@ def cpu_baseline(torch, sample_n, reps, speed_over_memory=True):
     sample = ("batch %d of the same layer (fp32, %s orchestration, torch CPU ops = oneDNN), median of %d steps"
               % (sample_n, "8-product" if speed_over_memory else "16-product", reps))
     return fl / t / 1e12, cores, sample, t
+
+
+LINE_LIMIT = 5000
+
+
+def compact(record):
+    """The printed line: the keys that name, value and qualify the measurement as they are in the record, of the others the numbers
+    and short words of the first two levels. Tables (lists) and notes stay in the record."""
+    kept = ("metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better", "scaling", "vs_baseline", "dtype", "data",
+            "config", "clocks", "gpu_launches")
+
+    def short(v, depth):
+        if isinstance(v, float):
+            return float("%.5g" % v)
+        if isinstance(v, dict):
+            if depth == 0:
+                return None
+            d = {k: short(w, depth - 1) for k, w in v.items()}
+            return {k: w for k, w in d.items() if w is not None} or None
+        if isinstance(v, list):
+            return None
+        return None if isinstance(v, str) and len(v) > 160 else v
+
+    line = {k: record[k] for k in kept if k in record}
+    for k, v in record.items():
+        if k not in line:
+            v = short(v, 1 if k in ("dense", "qresnet18", "sweep", "sweep_f32") else 2)
+            if v is not None:
+                line[k] = v
+    if "e2e" in record and record["e2e"]:
+        line["e2e"] = dict({k: v for k, v in record["e2e"].items() if not isinstance(v, dict)},
+                           **{k: short(v, 1) for k, v in record["e2e"].items() if isinstance(v, dict)})
+    for k in ("dense", "sweep", "sweep_f32"):                     # time of the whole table, by pass or type where it has them
+        if record.get(k):
+            rows = record[k].get("rows") if isinstance(record[k], dict) else None
+            if rows:
+                line[k] = {"rows": len(rows), "ms_sum": short(sum(r["ms"] for r in rows if r.get("ms")), 1)}
+            else:
+                line[k] = short(record[k], 2)
+    for k in ("kernel_sm_mhz", "sweep_f32", "sweep", "dense", "eight_product", "pct_of_tensor_peak"):
+        if len(json.dumps(line)) <= LINE_LIMIT:
+            break
+        line.pop(k, None)
+    return line
 
 
 def run_reference(args):
@@ -715,7 +760,13 @@ def run_ours(args):
         if cpu is not None:
             line["cpu_baseline"] = {"value": cpu[0], "unit": "TFLOP/s", "cores": cpu[1], "kind": "port", "sample": cpu[2],
                                     "sixteen_product": {"value": cpu16[0], "unit": "TFLOP/s", "sample": cpu16[2]}}
-        print(json.dumps(line), flush=True)
+        try:
+            with open(args.detail, "w") as f:
+                json.dump(line, f)
+                f.write("\n")
+        except OSError as e:
+            print("no detail record: %s" % e, file=sys.stderr)
+        print(json.dumps(compact(line)), flush=True)
     if world > 1:
         dist.barrier()
         dist.destroy_process_group()
@@ -726,6 +777,7 @@ def main():
     ap.add_argument("--gpus", type=int, default=1)
     ap.add_argument("--steps", type=int, default=200)
     ap.add_argument("--warmup", type=int, default=3)
+    ap.add_argument("--detail", default=os.path.join(ROOT, "bench_detail.json"), help="file for the full record")
     ap.add_argument("--impl", default="ours", choices=["ours", "reference"])
     ap.add_argument("--cpu-sample", type=int, default=32, help="batch size of the CPU baseline sample")
     ap.add_argument("--kernel-seconds", type=float, default=2.0, help="length of each kernel's sustained timing run")
