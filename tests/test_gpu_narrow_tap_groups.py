@@ -29,3 +29,24 @@ def test_tap_groups(oracle, taps, ci, co, h, w, dtype):
     dw, dx = gpu.run_conv_bwd(x, f, dy, (1, 1), pad, dtype, "16p", "tensor", True)
     assert np.all(np.isfinite(dw)) and rel_err(dw, rdw) <= TOL[dtype]
     assert np.all(np.isfinite(dx)) and rel_err(dx, rdx) <= TOL[dtype]
+
+
+@pytest.mark.parametrize("taps,stride,ci,dtype", [((11, 3), 2, 3, "f16"), ((12, 4), 2, 4, "bf16"), ((12, 4), 2, 1, "f16"), ((6, 2), 1, 16, "f16"), ((7, 7), 2, 3, "f16")])
+def test_rows_folded_by_halves(oracle, taps, stride, ci, dtype):
+    """Real-valued input: the filter rows share an MMA too, three of six here, two of four for the 7 x 7 stem."""
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import gpu_util as gpu
+    kh, kw = taps
+    n, h, w = 2, 34, 38
+    pad = ((kh - 1) // 2, (kw - 1) // 2, kh // 2, kw // 2)
+    x = gpu.rounded(uniform(34, (n, ci, h, w)), dtype)
+    f = gpu.rounded(normal(35, (4, 16, ci, kh, kw), std=(2.0 / (ci * kh * kw)) ** 0.5), dtype)
+    x4 = np.concatenate([x, np.zeros((3 * n, ci, h, w), np.float32)])            # the quaternions with zero imaginary parts
+    dy = gpu.rounded(normal(36, oracle.conv2d_fwd(x4, f, None, (stride, stride), (1, 1), pad).shape), dtype)
+    rdw, _ = oracle.conv2d_bwd(x4, f, dy, (stride, stride), (1, 1), pad)
+    _, desc = gpu.conv_descriptors(x.shape, f.shape, (stride, stride), pad, False, False, True)
+    out = torch.full(f.shape, float("nan"), dtype=gpu.TORCH_DTYPES[dtype], device="cuda")
+    gpu.pcb.conv2DBwd(gpu.dev(x, dtype), gpu.dev(f, dtype), gpu.dev(dy, dtype), out, None, desc, gpu.context("16p"), gpu.ENGINES["tensor"])
+    dw = gpu.host(out)
+    assert np.all(np.isfinite(dw)) and rel_err(dw, rdw) <= TOL[dtype]
