@@ -4,9 +4,9 @@
 // The reference layout (NCHW, components stacked on the batch axis) cannot feed tap-shifted TMA boxes: the
 // innermost TMA coordinate must be a multiple of 16 bytes, and a filter tap shifts the pixel axis by single
 // elements. So a convolution with taps first stages two small-or-cheap things in the caller's workspace:
-//   * the activations, channels-last:  xp[comp][img][h][w][c16]   (stage_compact_kernel and others)
+//   * the activations, channels-last:  xp[comp][img][h][w][c16]   (stage_compact, mostly)
 //   * the filters as the signed, permuted real matrix of the Hamilton product, one slab per tap:
-//       Wexp[tap][(d,co)][(l,ci)] = s(l,d) * w[l^d][co][ci][tap]                    (pack_filters_kernel)
+//       Wexp[tap][(d,co)][(l,ci)] = s(l,d) * w[l^d][co][ci][tap]                    (pack_filters_tile)
 //     (reference sign table src/algebras.cc:28-49; for backward-data the transposed block with flipped taps)
 // and then runs ONE implicit-GEMM kernel: D[(d,co), pixel] = sum over (tap, l, ci). With channels innermost a
 // tap is a shift of the *outer* TMA coordinates (free), stride 2 is the tensor map's element stride, and
@@ -700,7 +700,7 @@ int padded_channels(int c, bool tight) { return round_up(c, c <= 16 || tight ? 1
 int channel_slice(int c, bool tight) { const int p = padded_channels(c, tight); return p % 64 == 0 ? 64 : (p % 32 == 0 ? 32 : 16); }
 
 // Channels-last sources that have to be copied (padded to slices, or cut into blocks of 8 U channels for the filter gradient): 16-byte
-// units, C a multiple of 8. Destination as for stage_compact_kernel.
+// units, C a multiple of 8. Destination as for stage_compact.
 __device__ __forceinline__ void repack_channels_last(const StageJob& p, unsigned block) {
     const uint4* x = static_cast<const uint4*>(p.x);
     uint4* __restrict__ xp = static_cast<uint4*>(p.xp);

@@ -6,7 +6,8 @@
 // accumulator: hi*hi + hi*lo + lo*hi. What is dropped is lo*lo and the rounding of lo (both ~2^-22 relative), so
 // the result is as good as an fp32 FMA chain. Cost: 3 TF32 MMAs per product and twice the operand bytes.
 //
-// Structure as in conv_tc.cu: channels-last zero-padded activations and the signed/permuted filter matrix
+// Structure as in conv_tc.cu: channels-last activations (not padded: the zero fill of the tensor maps is
+// the padding) and the signed/permuted filter matrix
 // Wexp[tap][(d,co)][(l,ci)] (reference sign table src/algebras.cc:28-49) are staged in the workspace, here in fp32
 // and twice (hi, lo); the implicit-GEMM kernel is TMA-fed, 128 x 256 tile, double-buffered TMEM accumulator.
 // Dense layers are the 1x1 convolution of 1x1 images (pixels = batch); input-major dense filters and the

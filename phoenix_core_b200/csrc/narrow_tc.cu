@@ -448,7 +448,9 @@ void add_planar_job(PlanarPrologue& pro, const void* src, void* dst, int planes_
         j.blocks = grid_cap(units, NP_THREADS, 16);
     }
 }
-// `chain`: whether the main kernel may be chained to this launch (the copies' CTAs are capped at 16 per SM: a capped one is a long one).
+// `chain`: whether the main kernel may be chained to this launch (the copies' CTAs are capped at 16 per SM: a capped one is a long one.
+// Chained / not, us: 16 -> 16, 32 x 32, 3x3, forward, batch 256, below the cap 45.8 / 49.5, batch 16 12.8 / 14.8; above it 112 x 112, batch 64, both
+// gradients 350 / 340, the 7x7/2 stem at batch 128 350 / 245).
 int launch_prologue(PlanarPrologue& pro, StatusClear* sc, cudaStream_t stream, bool* chain) {
     unsigned copies = 0;
     for (int i = 0; i < pro.n_stages; ++i) copies += pro.stage[i].blocks;

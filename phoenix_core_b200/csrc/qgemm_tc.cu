@@ -12,12 +12,14 @@
 // The rows m are contiguous in the output of every pass, so the 32 lanes of an epilogue warp store 32 consecutive elements.
 // (replaces the 16 GEMM calls and accumulate passes of the reference, src/dense.hpp:21-379, src/backend/cudnn/dense.hpp:20-218.)
 //
-// Three groups of four warps load (plain loads: feature counts need no alignment, which a tensor map would ask for), expand and store the operands in the tcgen05 layouts, each group its own stages;
+// Three groups of four warps load (plain loads: feature counts need no alignment, which a tensor map would ask for), expand and store
+// the operands in the tcgen05 layouts, each group its own stages;
 // one thread of a thirteenth warp issues the MMAs. fp32 operands are split into hi + lo TF32 numbers on their way
 // (three MMAs per product, as in conv_tf32.cu). The reduced dimension of a tile is cut over the CTAs of a cluster, which add
 // their partial tiles through distributed shared memory in a fixed order (results do not depend on timing, nothing is zeroed or
 // cast in a second pass). What bounds a dense layer of a few hundred features is the latency of this chain (load, expand, MMA,
-// exchange, store), not bandwidth: hence one launch per call, no staging kernels, and a cluster split that fills the machine.
+// exchange, store), not bandwidth: hence one kernel per call (behind the reset of the status word), no staging
+// kernels, and a cluster split that fills the machine.
 // All mbarrier waits are bounded.
 #include "tc_common.cuh"
 #include "tensor_path.cuh"
@@ -521,8 +523,9 @@ bool dense_tc_supported(int dtype, int variant, const Geom& g) {
     if (g.H != 1 || g.W != 1 || g.KH != 1 || g.KW != 1 || !g.dw_io || g.groups != 1) return false;
     const int most = 8 * Q_F32_STAGES_PER_ACC * Q_F32_ACCS / 4 * 32;
     if (dtype == PCB_F32 && (g.Ci > most || g.Co > most || g.Nb > most)) return false;
-    // A wide fp32 layer runs faster from staged hi / lo operands: here every tile splits its operands again. Forward + backward,
-    // this kernel against the staged ones: 560 / 688 us at 1024 x 768 x 1024, 6099 / 5155 us at 2048 x 2048 x 2048.
+    // A wide fp32 layer runs faster from staged hi / lo operands: here every tile splits its operands again. This kernel against the
+    // staged ones, us: forward 2048 x 2048 x 2048 2069 / 1829, 1024 x 2048 x 2048 1051 / 1036 (not for a forward pass that is longer than
+    // wide, 2048 x 1024 x 1536 720 / 830, but one line serves both directions and backward is the longer one: preferred_route).
     if (dtype == PCB_F32 && (long long)g.Nb * g.Ci * g.Co > (1ll << 31)) return false;
     return true;
 }

@@ -299,9 +299,10 @@ inline int sm_count() {
 }
 
 // Whether a main kernel is chained to a prologue of that many CTAs: only behind a short one. Behind a longer prologue the gap does not
-// matter, and the main kernel, started CTA by CTA beside the last wave, runs 2 to 3 % slower for its whole length (fp32 3x3, 128
-// channels, 28 x 28, batch 128, forward + backward: 6825 us chained, 6790 not; 3x3/2 128 channels 616 / 609; the 7x7/2 stem 442 / 357). At 5
-// to 20 MB of copies it is worth 3 to 7 % (3x3 16 -> 16, 45 x 37, batch 32: 96 us chained, 102 not).
+// matter, and the main kernel, started CTA by CTA beside the last wave, can be the slower for it. Chained / not, us: fp32 3x3, 128
+// channels, 28 x 28, batch 128, forward 2196 / 2087; fp16 3x3 of the same size, filter gradient 482 / 446; the 7x7/2 stem, 224 x 224, batch 128,
+// forward 350 / 245 (but 3x3 64 -> 64, 56 x 56, batch 64 228 / 228). Behind short ones: 3x3 64 -> 64, 56 x 56, batch 8, forward 40.9 / 43.3, 3x3
+// 16 -> 16, 45 x 37, batch 32 26.8 / 29.0, 32 x 32, batch 16, forward 12.8 / 14.8, both gradients 31.4 / 37.3.
 inline bool chain_behind(unsigned prologue_blocks, unsigned per_sm) { return prologue_blocks <= per_sm * (unsigned)sm_count(); }
 
 inline int round_up(int v, int m) { return (v + m - 1) / m * m; }

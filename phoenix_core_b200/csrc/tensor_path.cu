@@ -460,10 +460,12 @@ struct StrideClass {
     size_t dx_off, w_off;   // byte offsets of the compact gradient / the class's filters in the scratch area
 };
 
-// Taken from 512 gradient rows (128 quaternion channels) up: each class pays its own staging pass and launch, and below that
-// width those cost more than the zero-insertion route's extra MMAs (measured at batch 128: 0.47 -> 0.38 ms at 128
-// channels and 28 x 28, 0.51 -> 0.34 ms at 256 and 14 x 14, but 0.12 -> 0.27 ms at 64 -> 128 channels and 14 x 14).
-// From 256 rows (64 quaternion channels) the classes also win when the gradient is large (at least ~200k pixels per component).
+// Taken from 512 gradient rows (128 quaternion channels) up, and from 256 rows (64 quaternion channels) when the gradient is large (at least
+// ~200k pixels per component): each class pays its own staging pass and launch. The line is that of 16-bit layers, which take this route
+// only for one-row filters and many taps (below): 3x3/2, batch 128, zero insertion -> classes 0.47 -> 0.38 ms at 128 channels and 28 x 28,
+// but 0.12 -> 0.27 ms at 64 -> 128 channels and 14 x 14. fp32 layers, 3x3/2, us, zero insertion / classes: 128 -> 256, 28 x 28, batch 128
+// 4326 / 1855, batch 8 351 / 214; 128 -> 128, 14 x 14, batch 128 614 / 398, batch 32 186 / 194; 64 -> 128, 56 x 56, batch 128 4199 / 2204. Below the
+// line the classes would be the faster ones for fp32: 64 -> 128, 28 x 28 1150 / 665, 14 x 14 330 / 244; 32 -> 64, 56 x 56 1194 / 910.
 bool strided_taps(const Geom& g) {
     const bool wide = g.nc * g.Ci >= 512 || (g.nc * g.Ci >= 256 && (long long)g.Nb * g.H * g.W >= 200000);
     return (g.KH > 1 || g.KW > 1) && (g.SH > 1 || g.SW > 1) && g.SH <= 2 && g.SW <= 2 && g.DH == 1 && g.DW == 1 && g.plain && !g.w_io &&

@@ -9,7 +9,7 @@ bool tensor_path_supported(Pass pass, int dtype, int variant, const Geom& g);
 // Scratch bytes (beyond the workspace header) the tensor-core kernel of this problem needs.
 size_t tensor_scratch_bytes(Pass pass, int dtype, int variant, int engine, const Geom& g);
 // Operand roles as for simt_launch. `status` is the device status word of the workspace header.
-// A staged tensor that another pass already made: where it lies and how it is padded.
+// A staged tensor that another pass already made: where it lies and how it is padded (copies for the narrow kernels are).
 struct StagedView {
     const void* base = nullptr;
     int Hp = 0, Wp = 0, pad_top = 0, pad_left = 0;   // padded plane and the position of pixel (0, 0) inside it
@@ -17,7 +17,7 @@ struct StagedView {
 // What a filter-gradient pass may take over from other passes instead of staging it again:
 // `kept_x`: the staged copy of x that the forward call of the same layer left in ITS workspace scratch (see
 //           forward_keeps_staged_input);
-// `dy`:     the padded copy of dy that the backward-data pass of the same call staged (see backward_shares_staged_dy);
+// `dy`:     the copy of dy that the backward-data pass of the same call staged (see backward_shares_staged_dy);
 // `scratch_offset`: bytes of the workspace scratch to leave alone (they hold that copy).
 struct PassExtras {
     const void* kept_x = nullptr;
@@ -40,8 +40,8 @@ struct StatusClear {
 int tensor_launch(Pass pass, int dtype, int variant, const Geom& g, const void* a, const void* b, const void* bias,
                   void* out, float* scratch, int* status, cudaStream_t stream, const PassExtras* extras = nullptr, StatusClear* sc = nullptr);
 // True when the backward-data pass of this layer stages dy (at the start of its scratch, `bytes` long) in a layout its
-// filter gradient can read through a tensor map: stride-1 layers on the narrow pair of kernels, or on the general pair with
-// one channel block per component. `view` receives the padded geometry (its base is left null).
+// filter gradient can read through a tensor map: the narrow pair of kernels (stride 1), or the general pair with one channel block per
+// component (stride 1, or 2 x 2 by pixel classes). `view` receives the padded geometry (its base is left null).
 bool backward_shares_staged_dy(int dtype, int variant, const Geom& g, StagedView* view, size_t* bytes);
 // True when the forward pass of this layer stages x, at the start of its scratch, in exactly the layout its filter
 // gradient reads: a narrow forward with a narrow filter gradient, or the general pair with one channel block per component.
