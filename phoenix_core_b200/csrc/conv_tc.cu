@@ -49,7 +49,9 @@ struct GParams {
                                  // the tile leaves through shared memory as one contiguous bulk copy per image
     // halo mode
     int Wt, Ht;
-    uint32_t stage_bytes;
+    int a_slots, a_taps;         // filter slices in flight, and the taps of one (a filter row, or one tap)
+    uint32_t halo_bytes;         // shared-memory pitch of one halo tile (n_stages of them)
+    uint32_t stage_bytes;        // the other forms: one stage of both operands
     int off_w, off_h;            // added to the pixel coordinates of every activation box: minus the padding (out-of-range coordinates
                                  // read zeros); 0 for a zero-inserted copy, which holds its padding
     int o_generic;               // the output is addressed through the element strides below (channels-last tensors, channel
@@ -129,12 +131,16 @@ __device__ __forceinline__ void plane_pack_exact(const uint32_t (&v)[32], int co
 }
 
 // 192 KB of operand stages, at most 12
+constexpr int H_MAX_SLOTS = 22, H_MAX_TILES = 3;               // halo form: filter slices and halo tiles in flight
 template <int KS, bool DUAL> constexpr int G_MAX_STAGES = KS == 64 ? (DUAL ? 6 : 4) : (KS == 32 ? (DUAL ? 12 : 8) : 12);
 
-// HALO (KS == 32, stride-1 correlation, tile = 8 x PH pixels of one image): a stage is one 32-channel slice of one
-// component -- the halo tile [Ht][Wt][32 channels] of the output tile and the filter slices of ALL taps -- and every
-// tap's MMAs read the same halo tile at a shifted start address. Per MMA the kernel then moves 5 KB from L2 instead
-// of 12 KB, which is what bounds the plain form.
+// HALO (KS == 32, stride-1 correlation, tile = 8 x PH pixels of one image): for every 32-channel slice of one component the halo
+// tile [Ht][Wt][32 channels] of the output tile is loaded once, and every tap's MMAs read it at a shifted start address; the filter
+// slices stream beside it. Per MMA the kernel then moves 5 KB from L2 instead of 12 KB, which is what bounds the plain form (an SM
+// takes in about 64 bytes per clock). The two operands have rings of their own: 2 or 3 halo tiles of some 20 KB, and as many filter
+// slices of one filter row (or tap) as fit; with both operands of all taps in one of two 90 KB stages the loads were exposed. Channels-last
+// 3x3, 64 -> 64, 56 x 56, batch 128, forward: 373 -> 356 us (first 20 launches), 424 -> 410 us under the power limit. Also open to 5x5
+// and larger filters, whose slices did not fit a stage. What bounds it now is the power limit: 1155 TFLOP/s at 990 W.
 //
 // DUAL (backward-data of a layer with strides 2 x 2): the input pixels fall into four classes by the parity of row and column,
 // and with r = (a + PT) mod 2, c = (a + PT) div 2 the gradient of row class a is dx[2 i + a] = sum over k of dy[i + c - k] w[r + 2 k]
@@ -148,20 +154,22 @@ __global__ void __launch_bounds__(G_THREADS, 1)
 qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GParams p,
                         const uint16_t* bias, uint16_t* __restrict__ out, int* __restrict__ status) {
     constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = (DUAL ? GN / 2 : GN) * KS * 2;
-    constexpr int MAX_STAGES = G_MAX_STAGES<KS, DUAL>;
-    const uint32_t STAGE = HALO ? p.stage_bytes : A_BYTES + B_BYTES;
-    const int STAGES = p.n_stages;
+    constexpr int MAX_STAGES = HALO ? H_MAX_SLOTS : G_MAX_STAGES<KS, DUAL>;
+    const uint32_t STAGE = HALO ? A_BYTES * p.a_taps : A_BYTES + B_BYTES;      // HALO: one slot of the filter ring
+    const int STAGES = HALO ? p.a_slots : p.n_stages;
     const int taps = p.KH * p.KW;
     extern __shared__ uint8_t smem_raw[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(base + STAGES * STAGE);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 5);
-    const uint32_t tiles_addr = smem_u32(base);
+    const uint32_t operand_bytes = STAGES * STAGE + (HALO ? p.n_stages * p.halo_bytes : 0u);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + operand_bytes);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_STAGES + 5 + 2 * H_MAX_TILES);
+    const uint32_t tiles_addr = smem_u32(base), halo_addr = tiles_addr + STAGES * STAGE;
     const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + MAX_STAGES);
     const uint32_t tmem_full = smem_u32(bars + 2 * MAX_STAGES), tmem_empty = smem_u32(bars + 2 * MAX_STAGES + 2);
     const uint32_t epi_bar = smem_u32(bars + 2 * MAX_STAGES + 4);
-    uint8_t* plane_buf = base + STAGES * STAGE + 512;              // plane mode only: [image][128 rows][HO * WO]
+    const uint32_t halo_full = smem_u32(bars + 2 * MAX_STAGES + 5), halo_empty = halo_full + 8 * H_MAX_TILES;      // HALO
+    uint8_t* plane_buf = base + operand_bytes + 512;               // plane mode only: [image][128 rows][HO * WO]
 
     const int tiles_px = p.tiles_w * p.tiles_h * p.tiles_n;
     const int n_tiles = tiles_px * p.tiles_m * (DUAL ? 2 : 1);
@@ -174,6 +182,8 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, 8); }
         mbar_init(epi_bar, 8);
+        if (HALO)
+            for (int s = 0; s < H_MAX_TILES; ++s) { mbar_init(halo_full + 8 * s, 1); mbar_init(halo_empty + 8 * s, 1); }
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
@@ -186,8 +196,10 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0) {
+        {
+            const bool el = elect_one();
             int s = 0, phase = 1;                  // ring position and the parity its `empty` barrier is waited with
+            int hs = 0, hphase = 1;                // the same of the halo tiles
             bool ok = true;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
                 const int tm = tile % p.tiles_m;
@@ -204,12 +216,14 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                             const int tap = taps - 1 - (kh * p.KW + kw);             // the packed filters hold the taps flipped
                             for (int l = 0; l < p.LK && ok; ++l) {
                                 for (int cs = 0; cs < c_steps; ++cs) {
-                                    ok = mbar_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+                                    ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
                                     if (!ok) break;
                                     const uint32_t a_dst = tiles_addr + s * STAGE, bar = full_bar + 8 * s;
-                                    mbar_arrive_expect_tx(bar, A_BYTES + p.b_tx);
-                                    tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, bar);
-                                    tma_load_5d(a_dst + A_BYTES, &map_x, cs * KS, col, row, n0, l, bar);
+                                    if (el) {
+                                        mbar_arrive_expect_tx(bar, A_BYTES + p.b_tx);
+                                        tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, bar);
+                                        tma_load_5d(a_dst + A_BYTES, &map_x, cs * KS, col, row, n0, l, bar);
+                                    }
                                     if (++s == STAGES) { s = 0; phase ^= 1; }
                                 }
                             }
@@ -220,14 +234,23 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 const int m0 = tm * GM, ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
                 if (HALO) {
                     for (int l = 0; l < p.LK && ok; ++l) {
-                        for (int cs = 0; cs < c_steps; ++cs) {
-                            ok = mbar_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+                        for (int cs = 0; cs < c_steps && ok; ++cs) {
+                            ok = warp_wait_bounded(halo_empty + 8 * hs, hphase, status, ST_G_PRODUCER);
                             if (!ok) break;
-                            const uint32_t a_dst = tiles_addr + s * STAGE, bar = full_bar + 8 * s;
-                            mbar_arrive_expect_tx(bar, taps * A_BYTES + (uint32_t)p.Wt * p.Ht * KS * 2);
-                            tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, 0, bar);                       // [tap][128 rows][32 channels]
-                            tma_load_5d(a_dst + taps * A_BYTES, &map_x, cs * KS, ow0 + p.off_w, oh0 + p.off_h, n0, l, bar);   // [Ht][Wt][32 channels]
-                            if (++s == STAGES) { s = 0; phase ^= 1; }
+                            if (el) {
+                                mbar_arrive_expect_tx(halo_full + 8 * hs, (uint32_t)p.Wt * p.Ht * KS * 2);
+                                tma_load_5d(halo_addr + hs * p.halo_bytes, &map_x, cs * KS, ow0 + p.off_w, oh0 + p.off_h, n0, l, halo_full + 8 * hs);   // [Ht][Wt][32 channels]
+                            }
+                            if (++hs == p.n_stages) { hs = 0; hphase ^= 1; }
+                            for (int tap = 0; tap < taps; tap += p.a_taps) {
+                                ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+                                if (!ok) break;
+                                if (el) {
+                                    mbar_arrive_expect_tx(full_bar + 8 * s, STAGE);
+                                    tma_load_3d(tiles_addr + s * STAGE, &map_w, l * p.Cp + cs * KS, m0, tap, full_bar + 8 * s);   // [taps][128 rows][32 channels]
+                                }
+                                if (++s == STAGES) { s = 0; phase ^= 1; }
+                            }
                         }
                     }
                     continue;
@@ -237,12 +260,14 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     const int wp0 = ow0 * p.SW + kw * p.DW + p.off_w, hp0 = oh0 * p.SH + kh * p.DH + p.off_h;
                     for (int l = 0; l < p.LK && ok; ++l) {
                         for (int cs = 0; cs < c_steps; ++cs) {
-                            ok = mbar_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+                            ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
                             if (!ok) break;
                             const uint32_t a_dst = tiles_addr + s * STAGE, bar = full_bar + 8 * s;
-                            mbar_arrive_expect_tx(bar, A_BYTES + p.b_tx);
-                            tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, bar);
-                            tma_load_5d(a_dst + A_BYTES, &map_x, cs * KS, wp0, hp0, n0, l, bar);
+                            if (el) {
+                                mbar_arrive_expect_tx(bar, A_BYTES + p.b_tx);
+                                tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, bar);
+                                tma_load_5d(a_dst + A_BYTES, &map_x, cs * KS, wp0, hp0, n0, l, bar);
+                            }
                             if (++s == STAGES) { s = 0; phase ^= 1; }
                         }
                     }
@@ -252,17 +277,17 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         __syncwarp();
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        // One thread runs the whole loop (waits, descriptor stepping, MMAs, commits): whatever it executes between two MMAs is
-        // time the tensor pipe idles, so there is no warp synchronisation inside and a stage's two descriptors are built once
-        // and stepped by adding to the address field of their low words (16-byte units, never carrying out of the field).
-        if (lane == 0) {
+        // One elected lane issues (umma.cuh: elect_one); a stage's two descriptors are built once and stepped by adding to the address
+        // field of their low words (16-byte units, never carrying out of the field).
+        {
+            const bool el = elect_one();
             const uint32_t idesc = make_idesc_f16(p.fmt, GM, DUAL ? GN / 2 : ((HALO || p.exact) ? p.n_cols : GN), false, false);
-            int s = 0, phase = 0, local_tile = 0;
+            int s = 0, phase = 0, hs = 0, hphase = 0, local_tile = 0;
             bool ok = true;
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local_tile) {
                 const int buf = local_tile & 1, use = local_tile >> 1;       // use-th time this accumulator buffer is filled
                 if (use > 0) {
-                    ok = mbar_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_G_MMA);
+                    ok = warp_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_G_MMA);
                     if (!ok) break;
                     tc_fence_after_sync();
                 }
@@ -273,52 +298,77 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     int kw = 0, left = inner, b = p.PL & 1;
                     uint32_t started = 0;                              // bit b: column class b's accumulator has been written
                     for (int k = 0; k < steps; ++k) {
-                        ok = mbar_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA);
+                        ok = warp_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA);
                         if (!ok) break;
                         tc_fence_after_sync();
                         const uint32_t a_addr = tiles_addr + s * STAGE;
                         const uint64_t ad = make_desc_kmajor_rows<KS>(a_addr), bd = make_desc_kmajor_rows<KS>(a_addr + A_BYTES);
+                        if (el) {
 #pragma unroll
-                        for (int j = 0; j < KS / 16; ++j)
-                            mma_f16_ss_words(d_tmem + b * (GN / 2), (uint32_t)ad + 2 * j, (uint32_t)(ad >> 32), (uint32_t)bd + 2 * j, (uint32_t)(bd >> 32),
-                                             idesc, (j > 0 || ((started >> b) & 1u)) ? 1u : 0u);
+                            for (int j = 0; j < KS / 16; ++j)
+                                mma_f16_ss_words(d_tmem + b * (GN / 2), (uint32_t)ad + 2 * j, (uint32_t)(ad >> 32), (uint32_t)bd + 2 * j, (uint32_t)(bd >> 32),
+                                                 idesc, (j > 0 || ((started >> b) & 1u)) ? 1u : 0u);
+                            mma_commit(empty_bar + 8 * s);
+                            if (k == steps - 1) mma_commit(tmem_full + 8 * buf);
+                        }
                         started |= 1u << b;
-                        mma_commit(empty_bar + 8 * s);
-                        if (k == steps - 1) mma_commit(tmem_full + 8 * buf);
                         if (++s == STAGES) { s = 0; phase ^= 1; }
                         if (--left == 0) { left = inner; b ^= 1; if (++kw == p.KW) { kw = 0; b = p.PL & 1; } }
                     }
                     continue;
                 }
+                if (HALO) {
+                    const uint32_t row_step = (uint32_t)(p.DH * p.Wt * KS * 2) >> 4, col_step = (uint32_t)(p.DW * KS * 2) >> 4;
+                    for (int k = 0; k < n_k && ok; ++k) {
+                        ok = warp_wait_bounded(halo_full + 8 * hs, hphase, status, ST_G_MMA);
+                        if (!ok) break;
+                        const uint64_t bd = make_desc_kmajor_sw64_groups(halo_addr + hs * p.halo_bytes, p.Wt * KS * 2);
+                        const uint32_t b_hi = (uint32_t)(bd >> 32);
+                        uint32_t b_row = (uint32_t)bd, b_tap = b_row;
+                        int kw = 0;
+                        for (int tap = 0; tap < taps && ok; tap += p.a_taps) {
+                            ok = warp_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA);
+                            if (!ok) break;
+                            tc_fence_after_sync();
+                            const uint64_t ad = make_desc_kmajor_rows<KS>(tiles_addr + s * STAGE);
+                            if (el) {
+                                uint32_t a_lo = (uint32_t)ad, b_lo = b_tap;
+                                const uint32_t a_hi = (uint32_t)(ad >> 32);
+                                for (int i = 0; i < p.a_taps; ++i) {
+#pragma unroll
+                                    for (int j = 0; j < KS / 16; ++j)
+                                        mma_f16_ss_words(d_tmem, a_lo + 2 * j, a_hi, b_lo + 2 * j, b_hi, idesc, (k > 0 || tap + i > 0 || j > 0) ? 1u : 0u);
+                                    a_lo += A_BYTES >> 4;
+                                    b_lo += col_step;
+                                }
+                                mma_commit(empty_bar + 8 * s);
+                            }
+                            // (a slot's taps lie in one filter row)
+                            if ((kw += p.a_taps) == p.KW) { kw = 0; b_row += row_step; b_tap = b_row; } else b_tap += col_step;
+                            if (++s == STAGES) { s = 0; phase ^= 1; }
+                        }
+                        if (el) {
+                            mma_commit(halo_empty + 8 * hs);
+                            if (k == n_k - 1) mma_commit(tmem_full + 8 * buf);
+                        }
+                        if (++hs == p.n_stages) { hs = 0; hphase ^= 1; }
+                    }
+                    continue;
+                }
                 for (int k = 0; k < n_k && ok; ++k) {
-                    ok = mbar_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA);
+                    ok = warp_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    const uint32_t a_addr = tiles_addr + s * STAGE, b_addr = a_addr + (HALO ? taps * A_BYTES : A_BYTES);
-                    const uint64_t ad = make_desc_kmajor_rows<KS>(a_addr);
-                    const uint32_t a_lo = (uint32_t)ad, a_hi = (uint32_t)(ad >> 32);
-                    if (HALO) {
-                        const uint64_t bd = make_desc_kmajor_sw64_groups(b_addr, p.Wt * KS * 2);
-                        const uint32_t b_lo = (uint32_t)bd, b_hi = (uint32_t)(bd >> 32);
-                        const uint32_t row_step = (uint32_t)(p.DH * p.Wt * KS * 2) >> 4, col_step = (uint32_t)(p.DW * KS * 2) >> 4;
-                        uint32_t a_tap = a_lo, b_row = b_lo, b_tap = b_lo;
-                        int kw = 0;
-                        for (int tap = 0; tap < taps; ++tap) {
-#pragma unroll
-                            for (int j = 0; j < KS / 16; ++j)
-                                mma_f16_ss_words(d_tmem, a_tap + 2 * j, a_hi, b_tap + 2 * j, b_hi, idesc, (k > 0 || tap > 0 || j > 0) ? 1u : 0u);
-                            a_tap += A_BYTES >> 4;
-                            if (++kw == p.KW) { kw = 0; b_row += row_step; b_tap = b_row; } else b_tap += col_step;
-                        }
-                    } else {
-                        const uint64_t bd = make_desc_kmajor_rows<KS>(b_addr);
-                        const uint32_t b_lo = (uint32_t)bd, b_hi = (uint32_t)(bd >> 32);
+                    const uint32_t a_addr = tiles_addr + s * STAGE;
+                    const uint64_t ad = make_desc_kmajor_rows<KS>(a_addr), bd = make_desc_kmajor_rows<KS>(a_addr + A_BYTES);
+                    const uint32_t a_lo = (uint32_t)ad, a_hi = (uint32_t)(ad >> 32), b_lo = (uint32_t)bd, b_hi = (uint32_t)(bd >> 32);
+                    if (el) {
 #pragma unroll
                         for (int j = 0; j < KS / 16; ++j)
                             mma_f16_ss_words(d_tmem, a_lo + 2 * j, a_hi, b_lo + 2 * j, b_hi, idesc, (k > 0 || j > 0) ? 1u : 0u);
+                        mma_commit(empty_bar + 8 * s);
+                        if (k == n_k - 1) mma_commit(tmem_full + 8 * buf);
                     }
-                    mma_commit(empty_bar + 8 * s);
-                    if (k == n_k - 1) mma_commit(tmem_full + 8 * buf);
                     if (++s == STAGES) { s = 0; phase ^= 1; }
                 }
             }
@@ -1056,7 +1106,8 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
     chain_next();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
+            const bool el = elect_one();
             // one copy per operand and stage (the staged tensors keep the channel-block index outermost, so the blocks of
             // a tile are one box even across components), and a running (tw, th, tn) of the pixel box: the thread that
             // issues the copies runs no division in this loop -- at a few hundred cycles per copy it used to bound the kernel
@@ -1064,27 +1115,30 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
             int s = 0, phase = 1;
             bool ok = true;
             for (int it = 0; it < n_steps && ok; ++it) {
-                ok = mbar_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+                ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
                 if (!ok) break;
                 const int ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
                 const uint32_t a_dst = tiles_addr + s * F_STAGE, b_dst = a_dst + GM * FK * 2, bar = full_bar + 8 * s;
                 if (++tw == p.tiles_w) { tw = 0; if (++th == p.tiles_h) { th = 0; ++tn; } }
                 if (++s == F_STAGES) { s = 0; phase ^= 1; }
-                mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
-                tma_load_5d(a_dst, &map_dy, 0, ow0, oh0, n0, blockA0, bar);
-                tma_load_5d(b_dst, &map_x, 0, ow0 * p.SW + kw * p.DW + p.off_w, oh0 * p.SH + kh * p.DH + p.off_h, n0, blockB0, bar);
+                if (el) {
+                    mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
+                    tma_load_5d(a_dst, &map_dy, 0, ow0, oh0, n0, blockA0, bar);
+                    tma_load_5d(b_dst, &map_x, 0, ow0 * p.SW + kw * p.DW + p.off_w, oh0 * p.SH + kh * p.DH + p.off_h, n0, blockB0, bar);
+                }
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         const uint32_t idesc = make_idesc_f16(p.fmt, GM, p.n_tile_cols, true, true);
         bool ok = true;
+        const bool el = elect_one();
         for (int it = 0; it < n_steps && ok; ++it) {
             const int s = it % F_STAGES;
-            ok = mbar_wait_bounded(full_bar + 8 * s, (it / F_STAGES) & 1, status, ST_G_MMA);
+            ok = warp_wait_bounded(full_bar + 8 * s, (it / F_STAGES) & 1, status, ST_G_MMA);
             if (!ok) break;
             tc_fence_after_sync();
-            if (lane == 0) {
+            if (el) {
                 const uint32_t a_addr = tiles_addr + s * F_STAGE, b_addr = a_addr + GM * FK * 2;
                 // consecutive MMAs alternate between two accumulators (summed by the epilogue): back-to-back MMAs into one
                 // accumulator run at about two thirds of the rate of independent ones
@@ -1192,7 +1246,8 @@ qconv_filter_xmajor_tc_kernel(const __grid_constant__ CUtensorMap map_x, const _
     chain_next();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
+            const bool el = elect_one();
             // per-tap offsets of the x boxes and the running (tw, th, tn) of the pixel box: no division in the loop
             int w_ofs[8], h_ofs[8], comp[8];
             for (int tl = 0; tl < p.TPG && tl < 8; ++tl) {
@@ -1205,28 +1260,31 @@ qconv_filter_xmajor_tc_kernel(const __grid_constant__ CUtensorMap map_x, const _
             int s = 0, phase = 1;
             bool ok = true;
             for (int it = 0; it < n_steps && ok; ++it) {
-                ok = mbar_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+                ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
                 if (!ok) break;
                 const int ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
                 const uint32_t a_dst = tiles_addr + s * F_STAGE, b_dst = a_dst + GM * FK * 2, bar = full_bar + 8 * s;
                 if (++tw == p.tiles_w) { tw = 0; if (++th == p.tiles_h) { th = 0; ++tn; } }
                 if (++s == F_STAGES) { s = 0; phase ^= 1; }
-                mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
-                for (int tl = 0; tl < p.TPG; ++tl)
-                    tma_load_5d(a_dst + tl * tap_bytes, &map_x, 0, ow0 * p.SW + w_ofs[tl] + p.off_w, oh0 * p.SH + h_ofs[tl] + p.off_h, n0, comp[tl], bar);
-                tma_load_5d(b_dst, &map_dy, 0, ow0, oh0, n0, 0, bar);
+                if (el) {
+                    mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
+                    for (int tl = 0; tl < p.TPG; ++tl)
+                        tma_load_5d(a_dst + tl * tap_bytes, &map_x, 0, ow0 * p.SW + w_ofs[tl] + p.off_w, oh0 * p.SH + h_ofs[tl] + p.off_h, n0, comp[tl], bar);
+                    tma_load_5d(b_dst, &map_dy, 0, ow0, oh0, n0, 0, bar);
+                }
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         const uint32_t idesc = make_idesc_f16(p.fmt, GM, n_cols, true, true);
         bool ok = true;
+        const bool el = elect_one();
         for (int it = 0; it < n_steps && ok; ++it) {
             const int s = it % F_STAGES;
-            ok = mbar_wait_bounded(full_bar + 8 * s, (it / F_STAGES) & 1, status, ST_G_MMA);
+            ok = warp_wait_bounded(full_bar + 8 * s, (it / F_STAGES) & 1, status, ST_G_MMA);
             if (!ok) break;
             tc_fence_after_sync();
-            if (lane == 0) {
+            if (el) {
                 const uint32_t a_addr = tiles_addr + s * F_STAGE, b_addr = a_addr + GM * FK * 2;
 #pragma unroll
                 for (int j = 0; j < FK / 16; ++j)           // two accumulators in turn, as in the general kernel
@@ -1469,17 +1527,24 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     const bool unaligned_rows = g.plain && p.store_vec < 8;
     const int epi_bytes = cl32 ? CL32_BYTES : (unaligned_rows ? ROWS_BYTES : 0);
     bool halo = false;
-    p.n_cols = 256; p.Wt = p.Ht = 0; p.n_stages = 0; p.stage_bytes = 0;
+    p.n_cols = 256; p.Wt = p.Ht = 0; p.n_stages = 0; p.stage_bytes = 0; p.a_slots = 0; p.a_taps = 1; p.halo_bytes = 0;
     if (!pl.dual && pl.Cp % 32 == 0 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
         const int rows = (pl.Hout + 31) / 32;
         const int ph = (((pl.Hout + rows - 1) / rows) + 1) & ~1;
         const int wt = 8 + (g.KW - 1) * g.DW, ht = ph + (g.KH - 1) * g.DH;
-        const uint32_t stage = ((uint32_t)taps * GM * 32 * 2 + (uint32_t)wt * ht * 64 + 1023) / 1024 * 1024;
-        const int n_stages = (int)((227 * 1024 - 1024 - 512 - epi_bytes) / stage);
-        if (ph >= 24 && wt <= 256 && ht <= 256 && taps <= 256 && n_stages >= 2) {
+        const uint32_t tile = ((uint32_t)wt * ht * 64 + 1023) / 1024 * 1024, tap_bytes = GM * 32 * 2;
+        const int room = 227 * 1024 - 1024 - 512 - epi_bytes;
+        // a slot of the filter ring holds a filter row where at least four of those fit beside two halo tiles, one tap otherwise
+        p.a_taps = room >= (int)(2 * tile + 4 * g.KW * tap_bytes) ? g.KW : 1;
+        const int slot = p.a_taps * (int)tap_bytes;
+        if (ph >= 24 && wt <= 256 && ht <= 256 && room >= (int)(2 * tile) + 4 * slot) {
             halo = true;
             p.PW = 8; p.PH = ph; p.PN = 1; p.n_cols = 8 * ph; p.Wt = wt; p.Ht = ht;
-            p.n_stages = n_stages > 8 ? 8 : n_stages; p.stage_bytes = stage;
+            p.halo_bytes = tile;
+            p.n_stages = room >= (int)(H_MAX_TILES * tile) + 6 * slot ? H_MAX_TILES : 2;
+            p.a_slots = (room - p.n_stages * (int)tile) / slot;
+            if (p.a_slots > H_MAX_SLOTS) p.a_slots = H_MAX_SLOTS;
+            p.stage_bytes = 0;
         }
     }
     {
@@ -1539,7 +1604,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     {
         const cuuint64_t dims[3] = {(cuuint64_t)pl.Kp, (cuuint64_t)pl.Mp, (cuuint64_t)taps};
         const cuuint64_t strides[2] = {(cuuint64_t)pl.Kp * 2, (cuuint64_t)pl.Mp * pl.Kp * 2};
-        const cuuint32_t box[3] = {(cuuint32_t)ks, GM, (cuuint32_t)(halo ? taps : 1)};
+        const cuuint32_t box[3] = {(cuuint32_t)ks, GM, (cuuint32_t)(halo ? p.a_taps : 1)};
         const cuuint32_t es[3] = {1, 1, 1};
         const CUresult r = encode(&map_w, dt, 3, wexp, dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1561,7 +1626,8 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
 
     const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * (pl.dual ? 2 : 1);
     const int grid = n_tiles < sm_count() ? n_tiles : sm_count();
-    size_t smem = 1024 + (size_t)p.n_stages * p.stage_bytes + 512 + tail_bytes;
+    const size_t operand_bytes = halo ? (size_t)p.a_slots * p.a_taps * GM * 64 + (size_t)p.n_stages * p.halo_bytes : (size_t)p.n_stages * p.stage_bytes;
+    size_t smem = 1024 + operand_bytes + 512 + tail_bytes;
     if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
     auto run = [&](auto* kernel) -> int {
         PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
