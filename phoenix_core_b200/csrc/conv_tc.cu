@@ -1037,6 +1037,8 @@ constexpr int FK = 64;                               // pixels per stage
 constexpr int F_STAGES = 4;
 constexpr uint32_t F_STAGE = (GM + GN) * FK * 2;     // 48 KB
 constexpr size_t FG_SMEM = 1024 + F_STAGES * F_STAGE + 512;
+constexpr int FP_STAGES = 6;                         // pairs of SMs: half of the N columns in each CTA
+constexpr uint32_t FP_STAGE = (GM + GN / 2) * FK * 2;
 
 struct FGParams {
     int Nb, Co, Ci, HO, WO;
@@ -1062,23 +1064,31 @@ __device__ __forceinline__ uint64_t make_desc_mn_blocks(uint32_t smem_addr, int 
            ((uint64_t)(((8u * cb * 2u) >> 4) & 0x3FFFu) << 32) | DESC_VERSION_SM100 | (layout << 61);
 }
 
+// PAIR: a cluster of two CTAs takes a 256-row M tile (128 rows each) and half of the N columns each; per SM 32 KB instead of 48 KB come
+// from L2 for every four MMAs of 512 clocks (an SM takes in about 64 bytes per clock). Forward + backward, before / after: 3x3 64 at 56,
+// channels-last, batch 128 1199 / 1164 us; 3x3 stride 2, 128 at 28 578 / 565; 1x1 256 at 14 304 / 295.
+template <bool PAIR>
 __global__ void __launch_bounds__(G_THREADS, 1)
 qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_constant__ CUtensorMap map_x, FGParams p,
                                float* __restrict__ dw32, int* __restrict__ status) {
+    constexpr int STAGES = PAIR ? FP_STAGES : F_STAGES;
+    constexpr uint32_t STAGE = PAIR ? FP_STAGE : F_STAGE;
     extern __shared__ uint8_t smem_raw[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
+    const int rank = PAIR ? (int)cluster_ctarank() : 0;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(base + F_STAGES * F_STAGE);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * F_STAGES + 1);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + STAGES * STAGE);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 1);
     const uint32_t tiles_addr = smem_u32(base);
-    const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + F_STAGES), tmem_full = smem_u32(bars + 2 * F_STAGES);
+    const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + STAGES), tmem_full = smem_u32(bars + 2 * STAGES);
 
-    // work item of this CTA
+    // work item of this CTA (pair)
     // items (tap, tiles) vary fastest so that the CTAs running at the same time read the same pixel slice (L2 reuse)
-    const int n_items = p.m_tiles * p.n_tiles * p.KH * p.KW;
-    int item = blockIdx.x % n_items;
-    const int split = blockIdx.x / n_items;
-    const int mt = item % p.m_tiles; item /= p.m_tiles;
+    const int m_tiles = PAIR ? p.m_tiles / 2 : p.m_tiles;
+    const int n_items = m_tiles * p.n_tiles * p.KH * p.KW, id = PAIR ? blockIdx.x / 2 : blockIdx.x;
+    int item = id % n_items;
+    const int split = id / n_items;
+    const int mt = PAIR ? 2 * (item % m_tiles) + rank : item % m_tiles; item /= m_tiles;
     const int nt = item % p.n_tiles;
     const int tap = item / p.n_tiles;
     const int kh = tap / p.KW, kw = tap - kh * p.KW;
@@ -1086,72 +1096,89 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
     const int step_beg = split * p.steps_per_split;
     const int n_steps = max(0, min(steps_total, step_beg + p.steps_per_split) - step_beg);
 
-    const int nblkA = GM / p.cbA, nblkB = p.n_tile_cols / p.cbB;
+    const int nblkA = GM / p.cbA, nblkB = p.n_tile_cols / p.cbB / (PAIR ? 2 : 1);        // blocks of this CTA's shared memory
     const int bpcA = p.Cop / p.cbA, bpcB = p.Cip / p.cbB;               // channel blocks per component
     const uint32_t blkA_bytes = FK * p.cbA * 2, blkB_bytes = FK * p.cbB * 2;
     const uint32_t a_bytes = nblkA * blkA_bytes, b_bytes = nblkB * blkB_bytes;
     const int blockA0 = mt * nblkA, blockB0 = nt * (GN / p.cbB);
 
     if (t == 0) {
-        for (int s = 0; s < F_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
         mbar_init(tmem_full, 1);
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
+    if (warp == 1) { if (PAIR) tmem_alloc_pair(smem_u32(tmem_slot), 512); else tmem_alloc(smem_u32(tmem_slot), 512); }
     tc_fence_before_sync();
     __syncthreads();
+    if (PAIR) cluster_sync_all();                     // both CTAs' barriers exist before anything signals them
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     chain_wait();
     chain_next();
 
     if (warp == 0) {
-        {
-            const bool el = elect_one();
-            // one copy per operand and stage (the staged tensors keep the channel-block index outermost, so the blocks of
-            // a tile are one box even across components), and a running (tw, th, tn) of the pixel box: the thread that
-            // issues the copies runs no division in this loop -- at a few hundred cycles per copy it used to bound the kernel
-            int tw = step_beg % p.tiles_w, th = (step_beg / p.tiles_w) % p.tiles_h, tn = step_beg / (p.tiles_w * p.tiles_h);
-            int s = 0, phase = 1;
-            bool ok = true;
-            for (int it = 0; it < n_steps && ok; ++it) {
-                ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
-                if (!ok) break;
+        // one copy per operand and stage (the staged tensors keep the channel-block index outermost, so the blocks of
+        // a tile are one box even across components), and a running (tw, th, tn) of the pixel box: the thread that
+        // issues the copies runs no division in this loop -- at a few hundred cycles per copy it used to bound the kernel
+        const bool el = elect_one();
+        int tw = step_beg % p.tiles_w, th = (step_beg / p.tiles_w) % p.tiles_h, tn = step_beg / (p.tiles_w * p.tiles_h);
+        int s = 0, phase = 1;
+        bool ok = true;
+        for (int it = 0; it < n_steps; ++it) {
+            ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
+            if (!ok) break;
+            if (el) {
                 const int ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
-                const uint32_t a_dst = tiles_addr + s * F_STAGE, b_dst = a_dst + GM * FK * 2, bar = full_bar + 8 * s;
-                if (++tw == p.tiles_w) { tw = 0; if (++th == p.tiles_h) { th = 0; ++tn; } }
-                if (++s == F_STAGES) { s = 0; phase ^= 1; }
-                if (el) {
+                const int wx = ow0 * p.SW + kw * p.DW + p.off_w, hx = oh0 * p.SH + kh * p.DH + p.off_h;
+                const uint32_t a_dst = tiles_addr + s * STAGE, b_dst = a_dst + GM * FK * 2, bar = full_bar + 8 * s;
+                if (PAIR) {
+                    const uint32_t lead = map_to_cta(bar, 0);
+                    if (rank == 0) mbar_arrive_expect_tx(bar, 2 * (a_bytes + b_bytes));
+                    tma_load_5d_pair(a_dst, &map_dy, 0, ow0, oh0, n0, blockA0, lead);
+                    tma_load_5d_pair(b_dst, &map_x, 0, wx, hx, n0, blockB0 + rank * nblkB, lead);
+                } else {
                     mbar_arrive_expect_tx(bar, a_bytes + b_bytes);
                     tma_load_5d(a_dst, &map_dy, 0, ow0, oh0, n0, blockA0, bar);
-                    tma_load_5d(b_dst, &map_x, 0, ow0 * p.SW + kw * p.DW + p.off_w, oh0 * p.SH + kh * p.DH + p.off_h, n0, blockB0, bar);
+                    tma_load_5d(b_dst, &map_x, 0, wx, hx, n0, blockB0, bar);
                 }
             }
+            if (++tw == p.tiles_w) { tw = 0; if (++th == p.tiles_h) { th = 0; ++tn; } }
+            if (++s == STAGES) { s = 0; phase ^= 1; }
         }
         __syncwarp();
     } else if (warp == 1) {
-        const uint32_t idesc = make_idesc_f16(p.fmt, GM, p.n_tile_cols, true, true);
-        bool ok = true;
-        const bool el = elect_one();
-        for (int it = 0; it < n_steps && ok; ++it) {
-            const int s = it % F_STAGES;
-            ok = warp_wait_bounded(full_bar + 8 * s, (it / F_STAGES) & 1, status, ST_G_MMA);
-            if (!ok) break;
-            tc_fence_after_sync();
-            if (el) {
-                const uint32_t a_addr = tiles_addr + s * F_STAGE, b_addr = a_addr + GM * FK * 2;
-                // consecutive MMAs alternate between two accumulators (summed by the epilogue): back-to-back MMAs into one
-                // accumulator run at about two thirds of the rate of independent ones
+        if (rank == 0) {
+            const uint32_t idesc = make_idesc_f16(p.fmt, PAIR ? 2 * GM : GM, p.n_tile_cols, true, true);
+            const uint32_t peer_empty = PAIR ? map_to_cta(empty_bar, 1) : 0u, peer_full = PAIR ? map_to_cta(tmem_full, 1) : 0u;
+            const bool el = elect_one();
+            int s = 0, phase = 0;
+            for (int it = 0; it < n_steps; ++it) {
+                if (!warp_wait_bounded(full_bar + 8 * s, phase, status, ST_G_MMA)) break;
+                tc_fence_after_sync();
+                if (el) {
+                    const uint32_t a_addr = tiles_addr + s * STAGE;
+                    const uint64_t ad = make_desc_mn_blocks(a_addr, p.cbA, blkA_bytes), bd = make_desc_mn_blocks(a_addr + GM * FK * 2, p.cbB, blkB_bytes);
+                    const uint32_t a_step = (16u * p.cbA * 2u) >> 4, b_step = (16u * p.cbB * 2u) >> 4;
 #pragma unroll
-                for (int j = 0; j < FK / 16; ++j)
-                    mma_f16_ss(tmem_base + (j & 1) * GN, make_desc_mn_blocks(a_addr + j * 16 * p.cbA * 2, p.cbA, blkA_bytes),
-                               make_desc_mn_blocks(b_addr + j * 16 * p.cbB * 2, p.cbB, blkB_bytes), idesc, (it > 0 || j > 1) ? 1u : 0u);
-                mma_commit(empty_bar + 8 * s);
-                if (it == n_steps - 1) mma_commit(tmem_full);
+                    for (int j = 0; j < FK / 16; ++j) {
+                        // two accumulators in turn: an MMA truncates when it adds (conv_tf32.cu), so half as many in each is half the error
+                        const uint32_t al = (uint32_t)ad + j * a_step, bl = (uint32_t)bd + j * b_step, acc = (it > 0 || j > 1) ? 1u : 0u, dst = tmem_base + (j & 1) * GN;
+                        if (PAIR) mma_f16_pair(dst, al, (uint32_t)(ad >> 32), bl, (uint32_t)(bd >> 32), idesc, acc);
+                        else mma_f16_ss_words(dst, al, (uint32_t)(ad >> 32), bl, (uint32_t)(bd >> 32), idesc, acc);
+                    }
+                    if (PAIR) {
+                        mma_commit_pair(empty_bar + 8 * s);
+                        mma_commit_pair(peer_empty + 8 * s);
+                        if (it == n_steps - 1) { mma_commit_pair(tmem_full); mma_commit_pair(peer_full); }
+                    } else {
+                        mma_commit(empty_bar + 8 * s);
+                        if (it == n_steps - 1) mma_commit(tmem_full);
+                    }
+                }
+                if (++s == STAGES) { s = 0; phase ^= 1; }
             }
-            __syncwarp();
+            if (n_steps == 0 && el) { mbar_arrive(tmem_full); if (PAIR) mbar_arrive_cluster(peer_full); }
         }
-        if (n_steps == 0 && lane == 0) mbar_arrive(tmem_full);
         __syncwarp();
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
@@ -1201,7 +1228,8 @@ qconv_filter_general_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, 512);
+    if (PAIR) cluster_sync_all();                     // nobody leaves while its peer may still signal its barriers or read its shared memory
+    if (warp == 1) { if (PAIR) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512); }
 }
 
 // ---------------------------------------------------------------------------------------------------
@@ -1774,8 +1802,9 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     const bool xmajor = filter_xmajor(g, f);
     p.TPG = xmajor ? GM / (p.LK * p.cbB) : 1;
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
-    const int items = xmajor ? (taps + p.TPG - 1) / p.TPG : taps * p.m_tiles * p.n_tiles;
-    int splits = split_count(items, sm_count());
+    const bool pair = !xmajor && p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0;
+    const int items = xmajor ? (taps + p.TPG - 1) / p.TPG : taps * p.m_tiles * p.n_tiles / (pair ? 2 : 1);
+    int splits = split_count(items, pair ? sm_count() / 2 : sm_count());
     if (splits > steps_total) splits = steps_total;
     if (splits < 1) splits = 1;
     p.steps_per_split = (steps_total + splits - 1) / splits;
@@ -1811,7 +1840,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
         const cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)Wd * Cd * 2, (cuuint64_t)Hd * Wd * Cd * 2,
                                        (cuuint64_t)g.Nb * Hd * Wd * Cd * 2};
         const cuuint32_t box[5] = {(cuuint32_t)p.cbB, (cuuint32_t)((p.PW - 1) * g.SW + 1), (cuuint32_t)((p.PH - 1) * g.SH + 1), (cuuint32_t)p.PN,
-                                   (cuuint32_t)(xmajor ? p.LK : p.n_tile_cols / p.cbB)};
+                                   (cuuint32_t)(xmajor ? p.LK : p.n_tile_cols / p.cbB / (pair ? 2 : 1))};
         const cuuint32_t es[5] = {1, (cuuint32_t)g.SW, (cuuint32_t)g.SH, 1, 1};
         const CUresult r = encode(&map_x, dt, 5, direct_x ? const_cast<void*>(x) : static_cast<void*>(xp), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, swz(p.cbB),
                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
@@ -1821,8 +1850,9 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
         PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_xmajor_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG_SMEM));
         PCB_CUDA_TRY(launch_chained_if(chain, qconv_filter_xmajor_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_x, map_dy, p, acc, status));
     } else {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_general_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG_SMEM));
-        PCB_CUDA_TRY(launch_chained_if(chain, qconv_filter_general_tc_kernel, items * p.splits, G_THREADS, FG_SMEM, stream, map_dy, map_x, p, acc, status));
+        auto* kernel = pair ? qconv_filter_general_tc_kernel<true> : qconv_filter_general_tc_kernel<false>;
+        PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)FG_SMEM));
+        PCB_CUDA_TRY(launch_clusters(pair ? 2 : 1, chain, kernel, items * p.splits * (pair ? 2 : 1), G_THREADS, FG_SMEM, stream, map_dy, map_x, p, acc, status));
     }
     PCB_CUDA_TRY(cudaGetLastError());
     const size_t per_tap = (size_t)g.nc * g.Co * g.Ci, total = per_tap * taps;

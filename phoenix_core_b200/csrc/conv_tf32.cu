@@ -1,15 +1,17 @@
-// fp32 quaternion convolution and dense on the tensor cores with error-compensated TF32 ("3xTF32").
+// fp32 quaternion convolution and dense on the tensor cores: hi * hi in TF32, the cross terms in bf16.
 //
 // tcgen05.mma.kind::tf32 keeps 10 mantissa bits of each fp32 operand, far from the 1e-5 parity the fp32 path
-// owes. Every operand is therefore split while it is staged into hi = x with the 13 low mantissa bits cleared
-// (exactly a TF32 number) and lo = x - hi (exact in fp32), and each K step issues three MMAs into the same fp32
-// accumulator: hi*hi + hi*lo + lo*hi. What is dropped is lo*lo and the rounding of lo (both ~2^-22 relative), so
-// the result is as good as an fp32 FMA chain. Cost: 3 TF32 MMAs per product and twice the operand bytes.
+// owes. Every operand is therefore split while it is staged into hi, x rounded to a TF32 number, and lo = x - hi
+// (exact, at most 2^-11 of x), and a product is hi*hi (TF32) + lo*x + x*lo, the latter with both factors rounded to bf16, which has the
+// exponents of fp32: an error of 2^-9 in a term of 2^-11 or less. Two MMAs of 8 and two of 16 K elements per 16 K elements, where all
+// three products in TF32 (lo too kept as a TF32 number, hi cut off) took six. Against 64 bits, 2-norm of the difference over that of the result,
+// TF32 alone / this: 3x3, 16 channels, 32 x 32, forward 1.3e-6 / 9.6e-7; 3x3, 128 channels, 28 x 28, batch 128, all three passes 2.1e-6 /
+// 1.4e-6 (less than before: the accumulators of hi*hi take a third of the MMAs, whose additions truncate).
 //
 // Structure as in conv_tc.cu: channels-last activations (not padded: the zero fill of the tensor maps is
 // the padding) and the signed/permuted filter matrix
 // Wexp[tap][(d,co)][(l,ci)] (reference sign table src/algebras.cc:28-49) are staged in the workspace, here in fp32
-// and twice (hi, lo); the implicit-GEMM kernel is TMA-fed, 128 x 256 tile, double-buffered TMEM accumulator.
+// (hi) and as pairs of bf16 (x and lo); the implicit-GEMM kernel is TMA-fed, 128 x 256 tile.
 // Dense layers are the 1x1 convolution of 1x1 images (pixels = batch); input-major dense filters and the
 // input-major dense filter gradient are handled while staging / unstaging. Replaces, for fp32 tensors, the scalar
 // fp32 library calls of src/backend/cudnn/conv2d.hpp:280-309, :447-488 and src/backend/cudnn/dense.hpp:102-133, :181-216.
@@ -27,6 +29,7 @@ constexpr int T_THREADS = 320;
 constexpr uint32_t TA_BYTES = TM * TKS * 4, TB_BYTES = TN * TKS * 4;
 constexpr uint32_t T_STAGE = 2 * (TA_BYTES + TB_BYTES);     // hi and lo of both operands: 48 KB
 constexpr int T_STAGES = 4;
+constexpr int T_MAX_SLOTS = 10, T_HALO_TILES = 2;           // halo form: filter slices and halo tiles in flight
 constexpr size_t T_SMEM = 1024 + T_STAGES * T_STAGE + 512;
 constexpr int ST_T_PRODUCER = 0x1000, ST_T_MMA = 0x2000, ST_T_EPILOGUE = 0x4000;
 
@@ -36,46 +39,62 @@ struct TParams {
     int PW, PH, PN;
     int tiles_w, tiles_h, tiles_n, tiles_m;
     int has_bias, LK, store_vec;
-    int n_cols;                       // pixels of a tile: 256, or 128 where few tiles leave most SMs idle
+    int n_cols;                       // pixels of a tile: 256, 128 where few tiles leave most SMs idle, 8 * PH in halo form
     int n_chunks, chunk_len;          // a work item's K range runs in n_chunks pieces of at most chunk_len stages
     int off_w, off_h;                 // added to the pixel coordinates of every activation box: minus the padding; 0 for a zero-inserted copy
     int rows_epi;                     // image rows not a multiple of 8 pixels: stored through shared memory (store_rows_f32)
     int splits, k_per_split;          // the K loop of a tile is cut into `splits` work items of k_per_split stages; with more than one
                                       // the partial results meet in the (zeroed) output by fp32 reductions
+    int Wt, Ht, a_slots;              // halo form: halo tile, filter slices in flight
+    uint32_t halo_bytes;              // halo form: shared-memory pitch of the hi (and of the lo) part of a halo tile
 };
 
-// K-major tile with 64-byte rows (16 fp32), 64-byte swizzle.
-__device__ __forceinline__ uint64_t desc_k64(uint32_t addr) {
-    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | DESC_VERSION_SM100 | (4ull << 61);
+// K-major tile with 64-byte rows, 64-byte swizzle, groups of 8 rows `group_bytes` apart (512, or the row pitch of a halo tile).
+__device__ __forceinline__ uint64_t desc_k64(uint32_t addr, uint32_t group_bytes = 512) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)((group_bytes >> 4) & 0x3FFFu) << 32) | DESC_VERSION_SM100 | (4ull << 61);
 }
 
 // Each MMA truncates when it adds into the TMEM accumulator, so the error of one accumulator grows with the number
 // of MMAs it takes (measured: about 3e-8 of the largest output per MMA). K loops are therefore cut into chunks of
-// at most T_CHUNK stages; chunks alternate between the two TMEM buffers (as whole tiles do when one chunk is
-// enough) and the epilogue warps add them up in registers, rounding to nearest.
-constexpr int T_CHUNK = 16;           // 16 stages = 96 MMAs = 256 fp32 of K
+// at most T_CHUNK stages; the epilogue warps add the chunks' sums of hi * hi up in registers, rounding to nearest. The sums of the
+// cross terms, 2^-11 of the size, stay in an accumulator of their own for the whole K loop.
+// Tensor memory: tiles of up to 128 columns have two accumulators of each kind, and the drain of one chunk overlaps the MMAs of the
+// next; wider tiles have one of each.
+constexpr int T_SPLIT = 16;           // fewest stages of a work item
+constexpr int T_CHUNK = 32;           // 32 stages = 64 MMAs of hi * hi = 512 fp32 of K
 
-template <bool CHUNKED>
+// HALO (stride-1 correlation, tile = 8 x PH pixels of one image): as in conv_tc.cu, the halo tile of 16 channels is loaded once and every
+// tap's MMAs read it at a shifted start address; the filter slices have a ring of their own. 20 KB instead of 48 KB from L2 per four MMAs of
+// 128 x 224: the four take 448 clocks, and an SM takes in about 64 bytes per clock. 3x3, 128 channels, 28 x 28, batch 128, forward: 2012 ->
+// 1580 us (first 20 launches), 2277 -> 1815 us under the power limit, of which 105 us are the staging.
+template <bool CHUNKED, bool HALO>
 __global__ void __launch_bounds__(T_THREADS, 1)
 qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __grid_constant__ CUtensorMap map_w_lo,
                           const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo, TParams p,
                           const float* bias, float* __restrict__ out, int* __restrict__ status) {
+    constexpr int MAX_SLOTS = HALO ? T_MAX_SLOTS : T_STAGES;
+    constexpr uint32_t SLOT = HALO ? 2 * TA_BYTES : T_STAGE;
+    const int slots = HALO ? p.a_slots : T_STAGES;
     extern __shared__ uint8_t smem_raw[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(base + T_STAGES * T_STAGE);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * T_STAGES + 4);
-    const uint32_t tiles_addr = smem_u32(base);
-    const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + T_STAGES);
-    const uint32_t tmem_full = smem_u32(bars + 2 * T_STAGES), tmem_empty = smem_u32(bars + 2 * T_STAGES + 2);
+    const uint32_t operand_bytes = slots * SLOT + (HALO ? T_HALO_TILES * 2 * p.halo_bytes : 0u);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + operand_bytes);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * MAX_SLOTS + 4 + 2 * T_HALO_TILES);
+    const uint32_t tiles_addr = smem_u32(base), halo_addr = tiles_addr + slots * SLOT;
+    const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + MAX_SLOTS);
+    const uint32_t tmem_full = smem_u32(bars + 2 * MAX_SLOTS), tmem_empty = smem_u32(bars + 2 * MAX_SLOTS + 2);
+    const uint32_t halo_full = smem_u32(bars + 2 * MAX_SLOTS + 4), halo_empty = halo_full + 8 * T_HALO_TILES;
 
     const int n_items = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * p.splits;
-    const int c_steps = p.Cp / TKS;
-    const int n_k = p.KH * p.KW * p.LK * c_steps;
+    const int c_steps = p.Cp / TKS, taps = p.KH * p.KW;
+    const int n_k = taps * p.LK * c_steps;
+    const int bufs = p.n_cols <= 128 ? 2 : 1;          // accumulators of each kind: columns 128 buf and 256 + 128 buf
 
     if (t == 0) {
-        for (int s = 0; s < T_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
+        for (int s = 0; s < MAX_SLOTS; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
         for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, 8); }
+        for (int s = 0; s < T_HALO_TILES; ++s) { mbar_init(halo_full + 8 * s, 1); mbar_init(halo_empty + 8 * s, 1); }
         fence_barrier_init();
     }
     if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
@@ -87,80 +106,125 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
     chain_next();
 
     if (warp == 0) {
-        if (lane == 0) {
-            int it = 0;
-            bool ok = true;
-            for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
-                const int tile = item / p.splits, split = item - tile * p.splits;
-                const int tm = tile % p.tiles_m;
-                int rest = tile / p.tiles_m;
-                const int tw = rest % p.tiles_w; rest /= p.tiles_w;
-                const int th = rest % p.tiles_h;
-                const int tn = rest / p.tiles_h;
-                const int m0 = tm * TM, ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
-                const int k0 = split * p.k_per_split, k1 = min(n_k, k0 + p.k_per_split);
-                // stage k = (tap * LK + l) * c_steps + cs
-                int cs = k0 % c_steps, l = (k0 / c_steps) % p.LK, tap = k0 / (c_steps * p.LK);
-                for (int k = k0; k < k1; ++k, ++it) {
-                    const int kh = tap / p.KW, kw = tap - kh * p.KW;
-                    const int wp0 = ow0 * p.SW + kw * p.DW + p.off_w, hp0 = oh0 * p.SH + kh * p.DH + p.off_h;
-                    const int s = it % T_STAGES;
-                    ok = mbar_wait_bounded(empty_bar + 8 * s, ((it / T_STAGES) & 1) ^ 1, status, ST_T_PRODUCER);
-                    if (!ok) break;
-                    const uint32_t dst = tiles_addr + s * T_STAGE, bar = full_bar + 8 * s;
+        const bool el = elect_one();
+        int s = 0, phase = 1, hs = 0, hphase = 1;
+        bool ok = true;
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+            const int tile = item / p.splits, split = item - tile * p.splits;
+            const int tm = tile % p.tiles_m;
+            int rest = tile / p.tiles_m;
+            const int tw = rest % p.tiles_w; rest /= p.tiles_w;
+            const int th = rest % p.tiles_h;
+            const int tn = rest / p.tiles_h;
+            const int m0 = tm * TM, ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
+            const int k0 = split * p.k_per_split, k1 = min(n_k, k0 + p.k_per_split);
+            if (HALO) {                                  // stage k = (l * c_steps + cs) * taps + tap
+                for (int l = 0; l < p.LK && ok; ++l)
+                    for (int cs = 0; cs < c_steps && ok; ++cs) {
+                        ok = warp_wait_bounded(halo_empty + 8 * hs, hphase, status, ST_T_PRODUCER);
+                        if (!ok) break;
+                        if (el) {
+                            const uint32_t dst = halo_addr + hs * 2 * p.halo_bytes, bar = halo_full + 8 * hs;
+                            mbar_arrive_expect_tx(bar, 2 * (uint32_t)p.Wt * p.Ht * TKS * 4);
+                            tma_load_5d(dst, &map_x_hi, cs * TKS, ow0 + p.off_w, oh0 + p.off_h, n0, l, bar);              // [Ht][Wt][16 channels]
+                            tma_load_5d(dst + p.halo_bytes, &map_x_lo, cs * TKS, ow0 + p.off_w, oh0 + p.off_h, n0, l, bar);
+                        }
+                        if (++hs == T_HALO_TILES) { hs = 0; hphase ^= 1; }
+                        for (int tap = 0; tap < taps; ++tap) {
+                            ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_T_PRODUCER);
+                            if (!ok) break;
+                            if (el) {
+                                const uint32_t dst = tiles_addr + s * SLOT, bar = full_bar + 8 * s;
+                                mbar_arrive_expect_tx(bar, SLOT);
+                                tma_load_3d(dst, &map_w_hi, l * p.Cp + cs * TKS, m0, tap, bar);
+                                tma_load_3d(dst + TA_BYTES, &map_w_lo, l * p.Cp + cs * TKS, m0, tap, bar);
+                            }
+                            if (++s == slots) { s = 0; phase ^= 1; }
+                        }
+                    }
+                continue;
+            }
+            // stage k = (tap * LK + l) * c_steps + cs
+            int cs = k0 % c_steps, l = (k0 / c_steps) % p.LK, tap = k0 / (c_steps * p.LK);
+            for (int k = k0; k < k1; ++k) {
+                const int kh = tap / p.KW, kw = tap - kh * p.KW;
+                const int wp0 = ow0 * p.SW + kw * p.DW + p.off_w, hp0 = oh0 * p.SH + kh * p.DH + p.off_h;
+                ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_T_PRODUCER);
+                if (!ok) break;
+                if (el) {
+                    const uint32_t dst = tiles_addr + s * SLOT, bar = full_bar + 8 * s;
                     mbar_arrive_expect_tx(bar, 2 * (TA_BYTES + (uint32_t)p.n_cols * TKS * 4));
                     tma_load_3d(dst, &map_w_hi, l * p.Cp + cs * TKS, m0, tap, bar);
                     tma_load_3d(dst + TA_BYTES, &map_w_lo, l * p.Cp + cs * TKS, m0, tap, bar);
                     tma_load_5d(dst + 2 * TA_BYTES, &map_x_hi, cs * TKS, wp0, hp0, n0, l, bar);
                     tma_load_5d(dst + 2 * TA_BYTES + TB_BYTES, &map_x_lo, cs * TKS, wp0, hp0, n0, l, bar);
-                    if (++cs == c_steps) { cs = 0; if (++l == p.LK) { l = 0; ++tap; } }
                 }
+                if (++s == slots) { s = 0; phase ^= 1; }
+                if (++cs == c_steps) { cs = 0; if (++l == p.LK) { l = 0; ++tap; } }
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        const uint32_t idesc = make_idesc_f16(2, TM, p.n_cols, false, false);
-        int it = 0, unit = 0;                       // unit = one accumulator's worth of work: a chunk of a tile
+        const bool el = elect_one();
+        const uint32_t idesc_main = make_idesc_f16(2, TM, p.n_cols, false, false), idesc_cross = make_idesc_f16(1, TM, p.n_cols, false, false);
+        const uint32_t row_step = (uint32_t)(p.DH * p.Wt * TKS * 4) >> 4, col_step = (uint32_t)(p.DW * TKS * 4) >> 4;      // HALO
+        int s = 0, phase = 0, hs = 0, hphase = 0, unit = 0, local_item = 0;      // unit = one accumulation of hi * hi: a chunk of a tile
         bool ok = true;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++local_item) {
             const int split = item % p.splits;
             const int k0 = split * p.k_per_split, k1 = min(n_k, k0 + p.k_per_split);
+            const uint32_t d_cross = tmem_base + 256 + (bufs == 2 ? (local_item & 1) * 128 : 0);
+            int tap = 0, kw = 0;
+            uint32_t b_row = 0;                                    // HALO: start-address offset of the tap's filter row
             for (int c = 0; c < p.n_chunks && ok; ++c, ++unit) {
-                const int buf = unit & 1, use = unit >> 1;
+                const int buf = bufs == 2 ? unit & 1 : 0, use = bufs == 2 ? unit >> 1 : unit;
                 if (use > 0) {
-                    ok = mbar_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_T_MMA);
+                    ok = warp_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_T_MMA);
                     if (!ok) break;
                     tc_fence_after_sync();
                 }
+                const uint32_t d_main = tmem_base + buf * 128;
                 const int k_beg = k0 + c * p.chunk_len, k_end = min(k1, k_beg + p.chunk_len);
-                for (int k = k_beg; k < k_end && ok; ++k, ++it) {
-                    const int s = it % T_STAGES;
-                    ok = mbar_wait_bounded(full_bar + 8 * s, (it / T_STAGES) & 1, status, ST_T_MMA);
+                for (int k = k_beg; k < k_end; ++k) {
+                    if (HALO && tap == 0) {
+                        ok = warp_wait_bounded(halo_full + 8 * hs, hphase, status, ST_T_MMA);
+                        if (!ok) break;
+                    }
+                    ok = warp_wait_bounded(full_bar + 8 * s, phase, status, ST_T_MMA);
                     if (!ok) break;
                     tc_fence_after_sync();
-                    if (lane == 0) {
-                        const uint32_t a_hi = tiles_addr + s * T_STAGE, a_lo = a_hi + TA_BYTES, b_hi = a_hi + 2 * TA_BYTES, b_lo = b_hi + TB_BYTES;
-                        const uint32_t d = tmem_base + buf * TN;
+                    if (el) {
+                        const uint32_t a_hi = tiles_addr + s * SLOT, b_hi = HALO ? halo_addr + hs * 2 * p.halo_bytes : a_hi + 2 * TA_BYTES;
+                        const uint64_t ad = desc_k64(a_hi), bd = desc_k64(b_hi, HALO ? p.Wt * TKS * 4 : 512);
+                        const uint32_t a0 = (uint32_t)ad, ah = (uint32_t)(ad >> 32), b0 = (uint32_t)bd + (HALO ? b_row + kw * col_step : 0u), bh = (uint32_t)(bd >> 32);
+                        const uint32_t a1 = a0 + (TA_BYTES >> 4), b1 = b0 + ((HALO ? p.halo_bytes : TB_BYTES) >> 4);
+                        // the rows of the lo parts hold [lo | x] of the filters and [x | lo] of the activations in bf16
 #pragma unroll
-                        for (int j = 0; j < TKS / 8; ++j) {             // 8 fp32 = 32 bytes per MMA along a row
-                            mma_tf32_ss(d, desc_k64(a_lo + j * 32), desc_k64(b_hi + j * 32), idesc, (k > k_beg || j > 0) ? 1u : 0u);   // small terms first
-                            mma_tf32_ss(d, desc_k64(a_hi + j * 32), desc_k64(b_lo + j * 32), idesc, 1u);
-                            mma_tf32_ss(d, desc_k64(a_hi + j * 32), desc_k64(b_hi + j * 32), idesc, 1u);
-                        }
+                        for (int j = 0; j < 2; ++j) mma_f16_ss_words(d_cross, a1 + 2 * j, ah, b1 + 2 * j, bh, idesc_cross, (k > k0 || j > 0) ? 1u : 0u);
+#pragma unroll
+                        for (int j = 0; j < 2; ++j) mma_tf32_ss_words(d_main, a0 + 2 * j, ah, b0 + 2 * j, bh, idesc_main, (k > k_beg || j > 0) ? 1u : 0u);
                         mma_commit(empty_bar + 8 * s);
+                        if (HALO && tap == taps - 1) mma_commit(halo_empty + 8 * hs);
                         if (k == k_end - 1) mma_commit(tmem_full + 8 * buf);
                     }
-                    __syncwarp();
+                    if (++s == slots) { s = 0; phase ^= 1; }
+                    if (HALO) {
+                        if (++kw == p.KW) { kw = 0; b_row += row_step; }
+                        if (++tap == taps) { tap = 0; kw = 0; b_row = 0; if (++hs == T_HALO_TILES) { hs = 0; hphase ^= 1; } }
+                    }
                 }
             }
         }
+        __syncwarp();
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
         const int sv = p.store_vec;                  // pixels per store: 8, 4, 2 or 1
-        int unit = 0;
+        const int half = p.n_cols > 128 ? 128 : p.n_cols / 2;       // columns of a warp: chalf * half and on
+        const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + chalf * half;
+        int unit = 0, local_item = 0;
         bool ok = true;
         const bool reduce = p.splits > 1;            // partial sums of a tile meet in the zeroed output
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++local_item) {
             const int tile = item / p.splits, split = item - tile * p.splits;
             const int tm = tile % p.tiles_m;
             int rest = tile / p.tiles_m;
@@ -172,6 +236,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
             const bool row_ok = m < p.Mvalid;
             const int d = row_ok ? m / p.Cout : 0, co = m - d * p.Cout;
             const float badd = (row_ok && p.has_bias && split == 0) ? ld_chained(bias + d * p.Cout + co) : 0.f;
+            const int cross = 256 + (bufs == 2 ? (local_item & 1) * 128 : 0);
             float part[CHUNKED ? 4 : 1][CHUNKED ? 32 : 1];          // this thread's 128 columns, summed over the chunks so far
             if (CHUNKED) {
 #pragma unroll
@@ -179,7 +244,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
 #pragma unroll
                     for (int e = 0; e < 32; ++e) part[cb][e] = 0.f;
                 for (int c = 0; c + 1 < p.n_chunks && ok; ++c, ++unit) {
-                    const int buf = unit & 1, use = unit >> 1;
+                    const int buf = bufs == 2 ? unit & 1 : 0, use = bufs == 2 ? unit >> 1 : unit;
                     const int seen = read_status(status);
                     ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
                     ok = warp_may_store(ok, seen);
@@ -187,9 +252,9 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                     tc_fence_after_sync();
 #pragma unroll
                     for (int cb = 0; cb < 4; ++cb) {
-                        if (cb * 64 >= p.n_cols) break;
+                        if (cb * 32 >= half || chalf * half + cb * 32 >= p.n_cols) break;
                         uint32_t v[32];
-                        tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * TN + chalf * (p.n_cols / 2) + cb * 32, v);
+                        tmem_ld_32x32b_x32(lane_addr + buf * 128 + cb * 32, v);
                         tmem_ld_wait();
 #pragma unroll
                         for (int e = 0; e < 32; ++e) part[cb][e] += __uint_as_float(v[e]);
@@ -200,7 +265,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                 }
                 if (!ok) break;
             }
-            const int buf = unit & 1, use = unit >> 1;
+            const int buf = bufs == 2 ? unit & 1 : 0, use = bufs == 2 ? unit >> 1 : unit;
             ++unit;
             const int seen = read_status(status);
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
@@ -210,20 +275,32 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
 #pragma unroll(CHUNKED ? 4 : 1)
             for (int cb = 0; cb < 4; ++cb) {
                 uint32_t v[32];
-                if (cb * 64 >= p.n_cols) break;
-                const int col0 = chalf * (p.n_cols / 2) + cb * 32;
-                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * TN + col0, v);
-                tmem_ld_wait();
-                if (!row_ok && !p.rows_epi) continue;
+                const int col0 = chalf * half + cb * 32;
+                if (cb * 32 >= half || col0 >= p.n_cols) break;
+                if (CHUNKED) {
+                    tmem_ld_32x32b_x32(lane_addr + cross + cb * 32, v);
+                    tmem_ld_wait();
 #pragma unroll
-                for (int e = 0; e < 32; ++e)
-                    v[e] = __float_as_uint(__uint_as_float(v[e]) + (CHUNKED ? part[cb][e] : 0.f) + badd);
+                    for (int e = 0; e < 32; ++e) part[cb][e] += __uint_as_float(v[e]);
+                    tmem_ld_32x32b_x32(lane_addr + buf * 128 + cb * 32, v);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + part[cb][e] + badd);
+                } else {
+                    uint32_t u[32];
+                    tmem_ld_32x32b_x32(lane_addr + buf * 128 + cb * 32, v);
+                    tmem_ld_32x32b_x32(lane_addr + cross + cb * 32, u);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + __uint_as_float(u[e]) + badd);
+                }
+                if (!row_ok && !p.rows_epi) continue;
                 if (p.rows_epi) {
-                    const uint32_t rbuf = smem_u32(base) + T_STAGES * T_STAGE + 512 + (uint32_t)(warp - 2) * EPI_ROWS_F32_BYTES;
+                    const uint32_t rbuf = smem_u32(base) + operand_bytes + 512 + (uint32_t)(warp - 2) * EPI_ROWS_F32_BYTES;
                     const int HWo = p.HO * p.WO, je = col0 + (sv == 1 ? lane : (sv == 2 ? (lane & 15) * 2 : (lane & 7) * 4));
                     const int wl = je % p.PW, hl = (je / p.PW) % p.PH, nl = je / (p.PW * p.PH);
                     const int ow = ow0 + wl, oh = oh0 + hl, img = n0 + nl;
-                    const int pix_off = (ow < p.WO && oh < p.HO && img < p.Nb) ? (img * p.Cout * p.HO + oh) * p.WO + ow : -1;
+                    const int pix_off = (je < p.n_cols && ow < p.WO && oh < p.HO && img < p.Nb) ? (img * p.Cout * p.HO + oh) * p.WO + ow : -1;
                     const int row_off = row_ok ? (d * p.Nb * p.Cout + co) * HWo : -1;
                     if (p.Mvalid <= 64) {
                         if (tm * TM + q * 32 >= p.Mvalid) continue;         // (a warp without rows)
@@ -238,6 +315,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
 #pragma unroll
                 for (int g8 = 0; g8 < 4; ++g8) {
                     const int j = col0 + g8 * 8;
+                    if (j >= p.n_cols) continue;
                     const int wl = j % p.PW, hl = (j / p.PW) % p.PH, nl = j / (p.PW * p.PH);
                     const int ow = ow0 + wl, oh = oh0 + hl, img = n0 + nl;
                     if (p.PW >= 8) {
@@ -277,16 +355,35 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
 }
 
 // ---- staging: fp32 -> (hi, lo) ------------------------------------------------------------------------
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-    hi = __uint_as_float(__float_as_uint(x) & 0xFFFFE000u);
-    lo = x - hi;
+// hi: x rounded to a TF32 number; xb and lb: x and x - hi (exact) rounded to bf16. Where rounding a finite x would overflow, it is cut off
+// instead. Infinities and NaN make lo a NaN.
+struct Split32 { float hi; uint16_t xb, lb; };
+__device__ __forceinline__ Split32 split_f32(float x) {
+    const uint32_t u = __float_as_uint(x);
+    uint32_t h = (u + 0x1000u) & 0xFFFFE000u, b = u + 0x7FFFu + ((u >> 16) & 1u);
+    if ((h & 0x7F800000u) == 0x7F800000u) h = u & 0xFFFFE000u;
+    if ((b & 0x7F800000u) == 0x7F800000u) b = u;
+    Split32 r;
+    r.hi = __uint_as_float(h);
+    r.xb = (uint16_t)(b >> 16);
+    r.lb = __bfloat16_as_ushort(__float2bfloat16_rn(x - r.hi));
+    return r;
 }
+// Four channels of a pixel (or four K columns of a filter row) at hi + o, o a multiple of 4; the bf16 parts at lb and xb.
+__device__ __forceinline__ void store_split(float4 f, float* hi, uint16_t* xb, uint16_t* lb) {
+    const Split32 a = split_f32(f.x), b = split_f32(f.y), c = split_f32(f.z), d = split_f32(f.w);
+    *reinterpret_cast<float4*>(hi) = make_float4(a.hi, b.hi, c.hi, d.hi);
+    *reinterpret_cast<uint2*>(xb) = make_uint2(a.xb | (uint32_t)b.xb << 16, c.xb | (uint32_t)d.xb << 16);
+    *reinterpret_cast<uint2*>(lb) = make_uint2(a.lb | (uint32_t)b.lb << 16, c.lb | (uint32_t)d.lb << 16);
+}
+// The place of x in the lo part (bf16 elements) of channels-last rows: element o of the hi part, 32 elements per 16 channels. lo is 16 behind it.
+__device__ __forceinline__ size_t row_lo(size_t o) { return 2 * o - (o & 15); }
 
 // A block takes 32 consecutive padded pixels of one plane and up to 64 channels at a time through shared memory: the NCHW reads
 // run along the pixels of one channel (coalesced), the channels-last writes along the channel groups of one pixel (coalesced;
 // a thread per (pixel, 4 channels) writes one float4 of hi and one of lo).
 __global__ void __launch_bounds__(256)
-pack_activations_f32_kernel(const float* __restrict__ x, float* __restrict__ hi, float* __restrict__ lo, int planes, int C,
+pack_activations_f32_kernel(const float* __restrict__ x, float* __restrict__ hi, uint16_t* __restrict__ lo, int planes, int C,
                             int H, int W, int Hp, int Wp, int Cp, int pad_top, int pad_left, int ins_h, int ins_w,
                             int cb, int Nb) {
     __shared__ float tile[64][33];
@@ -313,19 +410,15 @@ pack_activations_f32_kernel(const float* __restrict__ x, float* __restrict__ hi,
             for (int idx = threadIdx.x; idx < 32 * groups; idx += 256) {
                 const int g = idx % groups, px = idx / groups;
                 if (pp0 + px >= PP) continue;
-                float4 vh, vl;
-                split_tf32(tile[4 * g][px], vh.x, vl.x);
-                split_tf32(tile[4 * g + 1][px], vh.y, vl.y);
-                split_tf32(tile[4 * g + 2][px], vh.z, vl.z);
-                split_tf32(tile[4 * g + 3][px], vh.w, vl.w);
+                const float4 f = make_float4(tile[4 * g][px], tile[4 * g + 1][px], tile[4 * g + 2][px], tile[4 * g + 3][px]);
                 const int ch = c0 + 4 * g;
-                size_t o = ((size_t)plane * PP + pp0 + px) * Cp + ch;
-                if (cb > 0) {   // blocks of cb channels, block index outermost: [comp * (Cp / cb) + c / cb][img][hp][wp][cb]
+                size_t o = ((size_t)plane * PP + pp0 + px) * Cp + ch, ox = row_lo(o), ol = ox + 16;
+                if (cb > 0) {   // blocks of cb channels, block index outermost: [comp * (Cp / cb) + c / cb][img][hp][wp][cb]; lo: two planes per block
                     const int comp = plane / Nb, img = plane - comp * Nb, bl = ch / cb;
-                    o = ((((size_t)comp * (Cp / cb) + bl) * Nb + img) * PP + pp0 + px) * cb + (ch - bl * cb);
+                    const size_t blk = (size_t)comp * (Cp / cb) + bl, at = ((size_t)img * PP + pp0 + px) * cb + (ch - bl * cb), size = (size_t)Nb * PP * cb;
+                    o = blk * size + at; ox = 2 * blk * size + at; ol = ox + size;
                 }
-                *reinterpret_cast<float4*>(hi + o) = vh;
-                *reinterpret_cast<float4*>(lo + o) = vl;
+                store_split(f, hi + o, lo + ox, lo + ol);
             }
             __syncthreads();
         }
@@ -334,7 +427,7 @@ pack_activations_f32_kernel(const float* __restrict__ x, float* __restrict__ hi,
 
 // The same staging, one thread per (pixel, 4 channels), for planes of fewer than 32 padded pixels (dense layers are 1 x 1 images:
 // consecutive threads then walk the channel groups of one row, and both sides are contiguous).
-__global__ void pack_activations_f32_small_kernel(const float* __restrict__ x, float* __restrict__ hi, float* __restrict__ lo, int planes, int C,
+__global__ void pack_activations_f32_small_kernel(const float* __restrict__ x, float* __restrict__ hi, uint16_t* __restrict__ lo, int planes, int C,
                                                   int H, int W, int Hp, int Wp, int Cp, int pad_top, int pad_left, int ins_h, int ins_w,
                                                   int cb, int Nb) {
     const int groups = Cp / 4;
@@ -352,22 +445,19 @@ __global__ void pack_activations_f32_small_kernel(const float* __restrict__ x, f
             ih /= ins_h; iw /= ins_w;
         }
         inside = inside && ih < H && iw < W;
-        float4 vh, vl;
-        float* ph = &vh.x; float* pl = &vl.x;
+        float v[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const int c = grp * 4 + e;
-            float v = 0.f;
-            if (c < C && inside) v = __ldg(x + (((size_t)plane * C + c) * H + ih) * W + iw);
-            split_tf32(v, ph[e], pl[e]);
+            v[e] = (c < C && inside) ? __ldg(x + (((size_t)plane * C + c) * H + ih) * W + iw) : 0.f;
         }
-        size_t o = (((size_t)plane * Hp + hp) * Wp + wp) * Cp + grp * 4;
+        size_t o = (((size_t)plane * Hp + hp) * Wp + wp) * Cp + grp * 4, ox = row_lo(o), ol = ox + 16;
         if (cb > 0) {
             const int comp = plane / Nb, img = plane - comp * Nb, b = (grp * 4) / cb;
-            o = (((((size_t)comp * (Cp / cb) + b) * Nb + img) * Hp + hp) * Wp + wp) * cb + (grp * 4 - b * cb);
+            const size_t blk = (size_t)comp * (Cp / cb) + b, at = (((size_t)img * Hp + hp) * Wp + wp) * cb + (grp * 4 - b * cb), size = (size_t)Nb * Hp * Wp * cb;
+            o = blk * size + at; ox = 2 * blk * size + at; ol = ox + size;
         }
-        *reinterpret_cast<float4*>(hi + o) = vh;
-        *reinterpret_cast<float4*>(lo + o) = vl;
+        store_split(make_float4(v[0], v[1], v[2], v[3]), hi + o, lo + ox, lo + ol);
     }
 }
 
@@ -379,12 +469,24 @@ __global__ void pack_activations_f32_small_kernel(const float* __restrict__ x, f
 // 56 x 56, batch 32, 1 x 1, 99 / 120.
 struct StageJob32 {
     const float* x;
-    float *hi, *lo;
+    float* hi;
+    uint16_t* lo;
     unsigned total_px, HW, Nb;
     int C, nblk, U, V, blocked;
     unsigned units;                   // units of a pixel (all blocks)
     unsigned bx, blocks;
 };
+// Unit g (of U) of block `by` of pixel P (counted over all planes) of component `comp`.
+__device__ __forceinline__ void store_unit(const StageJob32& p, unsigned P, unsigned comp, unsigned by, unsigned g, unsigned U, float4 f) {
+    size_t o, ox, ol;
+    if (p.blocked) {
+        const size_t size = (size_t)p.Nb * p.HW * (4 * U), blk = (size_t)comp * p.nblk + by, at = ((size_t)P - (size_t)comp * p.Nb * p.HW) * (4 * U) + 4 * g;
+        o = blk * size + at; ox = 2 * blk * size + at; ol = ox + size;
+    } else {
+        o = 4 * ((size_t)P * p.units + by * U + g); ox = row_lo(o); ol = ox + 16;
+    }
+    store_split(f, p.hi + o, p.lo + ox, p.lo + ol);
+}
 template <int V, int U>
 __device__ __forceinline__ void stage_compact_f32(const StageJob32& p, unsigned block, float4* tile /*[STAGE_UNITS]*/) {
     constexpr int TPX = STAGE_UNITS / U;
@@ -413,14 +515,7 @@ __device__ __forceinline__ void stage_compact_f32(const StageJob32& p, unsigned 
         const int i = threadIdx.x + it * STAGE_THREADS, px = i / U, g = i % U;
         const unsigned P = px0 + px;
         if (P >= p.total_px || by * U + g >= p.units) continue;
-        size_t unit;
-        if (p.blocked) unit = ((size_t)P + (size_t)((P / HW / p.Nb) * (unsigned)(p.nblk - 1) + by) * p.Nb * HW) * U + g;
-        else unit = (size_t)P * p.units + by * U + g;
-        const float4 f = tile[stage_unit<V, U>(px, g)];
-        float4 h, lo;
-        split_tf32(f.x, h.x, lo.x); split_tf32(f.y, h.y, lo.y); split_tf32(f.z, h.z, lo.z); split_tf32(f.w, h.w, lo.w);
-        reinterpret_cast<float4*>(p.hi)[unit] = h;
-        reinterpret_cast<float4*>(p.lo)[unit] = lo;
+        store_unit(p, P, P / HW / p.Nb, by, g, U, tile[stage_unit<V, U>(px, g)]);
     }
 }
 template <int U>
@@ -440,21 +535,14 @@ __device__ __forceinline__ void stage_tiny_f32(const StageJob32& p, unsigned blo
         float f[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e) f[e] = ld_chained(src + (size_t)e * HW, (int)(4 * grp) + e < p.C);
-        const size_t P = (size_t)plane * HW + px;
-        size_t unit = P * groups + grp;
-        if (p.blocked) {
-            const unsigned comp = plane / p.Nb, b = grp / p.U;
-            unit = (P + (size_t)(comp * (unsigned)(p.nblk - 1) + b) * p.Nb * HW) * p.U + (grp - b * p.U);
-        }
-        float4 h, lo;
-        split_tf32(f[0], h.x, lo.x); split_tf32(f[1], h.y, lo.y); split_tf32(f[2], h.z, lo.z); split_tf32(f[3], h.w, lo.w);
-        reinterpret_cast<float4*>(p.hi)[unit] = h;
-        reinterpret_cast<float4*>(p.lo)[unit] = lo;
+        const unsigned b = grp / p.U;
+        store_unit(p, plane * HW + px, plane / p.Nb, b, grp - b * p.U, p.U, make_float4(f[0], f[1], f[2], f[3]));
     }
 }
 struct FilterJob32 {
     const float* w;
-    float *hi, *lo;
+    float* hi;
+    uint16_t* lo;
     int Co, Ci, taps, Mp, Kp, Cp, transposed, w_io, nc, ga;
     unsigned long long neg;
 };
@@ -467,7 +555,7 @@ __device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned 
     // one row (tap, m) of the expanded matrix per `wx` threads; the row is decoded once and its threads walk k
     const float* w = p.w;
     float* __restrict__ hi = p.hi;
-    float* __restrict__ lo = p.lo;
+    uint16_t* __restrict__ lo = p.lo;
     const int Co = p.Co, Ci = p.Ci, taps = p.taps, Mp = p.Mp, Kp = p.Kp, Cp = p.Cp, transposed = p.transposed, w_io = p.w_io, nc = p.nc, ga = p.ga;
     const unsigned long long neg = p.neg;
     const int Cm = transposed ? Ci : Co, Ck = transposed ? Co : Ci;
@@ -478,7 +566,7 @@ __device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned 
         const int cm_comp = m / Cm, cm = m - cm_comp * Cm;
         const int src_tap = transposed ? taps - 1 - tap : tap;
         float* hrow = hi + (size_t)row * Kp;
-        float* lrow = lo + (size_t)row * Kp;
+        uint16_t* lrow = lo + (size_t)row * Kp * 2;            // [lo | x] for every 16 columns
         for (int k = tx; k < Kp; k += wx) {
             const int ck_comp = k / Cp, ck = k - ck_comp * Cp;
             float v = 0.f;
@@ -490,10 +578,10 @@ __device__ __forceinline__ void pack_filters_f32(const FilterJob32& p, unsigned 
                 v = ld_chained(w + src);
                 if (alg_negative(neg, l, d)) v = -v;
             }
-            float h, lw;
-            split_tf32(v, h, lw);
-            hrow[k] = h;
-            lrow[k] = lw;
+            const Split32 sp = split_f32(v);
+            hrow[k] = sp.hi;
+            lrow[2 * k - (k & 15)] = sp.lb;
+            lrow[2 * k - (k & 15) + 16] = sp.xb;
         }
     }
 }
@@ -573,7 +661,7 @@ int launch_prologue(Prologue32& pro, StatusClear* sc, cudaStream_t stream, bool*
 // A job of the prologue launch for unpadded copies, a kernel of its own otherwise (zero-inserted gradients). As kernels of their own in
 // front of the prologue, with the filters packed behind them, the copies of planes of a few pixels cost a dense layer 1024 -> 1024 at
 // batch 3000 728 us forward and 552 us for the filter gradient instead of 709 and 508.
-void stage_activations_f32(Prologue32& pro, const float* x, float* hi, float* lo, int planes, int C, int H, int W, int Hp, int Wp, int Cp, int pad_top,
+void stage_activations_f32(Prologue32& pro, const float* x, float* hi, uint16_t* lo, int planes, int C, int H, int W, int Hp, int Wp, int Cp, int pad_top,
                            int pad_left, int ins_h, int ins_w, int cb, int Nb, cudaStream_t stream) {
     if (Hp == H && Wp == W && pad_top == 0 && pad_left == 0 && ins_h == 1 && ins_w == 1) {
         const int block = cb > 0 ? cb : (Cp > 32 ? 64 : (Cp > 16 ? 32 : 16));       // (cb is 0 or 32, and then Cp a multiple of 32)
@@ -596,12 +684,14 @@ void stage_activations_f32(Prologue32& pro, const float* x, float* hi, float* lo
 }
 
 // ---- backward-filter ------------------------------------------------------------------------------------
-// Both staged tensors MN-major (K = pixels, 16 per stage), M = (d, co), N = (l, ci); per K step of 8 pixels three
-// TF32 MMAs; the epilogue folds G[(d,co),(l,ci)] through the quaternion table into fp32 scratch [tap][r][co][ci].
+// Both staged tensors MN-major (K = pixels, 16 per stage), M = (d, co), N = (l, ci); per stage two TF32 MMAs of 8 pixels and two
+// bf16 MMAs of 16; the epilogue folds G[(d,co),(l,ci)] through the quaternion table into fp32 scratch [tap][r][co][ci].
 // 32-bit MN-major operands exist in one shared-memory layout only: 128-byte rows (32 channels) swizzled in 32-byte
 // units over groups of 4 rows (descriptor layout type 1, TMA swizzle 128B_ATOM_32B), so channels are padded to 32.
 constexpr int TFK = 16;
 constexpr uint32_t TF_STAGE = 2 * (TM + TN) * TFK * 4;      // 48 KB
+constexpr int TFP_STAGES = 6;                               // pairs of SMs: half of the N columns in each CTA, 32 KB
+constexpr uint32_t TFP_STAGE = 2 * (TM + TN / 2) * TFK * 4;
 struct TFParams {
     int Nb, Co, Ci, HO, WO, Cop, Cip, cbA, cbB;             // channel-block width in fp32 elements: 32
     int KH, KW, SH, SW, DH, DW, PW, PH, PN, tiles_w, tiles_h, tiles_n;
@@ -617,53 +707,69 @@ __device__ __forceinline__ uint64_t desc_mn_f32(uint32_t addr, int cb, uint32_t 
            ((uint64_t)(((4u * cb * 4u) >> 4) & 0x3FFFu) << 32) | DESC_VERSION_SM100 | (1ull << 61);
 }
 
+// The bf16 parts: per block of 32 channels a plane of x and one of lo, 64-byte rows (one per pixel), 64-byte swizzle.
+constexpr uint32_t LO_PLANE = TFK * 32 * 2;
+__device__ __forceinline__ uint64_t desc_mn_b16(uint32_t addr) {
+    return (uint64_t)((addr & 0x3FFFFu) >> 4) | ((uint64_t)((2 * LO_PLANE) >> 4) << 16) | ((uint64_t)(512 >> 4) << 32) | DESC_VERSION_SM100 | (4ull << 61);
+}
+
+// PAIR: as in conv_tc.cu, a cluster of two CTAs takes 256 rows and half of the N columns each. 3x3, 128 channels, 28 x 28, batch 128, forward
+// and backward under the power limit: 5543 -> 5239 us with it.
+template <bool PAIR>
 __global__ void __launch_bounds__(T_THREADS, 1)
 qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __grid_constant__ CUtensorMap map_dy_lo,
                          const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo, TFParams p,
                          float* __restrict__ dw32, int* __restrict__ status) {
+    constexpr int STAGES = PAIR ? TFP_STAGES : T_STAGES;
+    constexpr uint32_t STAGE = PAIR ? TFP_STAGE : TF_STAGE;
     extern __shared__ uint8_t smem_raw[];
+    const int rank = PAIR ? (int)cluster_ctarank() : 0;
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t* bars = reinterpret_cast<uint64_t*>(base + T_STAGES * TF_STAGE);
-    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * T_STAGES + 4);
+    uint64_t* bars = reinterpret_cast<uint64_t*>(base + STAGES * STAGE);
+    uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * STAGES + 4);
     const uint32_t tiles_addr = smem_u32(base);
-    const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + T_STAGES);
-    const uint32_t tmem_full = smem_u32(bars + 2 * T_STAGES), tmem_empty = smem_u32(bars + 2 * T_STAGES + 2);
+    const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + STAGES);
+    const uint32_t tmem_full = smem_u32(bars + 2 * STAGES), tmem_empty = smem_u32(bars + 2 * STAGES + 2);
 
-    const int n_items = p.m_tiles * p.n_tiles * p.KH * p.KW;
-    int item = blockIdx.x % n_items;
-    const int split = blockIdx.x / n_items;
-    const int mt = item % p.m_tiles; item /= p.m_tiles;
+    const int m_tiles = PAIR ? p.m_tiles / 2 : p.m_tiles, id = PAIR ? blockIdx.x / 2 : blockIdx.x;
+    const int n_items = m_tiles * p.n_tiles * p.KH * p.KW;
+    int item = id % n_items;
+    const int split = id / n_items;
+    const int mt = PAIR ? 2 * (item % m_tiles) + rank : item % m_tiles; item /= m_tiles;
     const int nt = item % p.n_tiles;
     const int tap = item / p.n_tiles;
     const int kh = tap / p.KW, kw = tap - kh * p.KW;
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
     const int step_beg = split * p.steps_per_split;
     const int n_steps = max(0, min(steps_total, step_beg + p.steps_per_split) - step_beg);
-    const int n_chunks = (n_steps + T_CHUNK - 1) / T_CHUNK;       // chunks alternate between the two TMEM buffers
+    const int n_chunks = (n_steps + T_CHUNK - 1) / T_CHUNK;
+    const int bufs = p.n_tile_cols <= 128 ? 2 : 1;                // accumulators of hi * hi, as in the kernel above; one of the cross terms
 
-    const int nblkA = TM / p.cbA, nblkB = p.n_tile_cols / p.cbB;
+    const int nblkA = TM / p.cbA, nblkB = p.n_tile_cols / p.cbB / (PAIR ? 2 : 1);      // blocks of this CTA's shared memory
     const int bpcA = p.Cop / p.cbA, bpcB = p.Cip / p.cbB;
     const uint32_t blkA_bytes = TFK * p.cbA * 4, blkB_bytes = TFK * p.cbB * 4;
     const uint32_t a_bytes = nblkA * blkA_bytes, b_bytes = nblkB * blkB_bytes;
-    const uint32_t A_REGION = TM * TFK * 4, B_REGION = TN * TFK * 4;      // 8 KB, 16 KB
+    const uint32_t A_REGION = TM * TFK * 4, B_REGION = (PAIR ? TN / 2 : TN) * TFK * 4;      // 8 KB, 16 (8) KB
     const int blockA0 = mt * nblkA, blockB0 = nt * (TN / p.cbB);
 
     if (t == 0) {
-        for (int s = 0; s < T_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, 8); }
+        for (int s = 0; s < STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, PAIR ? 16 : 8); }
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
+    if (warp == 1) { if (PAIR) tmem_alloc_pair(smem_u32(tmem_slot), 512); else tmem_alloc(smem_u32(tmem_slot), 512); }
     tc_fence_before_sync();
     __syncthreads();
+    if (PAIR) cluster_sync_all();                     // both CTAs' barriers exist before anything signals them
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     chain_wait();
     chain_next();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
+            const bool el = elect_one();
             // one copy per operand half and stage (the staged tensors keep the channel-block index outermost, so the blocks
             // of a tile are one box even across components) and a running (tw, th, tn) of the pixel box: no division in
             // this loop -- a division per copy used to bound the kernel
@@ -671,55 +777,83 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
             int s = 0, phase = 1;
             bool ok = true;
             for (int it = 0; it < n_steps && ok; ++it) {
-                ok = mbar_wait_bounded(empty_bar + 8 * s, phase, status, ST_T_PRODUCER);
+                ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_T_PRODUCER);
                 if (!ok) break;
                 const int ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
-                const uint32_t a_hi = tiles_addr + s * TF_STAGE, a_lo = a_hi + A_REGION, b_hi = a_hi + 2 * A_REGION, b_lo = b_hi + B_REGION;
+                const uint32_t a_hi = tiles_addr + s * STAGE, a_lo = a_hi + A_REGION, b_hi = a_hi + 2 * A_REGION, b_lo = b_hi + B_REGION;
                 const uint32_t bar = full_bar + 8 * s;
                 if (++tw == p.tiles_w) { tw = 0; if (++th == p.tiles_h) { th = 0; ++tn; } }
-                if (++s == T_STAGES) { s = 0; phase ^= 1; }
-                mbar_arrive_expect_tx(bar, 2 * (a_bytes + b_bytes));
-                tma_load_5d(a_hi, &map_dy_hi, 0, ow0, oh0, n0, blockA0, bar);
-                tma_load_5d(a_lo, &map_dy_lo, 0, ow0, oh0, n0, blockA0, bar);
+                if (++s == STAGES) { s = 0; phase ^= 1; }
                 const int wp0 = ow0 * p.SW + kw * p.DW + p.off_w, hp0 = oh0 * p.SH + kh * p.DH + p.off_h;
-                tma_load_5d(b_hi, &map_x_hi, 0, wp0, hp0, n0, blockB0, bar);
-                tma_load_5d(b_lo, &map_x_lo, 0, wp0, hp0, n0, blockB0, bar);
+                if (el && PAIR) {
+                    const uint32_t lead = map_to_cta(bar, 0);
+                    if (rank == 0) mbar_arrive_expect_tx(bar, 4 * (a_bytes + b_bytes));
+                    tma_load_5d_pair(a_hi, &map_dy_hi, 0, ow0, oh0, n0, blockA0, lead);
+                    tma_load_5d_pair(a_lo, &map_dy_lo, 0, ow0, oh0, n0, 2 * blockA0, lead);
+                    tma_load_5d_pair(b_hi, &map_x_hi, 0, wp0, hp0, n0, blockB0 + rank * nblkB, lead);
+                    tma_load_5d_pair(b_lo, &map_x_lo, 0, wp0, hp0, n0, 2 * (blockB0 + rank * nblkB), lead);
+                } else if (el) {
+                    mbar_arrive_expect_tx(bar, 2 * (a_bytes + b_bytes));
+                    tma_load_5d(a_hi, &map_dy_hi, 0, ow0, oh0, n0, blockA0, bar);
+                    tma_load_5d(a_lo, &map_dy_lo, 0, ow0, oh0, n0, 2 * blockA0, bar);
+                    tma_load_5d(b_hi, &map_x_hi, 0, wp0, hp0, n0, blockB0, bar);
+                    tma_load_5d(b_lo, &map_x_lo, 0, wp0, hp0, n0, 2 * blockB0, bar);
+                }
             }
         }
         __syncwarp();
     } else if (warp == 1) {
-        const uint32_t idesc = make_idesc_f16(2, TM, p.n_tile_cols, true, true);
-        bool ok = true;
-        for (int c = 0; c < n_chunks && ok; ++c) {
-            const int buf = c & 1, use = c >> 1;
-            if (use > 0) {
-                ok = mbar_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_T_MMA);
-                if (!ok) break;
-                tc_fence_after_sync();
-            }
-            const int k_beg = c * T_CHUNK, k_end = min(n_steps, k_beg + T_CHUNK);
-            const uint32_t dcol = tmem_base + buf * TN;
-            for (int it = k_beg; it < k_end && ok; ++it) {
-                const int s = it % T_STAGES;
-                ok = mbar_wait_bounded(full_bar + 8 * s, (it / T_STAGES) & 1, status, ST_T_MMA);
-                if (!ok) break;
-                tc_fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t a_hi = tiles_addr + s * TF_STAGE, a_lo = a_hi + A_REGION, b_hi = a_hi + 2 * A_REGION, b_lo = b_hi + B_REGION;
-#pragma unroll
-                    for (int j = 0; j < TFK / 8; ++j) {                   // 8 pixels (K rows) per MMA
-                        const uint32_t ao = j * 8 * p.cbA * 4, bo = j * 8 * p.cbB * 4;
-                        mma_tf32_ss(dcol, desc_mn_f32(a_lo + ao, p.cbA, blkA_bytes), desc_mn_f32(b_hi + bo, p.cbB, blkB_bytes), idesc, (it > k_beg || j > 0) ? 1u : 0u);
-                        mma_tf32_ss(dcol, desc_mn_f32(a_hi + ao, p.cbA, blkA_bytes), desc_mn_f32(b_lo + bo, p.cbB, blkB_bytes), idesc, 1u);
-                        mma_tf32_ss(dcol, desc_mn_f32(a_hi + ao, p.cbA, blkA_bytes), desc_mn_f32(b_hi + bo, p.cbB, blkB_bytes), idesc, 1u);
-                    }
-                    mma_commit(empty_bar + 8 * s);
-                    if (it == k_end - 1) mma_commit(tmem_full + 8 * buf);
+        if (rank == 0) {
+            constexpr int M = PAIR ? 2 * TM : TM;
+            const uint32_t idesc_main = make_idesc_f16(2, M, p.n_tile_cols, true, true), idesc_cross = make_idesc_f16(1, M, p.n_tile_cols, true, true);
+            const uint32_t d_cross = tmem_base + 256;
+            const uint32_t peer_empty = PAIR ? map_to_cta(empty_bar, 1) : 0u, peer_full = PAIR ? map_to_cta(tmem_full, 1) : 0u;
+            const bool el = elect_one();
+            bool ok = true;
+            int s = 0, phase = 0;
+            for (int c = 0; c < n_chunks && ok; ++c) {
+                const int buf = bufs == 2 ? c & 1 : 0, use = bufs == 2 ? c >> 1 : c;
+                if (use > 0) {
+                    ok = warp_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_T_MMA);
+                    if (!ok) break;
+                    tc_fence_after_sync();
                 }
-                __syncwarp();
+                const int k_beg = c * T_CHUNK, k_end = min(n_steps, k_beg + T_CHUNK);
+                const uint32_t d_main = tmem_base + buf * 128;
+                for (int it = k_beg; it < k_end; ++it) {
+                    ok = warp_wait_bounded(full_bar + 8 * s, phase, status, ST_T_MMA);
+                    if (!ok) break;
+                    tc_fence_after_sync();
+                    if (el) {
+                        const uint32_t a_hi = tiles_addr + s * STAGE, a_lo = a_hi + A_REGION, b_hi = a_hi + 2 * A_REGION, b_lo = b_hi + B_REGION;
+                        auto cross = [&](uint64_t ad, uint64_t bd, uint32_t acc) {
+                            if (PAIR) mma_f16_pair(d_cross, (uint32_t)ad, (uint32_t)(ad >> 32), (uint32_t)bd, (uint32_t)(bd >> 32), idesc_cross, acc);
+                            else mma_f16_ss(d_cross, ad, bd, idesc_cross, acc);
+                        };
+                        // lo: per channel block the planes of x and of lo, 16 pixels (one K step) each
+                        cross(desc_mn_b16(a_lo + LO_PLANE), desc_mn_b16(b_lo), it > 0 ? 1u : 0u);
+                        cross(desc_mn_b16(a_lo), desc_mn_b16(b_lo + LO_PLANE), 1u);
+#pragma unroll
+                        for (int j = 0; j < TFK / 8; ++j) {                   // 8 pixels (K rows) per MMA
+                            const uint64_t ad = desc_mn_f32(a_hi + j * 8 * p.cbA * 4, p.cbA, blkA_bytes), bd = desc_mn_f32(b_hi + j * 8 * p.cbB * 4, p.cbB, blkB_bytes);
+                            const uint32_t acc = (it > k_beg || j > 0) ? 1u : 0u;
+                            if (PAIR) mma_tf32_pair(d_main, (uint32_t)ad, (uint32_t)(ad >> 32), (uint32_t)bd, (uint32_t)(bd >> 32), idesc_main, acc);
+                            else mma_tf32_ss(d_main, ad, bd, idesc_main, acc);
+                        }
+                        if (PAIR) {
+                            mma_commit_pair(empty_bar + 8 * s);
+                            mma_commit_pair(peer_empty + 8 * s);
+                            if (it == k_end - 1) { mma_commit_pair(tmem_full + 8 * buf); mma_commit_pair(peer_full + 8 * buf); }
+                        } else {
+                            mma_commit(empty_bar + 8 * s);
+                            if (it == k_end - 1) mma_commit(tmem_full + 8 * buf);
+                        }
+                    }
+                    if (++s == STAGES) { s = 0; phase ^= 1; }
+                }
             }
+            if (n_steps == 0 && el) { mbar_arrive(tmem_full); if (PAIR) mbar_arrive_cluster(peer_full); }
         }
-        if (n_steps == 0 && lane == 0) mbar_arrive(tmem_full);
         __syncwarp();
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
@@ -730,7 +864,7 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
             for (int e = 0; e < 32; ++e) part[cb][e] = 0.f;
         bool ok = true;
         for (int c = 0; c + 1 < n_chunks && ok; ++c) {
-            const int buf = c & 1, use = c >> 1;
+            const int buf = bufs == 2 ? c & 1 : 0, use = bufs == 2 ? c >> 1 : c;
             const int seen = read_status(status);
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_T_EPILOGUE);
             ok = warp_may_store(ok, seen);
@@ -740,7 +874,7 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
             for (int cb = 0; cb < 4; ++cb) {
                 if (chalf * 128 + cb * 32 < p.n_tile_cols) {
                     uint32_t v[32];
-                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * TN + chalf * 128 + cb * 32, v);
+                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * 128 + chalf * 128 + cb * 32, v);
                     tmem_ld_wait();
 #pragma unroll
                     for (int e = 0; e < 32; ++e) part[cb][e] += __uint_as_float(v[e]);
@@ -748,12 +882,12 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
             }
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(tmem_empty + 8 * buf);
+            if (lane == 0) { if (PAIR) mbar_arrive_cluster(map_to_cta(tmem_empty + 8 * buf, 0)); else mbar_arrive(tmem_empty + 8 * buf); }
         }
-        const int last = n_chunks > 0 ? n_chunks - 1 : 0, lbuf = last & 1;
+        const int last = n_chunks > 0 ? n_chunks - 1 : 0, lbuf = bufs == 2 ? last & 1 : 0;
         if (ok) {
             const int seen = read_status(status);
-            ok = mbar_wait_bounded(tmem_full + 8 * lbuf, (last >> 1) & 1, status, ST_T_EPILOGUE);
+            ok = mbar_wait_bounded(tmem_full + 8 * lbuf, (bufs == 2 ? last >> 1 : last) & 1, status, ST_T_EPILOGUE);
             ok = warp_may_store(ok, seen);
         }
         tc_fence_after_sync();
@@ -769,7 +903,11 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
                 const int col0 = chalf * 128 + cb * 32;
                 if (col0 >= p.n_tile_cols) break;
                 uint32_t v[32];
-                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + lbuf * TN + col0, v);
+                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + 256 + col0, v);
+                tmem_ld_wait();
+#pragma unroll
+                for (int e = 0; e < 32; ++e) part[cb][e] += __uint_as_float(v[e]);
+                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + lbuf * 128 + col0, v);
                 tmem_ld_wait();
                 if (!row_ok) continue;
 #pragma unroll
@@ -797,7 +935,8 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, 512);
+    if (PAIR) cluster_sync_all();                     // nobody leaves while its peer may still signal its barriers or read its shared memory
+    if (warp == 1) { if (PAIR) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512); }
 }
 
 // scratch [tap][r][co][ci] -> dw [r][co][ci][tap], or [r][ci][co] for dense layers (input-major, one tap)
@@ -918,9 +1057,9 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     const int taps = g.KH * g.KW;
     uint8_t* s8 = static_cast<uint8_t*>(scratch);
     float* x_hi = reinterpret_cast<float*>(s8);
-    float* x_lo = reinterpret_cast<float*>(s8 + f.xp_bytes);
+    uint16_t* x_lo = reinterpret_cast<uint16_t*>(s8 + f.xp_bytes);
     float* y_hi = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes);
-    float* y_lo = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes + f.dyp_bytes);
+    uint16_t* y_lo = reinterpret_cast<uint16_t*>(s8 + 2 * f.xp_bytes + f.dyp_bytes);
     float* acc = reinterpret_cast<float*>(s8 + 2 * f.xp_bytes + 2 * f.dyp_bytes);
     bool chain = false;
     Prologue32 pro;
@@ -954,14 +1093,22 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     p.n_tiles = (n_cols + TN - 1) / TN;
     p.n_tile_cols = n_cols < TN ? n_cols : TN;
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
-    const int items = taps * p.m_tiles * p.n_tiles;
-    int splits = split_count(items, sm_count());
+    const bool pair = p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0;
+    const int items = taps * p.m_tiles * p.n_tiles / (pair ? 2 : 1);
+    int splits = split_count(items, pair ? sm_count() / 2 : sm_count());
     if (splits > steps_total) splits = steps_total;
     if (splits < 1) splits = 1;
     p.steps_per_split = (steps_total + splits - 1) / splits;
     p.splits = (steps_total + p.steps_per_split - 1) / p.steps_per_split;
 
     auto swz = [](int) { return CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B; };
+    // the lo part: the same bytes as two planes of bf16 per channel block
+    auto lo_map = [](CUtensorMap* map, const void* ptr, const cuuint64_t* dims, const cuuint64_t* strides, const cuuint32_t* box, const cuuint32_t* es, const char* what) {
+        const cuuint64_t d[5] = {dims[0], dims[1], dims[2], dims[3], 2 * dims[4]};
+        const cuuint64_t st[4] = {strides[0] / 2, strides[1] / 2, strides[2] / 2, strides[3] / 2};
+        const cuuint32_t b[5] = {box[0], box[1], box[2], box[3], 2 * box[4]};
+        return make_tensor_map(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, ptr, 5, d, st, b, es, CU_TENSOR_MAP_SWIZZLE_64B, what);
+    };
     alignas(64) CUtensorMap m_dy_hi, m_dy_lo, m_x_hi, m_x_lo;
     {
         // staged tensors: [component * blocks per component + channel block][image][h][w][32 channels]; the last box extent
@@ -971,7 +1118,7 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
                                        (cuuint64_t)g.Nb * g.HO * g.WO * p.cbA * 4};
         const cuuint32_t box[5] = {(cuuint32_t)p.cbA, (cuuint32_t)p.PW, (cuuint32_t)p.PH, (cuuint32_t)p.PN, (cuuint32_t)(TM / p.cbA)};
         int rc = make_tensor_map(&m_dy_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, y_hi, 5, dims, strides, box, nullptr, swz(p.cbA), "dy hi");
-        if (rc == PCB_OK) rc = make_tensor_map(&m_dy_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, y_lo, 5, dims, strides, box, nullptr, swz(p.cbA), "dy lo");
+        if (rc == PCB_OK) rc = lo_map(&m_dy_lo, y_lo, dims, strides, box, nullptr, "dy lo");
         if (rc != PCB_OK) return rc;
     }
     {
@@ -979,15 +1126,16 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
         const cuuint64_t strides[4] = {(cuuint64_t)p.cbB * 4, (cuuint64_t)f.W * p.cbB * 4, (cuuint64_t)f.H * f.W * p.cbB * 4,
                                        (cuuint64_t)g.Nb * f.H * f.W * p.cbB * 4};
         const cuuint32_t box[5] = {(cuuint32_t)p.cbB, (cuuint32_t)((p.PW - 1) * g.SW + 1), (cuuint32_t)((p.PH - 1) * g.SH + 1), (cuuint32_t)p.PN,
-                                   (cuuint32_t)(p.n_tile_cols / p.cbB)};
+                                   (cuuint32_t)(p.n_tile_cols / p.cbB / (pair ? 2 : 1))};
         const cuuint32_t es[5] = {1, (cuuint32_t)g.SW, (cuuint32_t)g.SH, 1, 1};
         int rc = make_tensor_map(&m_x_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_hi, 5, dims, strides, box, es, swz(p.cbB), "x hi");
-        if (rc == PCB_OK) rc = make_tensor_map(&m_x_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_lo, 5, dims, strides, box, es, swz(p.cbB), "x lo");
+        if (rc == PCB_OK) rc = lo_map(&m_x_lo, x_lo, dims, strides, box, es, "x lo");
         if (rc != PCB_OK) return rc;
     }
     constexpr size_t smem = 1024 + T_STAGES * TF_STAGE + 512;
-    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_filter_tf32_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    PCB_CUDA_TRY(launch_chained_if(chain, qconv_filter_tf32_kernel, items * p.splits, T_THREADS, smem, stream, m_dy_hi, m_dy_lo, m_x_hi, m_x_lo, p, acc, status));
+    auto* kernel = pair ? qconv_filter_tf32_kernel<true> : qconv_filter_tf32_kernel<false>;
+    PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+    PCB_CUDA_TRY(launch_clusters(pair ? 2 : 1, chain, kernel, items * p.splits * (pair ? 2 : 1), T_THREADS, smem, stream, m_dy_hi, m_dy_lo, m_x_hi, m_x_lo, p, acc, status));
     PCB_CUDA_TRY(cudaGetLastError());
     PCB_CUDA_TRY(launch_chained(unpack_filter_grad_f32_kernel, grid_cap((size_t)g.nc * g.Co * g.Ci * taps, 256, 16), 256, 0, stream, acc, dw, taps, g.Co, g.Ci, g.dw_io, g.nc));
     PCB_CUDA_TRY(cudaGetLastError());
@@ -1002,9 +1150,9 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     const int taps = g.KH * g.KW;
     uint8_t* s8 = static_cast<uint8_t*>(scratch);
     float* x_hi = reinterpret_cast<float*>(s8);
-    float* x_lo = reinterpret_cast<float*>(s8 + pl.xp_bytes);
+    uint16_t* x_lo = reinterpret_cast<uint16_t*>(s8 + pl.xp_bytes);
     float* w_hi = reinterpret_cast<float*>(s8 + 2 * pl.xp_bytes);
-    float* w_lo = reinterpret_cast<float*>(s8 + 2 * pl.xp_bytes + pl.w_bytes);
+    uint16_t* w_lo = reinterpret_cast<uint16_t*>(s8 + 2 * pl.xp_bytes + pl.w_bytes);
     const bool inserted = pl.ins_h != 1 || pl.ins_w != 1;
     bool chain = false;
     Prologue32 pro;
@@ -1034,25 +1182,48 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         p.tiles_m = pl.Mp / TM;
         const long long tiles = (long long)p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m;
         p.splits = 1;
-        if (2 * tiles <= sm_count() && n_k >= 2 * T_CHUNK) {
+        if (2 * tiles <= sm_count() && n_k >= 2 * T_SPLIT) {
             p.splits = sm_count() / (int)tiles;
-            if (p.splits > n_k / T_CHUNK) p.splits = n_k / T_CHUNK;
+            if (p.splits > n_k / T_SPLIT) p.splits = n_k / T_SPLIT;
             while (n_k % p.splits != 0) --p.splits;                  // equal work items: every chunk of every item holds stages
         }
         p.k_per_split = n_k / p.splits;
         const long long rounds = (tiles * p.splits + sm_count() - 1) / sm_count();
-        return rounds * p.k_per_split * (cols == 256 ? 128 : 80);        // clocks of an MMA
+        return rounds * (cols == 256 ? p.k_per_split * 750ll + 4500 : (p.k_per_split > 5 ? p.k_per_split * 512ll : 2500ll));
     };
-    // 128-pixel tiles where the longest CTA has less to do with them (an MMA of 128 columns takes 80 clocks, of 256 columns 128): only
-    // layers that leave SMs idle. Forward: 3x3, 16 channels, 32 x 32, batch 8: 25.0 -> 22.5 us; 1x1, 32 channels, 79 x 79, batch 6: 47 -> 40 us.
+    // Clocks of a stage: 750 with 256 pixels and 512 with 128 (48 and 32 KB at the 64 bytes per clock that an SM takes in), in halo form those of
+    // its four MMAs; tiles of 256 and halo tiles have single accumulators, so their epilogue (about 4500 clocks) is not hidden. 128-pixel
+    // tiles where the longest CTA has less to do with them: shallow layers and those that leave SMs idle. 3x3, 16 channels, 32 x 32, batch 8,
+    // forward: 20.3 -> 17.5 us with the present kernel (25.0 with three TF32 products and 256-pixel tiles).
     const long long narrow_cost = plan_tiles(128);
-    if (10 * plan_tiles(256) > 11 * narrow_cost) plan_tiles(128);
+    long long cost = plan_tiles(256);
+    if (10 * cost > 11 * narrow_cost) { cost = narrow_cost; plan_tiles(128); }
+    p.store_vec = 1;
+    while (p.store_vec < 8 && pl.Wout % (p.store_vec * 2) == 0 && (reinterpret_cast<uintptr_t>(out) % (size_t)(p.store_vec * 8)) == 0) p.store_vec *= 2;
+    bool halo = false;
+    p.Wt = p.Ht = p.a_slots = 0; p.halo_bytes = 0;
+    if (pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
+        const int rows = (pl.Hout + 31) / 32;
+        const int ph = (((pl.Hout + rows - 1) / rows) + 1) & ~1;
+        const int wt = 8 + (g.KW - 1) * g.DW, ht = ph + (g.KH - 1) * g.DH;
+        const uint32_t part = ((uint32_t)wt * ht * TKS * 4 + 1023) / 1024 * 1024;
+        const int room = 227 * 1024 - 1024 - 512 - (p.store_vec < 8 ? 8 * EPI_ROWS_F32_BYTES : 0) - (int)(T_HALO_TILES * 2 * part);
+        const long long tiles = (long long)((pl.Wout + 7) / 8) * ((pl.Hout + ph - 1) / ph) * g.Nb * (pl.Mp / TM);
+        const long long halo_cost = (tiles + sm_count() - 1) / sm_count() * (n_k * 16ll * ph + 4500);
+        if (ph >= 24 && wt <= 256 && ht <= 256 && room >= 6 * (int)(2 * TA_BYTES) && halo_cost < cost) {
+            halo = true;
+            p.PW = 8; p.PH = ph; p.PN = 1; p.n_cols = 8 * ph; p.Wt = wt; p.Ht = ht;
+            p.tiles_w = (pl.Wout + 7) / 8; p.tiles_h = (pl.Hout + ph - 1) / ph; p.tiles_n = g.Nb;
+            p.splits = 1; p.k_per_split = n_k;
+            p.halo_bytes = part;
+            p.a_slots = room / (int)(2 * TA_BYTES);
+            if (p.a_slots > T_MAX_SLOTS) p.a_slots = T_MAX_SLOTS;
+        }
+    }
     p.Nb = g.Nb; p.Cout = pl.Cout; p.Mvalid = g.nc * pl.Cout; p.HO = pl.Hout; p.WO = pl.Wout; p.Cp = pl.Cp;
     p.KH = g.KH; p.KW = g.KW; p.SH = pl.SH; p.SW = pl.SW; p.DH = g.DH; p.DW = g.DW;
     p.has_bias = (pass == PASS_FWD && g.has_bias) ? 1 : 0;
     p.LK = pl.LK;
-    p.store_vec = 1;
-    while (p.store_vec < 8 && pl.Wout % (p.store_vec * 2) == 0 && (reinterpret_cast<uintptr_t>(out) % (size_t)(p.store_vec * 8)) == 0) p.store_vec *= 2;
     p.rows_epi = (p.PW >= 8 && p.store_vec < 8) ? 1 : 0;
     p.off_w = inserted ? 0 : -pl.pad_left; p.off_h = inserted ? 0 : -pl.pad_top;
 
@@ -1069,7 +1240,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         const cuuint64_t dims[5] = {(cuuint64_t)pl.Cp, (cuuint64_t)pl.Wp, (cuuint64_t)pl.Hp, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
         const cuuint64_t strides[4] = {(cuuint64_t)pl.Cp * 4, (cuuint64_t)pl.Wp * pl.Cp * 4, (cuuint64_t)pl.Hp * pl.Wp * pl.Cp * 4,
                                        (cuuint64_t)g.Nb * pl.Hp * pl.Wp * pl.Cp * 4};
-        const cuuint32_t box[5] = {TKS, (cuuint32_t)((p.PW - 1) * pl.SW + 1), (cuuint32_t)((p.PH - 1) * pl.SH + 1), (cuuint32_t)p.PN, 1};
+        const cuuint32_t box[5] = {TKS, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : (p.PH - 1) * pl.SH + 1), (cuuint32_t)p.PN, 1};
         const cuuint32_t es[5] = {1, (cuuint32_t)pl.SW, (cuuint32_t)pl.SH, 1, 1};
         int rc = make_tensor_map(&m_x_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_hi, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_64B, "activations hi");
         if (rc == PCB_OK) rc = make_tensor_map(&m_x_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_lo, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_64B, "activations lo");
@@ -1090,14 +1261,16 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     const int grid = n_items < sm_count() ? n_items : sm_count();
     p.n_chunks = (p.k_per_split + T_CHUNK - 1) / T_CHUNK;
     p.chunk_len = (p.k_per_split + p.n_chunks - 1) / p.n_chunks;
-    const size_t smem = T_SMEM + (p.rows_epi ? 8 * EPI_ROWS_F32_BYTES : 0);
-    if (p.n_chunks > 1) {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
-        PCB_CUDA_TRY(launch_chained_if(chain, qconv_general_tf32_kernel<true>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
-    } else {
-        PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_general_tf32_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
-        PCB_CUDA_TRY(launch_chained_if(chain, qconv_general_tf32_kernel<false>, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
-    }
+    size_t smem = (halo ? 1024 + 512 + (size_t)p.a_slots * 2 * TA_BYTES + T_HALO_TILES * 2 * (size_t)p.halo_bytes : T_SMEM) + (p.rows_epi ? 8 * EPI_ROWS_F32_BYTES : 0);
+    if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
+    auto run = [&](auto* kernel) -> int {
+        PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
+        PCB_CUDA_TRY(launch_chained_if(chain, kernel, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
+        return PCB_OK;
+    };
+    const int rc = p.n_chunks > 1 ? (halo ? run(qconv_general_tf32_kernel<true, true>) : run(qconv_general_tf32_kernel<true, false>))
+                                  : (halo ? run(qconv_general_tf32_kernel<false, true>) : run(qconv_general_tf32_kernel<false, false>));
+    if (rc != PCB_OK) return rc;
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
