@@ -97,11 +97,14 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 
     if (warp == 0) {
         // ---------------------------------------------------------------- TMA producer
-        if (lane == 0 && blockIdx.x < n_tiles) {
-            mbar_arrive_expect_tx(a_full, a_bytes);
-            for (int tap = 0; tap < p.taps; ++tap)
-                for (int l = 0; l < p.LK; ++l)
-                    tma_load_4d(a_addr + (tap * p.LK + l) * NA_BYTES, &map_w, 0, 0, 2 * l, tap, a_full);   // [2 planes][128 rows][8]
+        if (blockIdx.x < n_tiles) {
+            const bool el = elect_one();
+            if (el) {
+                mbar_arrive_expect_tx(a_full, a_bytes);
+                for (int tap = 0; tap < p.taps; ++tap)
+                    for (int l = 0; l < p.LK; ++l)
+                        tma_load_4d(a_addr + (tap * p.LK + l) * NA_BYTES, &map_w, 0, 0, 2 * l, tap, a_full);   // [2 planes][128 rows][8]
+            }
             int it = 0;
             bool ok = true;
             const uint32_t tx = (uint32_t)p.Wt * p.Ht * 32;
@@ -110,10 +113,12 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                 const int th = r / p.tiles_w, tw = r - th * p.tiles_w;
                 for (int l = 0; l < p.LK; ++l, ++it) {
                     const int s = it % NB_STAGES;
-                    ok = mbar_wait_bounded(empty_bar + 8 * s, ((it / NB_STAGES) & 1) ^ 1, status, ST_N_PRODUCER);
+                    ok = warp_wait_bounded(empty_bar + 8 * s, ((it / NB_STAGES) & 1) ^ 1, status, ST_N_PRODUCER);
                     if (!ok) break;
-                    mbar_arrive_expect_tx(full_bar + 8 * s, tx);
-                    tma_load_5d(b_addr + s * p.stage_bytes, &map_x, tw * 64, th * p.PH, 0, img, l, full_bar + 8 * s);   // [2 planes][Ht][Wt][8]
+                    if (el) {
+                        mbar_arrive_expect_tx(full_bar + 8 * s, tx);
+                        tma_load_5d(b_addr + s * p.stage_bytes, &map_x, tw * 64, th * p.PH, 0, img, l, full_bar + 8 * s);   // [2 planes][Ht][Wt][8]
+                    }
                 }
             }
         }
@@ -122,27 +127,32 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         // ---------------------------------------------------------------- MMA issuer
         const uint32_t idesc = make_idesc_f16(p.fmt, NM, n_cols, false, false);
         int it = 0, local_tile = 0;
-        bool ok = blockIdx.x >= n_tiles || mbar_wait_bounded(a_full, 0, status, ST_N_MMA);
+        const bool el = elect_one();
+        bool ok = blockIdx.x >= n_tiles || warp_wait_bounded(a_full, 0, status, ST_N_MMA);
         for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local_tile) {
             const int buf = local_tile & 1, use = local_tile >> 1;
             if (use > 0) {
-                ok = mbar_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_N_MMA);
+                ok = warp_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_N_MMA);
                 if (!ok) break;
                 tc_fence_after_sync();
             }
             for (int l = 0; l < p.LK && ok; ++l, ++it) {
                 const int s = it % NB_STAGES;
-                ok = mbar_wait_bounded(full_bar + 8 * s, (it / NB_STAGES) & 1, status, ST_N_MMA);
+                ok = warp_wait_bounded(full_bar + 8 * s, (it / NB_STAGES) & 1, status, ST_N_MMA);
                 if (!ok) break;
                 tc_fence_after_sync();
-                if (lane == 0) {
-                    const uint32_t b0 = b_addr + s * p.stage_bytes;
-                    int kh = 0, kw = 0;
-                    for (int tap = 0; tap < p.taps; ++tap) {
-                        const uint32_t shift = (uint32_t)(kh * p.DH * p.Wt + kw * p.DW) * 16;
-                        if (++kw == p.KW) { kw = 0; ++kh; }
-                        mma_f16_ss(tmem_base + buf * 256, desc_plain(a_addr + (tap * p.LK + l) * NA_BYTES, NM * 16, 128),
-                                   desc_plain(b0 + shift, p.plane_bytes, p.Wt * 16), idesc, (l > 0 || tap > 0) ? 1u : 0u);
+                if (el) {
+                    const uint64_t ad = desc_plain(a_addr + l * NA_BYTES, NM * 16, 128), bd = desc_plain(b_addr + s * p.stage_bytes, p.plane_bytes, p.Wt * 16);
+                    const uint32_t a_step = (uint32_t)(p.LK * NA_BYTES) >> 4, a_hi = (uint32_t)(ad >> 32), b_hi = (uint32_t)(bd >> 32);
+                    uint32_t a_lo = (uint32_t)ad, b_row = (uint32_t)bd;
+                    for (int kh = 0; kh < p.KH; ++kh) {
+                        uint32_t b_lo = b_row;
+                        for (int kw = 0; kw < p.KW; ++kw) {
+                            mma_f16_ss_words(tmem_base + buf * 256, a_lo, a_hi, b_lo, b_hi, idesc, (l > 0 || kh > 0 || kw > 0) ? 1u : 0u);
+                            a_lo += a_step;
+                            b_lo += p.DW;
+                        }
+                        b_row += p.DH * p.Wt;
                     }
                     mma_commit(empty_bar + 8 * s);
                     if (l == p.LK - 1) mma_commit(tmem_full + 8 * buf);
@@ -553,39 +563,47 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
     chain_next();
 
     if (warp == 0) {
-        if (lane == 0) {
+        {
+            const bool el = elect_one();
             bool ok = true;
             int img = step_beg / tiles_img, th = (step_beg - img * tiles_img) / p.tiles_w, tw = step_beg - img * tiles_img - th * p.tiles_w;
             for (int it = 0; it < n_steps && ok; ++it) {
                 const int s = it % NF_STAGES;
-                ok = mbar_wait_bounded(empty_bar + 8 * s, ((it / NF_STAGES) & 1) ^ 1, status, ST_N_PRODUCER);
+                ok = warp_wait_bounded(empty_bar + 8 * s, ((it / NF_STAGES) & 1) ^ 1, status, ST_N_PRODUCER);
                 if (!ok) break;
                 const uint32_t dst = tiles_addr + s * p.stage_bytes, bar = full_bar + 8 * s;
-                mbar_arrive_expect_tx(bar, p.y_bytes + p.x_bytes);
-                tma_load_5d(dst, &map_dy, tw * 64, th * p.PH, 0, img, 0, bar);                 // [d][plane][PH][8 px][8]
-                if (p.fold > 1) tma_load_5d(dst + p.y_bytes, &map_x, tw * 64, th * p.PH, img * 2, 0, 0, bar);   // [kw][l][plane][Ht][8][8]
-                else tma_load_5d(dst + p.y_bytes, &map_x, tw * 64, th * p.PH, 0, img, 0, bar);                  // [l][plane][Ht][Wt][8]
+                if (el) {
+                    mbar_arrive_expect_tx(bar, p.y_bytes + p.x_bytes);
+                    tma_load_5d(dst, &map_dy, tw * 64, th * p.PH, 0, img, 0, bar);                 // [d][plane][PH][8 px][8]
+                    if (p.fold > 1) tma_load_5d(dst + p.y_bytes, &map_x, tw * 64, th * p.PH, img * 2, 0, 0, bar);   // [kw][l][plane][Ht][8][8]
+                    else tma_load_5d(dst + p.y_bytes, &map_x, tw * 64, th * p.PH, 0, img, 0, bar);                  // [l][plane][Ht][Wt][8]
+                }
                 if (++tw == p.tiles_w) { tw = 0; if (++th == p.tiles_h) { th = 0; ++img; } }
             }
         }
         __syncwarp();
     } else if (warp == 1) {
         const uint32_t idesc = make_idesc_f16(p.fmt, NM, ncols, true, true);
+        const bool el = elect_one();
         bool ok = true;
         for (int it = 0; it < n_steps && ok; ++it) {
             const int s = it % NF_STAGES;
-            ok = mbar_wait_bounded(full_bar + 8 * s, (it / NF_STAGES) & 1, status, ST_N_MMA);
+            ok = warp_wait_bounded(full_bar + 8 * s, (it / NF_STAGES) & 1, status, ST_N_MMA);
             if (!ok) break;
             tc_fence_after_sync();
-            if (lane == 0) {
+            if (el) {
                 const uint32_t y0 = tiles_addr + s * p.stage_bytes, x0 = y0 + p.y_bytes;
                 int kh = tap0 / p.KW, kw = tap0 - kh * p.KW;
                 for (int tl = 0; tl < n_taps; ++tl) {
                     const uint32_t shift = (uint32_t)(kh * p.DH * p.Wt + kw * p.DW) * 16;
                     if (++kw == p.KW) { kw = 0; ++kh; }
-                    for (int kk = 0; kk < p.PH / 2; ++kk)               // 16 pixels = two rows of the tile per MMA
-                        mma_f16_ss(tmem_base + tl * ncols, desc_plain(y0 + kk * 256, 128, p.PH * 128),
-                                   desc_plain(x0 + shift + kk * 2 * p.Wt * 16, p.Wt * 16, p.plane_bytes), idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                    const uint64_t ad = desc_plain(y0, 128, p.PH * 128), bd = desc_plain(x0 + shift, p.Wt * 16, p.plane_bytes);
+                    uint32_t a_lo = (uint32_t)ad, b_lo = (uint32_t)bd;
+                    for (int kk = 0; kk < p.PH / 2; ++kk) {             // 16 pixels = two rows of the tile per MMA
+                        mma_f16_ss_words(tmem_base + tl * ncols, a_lo, (uint32_t)(ad >> 32), b_lo, (uint32_t)(bd >> 32), idesc, (it > 0 || kk > 0) ? 1u : 0u);
+                        a_lo += 256 >> 4;
+                        b_lo += 2 * p.Wt;
+                    }
                 }
                 mma_commit(empty_bar + 8 * s);
                 if (it == n_steps - 1) mma_commit(tmem_full);
