@@ -42,7 +42,7 @@ constexpr int ST_N_PRODUCER = 0x10000, ST_N_MMA = 0x20000, ST_N_EPILOGUE = 0x400
 struct NParams {
     int Nb, Mvalid, Cout, HO, WO;        // batch; valid rows (components x Cout); output plane
     int KH, KW, DH, DW;
-    int PH;                              // output tile = 8 x PH pixels of one image (PH even, <= 32)
+    int PH;                              // output tile = 8 x PH pixels of one image (PH even, <= 32), 16 x PH (PH <= 16) in the wide form
     int Wt, Ht;                          // halo tile
     int tiles_w, tiles_h;
     int LK, taps;
@@ -60,9 +60,18 @@ __device__ __forceinline__ uint64_t desc_plain(uint32_t smem_addr, uint32_t lead
            DESC_VERSION_SM100;
 }
 
+// K-major operand with 64-byte rows, 64-byte swizzle.
+__device__ __forceinline__ uint64_t desc_rows64(uint32_t smem_addr) {
+    return (uint64_t)((smem_addr & 0x3FFFFu) >> 4) | ((uint64_t)1 << 16) | ((uint64_t)(512 >> 4) << 32) | DESC_VERSION_SM100 | (4ull << 61);
+}
+
 // ===================================================================================================
 // Forward / backward-data: D[(d,co), pixel] = sum over (tap, l, ci) of Wexp * x, tile 128 x (8 x PH pixels).
+// WIDE: the tile is two such blocks of 8 pixels side by side, an MMA each per tap, so that a lane stores runs of 16 pixels (whole 32-byte
+// sectors): taken where image rows are whole runs. The 16-byte runs of single blocks
+// bound the 7x7/2 stem (112 x 112 outputs): forward 158 -> 111 us at batch 128.
 // ===================================================================================================
+template <bool WIDE>
 __global__ void __launch_bounds__(NW_THREADS, 1)
 qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, NParams p,
                        const uint16_t* bias, uint16_t* __restrict__ out, int* __restrict__ status) {
@@ -79,7 +88,7 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 
     const int tiles_img = p.tiles_w * p.tiles_h;
     const int n_tiles = tiles_img * p.Nb;
-    const int n_cols = 8 * p.PH;
+    const int n_block = 8 * p.PH, n_cols = WIDE ? 2 * n_block : n_block;      // columns of an MMA, of the tile
 
     if (t == 0) {
         for (int s = 0; s < NB_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
@@ -117,7 +126,7 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                     if (!ok) break;
                     if (el) {
                         mbar_arrive_expect_tx(full_bar + 8 * s, tx);
-                        tma_load_5d(b_addr + s * p.stage_bytes, &map_x, tw * 64, th * p.PH, 0, img, l, full_bar + 8 * s);   // [2 planes][Ht][Wt][8]
+                        tma_load_5d(b_addr + s * p.stage_bytes, &map_x, tw * (WIDE ? 128 : 64), th * p.PH, 0, img, l, full_bar + 8 * s);   // [2 planes][Ht][Wt][8]
                     }
                 }
             }
@@ -125,7 +134,7 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
         __syncwarp();
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        const uint32_t idesc = make_idesc_f16(p.fmt, NM, n_cols, false, false);
+        const uint32_t idesc = make_idesc_f16(p.fmt, NM, n_block, false, false);
         int it = 0, local_tile = 0;
         const bool el = elect_one();
         bool ok = blockIdx.x >= n_tiles || warp_wait_bounded(a_full, 0, status, ST_N_MMA);
@@ -148,7 +157,9 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                     for (int kh = 0; kh < p.KH; ++kh) {
                         uint32_t b_lo = b_row;
                         for (int kw = 0; kw < p.KW; ++kw) {
-                            mma_f16_ss_words(tmem_base + buf * 256, a_lo, a_hi, b_lo, b_hi, idesc, (l > 0 || kh > 0 || kw > 0) ? 1u : 0u);
+                            const uint32_t acc = (l > 0 || kh > 0 || kw > 0) ? 1u : 0u;
+                            mma_f16_ss_words(tmem_base + buf * 256, a_lo, a_hi, b_lo, b_hi, idesc, acc);
+                            if (WIDE) mma_f16_ss_words(tmem_base + buf * 256 + n_block, a_lo, a_hi, b_lo + 8, b_hi, idesc, acc);
                             a_lo += a_step;
                             b_lo += p.DW;
                         }
@@ -181,7 +192,7 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
             const int buf = local_tile & 1, use = local_tile >> 1;
             const int img = tile / tiles_img, r = tile - img * tiles_img;
             const int th = r / p.tiles_w, tw = r - th * p.tiles_w;
-            const int ow0 = tw * 8, oh0 = th * p.PH;
+            const int ow0 = tw * (WIDE ? 16 : 8), oh0 = th * p.PH;
             // (no read of the status word here: 16 warps that all ask for it at every tile cost the 7x7/2 stem 3 to 6 %. Whoever gives up
             // a wait stops signalling, so a tile behind an expired wait is never announced.)
             ok = mbar_wait_bounded(tmem_full + 8 * buf, use & 1, status, ST_N_EPILOGUE);
@@ -191,8 +202,18 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
 #pragma unroll 1
             for (int col0 = part * 32; col0 < n_cols && some_rows; col0 += 128) {
                 uint32_t v[32];
-                tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256 + col0, v);
-                tmem_ld_wait();
+                if (WIDE) {                                              // two rows: eight pixels of each from either block
+                    uint32_t left[16], right[16];
+                    const uint32_t at = tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256 + col0 / 2;
+                    tmem_ld_32x32b_x16(at, left);
+                    tmem_ld_32x32b_x16(at + n_block, right);
+                    tmem_ld_wait();
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) { v[e] = left[e]; v[8 + e] = right[e]; v[16 + e] = left[8 + e]; v[24 + e] = right[8 + e]; }
+                } else {
+                    tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * 256 + col0, v);
+                    tmem_ld_wait();
+                }
                 if (!row_ok && !p.rows_epi) continue;
                 uint32_t packed[16];
 #pragma unroll
@@ -209,6 +230,15 @@ qconv_narrow_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_c
                     if (sv == 1) store_rows<1>(rbuf, packed, out, row_off, pix_off, lane);
                     else if (sv == 2) store_rows<2>(rbuf, packed, out, row_off, pix_off, lane);
                     else store_rows<4>(rbuf, packed, out, row_off, pix_off, lane);
+                    continue;
+                }
+                if (WIDE) {
+#pragma unroll
+                    for (int r = 0; r < 2; ++r) {
+                        const int oh = oh0 + (col0 >> 4) + r;
+                        if (col0 + r * 16 >= n_cols || oh >= p.HO) continue;
+                        st_global_v8(out + (((size_t)(d * p.Nb + img) * p.Cout + co) * p.HO + oh) * p.WO + ow0, &packed[8 * r]);
+                    }
                     continue;
                 }
 #pragma unroll
@@ -503,6 +533,10 @@ int launch_prologue(PlanarPrologue& pro, StatusClear* sc, cudaStream_t stream, b
 // A real-valued x (one component) leaves a map dimension free for the filter rows as well (stride: one staged row): the
 // box is then [kw][kh][plane][Ht][8 px][8] and one MMA of N = fold_h * KW * 16 columns serves fold_h filter rows: all of them (no halo
 // rows), or half of them from four rows up.
+// DIRECT: dy is read in place. Pixels are contiguous in NCHW, so a box of 32 pixels x all channels of all components x PH rows is a K-major
+// operand, 64-byte rows [row][(d, co)][32 pixels]; x boxes are 32 pixels wide too, and 16 pixels of one image row are the K of an MMA.
+// Layers whose dy nobody stages for another pass (no input gradient: the stem), where tiles of 32 pixels exceed the rows by a quarter at
+// most. Backward of the 7x7/2 stem, 224 x 224, batch 128: 209 -> 133 us, of which 70 us were the copy of dy.
 // ===================================================================================================
 constexpr int NF_STAGES = 2;
 constexpr int NF_MAX_GROUPS = 16;        // tap groups that can be given CTA shares of their own
@@ -522,7 +556,9 @@ struct NFParams {
     int fmt;
     uint32_t y_bytes, x_bytes, stage_bytes, plane_bytes;
 };
+constexpr int ND_W = 32;                 // pixels across a tile of the DIRECT form
 
+template <bool DIRECT>
 __global__ void __launch_bounds__(N_THREADS, 1)
 qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const __grid_constant__ CUtensorMap map_x, NFParams p,
                               float* __restrict__ dw32, int* __restrict__ status) {
@@ -574,8 +610,12 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
                 const uint32_t dst = tiles_addr + s * p.stage_bytes, bar = full_bar + 8 * s;
                 if (el) {
                     mbar_arrive_expect_tx(bar, p.y_bytes + p.x_bytes);
-                    tma_load_5d(dst, &map_dy, tw * 64, th * p.PH, 0, img, 0, bar);                 // [d][plane][PH][8 px][8]
-                    if (p.fold > 1) tma_load_5d(dst + p.y_bytes, &map_x, tw * 64, th * p.PH, img * 2, 0, 0, bar);   // [kw][l][plane][Ht][8][8]
+                    if (DIRECT) {
+                        tma_load_5d(dst, &map_dy, tw * ND_W, 0, 0, th * p.PH, img, bar);                            // [PH][d][co][32 px]
+                        tma_load_5d(dst + p.y_bytes, &map_x, tw * ND_W * 8, th * p.PH, img * 2, 0, 0, bar);         // [kw][l][plane][Ht][32][8]
+                    } else tma_load_5d(dst, &map_dy, tw * 64, th * p.PH, 0, img, 0, bar);                 // [d][plane][PH][8 px][8]
+                    if (DIRECT) {
+                    } else if (p.fold > 1) tma_load_5d(dst + p.y_bytes, &map_x, tw * 64, th * p.PH, img * 2, 0, 0, bar);   // [kw][l][plane][Ht][8][8]
                     else tma_load_5d(dst + p.y_bytes, &map_x, tw * 64, th * p.PH, 0, img, 0, bar);                  // [l][plane][Ht][Wt][8]
                 }
                 if (++tw == p.tiles_w) { tw = 0; if (++th == p.tiles_h) { th = 0; ++img; } }
@@ -583,7 +623,7 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
         }
         __syncwarp();
     } else if (warp == 1) {
-        const uint32_t idesc = make_idesc_f16(p.fmt, NM, ncols, true, true);
+        const uint32_t idesc = make_idesc_f16(p.fmt, NM, ncols, !DIRECT, true);
         const bool el = elect_one();
         bool ok = true;
         for (int it = 0; it < n_steps && ok; ++it) {
@@ -597,6 +637,20 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
                 for (int tl = 0; tl < n_taps; ++tl) {
                     const uint32_t shift = (uint32_t)(kh * p.DH * p.Wt + kw * p.DW) * 16;
                     if (++kw == p.KW) { kw = 0; ++kh; }
+                    if (DIRECT) {
+                        const uint64_t ad = desc_rows64(y0), bd = desc_plain(x0 + shift, 128, p.plane_bytes);
+                        uint32_t a_lo = (uint32_t)ad, b_lo = (uint32_t)bd;
+                        const uint32_t a_row = (uint32_t)(p.nc * p.Co * ND_W * 2) >> 4;
+                        for (int r = 0; r < p.PH; ++r) {
+#pragma unroll
+                            for (int j = 0; j < ND_W / 16; ++j)
+                                mma_f16_ss_words(tmem_base + tl * ncols, a_lo + 2 * j, (uint32_t)(ad >> 32), b_lo + 16 * j, (uint32_t)(bd >> 32), idesc,
+                                                 (it > 0 || r > 0 || j > 0) ? 1u : 0u);
+                            a_lo += a_row;
+                            b_lo += ND_W;
+                        }
+                        continue;
+                    }
                     const uint64_t ad = desc_plain(y0, 128, p.PH * 128), bd = desc_plain(x0 + shift, p.Wt * 16, p.plane_bytes);
                     uint32_t a_lo = (uint32_t)ad, b_lo = (uint32_t)bd;
                     for (int kk = 0; kk < p.PH / 2; ++kk) {             // 16 pixels = two rows of the tile per MMA
@@ -620,7 +674,7 @@ qconv_narrow_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, const 
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
             const int m = q * 32 + lane;                                // row -> (d, plane, channel within the plane)
-            const int chunk = m >> 3, d = chunk / p.y_planes, co = (chunk - d * p.y_planes) * 8 + (m & 7);
+            const int chunk = m >> 3, d = DIRECT ? m / p.Co : chunk / p.y_planes, co = DIRECT ? m - d * p.Co : (chunk - d * p.y_planes) * 8 + (m & 7);
             const bool row_ok = d < p.nc && co < p.Co;
             const size_t comp_stride = (size_t)p.Co * p.Ci;
             for (int tl = tsel; tl < n_taps; tl += 2) {
@@ -691,12 +745,13 @@ bool s2d_layer(const Geom& g) { return g.SH == 2 && g.SW == 2 && g.DH == 1 && g.
 struct NPlan {
     int Cin, Cout, Hin, Win, Hout, Wout, pad_top, pad_left, ins_h, ins_w;
     int s2d, KHe, KWe, DHe, DWe;         // effective (staged) filter
+    int wide;
     int LK, Hp, Wp, PH, Wt, Ht, tiles_w, tiles_h;
     uint32_t stage_bytes;
     size_t xp_bytes, w_bytes, smem;
 };
 
-NPlan make_nplan(Pass pass, const Geom& g) {
+NPlan make_nplan(Pass pass, const Geom& g, bool may_be_wide = true) {
     NPlan pl;
     if (pass == PASS_FWD) {
         pl.Cin = g.Ci; pl.Cout = g.Co; pl.Hin = g.H; pl.Win = g.W; pl.Hout = g.HO; pl.Wout = g.WO;
@@ -723,6 +778,17 @@ NPlan make_nplan(Pass pass, const Geom& g) {
     pl.xp_bytes = ((size_t)pl.LK * g.Nb * 2 * pl.Hp * pl.Wp * 16 + 1023) / 1024 * 1024;
     pl.w_bytes = ((size_t)pl.KHe * pl.KWe * pl.LK * NA_BYTES + 1023) / 1024 * 1024;
     pl.smem = 1024 + (size_t)pl.KHe * pl.KWe * pl.LK * NA_BYTES + (size_t)NB_STAGES * pl.stage_bytes + 256;
+    // the wide form on the same staged copy (rows past it read as zeros through the tensor map)
+    pl.wide = 0;
+    const int rows16 = (pl.Hout + 15) / 16, ph16 = (((pl.Hout + rows16 - 1) / rows16) + 1) & ~1;
+    const int wt16 = 16 + (pl.KWe - 1) * pl.DWe, ht16 = ph16 + (pl.KHe - 1) * pl.DHe;
+    const uint32_t stage16 = ((uint32_t)wt16 * ht16 * 32 + 1023) / 1024 * 1024;
+    const size_t smem16 = pl.smem - (size_t)NB_STAGES * pl.stage_bytes + (size_t)NB_STAGES * stage16;
+    if (may_be_wide && pl.Wout % 16 == 0 && wt16 <= 32 && ht16 <= 255 && smem16 <= 226 * 1024) {
+        pl.wide = 1;
+        pl.PH = ph16; pl.Wt = wt16; pl.Ht = ht16; pl.stage_bytes = stage16; pl.smem = smem16;
+        pl.tiles_h = (pl.Hout + ph16 - 1) / ph16; pl.tiles_w = pl.Wout / 16;
+    }
     return pl;
 }
 
@@ -753,7 +819,7 @@ size_t narrow_tc_scratch_bytes(Pass pass, const Geom& g) {
 int narrow_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const void* act, const void* bias, void* out, void* scratch,
                      int* status, cudaStream_t stream, StatusClear* sc) {
     const int fmt = dtype == PCB_F16 ? 0 : 1;
-    const NPlan pl = make_nplan(pass, g);
+    const NPlan pl = make_nplan(pass, g, reinterpret_cast<uintptr_t>(out) % 32 == 0);
     const int taps = pl.KHe * pl.KWe, Kp = pl.LK * 16;
     const int src_c = pl.s2d ? g.Ci : pl.Cin;            // channels of the tensor being staged
     uint8_t* xp = static_cast<uint8_t*>(scratch);
@@ -800,8 +866,9 @@ int narrow_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const v
     p.rows_epi = p.store_vec < 8 && pl.smem + N_EPI_WARPS * EPI_ROWS_BYTES <= 227 * 1024;
     size_t smem = pl.smem + (p.rows_epi ? N_EPI_WARPS * EPI_ROWS_BYTES : 0);
     if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
-    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
-    PCB_CUDA_TRY(launch_chained_if(chain, qconv_narrow_tc_kernel, grid, NW_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
+    auto* kernel = pl.wide ? qconv_narrow_tc_kernel<true> : qconv_narrow_tc_kernel<false>;
+    PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
+    PCB_CUDA_TRY(launch_chained_if(chain, kernel, grid, NW_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
 }
@@ -811,6 +878,7 @@ namespace {
 struct NFPlan {
     int s2d, KHe, KWe, DHe, DWe, Cie;    // effective (staged) filter and channels
     int LK, PH, Wt, Ht, tiles_w, tiles_h, Hp, Wp, HOp, WOp, y_planes, taps_per_group, n_groups;
+    int direct_ph;                       // tile height of the DIRECT form (0: not for this layer)
     int fold, fold_h, LKe, taps;         // kw / kh taps folded into one MMA (1 = none), columns / 16 of one MMA, MMAs per 16 pixels
     uint32_t y_bytes, x_bytes, stage_bytes;
     size_t xp_bytes, dyp_bytes, acc_bytes, smem;
@@ -862,6 +930,18 @@ NFPlan make_nfplan(const Geom& g) {
         f.smem = 1024 + 1024 + (size_t)NF_STAGES * f.stage_bytes + slack;
         if (f.smem <= 226 * 1024 || f.PH <= 2) break;
     }
+    // the DIRECT form: the tile height that two stages leave room for, and where 32-pixel tiles waste little of the rows
+    f.direct_ph = 0;
+    const int rows_m = g.nc * g.Co;
+    if (f.fold > 1 && g.plain && g.WO % 8 == 0 && rows_m % 8 == 0 && rows_m <= NM && g.Co <= 256 && 4 * round_up(g.WO, ND_W) <= 5 * g.WO) {
+        const uint32_t y_row = (uint32_t)rows_m * ND_W * 2, x_row = (uint32_t)f.LKe * 2 * ND_W * 16, halo = (f.KHe - f.fold_h) * f.DHe;
+        // (the M = 128 operand reads up to 8 KB from the start of a row of dy)
+        const int fit = ((226 * 1024 - 2048 - 8192) / NF_STAGES / 1024 * 1024 - (int)(halo * x_row)) / (int)(y_row + x_row);
+        if (fit >= 2) {
+            const int r = (g.HO + fit - 1) / fit;
+            f.direct_ph = (g.HO + r - 1) / r;
+        }
+    }
     f.xp_bytes = ((size_t)f.LK * g.Nb * 2 * f.Hp * f.Wp * 16 + 1023) / 1024 * 1024;
     f.dyp_bytes = ((size_t)g.nc * g.Nb * f.y_planes * f.HOp * f.WOp * 16 + 1023) / 1024 * 1024;
     f.acc_bytes = ((size_t)g.nc * g.Co * f.Cie * f.KHe * f.KWe * sizeof(float) + 1023) / 1024 * 1024;
@@ -898,7 +978,17 @@ bool narrow_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes) {
 int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* x, void* dw, void* scratch, int* status, cudaStream_t stream,
                             const void* kept_x, const StagedView* kept_dy, StatusClear* sc) {
     const int fmt = dtype == PCB_F16 ? 0 : 1;
-    const NFPlan f = make_nfplan(g);
+    NFPlan f = make_nfplan(g);
+    // dy in place, unless backward-data has staged it
+    const bool direct = !kept_dy && f.direct_ph > 0 && (reinterpret_cast<uintptr_t>(dy) & 15u) == 0;
+    if (direct) {
+        f.PH = f.direct_ph; f.tiles_h = (g.HO + f.PH - 1) / f.PH; f.tiles_w = (g.WO + ND_W - 1) / ND_W;
+        f.Ht = f.PH + (f.KHe - f.fold_h) * f.DHe; f.Wt = ND_W;
+        f.y_bytes = (uint32_t)g.nc * g.Co * ND_W * 2 * f.PH;
+        f.x_bytes = (uint32_t)f.LKe * 2 * f.Ht * ND_W * 16;
+        f.stage_bytes = (f.y_bytes + f.x_bytes + 1023) / 1024 * 1024;
+        f.smem = 1024 + 1024 + (size_t)NF_STAGES * f.stage_bytes + 8192;
+    }
     const int taps = f.KHe * f.KWe;                 // filter taps of the staged problem (the folded form issues KHe MMAs per 16 pixels)
     // the forward pass of a narrow layer stages x exactly as this one does: a copy it kept is read in place
     uint8_t* xp = kept_x ? static_cast<uint8_t*>(const_cast<void*>(kept_x)) : static_cast<uint8_t*>(scratch);
@@ -909,7 +999,7 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
         // x: padded planar copy (space-to-depth for the stride-2 stem); dy: planar copy rounded up to whole tiles
         PlanarPrologue pro;
         if (!kept_x) add_planar_job(pro, x, xp, f.LK * g.Nb, g.Ci, g.H, g.W, f.Hp, f.Wp, 2, g.PT, g.PL, 1, 1, f.s2d);
-        if (!kept_dy) add_planar_job(pro, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, f.HOp, f.WOp, f.y_planes, 0, 0, 1, 1, 0);
+        if (!kept_dy && !direct) add_planar_job(pro, dy, dyp, g.nc * g.Nb, g.Co, g.HO, g.WO, f.HOp, f.WOp, f.y_planes, 0, 0, 1, 1, 0);
         pro.zero = reinterpret_cast<uint4*>(acc);
         pro.zero_units = (unsigned)(f.acc_bytes / 16);
         pro.zero_blocks = grid_cap(pro.zero_units, 4 * NP_THREADS, 1);
@@ -959,7 +1049,13 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
                                        (cuuint64_t)g.Nb * f.y_planes * f.HOp * f.WOp * 16};
         const cuuint32_t box[5] = {64, (cuuint32_t)f.PH, (cuuint32_t)f.y_planes, 1, (cuuint32_t)g.nc};
         int rc;
-        if (kept_dy) {
+        if (direct) {   // (w, co, d, h, image) of the caller's tensor
+            const size_t plane = (size_t)g.HO * g.WO * 2;
+            const cuuint64_t ddims[5] = {(cuuint64_t)g.WO, (cuuint64_t)g.Co, (cuuint64_t)g.nc, (cuuint64_t)g.HO, (cuuint64_t)g.Nb};
+            const cuuint64_t dstrides[4] = {plane, (cuuint64_t)g.Nb * g.Co * plane, (cuuint64_t)g.WO * 2, (cuuint64_t)g.Co * plane};
+            const cuuint32_t dbox[5] = {ND_W, (cuuint32_t)g.Co, (cuuint32_t)g.nc, (cuuint32_t)f.PH, 1};
+            rc = make_tensor_map(&map_dy, dt, dy, 5, ddims, dstrides, dbox, nullptr, CU_TENSOR_MAP_SWIZZLE_64B, "narrow dy (in place)");
+        } else if (kept_dy) {
             // the copy backward-data staged: [d][img][2 planes][Hp][Wp][8] with pixel (0, 0) at (pad_top, pad_left); only the
             // HO x WO pixels are inside the map, so whatever a tile box takes beyond them reads as zeros
             const size_t plane = (size_t)kept_dy->Hp * kept_dy->Wp * 16;
@@ -984,7 +1080,7 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
                                     (cuuint64_t)f.fold};
         const cuuint64_t strides[4] = {(cuuint64_t)f.Wp * 16, plane, fh ? (cuuint64_t)f.DHe * f.Wp * 16 : (cuuint64_t)g.Nb * 2 * plane,
                                        (cuuint64_t)f.DWe * 16};
-        const cuuint32_t box[5] = {64, (cuuint32_t)f.Ht, 2, (cuuint32_t)(fh ? f.fold_h : f.LK), (cuuint32_t)f.fold};
+        const cuuint32_t box[5] = {(cuuint32_t)(direct ? ND_W * 8 : 64), (cuuint32_t)f.Ht, 2, (cuuint32_t)(fh ? f.fold_h : f.LK), (cuuint32_t)f.fold};
         const int rc = make_tensor_map(&map_x, dt, xp, 5, dims, strides, box, nullptr, CU_TENSOR_MAP_SWIZZLE_NONE, "narrow x (folded)");
         if (rc != PCB_OK) return rc;
     } else {   // xp[l][img][plane][Hp][Wp][8]; box = the halo tile of all components
@@ -996,8 +1092,9 @@ int narrow_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void
         if (rc != PCB_OK) return rc;
     }
     const size_t fsmem = f.smem < ONE_CTA_SMEM ? ONE_CTA_SMEM : f.smem;
-    PCB_CUDA_TRY(cudaFuncSetAttribute(qconv_narrow_filter_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
-    PCB_CUDA_TRY(launch_chained_if(chain, qconv_narrow_filter_tc_kernel, grid, N_THREADS, fsmem, stream, map_dy, map_x, p, acc, status));
+    auto* kernel = direct ? qconv_narrow_filter_tc_kernel<true> : qconv_narrow_filter_tc_kernel<false>;
+    PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
+    PCB_CUDA_TRY(launch_chained_if(chain, kernel, grid, N_THREADS, fsmem, stream, map_dy, map_x, p, acc, status));
     PCB_CUDA_TRY(cudaGetLastError());
     const size_t per_tap = (size_t)g.nc * g.Co * g.Ci;
     const int blocks = grid_cap(per_tap * g.KH * g.KW, 256, 16);
