@@ -62,6 +62,8 @@ struct GParams {
     int exact;                   // plane mode with a tile box of exactly PN whole planes (WO x HO x PN pixels, any plane size up to
                                  // 256 pixels): the MMAs are n_cols = PN * WO * HO rounded up to 16 columns wide
     uint32_t b_tx;               // bytes one activation box brings (plain and DUAL forms)
+    int split_h, split_n;        // PAIR: pixel rows and images from the even CTA's half of the tile box to the odd one's
+    int half_valid;              // PAIR, exact: pixels of a half (its columns are rounded up to 8)
     int rows_epi;                // NCHW output whose image rows are not 16-byte aligned: stored through shared memory (store_rows)
     int PT, PL;                  // DUAL form: padding of the strided layer
 };
@@ -115,18 +117,39 @@ __device__ __forceinline__ void plane_pack(const uint32_t (&v)[32], int col0, co
 
 // The same for a box of exactly PN whole planes: column j is pixel j % (HO * WO) of image j / (HO * WO) of the tile, in the
 // order the plane is stored, so a thread's columns are runs of consecutive elements of its channel plane.
+// PAIR: the second half of the columns starts with pixel half_valid.
+// EVEN: planes of an even number of pixels, two of which are stored at a time.
+template <bool PAIR, bool EVEN>
 __device__ __forceinline__ void plane_pack_exact(const uint32_t (&v)[32], int col0, const GParams& p, uint16_t* mine, int HWo, float badd) {
-    int nl = col0 / HWo, pix = col0 - nl * HWo;
-    const int valid = p.PN * HWo;
+    constexpr int S = EVEN ? 2 : 1;
+    const int half_cols = p.n_cols / 2;
+    int at = col0;                                       // pixel of the tile; `left`: columns until the padding of the half (or of the tile)
+    int left = PAIR ? p.half_valid - col0 : p.PN * HWo - col0;
+    if (PAIR && col0 >= half_cols) { at = p.half_valid + col0 - half_cols; left = 2 * p.half_valid - at; }
+    const int edge = PAIR ? half_cols - col0 : -1;       // (a multiple of 8)
+    int nl = at / HWo, pix = at - nl * HWo;
+    uint16_t* dst = mine + (size_t)nl * GM * HWo + pix;
 #pragma unroll
-    for (int e = 0; e < 32; ++e) {
-        if (col0 + e < valid) {
-            const float f = __uint_as_float(v[e]) + badd;
-            uint16_t bits;
-            if (p.fmt == 0) bits = __half_as_ushort(__float2half_rn(f)); else bits = __bfloat16_as_ushort(__float2bfloat16_rn(f));
-            mine[(size_t)nl * GM * HWo + pix] = bits;
+    for (int e = 0; e < 32; e += S) {
+        if (PAIR && e % 8 == 0 && e > 0 && e == edge) {
+            left = p.half_valid + e;
+            nl = p.half_valid / HWo; pix = p.half_valid - nl * HWo;
+            dst = mine + (size_t)nl * GM * HWo + pix;
         }
-        if (++pix == HWo) { pix = 0; ++nl; }
+        if (e < left) {
+            const float f0 = __uint_as_float(v[e]) + badd;
+            if (EVEN) {
+                const float f1 = __uint_as_float(v[e + 1]) + badd;
+                uint32_t both;
+                if (p.fmt == 0) { const __half2 h = __floats2half2_rn(f0, f1); both = *reinterpret_cast<const uint32_t*>(&h); }
+                else { const __nv_bfloat162 h = __floats2bfloat162_rn(f0, f1); both = *reinterpret_cast<const uint32_t*>(&h); }
+                *reinterpret_cast<uint32_t*>(dst) = both;
+            } else {
+                *dst = p.fmt == 0 ? __half_as_ushort(__float2half_rn(f0)) : __bfloat16_as_ushort(__float2bfloat16_rn(f0));
+            }
+        }
+        dst += S;
+        if ((pix += S) == HWo) { pix = 0; dst += (size_t)(GM - 1) * HWo; }
     }
 }
 
@@ -149,12 +172,19 @@ template <int KS, bool DUAL> constexpr int G_MAX_STAGES = KS == 64 ? (DUAL ? 6 :
 // and the epilogue interleaves the two accumulators into runs of neighbouring pixels of dx. The layer's FLOPs are executed once
 // (a convolution of a zero-inserted dy executes four times as many) from one compact copy of dy, in one launch. Bound by the
 // operand traffic from L2: 32 KB per four MMAs of 128 x 128 x 16.
-template <int KS, bool HALO, bool DUAL>
+//
+// PAIR (not DUAL): a cluster of two CTAs takes two neighbouring row tiles and half of the pixels of the tile box each (cta_group::2): per SM
+// 32 KB instead of 48 KB from L2 for four MMAs of 128 x 256 x 16, and 7.5 instead of 11 KB of operands from shared memory per MMA of the halo
+// form. Without / with, under the power limit: 1x1 256 at 14, bf16, forward 94 / 82 us; 3x3 stride 2, 128 at 28, forward 184 / 157; forward +
+// backward of 3x3 64 at 56 1471 / 1362, channels-last 1164 / 1116.
+template <int KS, bool HALO, bool DUAL, bool PAIR>
 __global__ void __launch_bounds__(G_THREADS, 1)
 qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GParams p,
                         const uint16_t* bias, uint16_t* __restrict__ out, int* __restrict__ status) {
-    constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = (DUAL ? GN / 2 : GN) * KS * 2;
-    constexpr int MAX_STAGES = HALO ? H_MAX_SLOTS : G_MAX_STAGES<KS, DUAL>;
+    static_assert(!(DUAL && PAIR), "forms");
+    constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = (DUAL || PAIR ? GN / 2 : GN) * KS * 2;
+    constexpr int MAX_STAGES = HALO ? H_MAX_SLOTS : G_MAX_STAGES<KS, DUAL || PAIR>;
+    const int rank = PAIR ? (int)cluster_ctarank() : 0, first = PAIR ? blockIdx.x / 2 : blockIdx.x, step = PAIR ? gridDim.x / 2 : gridDim.x;
     const uint32_t STAGE = HALO ? A_BYTES * p.a_taps : A_BYTES + B_BYTES;      // HALO: one slot of the filter ring
     const int STAGES = HALO ? p.a_slots : p.n_stages;
     const int taps = p.KH * p.KW;
@@ -172,7 +202,8 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
     uint8_t* plane_buf = base + operand_bytes + 512;               // plane mode only: [image][128 rows][HO * WO]
 
     const int tiles_px = p.tiles_w * p.tiles_h * p.tiles_n;
-    const int n_tiles = tiles_px * p.tiles_m * (DUAL ? 2 : 1);
+    const int tiles_m = PAIR ? p.tiles_m / 2 : p.tiles_m;
+    const int n_tiles = tiles_px * tiles_m * (DUAL ? 2 : 1);
     const int c_steps = p.Cp / KS;
     // DUAL: the row class with more taps comes first in the tile order
     const int first_class = p.PT & 1;               // (a + PT) mod 2 == 0: taps 0, 2, ...
@@ -180,15 +211,16 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
 
     if (t == 0) {
         for (int s = 0; s < MAX_STAGES; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, 8); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, PAIR ? 16 : 8); }
         mbar_init(epi_bar, 8);
         if (HALO)
             for (int s = 0; s < H_MAX_TILES; ++s) { mbar_init(halo_full + 8 * s, 1); mbar_init(halo_empty + 8 * s, 1); }
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
+    if (warp == 1) { if (PAIR) tmem_alloc_pair(smem_u32(tmem_slot), 512); else tmem_alloc(smem_u32(tmem_slot), 512); }
     tc_fence_before_sync();
     __syncthreads();
+    if (PAIR) cluster_sync_all();                     // both CTAs' barriers exist before anything signals them
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     chain_wait();
@@ -201,9 +233,9 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             int s = 0, phase = 1;                  // ring position and the parity its `empty` barrier is waited with
             int hs = 0, hphase = 1;                // the same of the halo tiles
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x) {
-                const int tm = tile % p.tiles_m;
-                int rest = tile / p.tiles_m;
+            for (int tile = first; tile < n_tiles && ok; tile += step) {
+                const int tm = PAIR ? 2 * (tile % tiles_m) + rank : tile % tiles_m;
+                int rest = tile / tiles_m;
                 const int tw = rest % p.tiles_w; rest /= p.tiles_w;
                 const int th = rest % p.tiles_h;
                 const int tn = rest / p.tiles_h;
@@ -231,13 +263,16 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     }
                     continue;
                 }
-                const int m0 = tm * GM, ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
+                const int m0 = tm * GM, ow0 = tw * p.PW, oh0 = th * p.PH + rank * p.split_h, n0 = tn * p.PN + rank * p.split_n;
                 if (HALO) {
                     for (int l = 0; l < p.LK && ok; ++l) {
                         for (int cs = 0; cs < c_steps && ok; ++cs) {
                             ok = warp_wait_bounded(halo_empty + 8 * hs, hphase, status, ST_G_PRODUCER);
                             if (!ok) break;
-                            if (el) {
+                            if (el && PAIR) {
+                                if (rank == 0) mbar_arrive_expect_tx(halo_full + 8 * hs, 2 * (uint32_t)p.Wt * p.Ht * KS * 2);
+                                tma_load_5d_pair(halo_addr + hs * p.halo_bytes, &map_x, cs * KS, ow0 + p.off_w, oh0 + p.off_h, n0, l, map_to_cta(halo_full + 8 * hs, 0));
+                            } else if (el) {
                                 mbar_arrive_expect_tx(halo_full + 8 * hs, (uint32_t)p.Wt * p.Ht * KS * 2);
                                 tma_load_5d(halo_addr + hs * p.halo_bytes, &map_x, cs * KS, ow0 + p.off_w, oh0 + p.off_h, n0, l, halo_full + 8 * hs);   // [Ht][Wt][32 channels]
                             }
@@ -245,7 +280,10 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                             for (int tap = 0; tap < taps; tap += p.a_taps) {
                                 ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
                                 if (!ok) break;
-                                if (el) {
+                                if (el && PAIR) {
+                                    if (rank == 0) mbar_arrive_expect_tx(full_bar + 8 * s, 2 * STAGE);
+                                    tma_load_3d_pair(tiles_addr + s * STAGE, &map_w, l * p.Cp + cs * KS, m0, tap, map_to_cta(full_bar + 8 * s, 0));
+                                } else if (el) {
                                     mbar_arrive_expect_tx(full_bar + 8 * s, STAGE);
                                     tma_load_3d(tiles_addr + s * STAGE, &map_w, l * p.Cp + cs * KS, m0, tap, full_bar + 8 * s);   // [taps][128 rows][32 channels]
                                 }
@@ -263,7 +301,12 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                             ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
                             if (!ok) break;
                             const uint32_t a_dst = tiles_addr + s * STAGE, bar = full_bar + 8 * s;
-                            if (el) {
+                            if (el && PAIR) {
+                                const uint32_t lead = map_to_cta(bar, 0);
+                                if (rank == 0) mbar_arrive_expect_tx(bar, 2 * (A_BYTES + p.b_tx));
+                                tma_load_3d_pair(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, lead);
+                                tma_load_5d_pair(a_dst + A_BYTES, &map_x, cs * KS, wp0, hp0, n0, l, lead);
+                            } else if (el) {
                                 mbar_arrive_expect_tx(bar, A_BYTES + p.b_tx);
                                 tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, bar);
                                 tma_load_5d(a_dst + A_BYTES, &map_x, cs * KS, wp0, hp0, n0, l, bar);
@@ -279,12 +322,20 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
         // ---------------------------------------------------------------- MMA issuer
         // One elected lane issues (umma.cuh: elect_one); a stage's two descriptors are built once and stepped by adding to the address
         // field of their low words (16-byte units, never carrying out of the field).
-        {
+        if (rank == 0) {                              // PAIR: the even CTA issues the MMAs of both
             const bool el = elect_one();
-            const uint32_t idesc = make_idesc_f16(p.fmt, GM, DUAL ? GN / 2 : ((HALO || p.exact) ? p.n_cols : GN), false, false);
+            auto mma = [](uint32_t d, uint32_t a_lo, uint32_t a_hi, uint32_t b_lo, uint32_t b_hi, uint32_t id, uint32_t acc) {
+                if (PAIR) mma_f16_pair(d, a_lo, a_hi, b_lo, b_hi, id, acc);
+                else mma_f16_ss_words(d, a_lo, a_hi, b_lo, b_hi, id, acc);
+            };
+            auto commit = [](uint32_t bar) {          // in both CTAs
+                if (PAIR) { mma_commit_pair(bar); mma_commit_pair(map_to_cta(bar, 1)); }
+                else mma_commit(bar);
+            };
+            const uint32_t idesc = make_idesc_f16(p.fmt, PAIR ? 2 * GM : GM, DUAL ? GN / 2 : ((HALO || p.exact) ? p.n_cols : GN), false, false);
             int s = 0, phase = 0, hs = 0, hphase = 0, local_tile = 0;
             bool ok = true;
-            for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local_tile) {
+            for (int tile = first; tile < n_tiles && ok; tile += step, ++local_tile) {
                 const int buf = local_tile & 1, use = local_tile >> 1;       // use-th time this accumulator buffer is filled
                 if (use > 0) {
                     ok = warp_wait_bounded(tmem_empty + 8 * buf, (use - 1) & 1, status, ST_G_MMA);
@@ -293,7 +344,7 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 }
                 const uint32_t d_tmem = tmem_base + buf * GN;
                 if (DUAL) {
-                    const int a = first_class ^ (tile / (tiles_px * p.tiles_m)), kh0 = (a + p.PT) & 1;
+                    const int a = first_class ^ (tile / (tiles_px * tiles_m)), kh0 = (a + p.PT) & 1;
                     const int inner = p.LK * c_steps, steps = (p.KH - kh0 + 1) / 2 * p.KW * inner;
                     int kw = 0, left = inner, b = p.PL & 1;
                     uint32_t started = 0;                              // bit b: column class b's accumulator has been written
@@ -306,10 +357,10 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                         if (el) {
 #pragma unroll
                             for (int j = 0; j < KS / 16; ++j)
-                                mma_f16_ss_words(d_tmem + b * (GN / 2), (uint32_t)ad + 2 * j, (uint32_t)(ad >> 32), (uint32_t)bd + 2 * j, (uint32_t)(bd >> 32),
+                                mma(d_tmem + b * (GN / 2), (uint32_t)ad + 2 * j, (uint32_t)(ad >> 32), (uint32_t)bd + 2 * j, (uint32_t)(bd >> 32),
                                                  idesc, (j > 0 || ((started >> b) & 1u)) ? 1u : 0u);
-                            mma_commit(empty_bar + 8 * s);
-                            if (k == steps - 1) mma_commit(tmem_full + 8 * buf);
+                            commit(empty_bar + 8 * s);
+                            if (k == steps - 1) commit(tmem_full + 8 * buf);
                         }
                         started |= 1u << b;
                         if (++s == STAGES) { s = 0; phase ^= 1; }
@@ -337,19 +388,19 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                                 for (int i = 0; i < p.a_taps; ++i) {
 #pragma unroll
                                     for (int j = 0; j < KS / 16; ++j)
-                                        mma_f16_ss_words(d_tmem, a_lo + 2 * j, a_hi, b_lo + 2 * j, b_hi, idesc, (k > 0 || tap + i > 0 || j > 0) ? 1u : 0u);
+                                        mma(d_tmem, a_lo + 2 * j, a_hi, b_lo + 2 * j, b_hi, idesc, (k > 0 || tap + i > 0 || j > 0) ? 1u : 0u);
                                     a_lo += A_BYTES >> 4;
                                     b_lo += col_step;
                                 }
-                                mma_commit(empty_bar + 8 * s);
+                                commit(empty_bar + 8 * s);
                             }
                             // (a slot's taps lie in one filter row)
                             if ((kw += p.a_taps) == p.KW) { kw = 0; b_row += row_step; b_tap = b_row; } else b_tap += col_step;
                             if (++s == STAGES) { s = 0; phase ^= 1; }
                         }
                         if (el) {
-                            mma_commit(halo_empty + 8 * hs);
-                            if (k == n_k - 1) mma_commit(tmem_full + 8 * buf);
+                            commit(halo_empty + 8 * hs);
+                            if (k == n_k - 1) commit(tmem_full + 8 * buf);
                         }
                         if (++hs == p.n_stages) { hs = 0; hphase ^= 1; }
                     }
@@ -365,9 +416,9 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     if (el) {
 #pragma unroll
                         for (int j = 0; j < KS / 16; ++j)
-                            mma_f16_ss_words(d_tmem, a_lo + 2 * j, a_hi, b_lo + 2 * j, b_hi, idesc, (k > 0 || j > 0) ? 1u : 0u);
-                        mma_commit(empty_bar + 8 * s);
-                        if (k == n_k - 1) mma_commit(tmem_full + 8 * buf);
+                            mma(d_tmem, a_lo + 2 * j, a_hi, b_lo + 2 * j, b_hi, idesc, (k > 0 || j > 0) ? 1u : 0u);
+                        commit(empty_bar + 8 * s);
+                        if (k == n_k - 1) commit(tmem_full + 8 * buf);
                     }
                     if (++s == STAGES) { s = 0; phase ^= 1; }
                 }
@@ -393,10 +444,10 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             ++epi_phase;
             return __all_sync(0xffffffffu, done);
         };
-        for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local_tile) {
+        for (int tile = first; tile < n_tiles && ok; tile += step, ++local_tile) {
             const int buf = local_tile & 1, use = local_tile >> 1;
-            const int tm = tile % p.tiles_m;
-            int rest = tile / p.tiles_m;
+            const int tm = PAIR ? 2 * (tile % tiles_m) + rank : tile % tiles_m;
+            int rest = tile / tiles_m;
             const int tw = rest % p.tiles_w; rest /= p.tiles_w;
             const int th = rest % p.tiles_h;
             int tn = rest / p.tiles_h, cls = 0;
@@ -431,13 +482,17 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     const int col0 = chalf * 128 + cb * 32;
                     tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + buf * GN + col0, v);
                     tmem_ld_wait();
-                    if (p.exact) { if (col0 < p.n_cols) plane_pack_exact(v, col0, p, mine, HWo, badd); }
+                    if (p.exact) {
+                        if (col0 >= p.n_cols) continue;
+                        if ((HWo & 1) == 0 && (!PAIR || (p.half_valid & 1) == 0)) plane_pack_exact<PAIR, true>(v, col0, p, mine, HWo, badd);
+                        else plane_pack_exact<PAIR, false>(v, col0, p, mine, HWo, badd);
+                    }
                     else if (p.lw == 3) plane_pack<3>(v, col0, p, mine, HWo, badd);
                     else plane_pack<4>(v, col0, p, mine, HWo, badd);
                 }
                 tc_fence_before_sync();
                 __syncwarp();
-                if (lane == 0) mbar_arrive(tmem_empty + 8 * buf);
+                if (lane == 0) { if (PAIR) mbar_arrive_cluster(map_to_cta(tmem_empty + 8 * buf, 0)); else mbar_arrive(tmem_empty + 8 * buf); }
                 fence_proxy_async_smem();
                 ok = epi_sync();
                 if (!ok) break;
@@ -552,14 +607,15 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
             }
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(tmem_empty + 8 * buf);
+            if (lane == 0) { if (PAIR) mbar_arrive_cluster(map_to_cta(tmem_empty + 8 * buf, 0)); else mbar_arrive(tmem_empty + 8 * buf); }
         }
         if (issuer) bulk_wait_read_all();                           // shared memory must outlive the last bulk store's reads
     }
 
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, 512);
+    if (PAIR) cluster_sync_all();                     // nobody leaves while its peer may still signal its barriers or read its shared memory
+    if (warp == 1) { if (PAIR) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512); }
 }
 
 // ---- staging kernels ------------------------------------------------------------------------------
@@ -1555,11 +1611,15 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     const bool unaligned_rows = g.plain && p.store_vec < 8;
     const int epi_bytes = cl32 ? CL32_BYTES : (unaligned_rows ? ROWS_BYTES : 0);
     bool halo = false;
+    // pairs of SMs: two row tiles at a time (with fewer tiles than SMs the single-SM form spreads them wider)
+    bool pair = !pl.dual && (pl.Mp / GM) % 2 == 0;
+    p.split_h = p.split_n = p.half_valid = 0;
     p.n_cols = 256; p.Wt = p.Ht = 0; p.n_stages = 0; p.stage_bytes = 0; p.a_slots = 0; p.a_taps = 1; p.halo_bytes = 0;
     if (!pl.dual && pl.Cp % 32 == 0 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
         const int rows = (pl.Hout + 31) / 32;
         const int ph = (((pl.Hout + rows - 1) / rows) + 1) & ~1;
-        const int wt = 8 + (g.KW - 1) * g.DW, ht = ph + (g.KH - 1) * g.DH;
+        // (a pair splits the rows of the tile in two; even the halves of 24 to 32 rows are 8 x PH / 2 >= 96 columns, a multiple of 8)
+        const int wt = 8 + (g.KW - 1) * g.DW, ht = (pair ? ph / 2 : ph) + (g.KH - 1) * g.DH;
         const uint32_t tile = ((uint32_t)wt * ht * 64 + 1023) / 1024 * 1024, tap_bytes = GM * 32 * 2;
         const int room = 227 * 1024 - 1024 - 512 - epi_bytes;
         // a slot of the filter ring holds a filter row where at least four of those fit beside two halo tiles, one tap otherwise
@@ -1568,6 +1628,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         if (ph >= 24 && wt <= 256 && ht <= 256 && room >= (int)(2 * tile) + 4 * slot) {
             halo = true;
             p.PW = 8; p.PH = ph; p.PN = 1; p.n_cols = 8 * ph; p.Wt = wt; p.Ht = ht;
+            p.split_h = pair ? ph / 2 : 0;
             p.halo_bytes = tile;
             p.n_stages = room >= (int)(H_MAX_TILES * tile) + 6 * slot ? H_MAX_TILES : 2;
             p.a_slots = (room - p.n_stages * (int)tile) / slot;
@@ -1606,13 +1667,30 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
             p.n_cols = round_up(p.PW * p.PH * p.PN, 16);
             p.lw = p.lh = 0;
         }
+        // a pair: as many whole planes in each half, or half a plane of an even number of rows
+        if (pair && (HWo <= 128 || (pl.Hout % 2 == 0 && HWo <= 256))) {
+            const int planes = HWo <= 128 ? 128 / HWo : 1;
+            p.exact = 1; p.plane_mode = 1;
+            p.PW = pl.Wout; p.PH = pl.Hout; p.PN = HWo <= 128 ? 2 * planes : 1;
+            p.split_n = HWo <= 128 ? planes : 0;
+            p.split_h = HWo <= 128 ? 0 : pl.Hout / 2;
+            p.half_valid = HWo <= 128 ? planes * HWo : HWo / 2;
+            p.n_cols = 2 * round_up(p.half_valid, 8);
+            p.lw = p.lh = 0;
+        } else if (p.exact) {
+            pair = false;
+        }
+    }
+    if (pair && !halo && !p.exact) {               // halves of the power-of-two box, in the order of its columns
+        if (p.PN >= 2) p.split_n = p.PN / 2;
+        else p.split_h = p.PH / 2;
     }
     p.rows_epi = (unaligned_rows && !p.o_generic && !p.plane_mode) ? 1 : 0;
-    const int b_rows = pl.dual ? GN / 2 : GN;
-    p.b_tx = (uint32_t)(p.exact ? p.PW * p.PH * p.PN : b_rows) * (uint32_t)pl.KS * 2u;
+    const int b_rows = pl.dual || pair ? GN / 2 : GN;
+    p.b_tx = (uint32_t)(p.exact ? (pair ? p.half_valid : p.PW * p.PH * p.PN) : b_rows) * (uint32_t)pl.KS * 2u;
     const int tail_bytes = p.plane_mode ? (int)G_PLANE_BYTES : (p.o_cl32 ? CL32_BYTES : (p.rows_epi ? ROWS_BYTES : 0));
     if (!halo) {
-        const int max_stages = pl.KS == 64 ? G_MAX_STAGES<64, false> + 2 * pl.dual : (pl.KS == 32 ? G_MAX_STAGES<32, false> + 4 * pl.dual : G_MAX_STAGES<16, false>);
+        const int small = pl.dual || pair, max_stages = pl.KS == 64 ? G_MAX_STAGES<64, false> + 2 * small : (pl.KS == 32 ? G_MAX_STAGES<32, false> + 4 * small : G_MAX_STAGES<16, false>);
         const int fit = (int)((227 * 1024 - 1024 - 512 - tail_bytes) / ((GM + b_rows) * pl.KS * 2));
         p.n_stages = fit < max_stages ? fit : max_stages;
         p.stage_bytes = (uint32_t)(GM + b_rows) * pl.KS * 2;
@@ -1644,28 +1722,31 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         const cuuint64_t dims[5] = {(cuuint64_t)Cd, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
         const cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)Wd * Cd * 2, (cuuint64_t)Hd * Wd * Cd * 2, (cuuint64_t)g.Nb * Hd * Wd * Cd * 2};
         // with an element stride s the box extent is given in input elements: s * (pixels - 1) + 1 of them hold the pixels loaded
-        const cuuint32_t box[5] = {(cuuint32_t)ks, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : (p.PH - 1) * pl.SH + 1),
-                                   (cuuint32_t)p.PN, 1};
+        const int rows = p.split_h > 0 ? p.split_h : p.PH;
+        const cuuint32_t box[5] = {(cuuint32_t)ks, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : (rows - 1) * pl.SH + 1),
+                                   (cuuint32_t)(p.split_n > 0 ? p.split_n : p.PN), 1};
         const cuuint32_t es[5] = {1, (cuuint32_t)pl.SW, (cuuint32_t)pl.SH, 1, 1};
         const CUresult r = encode(&map_x, dt, 5, direct ? const_cast<void*>(act) : static_cast<void*>(xp), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
                                   CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
         if (r != CUDA_SUCCESS) { set_error("cuTensorMapEncodeTiled (activations) failed with code %d", (int)r); return PCB_ERR_CUDA; }
     }
 
-    const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * (pl.dual ? 2 : 1);
-    const int grid = n_tiles < sm_count() ? n_tiles : sm_count();
+    const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * (pl.dual ? 2 : 1) / (pair ? 2 : 1);
+    const int most = pair ? sm_count() / 2 : sm_count(), grid = (n_tiles < most ? n_tiles : most) * (pair ? 2 : 1);
     const size_t operand_bytes = halo ? (size_t)p.a_slots * p.a_taps * GM * 64 + (size_t)p.n_stages * p.halo_bytes : (size_t)p.n_stages * p.stage_bytes;
     size_t smem = 1024 + operand_bytes + 512 + tail_bytes;
     if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
     auto run = [&](auto* kernel) -> int {
         PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
-        PCB_CUDA_TRY(launch_chained_if(chain, kernel, grid, G_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
+        PCB_CUDA_TRY(launch_clusters(pair ? 2 : 1, chain, kernel, grid, G_THREADS, smem, stream, map_w, map_x, p, (const uint16_t*)bias, (uint16_t*)out, status));
         return PCB_OK;
     };
+    auto by_slice = [&](auto* k64, auto* k32, auto* k16) -> int { return pl.KS == 64 ? run(k64) : (pl.KS == 32 ? run(k32) : run(k16)); };
     int rc;
-    if (pl.dual) rc = pl.KS == 64 ? run(qconv_general_tc_kernel<64, false, true>) : (pl.KS == 32 ? run(qconv_general_tc_kernel<32, false, true>) : run(qconv_general_tc_kernel<16, false, true>));
-    else if (halo) rc = run(qconv_general_tc_kernel<32, true, false>);
-    else rc = pl.KS == 64 ? run(qconv_general_tc_kernel<64, false, false>) : (pl.KS == 32 ? run(qconv_general_tc_kernel<32, false, false>) : run(qconv_general_tc_kernel<16, false, false>));
+    if (pl.dual) rc = by_slice(qconv_general_tc_kernel<64, false, true, false>, qconv_general_tc_kernel<32, false, true, false>, qconv_general_tc_kernel<16, false, true, false>);
+    else if (halo) rc = pair ? run(qconv_general_tc_kernel<32, true, false, true>) : run(qconv_general_tc_kernel<32, true, false, false>);
+    else if (pair) rc = by_slice(qconv_general_tc_kernel<64, false, false, true>, qconv_general_tc_kernel<32, false, false, true>, qconv_general_tc_kernel<16, false, false, true>);
+    else rc = by_slice(qconv_general_tc_kernel<64, false, false, false>, qconv_general_tc_kernel<32, false, false, false>, qconv_general_tc_kernel<16, false, false, false>);
     if (rc != PCB_OK) return rc;
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;

@@ -1,0 +1,65 @@
+"""General 16-bit kernel on pairs of SMs (an even number of 128-row tiles): whole planes in each half of a tile, half a plane, planes of an odd
+number of rows (which stay on single SMs), power-of-two boxes split by images and by rows, halo tiles; batches that leave halves empty; odd
+and even planes; slices of 16, 32 and 64 channels; strides, bias, channels-last."""
+import numpy as np
+import pytest
+import torch
+
+from helpers import normal, rel_err, uniform
+
+pytestmark = pytest.mark.gpu
+
+TOL = {"f16": 2.0 ** -10, "bf16": 2.0 ** -7}      # half a unit in the last place of max|ref|, twice for the sums' own error
+
+
+@pytest.fixture(scope="module")
+def gpu():
+    if not torch.cuda.is_available():
+        pytest.skip("no CUDA device")
+    import gpu_util
+    return gpu_util
+
+
+def _same(size, k, s):
+    out = -(-size // s)
+    total = max((out - 1) * s + k - size, 0)
+    return total // 2, total - total // 2
+
+
+# n, ci, co, h, w, k, stride
+@pytest.mark.parametrize("dtype,case", [
+    ("bf16", (3, 64, 128, 14, 14, 1, 1)), ("f16", (1, 40, 128, 7, 7, 3, 1)), ("f16", (5, 72, 128, 7, 7, 1, 1)), ("f16", (2, 64, 128, 13, 13, 1, 1)),
+    ("bf16", (2, 24, 256, 12, 15, 3, 1)), ("f16", (3, 48, 128, 28, 28, 3, 2)), ("f16", (1, 16, 128, 16, 16, 1, 1)), ("f16", (9, 20, 128, 5, 4, 3, 1)),
+    ("f16", (2, 64, 64, 20, 24, 1, 1)), ("bf16", (1, 40, 48, 33, 40, 3, 2)), ("f16", (3, 36, 64, 9, 11, 3, 1)), ("f16", (300, 24, 64, 2, 2, 2, 1)),
+    ("f16", (1, 64, 64, 25, 17, 3, 1)), ("bf16", (2, 32, 100, 11, 130, 3, 1)), ("f16", (1, 18, 64, 40, 300, 1, 2)),
+])
+def test_pairs(gpu, oracle, dtype, case):
+    n, ci, co, h, w, k, s = case
+    (pt, pb), (pl, pr) = _same(h, k, s), _same(w, k, s)
+    pad = (pt, pl, pb, pr)
+    x = gpu.rounded(uniform(51, (4 * n, ci, h, w)), dtype)
+    f = gpu.rounded(normal(52, (4, co, ci, k, k), std=(2.0 / (4 * ci * k * k)) ** 0.5), dtype)
+    b = gpu.rounded(uniform(53, (4, co)), dtype)
+    ref = oracle.conv2d_fwd(x, f, b, (s, s), (1, 1), pad)
+    y = gpu.run_conv_fwd(x, f, b, (s, s), pad, dtype, "16p", "tensor")
+    assert np.all(np.isfinite(y)) and rel_err(y, ref) <= TOL[dtype]
+    dy = gpu.rounded(normal(54, ref.shape), dtype)
+    rdw, rdx = oracle.conv2d_bwd(x, f, dy, (s, s), (1, 1), pad)
+    dw, dx = gpu.run_conv_bwd(x, f, dy, (s, s), pad, dtype, "16p", "tensor", True)
+    for got, want, what in ((dx, rdx, "dx"), (dw, rdw, "dw")):
+        assert np.all(np.isfinite(got)) and rel_err(got, want) <= TOL[dtype], (what, rel_err(got, want))
+
+
+@pytest.mark.parametrize("co,h,w", [(64, 26, 24), (96, 9, 10)])
+def test_pairs_channels_last(gpu, oracle, co, h, w):
+    import phoenix_core_b200 as pcb
+    n, ci = 2, 48
+    x = gpu.rounded(uniform(55, (4 * n, ci, h, w)), "f16")
+    f = gpu.rounded(normal(56, (4, co, ci, 3, 3), std=0.03), "f16")
+    ref = oracle.conv2d_fwd(x, f, None, (1, 1), (1, 1), (1, 1, 1, 1))
+    xd = torch.from_numpy(x).permute(0, 2, 3, 1).contiguous().half().cuda()
+    wd = torch.from_numpy(f).permute(0, 1, 3, 4, 2).contiguous().half().cuda()
+    desc = pcb.Conv2DFwdDescriptor(tuple(xd.shape), tuple(wd.shape), 1, 1, pcb.Padding.SAME, (), 1, pcb.Algebra.QUATERNION, pcb.DataFormat.NHWC, pcb.FilterLayout.OHWI, False)
+    y = torch.full(desc.getOutputShape(), float("nan"), dtype=torch.float16, device="cuda")
+    pcb.conv2DFwd(xd, wd, None, y, desc, gpu.context("16p"), gpu.ENGINES["tensor"])
+    assert rel_err(y.float().cpu().permute(0, 3, 1, 2).numpy(), ref) <= TOL["f16"]
