@@ -28,7 +28,7 @@ constexpr int TM = 128, TN = 256, TKS = 16;                 // tile, channels (f
 constexpr int T_THREADS = 320;
 constexpr uint32_t TA_BYTES = TM * TKS * 4, TB_BYTES = TN * TKS * 4;
 constexpr uint32_t T_STAGE = 2 * (TA_BYTES + TB_BYTES);     // hi and lo of both operands: 48 KB
-constexpr int T_STAGES = 4;
+constexpr int T_STAGES = 4, TP_STAGES = 6;                  // PAIR: half of the pixels in each CTA, 32 KB
 constexpr int T_MAX_SLOTS = 10, T_HALO_TILES = 2;           // halo form: filter slices and halo tiles in flight
 constexpr size_t T_SMEM = 1024 + T_STAGES * T_STAGE + 512;
 constexpr int ST_T_PRODUCER = 0x1000, ST_T_MMA = 0x2000, ST_T_EPILOGUE = 0x4000;
@@ -46,6 +46,7 @@ struct TParams {
     int splits, k_per_split;          // the K loop of a tile is cut into `splits` work items of k_per_split stages; with more than one
                                       // the partial results meet in the (zeroed) output by fp32 reductions
     int Wt, Ht, a_slots;              // halo form: halo tile, filter slices in flight
+    int split_h, split_n;             // PAIR: pixel rows and images from the even CTA's half of the tile box to the odd one's
     uint32_t halo_bytes;              // halo form: shared-memory pitch of the hi (and of the lo) part of a halo tile
 };
 
@@ -67,14 +68,17 @@ constexpr int T_CHUNK = 32;           // 32 stages = 64 MMAs of hi * hi = 512 fp
 // tap's MMAs read it at a shifted start address; the filter slices have a ring of their own. 20 KB instead of 48 KB from L2 per four MMAs of
 // 128 x 224: the four take 448 clocks, and an SM takes in about 64 bytes per clock. 3x3, 128 channels, 28 x 28, batch 128, forward: 2012 ->
 // 1580 us (first 20 launches), 2277 -> 1815 us under the power limit, of which 105 us are the staging.
-template <bool CHUNKED, bool HALO>
+// PAIR: a cluster of two CTAs takes two neighbouring row tiles and half of the pixels each, as in conv_tc.cu. 3x3, 128 channels, 28 x 28, batch 128,
+// forward and backward: 5239 -> 5156 us.
+template <bool CHUNKED, bool HALO, bool PAIR>
 __global__ void __launch_bounds__(T_THREADS, 1)
 qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __grid_constant__ CUtensorMap map_w_lo,
                           const __grid_constant__ CUtensorMap map_x_hi, const __grid_constant__ CUtensorMap map_x_lo, TParams p,
                           const float* bias, float* __restrict__ out, int* __restrict__ status) {
-    constexpr int MAX_SLOTS = HALO ? T_MAX_SLOTS : T_STAGES;
-    constexpr uint32_t SLOT = HALO ? 2 * TA_BYTES : T_STAGE;
-    const int slots = HALO ? p.a_slots : T_STAGES;
+    constexpr int MAX_SLOTS = HALO ? T_MAX_SLOTS : (PAIR ? TP_STAGES : T_STAGES);
+    constexpr uint32_t B_PART = PAIR ? TB_BYTES / 2 : TB_BYTES, SLOT = HALO ? 2 * TA_BYTES : 2 * (TA_BYTES + B_PART);
+    const int slots = HALO ? p.a_slots : MAX_SLOTS;
+    const int rank = PAIR ? (int)cluster_ctarank() : 0, first = PAIR ? blockIdx.x / 2 : blockIdx.x, step = PAIR ? gridDim.x / 2 : gridDim.x;
     extern __shared__ uint8_t smem_raw[];
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -86,20 +90,21 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
     const uint32_t tmem_full = smem_u32(bars + 2 * MAX_SLOTS), tmem_empty = smem_u32(bars + 2 * MAX_SLOTS + 2);
     const uint32_t halo_full = smem_u32(bars + 2 * MAX_SLOTS + 4), halo_empty = halo_full + 8 * T_HALO_TILES;
 
-    const int n_items = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * p.splits;
+    const int tiles_m = PAIR ? p.tiles_m / 2 : p.tiles_m, n_items = p.tiles_w * p.tiles_h * p.tiles_n * tiles_m * p.splits;
     const int c_steps = p.Cp / TKS, taps = p.KH * p.KW;
     const int n_k = taps * p.LK * c_steps;
     const int bufs = p.n_cols <= 128 ? 2 : 1;          // accumulators of each kind: columns 128 buf and 256 + 128 buf
 
     if (t == 0) {
         for (int s = 0; s < MAX_SLOTS; ++s) { mbar_init(full_bar + 8 * s, 1); mbar_init(empty_bar + 8 * s, 1); }
-        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, 8); }
+        for (int b = 0; b < 2; ++b) { mbar_init(tmem_full + 8 * b, 1); mbar_init(tmem_empty + 8 * b, PAIR ? 16 : 8); }
         for (int s = 0; s < T_HALO_TILES; ++s) { mbar_init(halo_full + 8 * s, 1); mbar_init(halo_empty + 8 * s, 1); }
         fence_barrier_init();
     }
-    if (warp == 1) tmem_alloc(smem_u32(tmem_slot), 512);
+    if (warp == 1) { if (PAIR) tmem_alloc_pair(smem_u32(tmem_slot), 512); else tmem_alloc(smem_u32(tmem_slot), 512); }
     tc_fence_before_sync();
     __syncthreads();
+    if (PAIR) cluster_sync_all();                     // both CTAs' barriers exist before anything signals them
     tc_fence_after_sync();
     const uint32_t tmem_base = *tmem_slot;
     chain_wait();
@@ -109,21 +114,26 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
         const bool el = elect_one();
         int s = 0, phase = 1, hs = 0, hphase = 1;
         bool ok = true;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x) {
+        for (int item = first; item < n_items && ok; item += step) {
             const int tile = item / p.splits, split = item - tile * p.splits;
-            const int tm = tile % p.tiles_m;
-            int rest = tile / p.tiles_m;
+            const int tm = PAIR ? 2 * (tile % tiles_m) + rank : tile % tiles_m;
+            int rest = tile / tiles_m;
             const int tw = rest % p.tiles_w; rest /= p.tiles_w;
             const int th = rest % p.tiles_h;
             const int tn = rest / p.tiles_h;
-            const int m0 = tm * TM, ow0 = tw * p.PW, oh0 = th * p.PH, n0 = tn * p.PN;
+            const int m0 = tm * TM, ow0 = tw * p.PW, oh0 = th * p.PH + rank * p.split_h, n0 = tn * p.PN + rank * p.split_n;
             const int k0 = split * p.k_per_split, k1 = min(n_k, k0 + p.k_per_split);
             if (HALO) {                                  // stage k = (l * c_steps + cs) * taps + tap
                 for (int l = 0; l < p.LK && ok; ++l)
                     for (int cs = 0; cs < c_steps && ok; ++cs) {
                         ok = warp_wait_bounded(halo_empty + 8 * hs, hphase, status, ST_T_PRODUCER);
                         if (!ok) break;
-                        if (el) {
+                        if (el && PAIR) {
+                            const uint32_t dst = halo_addr + hs * 2 * p.halo_bytes, lead = map_to_cta(halo_full + 8 * hs, 0);
+                            if (rank == 0) mbar_arrive_expect_tx(halo_full + 8 * hs, 4 * (uint32_t)p.Wt * p.Ht * TKS * 4);
+                            tma_load_5d_pair(dst, &map_x_hi, cs * TKS, ow0 + p.off_w, oh0 + p.off_h, n0, l, lead);
+                            tma_load_5d_pair(dst + p.halo_bytes, &map_x_lo, cs * TKS, ow0 + p.off_w, oh0 + p.off_h, n0, l, lead);
+                        } else if (el) {
                             const uint32_t dst = halo_addr + hs * 2 * p.halo_bytes, bar = halo_full + 8 * hs;
                             mbar_arrive_expect_tx(bar, 2 * (uint32_t)p.Wt * p.Ht * TKS * 4);
                             tma_load_5d(dst, &map_x_hi, cs * TKS, ow0 + p.off_w, oh0 + p.off_h, n0, l, bar);              // [Ht][Wt][16 channels]
@@ -133,7 +143,12 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                         for (int tap = 0; tap < taps; ++tap) {
                             ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_T_PRODUCER);
                             if (!ok) break;
-                            if (el) {
+                            if (el && PAIR) {
+                                const uint32_t dst = tiles_addr + s * SLOT, lead = map_to_cta(full_bar + 8 * s, 0);
+                                if (rank == 0) mbar_arrive_expect_tx(full_bar + 8 * s, 2 * SLOT);
+                                tma_load_3d_pair(dst, &map_w_hi, l * p.Cp + cs * TKS, m0, tap, lead);
+                                tma_load_3d_pair(dst + TA_BYTES, &map_w_lo, l * p.Cp + cs * TKS, m0, tap, lead);
+                            } else if (el) {
                                 const uint32_t dst = tiles_addr + s * SLOT, bar = full_bar + 8 * s;
                                 mbar_arrive_expect_tx(bar, SLOT);
                                 tma_load_3d(dst, &map_w_hi, l * p.Cp + cs * TKS, m0, tap, bar);
@@ -151,7 +166,14 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                 const int wp0 = ow0 * p.SW + kw * p.DW + p.off_w, hp0 = oh0 * p.SH + kh * p.DH + p.off_h;
                 ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_T_PRODUCER);
                 if (!ok) break;
-                if (el) {
+                if (el && PAIR) {
+                    const uint32_t dst = tiles_addr + s * SLOT, lead = map_to_cta(full_bar + 8 * s, 0);
+                    if (rank == 0) mbar_arrive_expect_tx(full_bar + 8 * s, 2 * SLOT);
+                    tma_load_3d_pair(dst, &map_w_hi, l * p.Cp + cs * TKS, m0, tap, lead);
+                    tma_load_3d_pair(dst + TA_BYTES, &map_w_lo, l * p.Cp + cs * TKS, m0, tap, lead);
+                    tma_load_5d_pair(dst + 2 * TA_BYTES, &map_x_hi, cs * TKS, wp0, hp0, n0, l, lead);
+                    tma_load_5d_pair(dst + 2 * TA_BYTES + B_PART, &map_x_lo, cs * TKS, wp0, hp0, n0, l, lead);
+                } else if (el) {
                     const uint32_t dst = tiles_addr + s * SLOT, bar = full_bar + 8 * s;
                     mbar_arrive_expect_tx(bar, 2 * (TA_BYTES + (uint32_t)p.n_cols * TKS * 4));
                     tma_load_3d(dst, &map_w_hi, l * p.Cp + cs * TKS, m0, tap, bar);
@@ -166,11 +188,16 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
         __syncwarp();
     } else if (warp == 1) {
         const bool el = elect_one();
-        const uint32_t idesc_main = make_idesc_f16(2, TM, p.n_cols, false, false), idesc_cross = make_idesc_f16(1, TM, p.n_cols, false, false);
+        constexpr int M = PAIR ? 2 * TM : TM;
+        const uint32_t idesc_main = make_idesc_f16(2, M, p.n_cols, false, false), idesc_cross = make_idesc_f16(1, M, p.n_cols, false, false);
+        auto commit = [](uint32_t bar) {              // in both CTAs
+            if (PAIR) { mma_commit_pair(bar); mma_commit_pair(map_to_cta(bar, 1)); }
+            else mma_commit(bar);
+        };
         const uint32_t row_step = (uint32_t)(p.DH * p.Wt * TKS * 4) >> 4, col_step = (uint32_t)(p.DW * TKS * 4) >> 4;      // HALO
         int s = 0, phase = 0, hs = 0, hphase = 0, unit = 0, local_item = 0;      // unit = one accumulation of hi * hi: a chunk of a tile
-        bool ok = true;
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++local_item) {
+        bool ok = rank == 0;                          // PAIR: the even CTA issues the MMAs of both
+        for (int item = first; item < n_items && ok; item += step, ++local_item) {
             const int split = item % p.splits;
             const int k0 = split * p.k_per_split, k1 = min(n_k, k0 + p.k_per_split);
             const uint32_t d_cross = tmem_base + 256 + (bufs == 2 ? (local_item & 1) * 128 : 0);
@@ -197,15 +224,23 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                         const uint32_t a_hi = tiles_addr + s * SLOT, b_hi = HALO ? halo_addr + hs * 2 * p.halo_bytes : a_hi + 2 * TA_BYTES;
                         const uint64_t ad = desc_k64(a_hi), bd = desc_k64(b_hi, HALO ? p.Wt * TKS * 4 : 512);
                         const uint32_t a0 = (uint32_t)ad, ah = (uint32_t)(ad >> 32), b0 = (uint32_t)bd + (HALO ? b_row + kw * col_step : 0u), bh = (uint32_t)(bd >> 32);
-                        const uint32_t a1 = a0 + (TA_BYTES >> 4), b1 = b0 + ((HALO ? p.halo_bytes : TB_BYTES) >> 4);
+                        const uint32_t a1 = a0 + (TA_BYTES >> 4), b1 = b0 + ((HALO ? p.halo_bytes : B_PART) >> 4);
                         // the rows of the lo parts hold [lo | x] of the filters and [x | lo] of the activations in bf16
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) mma_f16_ss_words(d_cross, a1 + 2 * j, ah, b1 + 2 * j, bh, idesc_cross, (k > k0 || j > 0) ? 1u : 0u);
+                        for (int j = 0; j < 2; ++j) {
+                            const uint32_t acc = (k > k0 || j > 0) ? 1u : 0u;
+                            if (PAIR) mma_f16_pair(d_cross, a1 + 2 * j, ah, b1 + 2 * j, bh, idesc_cross, acc);
+                            else mma_f16_ss_words(d_cross, a1 + 2 * j, ah, b1 + 2 * j, bh, idesc_cross, acc);
+                        }
 #pragma unroll
-                        for (int j = 0; j < 2; ++j) mma_tf32_ss_words(d_main, a0 + 2 * j, ah, b0 + 2 * j, bh, idesc_main, (k > k_beg || j > 0) ? 1u : 0u);
-                        mma_commit(empty_bar + 8 * s);
-                        if (HALO && tap == taps - 1) mma_commit(halo_empty + 8 * hs);
-                        if (k == k_end - 1) mma_commit(tmem_full + 8 * buf);
+                        for (int j = 0; j < 2; ++j) {
+                            const uint32_t acc = (k > k_beg || j > 0) ? 1u : 0u;
+                            if (PAIR) mma_tf32_pair(d_main, a0 + 2 * j, ah, b0 + 2 * j, bh, idesc_main, acc);
+                            else mma_tf32_ss_words(d_main, a0 + 2 * j, ah, b0 + 2 * j, bh, idesc_main, acc);
+                        }
+                        commit(empty_bar + 8 * s);
+                        if (HALO && tap == taps - 1) commit(halo_empty + 8 * hs);
+                        if (k == k_end - 1) commit(tmem_full + 8 * buf);
                     }
                     if (++s == slots) { s = 0; phase ^= 1; }
                     if (HALO) {
@@ -224,10 +259,10 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
         int unit = 0, local_item = 0;
         bool ok = true;
         const bool reduce = p.splits > 1;            // partial sums of a tile meet in the zeroed output
-        for (int item = blockIdx.x; item < n_items && ok; item += gridDim.x, ++local_item) {
+        for (int item = first; item < n_items && ok; item += step, ++local_item) {
             const int tile = item / p.splits, split = item - tile * p.splits;
-            const int tm = tile % p.tiles_m;
-            int rest = tile / p.tiles_m;
+            const int tm = PAIR ? 2 * (tile % tiles_m) + rank : tile % tiles_m;
+            int rest = tile / tiles_m;
             const int tw = rest % p.tiles_w; rest /= p.tiles_w;
             const int th = rest % p.tiles_h;
             const int tn = rest / p.tiles_h;
@@ -261,7 +296,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
                     }
                     tc_fence_before_sync();
                     __syncwarp();
-                    if (lane == 0) mbar_arrive(tmem_empty + 8 * buf);
+                    if (lane == 0) { if (PAIR) mbar_arrive_cluster(map_to_cta(tmem_empty + 8 * buf, 0)); else mbar_arrive(tmem_empty + 8 * buf); }
                 }
                 if (!ok) break;
             }
@@ -346,12 +381,13 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
             }
             tc_fence_before_sync();
             __syncwarp();
-            if (lane == 0) mbar_arrive(tmem_empty + 8 * buf);
+            if (lane == 0) { if (PAIR) mbar_arrive_cluster(map_to_cta(tmem_empty + 8 * buf, 0)); else mbar_arrive(tmem_empty + 8 * buf); }
         }
     }
     tc_fence_before_sync();
     __syncthreads();
-    if (warp == 1) tmem_dealloc(tmem_base, 512);
+    if (PAIR) cluster_sync_all();                     // nobody leaves while its peer may still signal its barriers or read its shared memory
+    if (warp == 1) { if (PAIR) tmem_dealloc_pair(tmem_base, 512); else tmem_dealloc(tmem_base, 512); }
 }
 
 // ---- staging: fp32 -> (hi, lo) ------------------------------------------------------------------------
@@ -1182,6 +1218,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         p.tiles_m = pl.Mp / TM;
         const long long tiles = (long long)p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m;
         p.splits = 1;
+        const bool two = cols == 256 && p.tiles_m % 2 == 0;         // on pairs of SMs
         if (2 * tiles <= sm_count() && n_k >= 2 * T_SPLIT) {
             p.splits = sm_count() / (int)tiles;
             if (p.splits > n_k / T_SPLIT) p.splits = n_k / T_SPLIT;
@@ -1189,9 +1226,9 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         }
         p.k_per_split = n_k / p.splits;
         const long long rounds = (tiles * p.splits + sm_count() - 1) / sm_count();
-        return rounds * (cols == 256 ? p.k_per_split * 750ll + 4500 : (p.k_per_split > 5 ? p.k_per_split * 512ll : 2500ll));
+        return rounds * (cols == 256 ? p.k_per_split * (two ? 540ll : 750ll) + 4500 : (p.k_per_split > 5 ? p.k_per_split * 512ll : 2500ll));
     };
-    // Clocks of a stage: 750 with 256 pixels and 512 with 128 (48 and 32 KB at the 64 bytes per clock that an SM takes in), in halo form those of
+    // Clocks of a stage: 750 with 256 pixels (540 on pairs) and 512 with 128 (48 and 32 KB at the 64 bytes per clock that an SM takes in), in halo form those of
     // its four MMAs; tiles of 256 and halo tiles have single accumulators, so their epilogue (about 4500 clocks) is not hidden. 128-pixel
     // tiles where the longest CTA has less to do with them: shallow layers and those that leave SMs idle. 3x3, 16 channels, 32 x 32, batch 8,
     // forward: 20.3 -> 17.5 us with the present kernel (25.0 with three TF32 products and 256-pixel tiles).
@@ -1205,7 +1242,8 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     if (pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
         const int rows = (pl.Hout + 31) / 32;
         const int ph = (((pl.Hout + rows - 1) / rows) + 1) & ~1;
-        const int wt = 8 + (g.KW - 1) * g.DW, ht = ph + (g.KH - 1) * g.DH;
+        const bool two = pl.Mp / TM % 2 == 0;
+        const int wt = 8 + (g.KW - 1) * g.DW, ht = (two ? ph / 2 : ph) + (g.KH - 1) * g.DH;
         const uint32_t part = ((uint32_t)wt * ht * TKS * 4 + 1023) / 1024 * 1024;
         const int room = 227 * 1024 - 1024 - 512 - (p.store_vec < 8 ? 8 * EPI_ROWS_F32_BYTES : 0) - (int)(T_HALO_TILES * 2 * part);
         const long long tiles = (long long)((pl.Wout + 7) / 8) * ((pl.Hout + ph - 1) / ph) * g.Nb * (pl.Mp / TM);
@@ -1224,6 +1262,9 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     p.KH = g.KH; p.KW = g.KW; p.SH = pl.SH; p.SW = pl.SW; p.DH = g.DH; p.DW = g.DW;
     p.has_bias = (pass == PASS_FWD && g.has_bias) ? 1 : 0;
     p.LK = pl.LK;
+    const bool pair = p.tiles_m % 2 == 0 && (halo || p.n_cols == 256);
+    p.split_h = p.split_n = 0;
+    if (pair) { if (p.PN >= 2) p.split_n = p.PN / 2; else p.split_h = p.PH / 2; }
     p.rows_epi = (p.PW >= 8 && p.store_vec < 8) ? 1 : 0;
     p.off_w = inserted ? 0 : -pl.pad_left; p.off_h = inserted ? 0 : -pl.pad_top;
 
@@ -1240,7 +1281,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         const cuuint64_t dims[5] = {(cuuint64_t)pl.Cp, (cuuint64_t)pl.Wp, (cuuint64_t)pl.Hp, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
         const cuuint64_t strides[4] = {(cuuint64_t)pl.Cp * 4, (cuuint64_t)pl.Wp * pl.Cp * 4, (cuuint64_t)pl.Hp * pl.Wp * pl.Cp * 4,
                                        (cuuint64_t)g.Nb * pl.Hp * pl.Wp * pl.Cp * 4};
-        const cuuint32_t box[5] = {TKS, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : (p.PH - 1) * pl.SH + 1), (cuuint32_t)p.PN, 1};
+        const cuuint32_t box[5] = {TKS, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : ((p.split_h ? p.split_h : p.PH) - 1) * pl.SH + 1), (cuuint32_t)(p.split_n ? p.split_n : p.PN), 1};
         const cuuint32_t es[5] = {1, (cuuint32_t)pl.SW, (cuuint32_t)pl.SH, 1, 1};
         int rc = make_tensor_map(&m_x_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_hi, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_64B, "activations hi");
         if (rc == PCB_OK) rc = make_tensor_map(&m_x_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_lo, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_64B, "activations lo");
@@ -1257,19 +1298,22 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         if (rc != PCB_OK) return rc;
         if (p.splits > 1 && !cleared) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
     }
-    const int n_items = n_tiles * p.splits;
-    const int grid = n_items < sm_count() ? n_items : sm_count();
+    const int n_items = n_tiles * p.splits / (pair ? 2 : 1), most = pair ? sm_count() / 2 : sm_count();
+    const int grid = (n_items < most ? n_items : most) * (pair ? 2 : 1);
     p.n_chunks = (p.k_per_split + T_CHUNK - 1) / T_CHUNK;
     p.chunk_len = (p.k_per_split + p.n_chunks - 1) / p.n_chunks;
     size_t smem = (halo ? 1024 + 512 + (size_t)p.a_slots * 2 * TA_BYTES + T_HALO_TILES * 2 * (size_t)p.halo_bytes : T_SMEM) + (p.rows_epi ? 8 * EPI_ROWS_F32_BYTES : 0);
     if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
     auto run = [&](auto* kernel) -> int {
         PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, MAX_CTA_SMEM));
-        PCB_CUDA_TRY(launch_chained_if(chain, kernel, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
+        PCB_CUDA_TRY(launch_clusters(pair ? 2 : 1, chain, kernel, grid, T_THREADS, smem, stream, m_w_hi, m_w_lo, m_x_hi, m_x_lo, p, (const float*)bias, (float*)out, status));
         return PCB_OK;
     };
-    const int rc = p.n_chunks > 1 ? (halo ? run(qconv_general_tf32_kernel<true, true>) : run(qconv_general_tf32_kernel<true, false>))
-                                  : (halo ? run(qconv_general_tf32_kernel<false, true>) : run(qconv_general_tf32_kernel<false, false>));
+    int rc;
+    if (p.n_chunks > 1) rc = halo ? (pair ? run(qconv_general_tf32_kernel<true, true, true>) : run(qconv_general_tf32_kernel<true, true, false>))
+                                  : (pair ? run(qconv_general_tf32_kernel<true, false, true>) : run(qconv_general_tf32_kernel<true, false, false>));
+    else rc = halo ? (pair ? run(qconv_general_tf32_kernel<false, true, true>) : run(qconv_general_tf32_kernel<false, true, false>))
+                   : (pair ? run(qconv_general_tf32_kernel<false, false, true>) : run(qconv_general_tf32_kernel<false, false, false>));
     if (rc != PCB_OK) return rc;
     PCB_CUDA_TRY(cudaGetLastError());
     return PCB_OK;
