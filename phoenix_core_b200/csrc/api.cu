@@ -530,16 +530,17 @@ int pcb_qdense_fwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     if (rc != PCB_OK) return rc;
     if (g.Nb == 0) return PCB_OK;
     if (!x || !w || !y || (g.has_bias && !bias)) { set_error("null tensor pointer"); return PCB_ERR_INVALID_ARGUMENT; }
-    rc = reset_status(workspace, workspace_bytes_, (cudaStream_t)stream);
-    if (rc != PCB_OK) return rc;
+    StatusClear sc = owe_status(workspace, workspace_bytes_);
     const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(y);
     const DenseBytes n = dense_bytes(desc->dtype, g);
     const bool apart = !overlaps(y, n.y, x, n.x) && !overlaps(y, n.y, w, n.w);
     if (dense_route(desc, g, all, apart, false, workspace, workspace_bytes_) == DENSE_DIRECT) {
         forget_kept(workspace);
-        return dense_tc_fwd(desc->dtype, g, x, w, bias, y, static_cast<int*>(workspace), (cudaStream_t)stream);
+        rc = dense_tc_fwd(desc->dtype, g, x, w, bias, y, static_cast<int*>(workspace), (cudaStream_t)stream, sc);
+    } else {
+        rc = run_pass(PASS_FWD, desc->dtype, variant_for(g, desc->variant), desc->engine, g, w, x, bias, y, workspace, workspace_bytes_, (cudaStream_t)stream, nullptr, &sc);
     }
-    return run_pass(PASS_FWD, desc->dtype, variant_for(g, desc->variant), desc->engine, g, w, x, bias, y, workspace, workspace_bytes_, (cudaStream_t)stream);
+    return finish_status(sc, rc, (cudaStream_t)stream);
 }
 
 int pcb_qdense_bwd(const pcb_dense_desc* desc, const void* x, const void* w, const void* dy, void* dw, void* dx,
@@ -553,8 +554,7 @@ int pcb_qdense_bwd(const pcb_dense_desc* desc, const void* x, const void* w, con
         return PCB_OK;
     }
     if (!x || !w || !dy || (desc->require_input_grad && !dx)) { set_error("null tensor pointer"); return PCB_ERR_INVALID_ARGUMENT; }
-    rc = reset_status(workspace, workspace_bytes_, (cudaStream_t)stream);
-    if (rc != PCB_OK) return rc;
+    StatusClear sc = owe_status(workspace, workspace_bytes_);
     void* gx = desc->require_input_grad ? dx : nullptr;
     const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(dy) |
                           reinterpret_cast<uintptr_t>(dw) | reinterpret_cast<uintptr_t>(gx);
@@ -564,14 +564,13 @@ int pcb_qdense_bwd(const pcb_dense_desc* desc, const void* x, const void* w, con
     const DenseRoute route = dense_route(desc, g, all, apart, true, workspace, workspace_bytes_);
     if (route != DENSE_STAGED) {
         forget_kept(workspace);
-        rc = dense_tc_bwd(desc->dtype, g, x, w, dy, dw, route == DENSE_DIRECT ? gx : nullptr, static_cast<int*>(workspace), (cudaStream_t)stream);
+        rc = dense_tc_bwd(desc->dtype, g, x, w, dy, dw, route == DENSE_DIRECT ? gx : nullptr, static_cast<int*>(workspace), (cudaStream_t)stream, sc);
     } else {
-        rc = run_pass(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g, dy, x, nullptr, dw, workspace, workspace_bytes_, (cudaStream_t)stream);
+        rc = run_pass(PASS_BWD_FILTER, desc->dtype, variant_for(g, desc->variant), desc->engine, g, dy, x, nullptr, dw, workspace, workspace_bytes_, (cudaStream_t)stream, nullptr, &sc);
     }
-    if (rc != PCB_OK || route == DENSE_DIRECT) return rc;
-    if (desc->require_input_grad)
-        rc = run_pass(PASS_BWD_DATA, desc->dtype, variant_for(g, desc->variant), desc->engine, g, w, dy, nullptr, dx, workspace, workspace_bytes_, (cudaStream_t)stream);
-    return rc;
+    if (rc == PCB_OK && route != DENSE_DIRECT && desc->require_input_grad)
+        rc = run_pass(PASS_BWD_DATA, desc->dtype, variant_for(g, desc->variant), desc->engine, g, w, dy, nullptr, dx, workspace, workspace_bytes_, (cudaStream_t)stream, nullptr, &sc);
+    return finish_status(sc, rc, (cudaStream_t)stream);
 }
 
 int pcb_qconv2d_engine_for(const pcb_conv2d_desc* desc, int pass) {

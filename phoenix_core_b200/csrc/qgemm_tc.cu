@@ -55,8 +55,8 @@ struct QProblem {
     int M, N, K;
     int o_c, o_n;        // output element (c, n, m) at c * o_c + n * o_n + m
     int tiles_m, tiles_n;
-    int chunks;          // K chunks of 64 (fp32: 32) elements
-    int split;           // CTAs that share a tile, neighbours in a cluster: slices of the K chunks
+    int stages;          // of a tile: four (one per component of A) for every K chunk of 64 (fp32: 32) elements
+    int split;           // CTAs that share a tile, neighbours in a cluster: slices of the stages
     uint32_t neg;        // bit 4 * kc + c: component c ^ kc of B enters block c negated
 };
 struct QParams {
@@ -64,6 +64,7 @@ struct QParams {
     int first_blocks;    // CTAs of prob[0]; the rest work on prob[1]
     int cluster;         // CTAs of a cluster (the larger of the two splits)
     int fmt;             // 0 = fp16, 1 = bf16, 2 = fp32 as TF32
+    int* clear;          // the call's status word, if this launch is to reset it
 };
 
 __device__ __forceinline__ uint32_t q_cluster_rank() {
@@ -82,6 +83,7 @@ __device__ __forceinline__ float ld_cluster_f32(uint32_t local_addr, uint32_t ra
     asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(v) : "r"(a) : "memory");
     return v;
 }
+__device__ __forceinline__ uint32_t ld_cluster_u32(uint32_t local_addr, uint32_t rank) { return __float_as_uint(ld_cluster_f32(local_addr, rank)); }
 __device__ __forceinline__ void st_shared_u32(uint32_t addr, uint32_t v) { asm volatile("st.shared.u32 [%0], %1;" ::"r"(addr), "r"(v) : "memory"); }
 __device__ __forceinline__ void st_shared_v2(uint32_t addr, uint32_t a, uint32_t b) {
     asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(addr), "r"(a), "r"(b) : "memory");
@@ -235,20 +237,19 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
     const int split = p.split, tile = block / split, rank = block - tile * split;
     const int m0 = (tile % p.tiles_m) * QM, n0 = (tile / p.tiles_m) * NT;
-    const int per = (p.chunks + split - 1) / split;
-    const int c_beg = min(p.chunks, rank * per), c_end = min(p.chunks, c_beg + per);
-    // stage st: chunk c_beg + st / 4, component st % 4 of A. (The grid is padded to whole clusters: CTAs past the last tile do nothing.)
-    const int n_stages = tile < p.tiles_m * p.tiles_n ? (c_end - c_beg) * 4 : 0;
+    const int per = (p.stages + split - 1) / split;
+    const int s_beg = min(p.stages, rank * per), s_end = min(p.stages, s_beg + per);
+    // stage s: chunk s / 4, component s % 4 of A. (The grid is padded to whole clusters: CTAs past the last tile do nothing.)
+    const int n_stages = tile < p.tiles_m * p.tiles_n ? s_end - s_beg : 0;
 
     bool ok = true;
-    const int seen = read_status(status);                              // asked before the first stage, needed behind the last
     if (t < Q_LOADERS) {
         // ------------------------------------------------------------------------------------------ loaders
         // group g fills stages g, g + Q_GROUPS, ...: while one group waits for its loads the others write theirs
         const int tg = t % Q_GROUP;
         constexpr int HALF = NT == 32 ? 4 : 2;                     // components of B in registers at a time
         for (int st = t / Q_GROUP; st < n_stages && ok; st += Q_GROUPS) {
-            const int kc = st & 3, k0 = (c_beg + (st >> 2)) * KC, s = st % L::STAGES;
+            const int kc = (s_beg + st) & 3, k0 = ((s_beg + st) >> 2) * KC, s = st % L::STAGES;
             uint32_t ra[QM / 4], rb[HALF][NT / 4];
             load_tile<F32, AK, QM>(ra, p.a, kc, m0, k0, tg);
 #pragma unroll
@@ -274,7 +275,7 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
             ok = __all_sync(0xffffffffu, ok);
             if (ok && lane == 0) mbar_arrive(full_bar + 8 * s);    // (not after an expired wait: the MMA thread's own wait then runs out)
         }
-    } else if (lane == 0 && n_stages > 0) {
+    } else if (n_stages > 0) {
         // ------------------------------------------------------------------------------------------ MMA issuer
         const uint32_t idesc = make_idesc_f16(F32 ? 2 : fmt, QM, L::N, !AK, !BK);
         constexpr uint32_t KROWS = F32 ? 32 : 64, KSTEP = F32 ? 8 : 16;          // K rows of a stage, K of one MMA
@@ -282,29 +283,32 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
         auto desc = [](uint32_t addr, bool kmajor) {
             return kmajor ? make_desc_kmajor(addr) : (F32 ? make_desc_mn_f32(addr, KROWS * Q_ROW_BYTES) : make_desc_mnmajor(addr, KROWS * Q_ROW_BYTES));
         };
+        const bool el = elect_one();
         int s = 0, phase = 0;
         for (int st = 0; st < n_stages; ++st) {
-            if (!mbar_wait_bounded(full_bar + 8 * s, phase, status, ST_Q_MMA)) break;
+            if (!warp_wait_bounded(full_bar + 8 * s, phase, status, ST_Q_MMA)) break;
             tc_fence_after_sync();
-            const uint32_t a_tile = tiles + s * L::STAGE, b_tile = a_tile + L::A_TILE * (F32 ? 2 : 1);
-            const uint64_t ah = desc(a_tile, AK), bh = desc(b_tile, BK);
-            if (F32) {
-                // stage st adds into accumulator st mod 4; small terms first
-                const uint32_t d = tmem_base + (uint32_t)((st % L::ACCS) * L::N);
-                const uint64_t al = desc(a_tile + L::A_TILE, AK), bl = desc(b_tile + L::B_TILE, BK);
+            if (el) {
+                const uint32_t a_tile = tiles + s * L::STAGE, b_tile = a_tile + L::A_TILE * (F32 ? 2 : 1);
+                const uint64_t ah = desc(a_tile, AK), bh = desc(b_tile, BK);
+                if (F32) {
+                    // stage st adds into accumulator st mod 4; small terms first
+                    const uint32_t d = tmem_base + (uint32_t)((st % L::ACCS) * L::N);
+                    const uint64_t al = desc(a_tile + L::A_TILE, AK), bl = desc(b_tile + L::B_TILE, BK);
 #pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                    mma_tf32_ss(d, al + AS * j, bh + BS * j, idesc, (st >= L::ACCS || j > 0) ? 1u : 0u);
-                    mma_tf32_ss(d, ah + AS * j, bl + BS * j, idesc, 1u);
-                    mma_tf32_ss(d, ah + AS * j, bh + BS * j, idesc, 1u);
+                    for (int j = 0; j < 4; ++j) {
+                        mma_tf32_ss(d, al + AS * j, bh + BS * j, idesc, (st >= L::ACCS || j > 0) ? 1u : 0u);
+                        mma_tf32_ss(d, ah + AS * j, bl + BS * j, idesc, 1u);
+                        mma_tf32_ss(d, ah + AS * j, bh + BS * j, idesc, 1u);
+                    }
+                } else {
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)                            // two accumulators in turn
+                        mma_f16_ss(tmem_base + (uint32_t)((j & 1) * L::N), ah + AS * j, bh + BS * j, idesc, (st > 0 || j > 1) ? 1u : 0u);
                 }
-            } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j)                            // two accumulators in turn
-                    mma_f16_ss(tmem_base + (uint32_t)((j & 1) * L::N), ah + AS * j, bh + BS * j, idesc, (st > 0 || j > 1) ? 1u : 0u);
+                mma_commit(empty_bar + 8 * s);
+                if (st == n_stages - 1) mma_commit(done_bar);
             }
-            mma_commit(empty_bar + 8 * s);
-            if (st == n_stages - 1) mma_commit(done_bar);
             if (++s == L::STAGES) { s = 0; phase ^= 1; }
         }
     }
@@ -314,7 +318,7 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
     const int q = warp & 3, half = warp >> 2;                          // TMEM lane quadrant, half of the columns (warps 0 .. 7)
     if (warp < 8) {
         if (n_stages > 0) ok = mbar_wait_bounded(done_bar, 0, status, ST_Q_EPILOGUE) && ok;
-        ok = warp_may_store(ok, seen);
+        ok = warp_may_store(ok, read_status(status));
         tc_fence_after_sync();
         const int row = q * 32 + lane, m = m0 + row;
 #pragma unroll 1
@@ -326,7 +330,7 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
             if (ok && n_stages > 0) {
 #pragma unroll
                 for (int acc = 0; acc < L::ACCS; ++acc) {
-                    if (F32 && acc >= n_stages) break;                 // fewer stages than accumulators (n_stages is a multiple of 4)
+                    if (F32 && acc >= n_stages) break;                 // fewer stages than accumulators
                     uint32_t v[32];
                     tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc * L::N) + col0, v);
                     tmem_ld_wait();
@@ -353,9 +357,10 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
         if (split > 1 && t < Q_LOADERS) {
             // every CTA of the tile finishes N / split columns: the partial tiles are added in rank order, four columns at a time
             // so that their reads from the other SMs overlap
-            const bool good = *reinterpret_cast<volatile int*>(status) == 0;
             const int row = t % QM, m = m0 + row, cols = L::N / split, col_beg = rank * cols;
             const uint32_t peer0 = q_cluster_rank() - (uint32_t)rank;
+            bool good = true;                                          // no CTA of the tile has given up a wait
+            for (int r = 0; r < split; ++r) good = good && ld_cluster_u32(smem_u32(status), peer0 + r) == 0u;
             constexpr int BATCH = 4;
             if (good && m < p.M) {
                 for (int col = col_beg + (t / QM) * BATCH; col < col_beg + cols; col += Q_GROUPS * BATCH) {
@@ -383,6 +388,10 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
 }
 
 // PAIR: prob[0] has layouts (AK, BK), prob[1] (AK1, BK1) -- both gradients of a dense layer in one launch.
+// The status word: every CTA keeps its own in shared memory (its waits look at no other), and ORs it into the call's word when it ends. The
+// first CTA resets that word when it starts (p.clear), instead of a launch in front of this one, which cost 2 to 3 us of a call: a CTA
+// has something to OR only after a wait of 2^31 clocks has run out, a second behind the start of its wave, and the first CTA is of the
+// first wave.
 template <bool F32, int NT, bool AK, bool BK, bool PAIR, bool AK1, bool BK1>
 __global__ void __launch_bounds__(Q_THREADS, 1) qgemm_tc_kernel(const __grid_constant__ QParams p, int* __restrict__ status) {
     typedef QLayout<F32, NT> L;
@@ -391,8 +400,10 @@ __global__ void __launch_bounds__(Q_THREADS, 1) qgemm_tc_kernel(const __grid_con
     uint8_t* base = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
     uint64_t* bars = reinterpret_cast<uint64_t*>(base + L::BODY);
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 2 * Q_MAX_STAGES + 1);
+    int* own_status = reinterpret_cast<int*>(tmem_slot + 1);
     const uint32_t full_bar = smem_u32(bars), empty_bar = smem_u32(bars + Q_MAX_STAGES), done_bar = smem_u32(bars + 2 * Q_MAX_STAGES);
     if (t == 0) {
+        *own_status = 0;
         for (int s = 0; s < L::STAGES; ++s) { mbar_init(full_bar + 8 * s, Q_GROUP / 32); mbar_init(empty_bar + 8 * s, 1); }
         mbar_init(done_bar, 1);
         fence_barrier_init();
@@ -405,17 +416,19 @@ __global__ void __launch_bounds__(Q_THREADS, 1) qgemm_tc_kernel(const __grid_con
     chain_wait();
     chain_next();
     const int block = blockIdx.x;
+    if (block == 0 && t == 0 && p.clear) *p.clear = 0;
     if (!PAIR || block < p.first_blocks)
-        q_tile<F32, NT, AK, BK>(p.prob[0], block, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, status);
+        q_tile<F32, NT, AK, BK>(p.prob[0], block, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, own_status);
     else
-        q_tile<F32, NT, AK1, BK1>(p.prob[1], block - p.first_blocks, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, status);
+        q_tile<F32, NT, AK1, BK1>(p.prob[1], block - p.first_blocks, p.cluster, p.fmt, tmem_base, smem_u32(base), full_bar, empty_bar, done_bar, own_status);
     tc_fence_before_sync();
     __syncthreads();
+    if (t == 0 && *own_status != 0) atomicOr(status, *own_status);
     if (warp == Q_LOADERS / 32) tmem_dealloc(tmem_base, L::ACCS * L::N);
 }
 
 template <bool F32, int NT, bool AK, bool BK, bool PAIR, bool AK1, bool BK1>
-int q_launch(const QParams& p, int blocks, int* status, cudaStream_t stream) {
+int q_launch(QParams p, int blocks, int* status, cudaStream_t stream, StatusClear& sc) {
     typedef QLayout<F32, NT> L;
     auto* kernel = qgemm_tc_kernel<F32, NT, AK, BK, PAIR, AK1, BK1>;
     PCB_CUDA_TRY(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::SMEM));
@@ -431,6 +444,8 @@ int q_launch(const QParams& p, int blocks, int* status, cudaStream_t stream) {
     attr[0].val.clusterDim.x = (unsigned)p.cluster; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
     cfg.attrs = attr;
     cfg.numAttrs = 2;
+    p.clear = nullptr;
+    if (sc.pending) { p.clear = sc.word; sc.pending = false; }
     PCB_CUDA_TRY(cudaLaunchKernelEx(&cfg, kernel, p, status));
     return PCB_OK;
 }
@@ -449,7 +464,7 @@ QOperand q_operand(const void* ptr, int cs, int ld, int nu, int nv, int f32) {
 void q_finish(QProblem& p, int NT, int f32, uint32_t neg) {
     p.tiles_m = (p.M + QM - 1) / QM;
     p.tiles_n = (p.N + NT - 1) / NT;
-    p.chunks = (p.K + (f32 ? 32 : 64) - 1) / (f32 ? 32 : 64);
+    p.stages = (p.K + (f32 ? 32 : 64) - 1) / (f32 ? 32 : 64) * 4;
     p.neg = neg;
 }
 uint32_t q_signs(Pass pass) {
@@ -461,7 +476,7 @@ uint32_t q_signs(Pass pass) {
         }
     return neg;
 }
-// Picks the slices of the reduced dimension of the one or two problems of a launch, and the cluster that holds them: powers of
+// Picks the slices of the stages of the one or two problems of a launch, and the cluster that holds them: powers of
 // two up to 8 (a portable cluster). The cost of a choice is rounds of the machine x (stages of the longest CTA + the fixed part
 // of a CTA, about as long as 6 stages). A cluster lies inside one group of 16 to 20 SMs and every CTA takes an SM, so clusters
 // of 4 and 8 fill only about 7/8 of the SMs at once. fp32: every slice short enough for its accumulators.
@@ -469,18 +484,18 @@ int q_plan(QParams& p, bool two, int f32) {
     long long best = -1;
     int blocks = 0;
     QProblem &a = p.prob[0], &b = p.prob[1];
-    const int most = Q_F32_STAGES_PER_ACC * Q_F32_ACCS / 4;            // chunks of an fp32 slice
+    const int most = Q_F32_STAGES_PER_ACC * Q_F32_ACCS;                // stages of an fp32 slice
     const int ta = a.tiles_m * a.tiles_n, tb = two ? b.tiles_m * b.tiles_n : 0;
     int sa_best = 1, sb_best = 1;
     for (int sa = 1; sa <= 8; sa *= 2)
         for (int sb = 1; sb <= (two ? 8 : 1); sb *= 2) {
-            const int la = (a.chunks + sa - 1) / sa, lb = two ? (b.chunks + sb - 1) / sb : 0;
-            if ((sa > 1 && sa > a.chunks) || (two && sb > 1 && sb > b.chunks)) continue;
+            const int la = (a.stages + sa - 1) / sa, lb = two ? (b.stages + sb - 1) / sb : 0;
+            if ((sa > 1 && sa > a.stages) || (two && sb > 1 && sb > b.stages)) continue;
             if (f32 && (la > most || lb > most)) continue;
             const int cl = sa > sb ? sa : sb;
             const int na = round_up(ta * sa, cl), nb = round_up(tb * sb, cl), slots = cl > 2 ? sm_count() * 7 / 8 / cl * cl : sm_count() / cl * cl;
             if (slots < cl) continue;
-            const long long cost = (long long)((na + nb + slots - 1) / slots) * ((la > lb ? la : lb) * 4 + 6 + (cl > 1 ? 1 : 0));
+            const long long cost = (long long)((na + nb + slots - 1) / slots) * ((la > lb ? la : lb) + 6 + (cl > 1 ? 1 : 0));
             if (best < 0 || cost < best) { best = cost; sa_best = sa; sb_best = sb; p.cluster = cl; p.first_blocks = na; blocks = na + nb; }
         }
     a.split = sa_best;
@@ -612,33 +627,35 @@ DenseRoute dense_tc_route(int dtype, const Geom& g, bool backward, bool need_dx)
     return fits ? route : DENSE_STAGED;
 }
 
-int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream) {
+int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream,
+                 StatusClear& sc) {
     const DensePlan d = plan_fwd(dtype, g, x, w, bias, y);
     if (d.blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
-    if (d.p.fmt == 2) return g.w_io ? q_launch<true, 32, false, true, false, false, false>(d.p, d.blocks, status, stream)
-                                    : q_launch<true, 32, true, true, false, false, false>(d.p, d.blocks, status, stream);
-    if (d.wide) return g.w_io ? q_launch<false, 64, false, true, false, false, false>(d.p, d.blocks, status, stream)
-                              : q_launch<false, 64, true, true, false, false, false>(d.p, d.blocks, status, stream);
-    return g.w_io ? q_launch<false, 32, false, true, false, false, false>(d.p, d.blocks, status, stream)
-                  : q_launch<false, 32, true, true, false, false, false>(d.p, d.blocks, status, stream);
+    if (d.p.fmt == 2) return g.w_io ? q_launch<true, 32, false, true, false, false, false>(d.p, d.blocks, status, stream, sc)
+                                    : q_launch<true, 32, true, true, false, false, false>(d.p, d.blocks, status, stream, sc);
+    if (d.wide) return g.w_io ? q_launch<false, 64, false, true, false, false, false>(d.p, d.blocks, status, stream, sc)
+                              : q_launch<false, 64, true, true, false, false, false>(d.p, d.blocks, status, stream, sc);
+    return g.w_io ? q_launch<false, 32, false, true, false, false, false>(d.p, d.blocks, status, stream, sc)
+                  : q_launch<false, 32, true, true, false, false, false>(d.p, d.blocks, status, stream, sc);
 }
 
 // dw, and dx unless it is null, in one launch.
-int dense_tc_bwd(int dtype, const Geom& g, const void* x, const void* w, const void* dy, void* dw, void* dx, int* status, cudaStream_t stream) {
+int dense_tc_bwd(int dtype, const Geom& g, const void* x, const void* w, const void* dy, void* dw, void* dx, int* status, cudaStream_t stream,
+                 StatusClear& sc) {
     const DensePlan d = plan_bwd(dtype, g, x, w, dy, dw, dx, dx != nullptr);
     if (d.blocks == 0) { set_error("no split of this dense layer"); return PCB_ERR_UNSUPPORTED; }
     const bool f32 = d.p.fmt == 2;
     if (!dx) {
-        if (f32) return q_launch<true, 32, false, false, false, false, false>(d.p, d.blocks, status, stream);
-        return d.wide ? q_launch<false, 64, false, false, false, false, false>(d.p, d.blocks, status, stream)
-                      : q_launch<false, 32, false, false, false, false, false>(d.p, d.blocks, status, stream);
+        if (f32) return q_launch<true, 32, false, false, false, false, false>(d.p, d.blocks, status, stream, sc);
+        return d.wide ? q_launch<false, 64, false, false, false, false, false>(d.p, d.blocks, status, stream, sc)
+                      : q_launch<false, 32, false, false, false, false, false>(d.p, d.blocks, status, stream, sc);
     }
-    if (f32) return g.w_io ? q_launch<true, 32, false, false, true, true, true>(d.p, d.blocks, status, stream)
-                           : q_launch<true, 32, false, false, true, false, true>(d.p, d.blocks, status, stream);
-    if (d.wide) return g.w_io ? q_launch<false, 64, false, false, true, true, true>(d.p, d.blocks, status, stream)
-                              : q_launch<false, 64, false, false, true, false, true>(d.p, d.blocks, status, stream);
-    return g.w_io ? q_launch<false, 32, false, false, true, true, true>(d.p, d.blocks, status, stream)
-                  : q_launch<false, 32, false, false, true, false, true>(d.p, d.blocks, status, stream);
+    if (f32) return g.w_io ? q_launch<true, 32, false, false, true, true, true>(d.p, d.blocks, status, stream, sc)
+                           : q_launch<true, 32, false, false, true, false, true>(d.p, d.blocks, status, stream, sc);
+    if (d.wide) return g.w_io ? q_launch<false, 64, false, false, true, true, true>(d.p, d.blocks, status, stream, sc)
+                              : q_launch<false, 64, false, false, true, false, true>(d.p, d.blocks, status, stream, sc);
+    return g.w_io ? q_launch<false, 32, false, false, true, true, true>(d.p, d.blocks, status, stream, sc)
+                  : q_launch<false, 32, false, false, true, false, true>(d.p, d.blocks, status, stream, sc);
 }
 
 }  // namespace pcb

@@ -112,8 +112,9 @@ bool dense_tc_supported(int dtype, int variant, const Geom& g);
 // faster, where the launch cannot be cut to fit the machine, or where it would not leave the SMs free that it should.
 enum DenseRoute { DENSE_STAGED, DENSE_DIRECT, DENSE_FILTER_DIRECT };
 DenseRoute dense_tc_route(int dtype, const Geom& g, bool backward, bool need_dx);
-int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream);
-int dense_tc_bwd(int dtype, const Geom& g, const void* x, const void* w, const void* dy, void* dw, void* dx /*or null*/, int* status,
-                 cudaStream_t stream);
+// (`sc`: the pending reset of the status word, done by the launch)
+int dense_tc_fwd(int dtype, const Geom& g, const void* x, const void* w, const void* bias, void* y, int* status, cudaStream_t stream, StatusClear& sc);
+int dense_tc_bwd(int dtype, const Geom& g, const void* x, const void* w, const void* dy, void* dw, void* dx /*or null*/, int* status, cudaStream_t stream,
+                 StatusClear& sc);
 
 }  // namespace pcb
