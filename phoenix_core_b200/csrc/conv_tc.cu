@@ -1611,8 +1611,9 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     const bool unaligned_rows = g.plain && p.store_vec < 8;
     const int epi_bytes = cl32 ? CL32_BYTES : (unaligned_rows ? ROWS_BYTES : 0);
     bool halo = false;
-    // pairs of SMs: two row tiles at a time (with fewer tiles than SMs the single-SM form spreads them wider)
-    bool pair = !pl.dual && (pl.Mp / GM) % 2 == 0;
+    // pairs of SMs: two row tiles at a time
+    bool pair = !pl.dual && (pl.Mp / GM) % 2 == 0 &&
+                worth_pairs((double)g.Nb * pl.Hout * pl.Wout / 256 * (pl.Mp / GM) * taps * pl.LK * (pl.Cp / 16));
     p.split_h = p.split_n = p.half_valid = 0;
     p.n_cols = 256; p.Wt = p.Ht = 0; p.n_stages = 0; p.stage_bytes = 0; p.a_slots = 0; p.a_taps = 1; p.halo_bytes = 0;
     if (!pl.dual && pl.Cp % 32 == 0 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
@@ -1883,7 +1884,8 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     const bool xmajor = filter_xmajor(g, f);
     p.TPG = xmajor ? GM / (p.LK * p.cbB) : 1;
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
-    const bool pair = !xmajor && p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0;
+    const bool pair = !xmajor && p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0 &&
+                      worth_pairs((double)taps * p.m_tiles * p.n_tiles * steps_total * (FK / 16) * p.n_tile_cols / GN);
     const int items = xmajor ? (taps + p.TPG - 1) / p.TPG : taps * p.m_tiles * p.n_tiles / (pair ? 2 : 1);
     int splits = split_count(items, pair ? sm_count() / 2 : sm_count());
     if (splits > steps_total) splits = steps_total;

@@ -1168,7 +1168,7 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     p.n_tiles = (n_cols + TN - 1) / TN;
     p.n_tile_cols = n_cols < TN ? n_cols : TN;
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
-    const bool pair = p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0;
+    const bool pair = p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0 && worth_pairs((double)taps * p.m_tiles * p.n_tiles * steps_total * 4 * p.n_tile_cols / TN);
     const int items = taps * p.m_tiles * p.n_tiles / (pair ? 2 : 1);
     int splits = split_count(items, pair ? sm_count() / 2 : sm_count());
     if (splits > steps_total) splits = steps_total;
@@ -1241,6 +1241,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     const int n_k = taps * pl.LK * (pl.Cp / TKS);
     p.store_vec = 1;
     while (p.store_vec < 8 && pl.Wout % (p.store_vec * 2) == 0 && (reinterpret_cast<uintptr_t>(out) % (size_t)(p.store_vec * 8)) == 0) p.store_vec *= 2;
+    const bool deep = worth_pairs((double)g.Nb * pl.Hout * pl.Wout / 256 * (pl.Mp / TM) * n_k * 4);
     // clocks of storing 256 pixels of 128 rows, about: aligned rows, and rows that go through shared memory
     const long long epilogue = p.store_vec < 8 ? 18000 : 5000;
     // Box of `cols` pixels that wastes the fewest columns, and the cut of its K loop. Too few tiles for the SMs (dense layers, small
@@ -1261,7 +1262,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         p.tiles_m = pl.Mp / TM;
         const long long tiles = (long long)p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m;
         p.splits = 1;
-        const bool two = cols == 256 && p.tiles_m % 2 == 0;         // on pairs of SMs
+        const bool two = cols == 256 && p.tiles_m % 2 == 0 && deep;  // on pairs of SMs
         if (2 * tiles <= sm_count() && n_k >= 2 * T_SPLIT) {
             p.splits = sm_count() / (int)tiles;
             if (p.splits > n_k / T_SPLIT) p.splits = n_k / T_SPLIT;
@@ -1284,7 +1285,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     if (pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
         const int rows = (pl.Hout + 31) / 32;
         const int ph = (((pl.Hout + rows - 1) / rows) + 1) & ~1;
-        const bool two = pl.Mp / TM % 2 == 0;
+        const bool two = pl.Mp / TM % 2 == 0 && deep;
         const int wt = 8 + (g.KW - 1) * g.DW, ht = (two ? ph / 2 : ph) + (g.KH - 1) * g.DH;
         const uint32_t part = ((uint32_t)wt * ht * TKS * 4 + 1023) / 1024 * 1024;
         const int room = 227 * 1024 - 1024 - 512 - (p.store_vec < 8 ? 8 * EPI_ROWS_F32_BYTES : 0) - (int)(T_HALO_TILES * 2 * part);
@@ -1304,7 +1305,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     p.KH = g.KH; p.KW = g.KW; p.SH = pl.SH; p.SW = pl.SW; p.DH = g.DH; p.DW = g.DW;
     p.has_bias = (pass == PASS_FWD && g.has_bias) ? 1 : 0;
     p.LK = pl.LK;
-    const bool pair = p.tiles_m % 2 == 0 && (halo || p.n_cols == 256);
+    const bool pair = p.tiles_m % 2 == 0 && deep && (halo || p.n_cols == 256);
     p.split_h = p.split_n = 0;
     if (pair) { if (p.PN >= 2) p.split_n = p.PN / 2; else p.split_h = p.PH / 2; }
     p.rows_epi = (p.PW >= 8 && p.store_vec < 8) ? 1 : 0;

@@ -389,6 +389,12 @@ inline int sm_count() {
 // 16 -> 16, 45 x 37, batch 32 26.8 / 29.0, 32 x 32, batch 16, forward 12.8 / 14.8, both gradients 31.4 / 37.3.
 inline bool chain_behind(unsigned prologue_blocks, unsigned per_sm) { return prologue_blocks <= per_sm * (unsigned)sm_count(); }
 
+// Whether a kernel of row tiles of 128 takes them two at a time on pairs of SMs (clusters of two): only where an SM has some 64 MMAs of
+// 256 columns (8192 clocks) to issue. A cluster launch starts later than a plain one. 1x1 layers, fp16, forward + backward, pairs / single, us:
+// 48 -> 56 channels, 10 x 10, batch 15 39.0 / 37.6; 56 -> 56, 30 x 30, batch 5 40.7 / 39.1; 24 -> 45, 55 x 59, batch 5 54.6 / 52.4; above the line
+// 3x3 24 -> 40, 45 x 37, batch 10, forward 24.9 / 25.7.
+inline bool worth_pairs(double mmas) { return mmas >= 64.0 * sm_count(); }
+
 inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
 // Number of slices to cut each of `items` work items into when every CTA occupies a whole SM: the CTAs must fill
 // one, two or three rounds of the machine as exactly as possible (one CTA more than a round costs a whole round). A further
