@@ -62,7 +62,7 @@ struct GParams {
     int exact;                   // plane mode with a tile box of exactly PN whole planes (WO x HO x PN pixels, any plane size up to
                                  // 256 pixels): the MMAs are n_cols = PN * WO * HO rounded up to 16 columns wide
     uint32_t b_tx;               // bytes one activation box brings (plain and DUAL forms)
-    int split_h, split_n;        // PAIR: pixel rows and images from the even CTA's half of the tile box to the odd one's
+    int split_w, split_h, split_n;   // PAIR: pixels, pixel rows and images from the even CTA's half of the tile box to the odd one's
     int half_valid;              // PAIR, exact: pixels of a half (its columns are rounded up to 8)
     int rows_epi;                // NCHW output whose image rows are not 16-byte aligned: stored through shared memory (store_rows)
     int PT, PL;                  // DUAL form: padding of the strided layer
@@ -263,7 +263,7 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                     }
                     continue;
                 }
-                const int m0 = tm * GM, ow0 = tw * p.PW, oh0 = th * p.PH + rank * p.split_h, n0 = tn * p.PN + rank * p.split_n;
+                const int m0 = tm * GM, ow0 = tw * p.PW + rank * p.split_w, oh0 = th * p.PH + rank * p.split_h, n0 = tn * p.PN + rank * p.split_n;
                 if (HALO) {
                     for (int l = 0; l < p.LK && ok; ++l) {
                         for (int cs = 0; cs < c_steps && ok; ++cs) {
@@ -1528,11 +1528,14 @@ size_t conv_tc_scratch_bytes(Pass pass, const Geom& g) {
     return pl.xp_bytes + pl.w_bytes;
 }
 
-int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const void* act, const void* bias, void* out,
+int conv_tc_launch(Pass pass, int dtype, const Geom& layer, const void* w, const void* act, const void* bias, void* out,
                    void* scratch, int* status, cudaStream_t stream, StatusClear* sc) {
     EncodeTiledFn encode = encode_fn();
     if (!encode) { set_error("cuTensorMapEncodeTiled is not available from the driver"); return PCB_ERR_CUDA; }
     const int fmt = dtype == PCB_F16 ? 0 : 1;
+    // (planes that leave whole, see the plane mode below, stay planes)
+    const bool planes = layer.H * layer.W <= 256 && (pass == PASS_FWD ? layer.Co : layer.Ci) % GM == 0;
+    const Geom g = planes ? layer : flat_pixels(layer);
     const Plan pl = make_plan(pass, g);
     const int taps = g.KH * g.KW;
     uint8_t* xp = static_cast<uint8_t*>(scratch);
@@ -1584,7 +1587,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         long long best = -1;
         // (dense layers are 1 x 1 images: their box is 1 x 1 x 256, so that the columns of a tile are batch rows and none is wasted)
         const bool dense_like = pl.Wout == 1 && pl.Hout == 1;
-        for (int pw = dense_like ? 1 : 8; pw <= 128; pw *= 2)
+        for (int pw = dense_like ? 1 : 8; pw <= 256; pw *= 2)
             for (int ph = 1; ph * pw <= 256; ph *= 2) {
                 const int pn = 256 / (pw * ph);
                 if (pw * pl.SW > 256 || ph * pl.SH > 256) continue;
@@ -1614,7 +1617,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     // pairs of SMs: two row tiles at a time
     bool pair = !pl.dual && (pl.Mp / GM) % 2 == 0 &&
                 worth_pairs((double)g.Nb * pl.Hout * pl.Wout / 256 * (pl.Mp / GM) * taps * pl.LK * (pl.Cp / 16));
-    p.split_h = p.split_n = p.half_valid = 0;
+    p.split_w = p.split_h = p.split_n = p.half_valid = 0;
     p.n_cols = 256; p.Wt = p.Ht = 0; p.n_stages = 0; p.stage_bytes = 0; p.a_slots = 0; p.a_taps = 1; p.halo_bytes = 0;
     if (!pl.dual && pl.Cp % 32 == 0 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
         const int rows = (pl.Hout + 31) / 32;
@@ -1684,7 +1687,8 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
     }
     if (pair && !halo && !p.exact) {               // halves of the power-of-two box, in the order of its columns
         if (p.PN >= 2) p.split_n = p.PN / 2;
-        else p.split_h = p.PH / 2;
+        else if (p.PH >= 2) p.split_h = p.PH / 2;
+        else p.split_w = p.PW / 2;
     }
     p.rows_epi = (unaligned_rows && !p.o_generic && !p.plane_mode) ? 1 : 0;
     const int b_rows = pl.dual || pair ? GN / 2 : GN;
@@ -1723,8 +1727,8 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& g, const void* w, const voi
         const cuuint64_t dims[5] = {(cuuint64_t)Cd, (cuuint64_t)Wd, (cuuint64_t)Hd, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
         const cuuint64_t strides[4] = {(cuuint64_t)Cd * 2, (cuuint64_t)Wd * Cd * 2, (cuuint64_t)Hd * Wd * Cd * 2, (cuuint64_t)g.Nb * Hd * Wd * Cd * 2};
         // with an element stride s the box extent is given in input elements: s * (pixels - 1) + 1 of them hold the pixels loaded
-        const int rows = p.split_h > 0 ? p.split_h : p.PH;
-        const cuuint32_t box[5] = {(cuuint32_t)ks, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : (rows - 1) * pl.SH + 1),
+        const int rows = p.split_h > 0 ? p.split_h : p.PH, width = p.split_w > 0 ? p.split_w : p.PW;
+        const cuuint32_t box[5] = {(cuuint32_t)ks, (cuuint32_t)(halo ? p.Wt : (width - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : (rows - 1) * pl.SH + 1),
                                    (cuuint32_t)(p.split_n > 0 ? p.split_n : p.PN), 1};
         const cuuint32_t es[5] = {1, (cuuint32_t)pl.SW, (cuuint32_t)pl.SH, 1, 1};
         const CUresult r = encode(&map_x, dt, 5, direct ? const_cast<void*>(act) : static_cast<void*>(xp), dims, strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE, sw,
@@ -1827,11 +1831,12 @@ bool conv_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes) {
     return true;
 }
 
-int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* x, void* dw, void* scratch, int* status,
+int conv_filter_tc_launch(int dtype, const Geom& layer, const void* dy, const void* x, void* dw, void* scratch, int* status,
                           cudaStream_t stream, const void* kept_x, const StagedView* kept_dy, StatusClear* sc) {
     EncodeTiledFn encode = encode_fn();
     if (!encode) { set_error("cuTensorMapEncodeTiled is not available from the driver"); return PCB_ERR_CUDA; }
     const int fmt = dtype == PCB_F16 ? 0 : 1;
+    const Geom g = flat_pixels(layer);
     const FilterPlan f = make_filter_plan(g);
     const int taps = g.KH * g.KW;
     // with one channel block per component the staged x is the forward pass's: a copy it kept is read in place
@@ -1865,12 +1870,12 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
     p.Nb = g.Nb; p.Co = g.Co; p.Ci = g.Ci; p.HO = g.HO; p.WO = g.WO; p.Cop = f.Cop; p.Cip = f.Cip;
     p.cbA = f.cby; p.cbB = f.cbx;
     p.KH = g.KH; p.KW = g.KW; p.SH = g.SH; p.SW = g.SW; p.DH = g.DH; p.DW = g.DW; p.fmt = fmt;
-    {   // pixel box of FK pixels wasting the fewest K rows
+    {   // pixel box of FK pixels wasting the fewest K rows (boxes of less than four pixels side by side are slow to load: conv_tf32.cu)
         long long best = -1;
         for (int pw = 1; pw <= FK; pw *= 2)
             for (int ph = 1; ph * pw <= FK; ph *= 2) {
                 const int pn = FK / (pw * ph);
-                const long long vol = (long long)round_up(g.WO, pw) * round_up(g.HO, ph) * round_up(g.Nb, pn);
+                const long long vol = (long long)round_up(g.WO, pw) * round_up(g.HO, ph) * round_up(g.Nb, pn) * (pw >= 4 ? 16 : (pw == 2 ? 17 : 19));
                 if (best < 0 || vol < best || (vol == best && pw > p.PW)) { best = vol; p.PW = pw; p.PH = ph; p.PN = pn; }
             }
     }

@@ -46,7 +46,7 @@ struct TParams {
     int splits, k_per_split;          // the K loop of a tile is cut into `splits` work items of k_per_split stages; with more than one
                                       // the partial results meet in the (zeroed) output by fp32 reductions
     int Wt, Ht, a_slots;              // halo form: halo tile, filter slices in flight
-    int split_h, split_n;             // PAIR: pixel rows and images from the even CTA's half of the tile box to the odd one's
+    int split_w, split_h, split_n;    // PAIR: pixels, pixel rows and images from the even CTA's half of the tile box to the odd one's
     uint32_t halo_bytes;              // halo form: shared-memory pitch of the hi (and of the lo) part of a halo tile
 };
 
@@ -121,7 +121,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
             const int tw = rest % p.tiles_w; rest /= p.tiles_w;
             const int th = rest % p.tiles_h;
             const int tn = rest / p.tiles_h;
-            const int m0 = tm * TM, ow0 = tw * p.PW, oh0 = th * p.PH + rank * p.split_h, n0 = tn * p.PN + rank * p.split_n;
+            const int m0 = tm * TM, ow0 = tw * p.PW + rank * p.split_w, oh0 = th * p.PH + rank * p.split_h, n0 = tn * p.PN + rank * p.split_n;
             const int k0 = split * p.k_per_split, k1 = min(n_k, k0 + p.k_per_split);
             if (HALO) {                                  // stage k = (l * c_steps + cs) * taps + tap
                 for (int l = 0; l < p.LK && ok; ++l)
@@ -1127,7 +1127,8 @@ size_t conv_tf32_scratch_bytes(Pass pass, const Geom& g) {
     return 2 * (pl.xp_bytes + pl.w_bytes);
 }
 
-static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* x, float* dw, void* scratch, int* status, cudaStream_t stream, StatusClear* sc) {
+static int conv_tf32_filter_launch(const Geom& layer, const float* dy, const float* x, float* dw, void* scratch, int* status, cudaStream_t stream, StatusClear* sc) {
+    const Geom g = flat_pixels(layer);
     const FilterPlan32 f = make_filter_plan32(g);
     const int taps = g.KH * g.KW;
     uint8_t* s8 = static_cast<uint8_t*>(scratch);
@@ -1158,7 +1159,9 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
         for (int pw = 1; pw <= TFK; pw *= 2)
             for (int ph = 1; ph * pw <= TFK; ph *= 2) {
                 const int pn = TFK / (pw * ph);
-                const long long vol = (long long)round_up(g.WO, pw) * round_up(g.HO, ph) * round_up(g.Nb, pn);
+                // (a pixel of the lo part is two rows of 64 bytes: boxes of less than four pixels side by side are slow to load. 3x3, 16 -> 24
+                // channels, 101 x 101, batch 32: filter gradient 1173 us with the 1 x 1 x 16 boxes that waste nothing, 442 with these)
+                const long long vol = (long long)round_up(g.WO, pw) * round_up(g.HO, ph) * round_up(g.Nb, pn) * (pw >= 4 ? 16 : (pw == 2 ? 17 : 19));
                 if (best < 0 || vol < best || (vol == best && pw > p.PW)) { best = vol; p.PW = pw; p.PH = ph; p.PN = pn; }
             }
     }
@@ -1217,10 +1220,11 @@ static int conv_tf32_filter_launch(const Geom& g, const float* dy, const float* 
     return PCB_OK;
 }
 
-int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, const void* bias, void* out, void* scratch, int* status,
+int conv_tf32_launch(Pass pass, const Geom& layer, const void* a, const void* b, const void* bias, void* out, void* scratch, int* status,
                      cudaStream_t stream, StatusClear* sc) {
     // operand roles as for the other launchers: forward/backward-data a = filters, b = activations; backward-filter a = dy, b = x
-    if (pass == PASS_BWD_FILTER) return conv_tf32_filter_launch(g, (const float*)a, (const float*)b, (float*)out, scratch, status, stream, sc);
+    if (pass == PASS_BWD_FILTER) return conv_tf32_filter_launch(layer, (const float*)a, (const float*)b, (float*)out, scratch, status, stream, sc);
+    const Geom g = flat_pixels(layer);
     const Plan32 pl = make_plan32(pass, g);
     const int taps = g.KH * g.KW;
     uint8_t* s8 = static_cast<uint8_t*>(scratch);
@@ -1242,15 +1246,17 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     p.store_vec = 1;
     while (p.store_vec < 8 && pl.Wout % (p.store_vec * 2) == 0 && (reinterpret_cast<uintptr_t>(out) % (size_t)(p.store_vec * 8)) == 0) p.store_vec *= 2;
     const bool deep = worth_pairs((double)g.Nb * pl.Hout * pl.Wout / 256 * (pl.Mp / TM) * n_k * 4);
-    // clocks of storing 256 pixels of 128 rows, about: aligned rows, and rows that go through shared memory
-    const long long epilogue = p.store_vec < 8 ? 18000 : 5000;
+    // clocks of storing 256 pixels of 128 rows, about: aligned rows, and rows that go through shared memory, 4, 2 or 1 pixels per lane
+    long long epilogue = p.store_vec == 8 ? 5000 : (p.store_vec == 4 ? 15000 : (p.store_vec == 2 ? 24000 : 35000));
+    if (g.nc * pl.Cout <= 64 && p.store_vec < 8) epilogue /= 3;          // (store_rows_f32_few)
+    if (pl.Wout < 8) epilogue = 60000;                                   // (an element of 32 planes per store)
     // Box of `cols` pixels that wastes the fewest columns, and the cut of its K loop. Too few tiles for the SMs (dense layers, small
     // planes): the K loop of every tile is cut into work items of at least one chunk each; their partial sums meet in the output, zeroed
     // first, by fp32 reductions (the order of which is not fixed).
     auto plan_tiles = [&](int cols) -> long long {
         long long best = -1;
         p.n_cols = cols;
-        for (int pw = 1; pw <= 128; pw *= 2)
+        for (int pw = 1; pw <= cols; pw *= 2)
             for (int ph = 1; ph * pw <= cols; ph *= 2) {
                 const int pn = cols / (pw * ph);
                 if (pn > 256 || (pw - 1) * pl.SW + 1 > 256 || (ph - 1) * pl.SH + 1 > 256) continue;
@@ -1270,29 +1276,32 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         }
         p.k_per_split = n_k / p.splits;
         const long long rounds = (tiles * p.splits + sm_count() - 1) / sm_count();
-        const long long wide = p.k_per_split * (two ? 540ll : 750ll) + epilogue, narrow = p.k_per_split * 512ll;
+        const long long wide = p.k_per_split * (two ? 540ll : 750ll) + epilogue, narrow = p.k_per_split * 650ll;
         return rounds * (cols == 256 ? wide : (narrow > epilogue / 2 ? narrow : epilogue / 2));
     };
-    // Clocks of a stage: 750 with 256 pixels (540 on pairs) and 512 with 128 (48 and 32 KB at the 64 bytes per clock that an SM takes in), in halo form those of
-    // its four MMAs; tiles of 256 and halo tiles have single accumulators, so their epilogue is not hidden, and tiles of 128 take no less than
+    // Clocks of a stage: 750 with 256 pixels (540 on pairs; 48 KB at the 64 bytes per clock that an SM takes in), 650 with 128, in halo form those of
+    // its four MMAs or 580; tiles of 256 and halo tiles have single accumulators, so their epilogue is not hidden, and tiles of 128 take no less than
     // theirs. 128-pixel tiles where the longest CTA has less to do with them: shallow layers and those that leave SMs idle. 3x3, 16 channels, 32 x 32, batch 8,
     // forward: 20.3 -> 17.5 us with the present kernel (25.0 with three TF32 products and 256-pixel tiles).
     const long long narrow_cost = plan_tiles(128);
     long long cost = plan_tiles(256);
     if (10 * cost > 11 * narrow_cost) { cost = narrow_cost; plan_tiles(128); }
+    // Halo tiles of up to 32 rows, or of up to 16, which are 128 pixels with double accumulators: shallow layers with slow stores.
     bool halo = false;
     p.Wt = p.Ht = p.a_slots = 0; p.halo_bytes = 0;
-    if (pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
-        const int rows = (pl.Hout + 31) / 32;
+    for (int cap = 32; cap >= 16 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8; cap -= 16) {
+        const int rows = (pl.Hout + cap - 1) / cap;
         const int ph = (((pl.Hout + rows - 1) / rows) + 1) & ~1;
         const bool two = pl.Mp / TM % 2 == 0 && deep;
         const int wt = 8 + (g.KW - 1) * g.DW, ht = (two ? ph / 2 : ph) + (g.KH - 1) * g.DH;
         const uint32_t part = ((uint32_t)wt * ht * TKS * 4 + 1023) / 1024 * 1024;
         const int room = 227 * 1024 - 1024 - 512 - (p.store_vec < 8 ? 8 * EPI_ROWS_F32_BYTES : 0) - (int)(T_HALO_TILES * 2 * part);
         const long long tiles = (long long)((pl.Wout + 7) / 8) * ((pl.Hout + ph - 1) / ph) * g.Nb * (pl.Mp / TM);
-        const long long halo_cost = (tiles + sm_count() - 1) / sm_count() * (n_k * 16ll * ph + epilogue);
-        if (ph >= 24 && wt <= 256 && ht <= 256 && room >= 6 * (int)(2 * TA_BYTES) && halo_cost < cost) {
+        const long long stages = n_k * (cap == 32 ? 16ll * ph : 580ll), each = cap == 32 ? stages + epilogue : (stages > epilogue / 2 ? stages : epilogue / 2);
+        const long long halo_cost = (tiles + sm_count() - 1) / sm_count() * each;
+        if (ph >= cap * 3 / 4 && wt <= 256 && ht <= 256 && room >= 6 * (int)(2 * TA_BYTES) && halo_cost < cost) {
             halo = true;
+            cost = halo_cost;
             p.PW = 8; p.PH = ph; p.PN = 1; p.n_cols = 8 * ph; p.Wt = wt; p.Ht = ht;
             p.tiles_w = (pl.Wout + 7) / 8; p.tiles_h = (pl.Hout + ph - 1) / ph; p.tiles_n = g.Nb;
             p.splits = 1; p.k_per_split = n_k;
@@ -1306,8 +1315,8 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
     p.has_bias = (pass == PASS_FWD && g.has_bias) ? 1 : 0;
     p.LK = pl.LK;
     const bool pair = p.tiles_m % 2 == 0 && deep && (halo || p.n_cols == 256);
-    p.split_h = p.split_n = 0;
-    if (pair) { if (p.PN >= 2) p.split_n = p.PN / 2; else p.split_h = p.PH / 2; }
+    p.split_w = p.split_h = p.split_n = 0;
+    if (pair) { if (p.PN >= 2) p.split_n = p.PN / 2; else if (p.PH >= 2) p.split_h = p.PH / 2; else p.split_w = p.PW / 2; }
     p.rows_epi = (p.PW >= 8 && p.store_vec < 8) ? 1 : 0;
     p.off_w = inserted ? 0 : -pl.pad_left; p.off_h = inserted ? 0 : -pl.pad_top;
 
@@ -1324,7 +1333,7 @@ int conv_tf32_launch(Pass pass, const Geom& g, const void* a, const void* b, con
         const cuuint64_t dims[5] = {(cuuint64_t)pl.Cp, (cuuint64_t)pl.Wp, (cuuint64_t)pl.Hp, (cuuint64_t)g.Nb, (cuuint64_t)pl.LK};
         const cuuint64_t strides[4] = {(cuuint64_t)pl.Cp * 4, (cuuint64_t)pl.Wp * pl.Cp * 4, (cuuint64_t)pl.Hp * pl.Wp * pl.Cp * 4,
                                        (cuuint64_t)g.Nb * pl.Hp * pl.Wp * pl.Cp * 4};
-        const cuuint32_t box[5] = {TKS, (cuuint32_t)(halo ? p.Wt : (p.PW - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : ((p.split_h ? p.split_h : p.PH) - 1) * pl.SH + 1), (cuuint32_t)(p.split_n ? p.split_n : p.PN), 1};
+        const cuuint32_t box[5] = {TKS, (cuuint32_t)(halo ? p.Wt : ((p.split_w ? p.split_w : p.PW) - 1) * pl.SW + 1), (cuuint32_t)(halo ? p.Ht : ((p.split_h ? p.split_h : p.PH) - 1) * pl.SH + 1), (cuuint32_t)(p.split_n ? p.split_n : p.PN), 1};
         const cuuint32_t es[5] = {1, (cuuint32_t)pl.SW, (cuuint32_t)pl.SH, 1, 1};
         int rc = make_tensor_map(&m_x_hi, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_hi, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_64B, "activations hi");
         if (rc == PCB_OK) rc = make_tensor_map(&m_x_lo, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, x_lo, 5, dims, strides, box, es, CU_TENSOR_MAP_SWIZZLE_64B, "activations lo");

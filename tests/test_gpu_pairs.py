@@ -1,4 +1,4 @@
-"""General 16-bit kernel on pairs of SMs (an even number of 128-row tiles): whole planes in each half of a tile, half a plane, planes of an odd
+"""General kernels on pairs of SMs (an even number of 128-row tiles and enough work; smaller layers stay on single SMs): whole planes in each half of a tile, half a plane, planes of an odd
 number of rows (which stay on single SMs), power-of-two boxes split by images and by rows, halo tiles; batches that leave halves empty; odd
 and even planes; slices of 16, 32 and 64 channels; strides, bias, channels-last."""
 import numpy as np
@@ -63,3 +63,32 @@ def test_pairs_channels_last(gpu, oracle, co, h, w):
     y = torch.full(desc.getOutputShape(), float("nan"), dtype=torch.float16, device="cuda")
     pcb.conv2DFwd(xd, wd, None, y, desc, gpu.context("16p"), gpu.ENGINES["tensor"])
     assert rel_err(y.float().cpu().permute(0, 3, 1, 2).numpy(), ref) <= TOL["f16"]
+
+
+# Layers with enough MMAs for pairs, and pointwise layers whose planes are taken as rows of pixels (odd and even planes, planes of less and more
+# than a tile, tiles of whole rows and of several images). The reference is the fp32 kernel of the CUDA cores on the same rounded inputs.
+@pytest.mark.parametrize("dtype,case", [
+    ("bf16", (27, 256, 256, 14, 14, 1, 1)), ("f16", (21, 64, 128, 14, 14, 3, 1)), ("f16", (46, 64, 128, 7, 7, 3, 1)), ("f16", (24, 64, 128, 13, 13, 3, 1)),
+    ("f16", (17, 64, 128, 28, 28, 3, 2)), ("bf16", (9, 64, 64, 40, 24, 3, 1)), ("f16", (7, 48, 64, 31, 44, 3, 1)), ("f16", (5, 96, 64, 26, 57, 5, 1)),
+    ("f16", (41, 96, 64, 20, 18, 3, 2)), ("f16", (33, 128, 192, 23, 20, 1, 1)), ("bf16", (7, 128, 192, 61, 51, 1, 1)), ("f16", (80, 128, 128, 5, 9, 3, 1)),
+    ("f16", (64, 16, 64, 24, 24, 3, 1)), ("f16", (9, 48, 40, 41, 47, 1, 1)), ("bf16", (50, 24, 56, 12, 11, 1, 1)),
+    ("f32", (5, 64, 64, 56, 28, 3, 1)), ("f32", (40, 64, 64, 14, 15, 3, 1)), ("f32", (21, 128, 128, 19, 17, 1, 1)), ("f32", (12, 40, 48, 33, 41, 3, 1)),
+    ("f32", (9, 40, 24, 41, 47, 1, 1)), ("f32", (33, 96, 64, 24, 20, 3, 2)), ("f32", (3, 16, 24, 101, 37, 3, 1)), ("f32", (5, 24, 32, 40, 51, 1, 1)),
+    ("f32", (10, 24, 30, 47, 47, 3, 1)),
+])
+def test_large_layers(gpu, dtype, case):
+    n, ci, co, h, w, k, s = case
+    (pt, pb), (pl, pr) = _same(h, k, s), _same(w, k, s)
+    pad = (pt, pl, pb, pr)
+    x = gpu.rounded(uniform(57, (4 * n, ci, h, w)), dtype)
+    f = gpu.rounded(normal(58, (4, co, ci, k, k), std=(2.0 / (4 * ci * k * k)) ** 0.5), dtype)
+    b = gpu.rounded(uniform(59, (4, co)), dtype)
+    tol = TOL.get(dtype, 1e-5)
+    ref = gpu.run_conv_fwd(x, f, b, (s, s), pad, "f32", "16p", "simt")
+    y = gpu.run_conv_fwd(x, f, b, (s, s), pad, dtype, "16p", "tensor")
+    assert np.all(np.isfinite(y)) and rel_err(y, ref) <= tol, rel_err(y, ref)
+    dy = gpu.rounded(normal(60, ref.shape), dtype)
+    rdw, rdx = gpu.run_conv_bwd(x, f, dy, (s, s), pad, "f32", "16p", "simt", True)
+    dw, dx = gpu.run_conv_bwd(x, f, dy, (s, s), pad, dtype, "16p", "tensor", True)
+    for got, want, what in ((dx, rdx, "dx"), (dw, rdw, "dw")):
+        assert np.all(np.isfinite(got)) and rel_err(got, want) <= tol, (what, rel_err(got, want))
