@@ -124,8 +124,9 @@ qconv_pointwise_pair_tc_kernel(const __grid_constant__ CUtensorMap map_w, const 
         }
         __syncwarp();
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer (even CTA, one thread)
-        if (lane == 0 && rank == 0) {
+        // ---------------------------------------------------------------- MMA issuer (even CTA, one elected lane)
+        if (rank == 0) {
+            const bool el = elect_one();
             int s = 0, local_tile = 0;
             uint32_t par = 0;
             bool ok = true;
@@ -145,15 +146,15 @@ qconv_pointwise_pair_tc_kernel(const __grid_constant__ CUtensorMap map_w, const 
             // phase A computes: the turnover of the single-buffered accumulators costs no tensor time (with one pass over
             // the slices, both pairs completed at the very end of the tile and the next tile waited for their drain).
             // Inside a phase the MMAs alternate between the two accumulators of the pair.
-            if (pair < n_tiles) ok = mbar_wait_bounded(a_full, 0, status, ST_P_MMA);
+            if (pair < n_tiles) ok = warp_wait_bounded(a_full, 0, status, ST_P_MMA);
             uint32_t a_lo_k[P_MAX_K], a_hi_k[P_MAX_K], b_lo_k[P_MAX_K], b_hi_k[P_MAX_K];
             int s_k[P_MAX_K];
             for (int tile = pair; tile < n_tiles && ok; tile += n_pairs, ++local_tile) {
 #pragma unroll
                 for (int ph = 0; ph < 2; ++ph) {
                     if (local_tile > 0) {           // both CTAs' epilogues have drained this pair of the previous tile
-                        ok = ok && mbar_wait_bounded(tmem_empty + 8 * (2 * ph), (local_tile - 1) & 1, status, ST_P_MMA) &&
-                             mbar_wait_bounded(tmem_empty + 8 * (2 * ph + 1), (local_tile - 1) & 1, status, ST_P_MMA);
+                        ok = ok && warp_wait_bounded(tmem_empty + 8 * (2 * ph), (local_tile - 1) & 1, status, ST_P_MMA) &&
+                             warp_wait_bounded(tmem_empty + 8 * (2 * ph + 1), (local_tile - 1) & 1, status, ST_P_MMA);
                         if (!ok) break;
                         tc_fence_after_sync();
                     }
@@ -161,7 +162,7 @@ qconv_pointwise_pair_tc_kernel(const __grid_constant__ CUtensorMap map_w, const 
                     for (int k = 0; k < P_MAX_K; ++k) {
                         if (k >= n_k) break;
                         if (ph == 0) {              // first touch of the slice: wait for its data, keep its descriptors
-                            ok = mbar_wait_bounded(full_bar + 8 * s, par, status, ST_P_MMA);
+                            ok = warp_wait_bounded(full_bar + 8 * s, par, status, ST_P_MMA);
                             if (!ok) break;
                             tc_fence_after_sync();
                             const uint64_t ad = desc_kmajor_sw64_p(a_slot(k));
@@ -171,20 +172,24 @@ qconv_pointwise_pair_tc_kernel(const __grid_constant__ CUtensorMap map_w, const 
                             if (++s == P_STAGES) { s = 0; par ^= 1u; }
                         }
                         a_lo = a_lo_k[k]; a_hi = a_hi_k[k]; b_lo = b_lo_k[k]; b_hi = b_hi_k[k];
+                        if (el) {
 #pragma unroll
-                        for (int j = 0; j < P_KS / 16; ++j)
+                            for (int j = 0; j < P_KS / 16; ++j)
 #pragma unroll
-                            for (int i = 0; i < 4; ++i)
+                                for (int i = 0; i < 4; ++i)
 #pragma unroll
-                                for (int oo = 0; oo < 2; ++oo) issue(j, i, 2 * ph + oo, (k > 0 || j > 0 || i > 0) ? 1u : 0u);
-                        if (ph == 1) {              // the stage is free in both CTAs
-                            mma_commit_pair(empty_bar + 8 * s_k[k]);
-                            mma_commit_pair(peer_empty + 8 * s_k[k]);
+                                    for (int oo = 0; oo < 2; ++oo) issue(j, i, 2 * ph + oo, (k > 0 || j > 0 || i > 0) ? 1u : 0u);
+                            if (ph == 1) {          // the stage is free in both CTAs
+                                mma_commit_pair(empty_bar + 8 * s_k[k]);
+                                mma_commit_pair(peer_empty + 8 * s_k[k]);
+                            }
                         }
                     }
                     if (!ok) break;
-                    mma_commit_pair(ph == 0 ? tmem_full0 : tmem_full1);
-                    mma_commit_pair(ph == 0 ? peer_full0 : peer_full1);
+                    if (el) {
+                        mma_commit_pair(ph == 0 ? tmem_full0 : tmem_full1);
+                        mma_commit_pair(ph == 0 ? peer_full0 : peer_full1);
+                    }
                 }
             }
         }
@@ -340,8 +345,9 @@ qconv_pointwise_filter_pair_tc_kernel(const __grid_constant__ CUtensorMap map_dy
         }
         __syncwarp();
     } else if (warp == 1) {
-        // ---------------------------------------------------------------- MMA issuer (even CTA, one thread)
-        if (lane == 0 && rank == 0) {
+        // ---------------------------------------------------------------- MMA issuer (even CTA, one elected lane)
+        if (rank == 0) {
+            const bool el = elect_one();
             bool ok = true;
             int s = 0;
             uint32_t par = 0;
@@ -349,31 +355,33 @@ qconv_pointwise_filter_pair_tc_kernel(const __grid_constant__ CUtensorMap map_dy
             const uint32_t idesc_neg = make_idesc_f16(p.fmt, 256, 128, false, false, true, false);
             const uint32_t peer_empty = map_to_cta(empty_bar, 1), peer_tmem_full = map_to_cta(tmem_full, 1);
             for (int it = 0; it < n_steps && ok; ++it) {
-                ok = mbar_wait_bounded(full_bar + 8 * s, par, status, ST_P_MMA);
+                ok = warp_wait_bounded(full_bar + 8 * s, par, status, ST_P_MMA);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint64_t ad = desc_kmajor_sw64_p(tiles_addr + s * PF_STAGE_BYTES);
                 const uint64_t bd = desc_kmajor_sw64_p(tiles_addr + s * PF_STAGE_BYTES + PF_A_BYTES);
                 const uint32_t a_lo = (uint32_t)ad, a_hi = (uint32_t)(ad >> 32), b_lo = (uint32_t)bd, b_hi = (uint32_t)(bd >> 32);
+                if (el) {
 #pragma unroll
-                for (int j = 0; j < PF_KP / 16; ++j) {
+                    for (int j = 0; j < PF_KP / 16; ++j) {
 #pragma unroll
-                    for (int l = 0; l < 4; ++l) {
+                        for (int l = 0; l < 4; ++l) {
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            const int d = l ^ r;
-                            const uint32_t a_off = (uint32_t)(d * (128 * PF_KP * 2) + j * 32) >> 4, b_off = (uint32_t)(l * (64 * PF_KP * 2) + j * 32) >> 4;
-                            mma_f16_pair(tmem_base + r * 128, a_lo + a_off, a_hi, b_lo + b_off, b_hi, quat_negative(l, d) ? idesc_neg : idesc_pos,
-                                         (it > 0 || j > 0 || l > 0) ? 1u : 0u);
+                            for (int r = 0; r < 4; ++r) {
+                                const int d = l ^ r;
+                                const uint32_t a_off = (uint32_t)(d * (128 * PF_KP * 2) + j * 32) >> 4, b_off = (uint32_t)(l * (64 * PF_KP * 2) + j * 32) >> 4;
+                                mma_f16_pair(tmem_base + r * 128, a_lo + a_off, a_hi, b_lo + b_off, b_hi, quat_negative(l, d) ? idesc_neg : idesc_pos,
+                                             (it > 0 || j > 0 || l > 0) ? 1u : 0u);
+                            }
                         }
                     }
+                    mma_commit_pair(empty_bar + 8 * s);
+                    mma_commit_pair(peer_empty + 8 * s);
+                    if (it == n_steps - 1) { mma_commit_pair(tmem_full); mma_commit_pair(peer_tmem_full); }
                 }
-                mma_commit_pair(empty_bar + 8 * s);
-                mma_commit_pair(peer_empty + 8 * s);
-                if (it == n_steps - 1) { mma_commit_pair(tmem_full); mma_commit_pair(peer_tmem_full); }
                 if (++s == PF_STAGES) { s = 0; par ^= 1u; }
             }
-            if (n_steps == 0) { mbar_arrive(tmem_full); mbar_arrive_cluster(peer_tmem_full); }
+            if (n_steps == 0 && el) { mbar_arrive(tmem_full); mbar_arrive_cluster(peer_tmem_full); }
         }
         __syncwarp();
     } else {

@@ -151,12 +151,12 @@ qconv_pointwise_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
         __syncwarp();
     } else if (warp == 1) {
         // ---------------------------------------------------------------- MMA issuer
-        // ONE thread runs this whole loop: waits, descriptor arithmetic and tcgen05.mma / commit. What that thread executes
-        // between two MMAs is time the tensor pipe idles (its queue is shallow), so the loop carries no division, no warp
-        // synchronisation and no descriptor construction: the two 64-bit shared-memory descriptors of a stage are built
-        // once, and an MMA's descriptors are those with a constant added to the address field of the low word (addresses
-        // are 16-byte units below 2^14, so the addition never carries into the neighbouring field).
-        if (lane == 0) {
+        // One elected lane issues (umma.cuh: elect_one). What is executed between two MMAs is time the tensor pipe idles (its queue is
+        // shallow), so the loop carries no division and no descriptor construction: the two 64-bit shared-memory descriptors of a
+        // stage are built once, and an MMA's descriptors are those with a constant added to the address field of the low word
+        // (addresses are 16-byte units below 2^14, so the addition never carries into the neighbouring field).
+        {
+            const bool el = elect_one();
             int s = 0, local_tile = 0;
             uint32_t par = 0;                                    // phase parity of stage s
             bool ok = true;
@@ -170,10 +170,10 @@ qconv_pointwise_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                 const uint32_t b_off = (uint32_t)(i * (KS * 128) + j * 2048) >> 4;
                 mma_f16_ss_words(tmem_base + o * PT, a_lo + a_off, a_hi, b_lo + b_off, b_hi, neg ? idesc_neg : idesc_pos, accumulate);
             };
-            if (resident && blockIdx.x < n_tiles) ok = mbar_wait_bounded(a_full, 0, status, ST_U_MMA);
+            if (resident && blockIdx.x < n_tiles) ok = warp_wait_bounded(a_full, 0, status, ST_U_MMA);
             for (int tile = blockIdx.x; tile < n_tiles && ok; tile += gridDim.x, ++local_tile) {
                 for (int k = 0; k < n_k && ok; ++k) {
-                    ok = mbar_wait_bounded(full_bar + 8 * s, par, status, ST_U_MMA);
+                    ok = warp_wait_bounded(full_bar + 8 * s, par, status, ST_U_MMA);
                     if (!ok) break;
                     tc_fence_after_sync();
                     {
@@ -195,11 +195,11 @@ qconv_pointwise_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
 #pragma unroll
                         for (int pair = 0; pair < 2; ++pair) {
                             if (local_tile > 0) {
-                                ok = ok && mbar_wait_bounded(tmem_empty + 8 * (2 * pair), (local_tile - 1) & 1, status, ST_U_MMA) &&
-                                     mbar_wait_bounded(tmem_empty + 8 * (2 * pair + 1), (local_tile - 1) & 1, status, ST_U_MMA);
+                                ok = ok && warp_wait_bounded(tmem_empty + 8 * (2 * pair), (local_tile - 1) & 1, status, ST_U_MMA) &&
+                                     warp_wait_bounded(tmem_empty + 8 * (2 * pair + 1), (local_tile - 1) & 1, status, ST_U_MMA);
                                 tc_fence_after_sync();
                             }
-                            if (ok) {
+                            if (ok && el) {
 #pragma unroll
                                 for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -207,34 +207,36 @@ qconv_pointwise_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                             }
                         }
                         if (!ok) break;
-                    } else {
+                    } else if (el) {
 #pragma unroll
                         for (int i = 0; i < 4; ++i)
 #pragma unroll
                             for (int o = 0; o < 4; ++o) issue(0, i, o, 1u);
                     }
+                    if (el) {
 #pragma unroll
-                    for (int j = 1; j < J - 1; ++j)
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-#pragma unroll
-                            for (int o = 0; o < 4; ++o) issue(j, i, o, 1u);
-                    if (last) {
-#pragma unroll
-                        for (int pair = 0; pair < 2; ++pair) {
+                        for (int j = 1; j < J - 1; ++j)
 #pragma unroll
                             for (int i = 0; i < 4; ++i)
 #pragma unroll
-                                for (int oo = 0; oo < 2; ++oo) issue(J - 1, i, 2 * pair + oo, 1u);
-                            mma_commit(pair == 0 ? tmem_full0 : tmem_full1);
+                                for (int o = 0; o < 4; ++o) issue(j, i, o, 1u);
+                        if (last) {
+#pragma unroll
+                            for (int pair = 0; pair < 2; ++pair) {
+#pragma unroll
+                                for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                    for (int oo = 0; oo < 2; ++oo) issue(J - 1, i, 2 * pair + oo, 1u);
+                                mma_commit(pair == 0 ? tmem_full0 : tmem_full1);
+                            }
+                        } else {
+#pragma unroll
+                            for (int i = 0; i < 4; ++i)
+#pragma unroll
+                                for (int o = 0; o < 4; ++o) issue(J - 1, i, o, 1u);
                         }
-                    } else {
-#pragma unroll
-                        for (int i = 0; i < 4; ++i)
-#pragma unroll
-                            for (int o = 0; o < 4; ++o) issue(J - 1, i, o, 1u);
+                        mma_commit(empty_bar + 8 * s);
                     }
-                    mma_commit(empty_bar + 8 * s);
                     if (++s == n_stages) { s = 0; par ^= 1u; }
                 }
             }
@@ -389,37 +391,40 @@ qconv_pointwise_filter_tc_kernel(const __grid_constant__ CUtensorMap map_dy, con
         }
         __syncwarp();
     } else if (warp == 1) {
-        if (lane == 0) {                       // one thread: waits, stepped descriptors, MMAs (see the forward kernel)
+        {                                      // (see the forward kernel)
+            const bool el = elect_one();
             bool ok = true;
             int s = 0;
             uint32_t par = 0;
             const uint32_t idesc_pos = make_idesc_f16(p.fmt, 128, 128, false, false, false, false);
             const uint32_t idesc_neg = make_idesc_f16(p.fmt, 128, 128, false, false, true, false);
             for (int it = 0; it < n_steps && ok; ++it) {
-                ok = mbar_wait_bounded(full_bar + 8 * s, par, status, ST_U_MMA);
+                ok = warp_wait_bounded(full_bar + 8 * s, par, status, ST_U_MMA);
                 if (!ok) break;
                 tc_fence_after_sync();
                 const uint64_t ad = make_desc_kmajor_sw64(tiles_addr + s * F_STAGE_BYTES);
                 const uint64_t bd = make_desc_kmajor_sw64(tiles_addr + s * F_STAGE_BYTES + F_OP_BYTES);
                 const uint32_t a_lo = (uint32_t)ad, a_hi = (uint32_t)(ad >> 32), b_lo = (uint32_t)bd, b_hi = (uint32_t)(bd >> 32);
+                if (el) {
 #pragma unroll
-                for (int j = 0; j < FKP / 16; ++j) {
+                    for (int j = 0; j < FKP / 16; ++j) {
 #pragma unroll
-                    for (int l = 0; l < 4; ++l) {
+                        for (int l = 0; l < 4; ++l) {
 #pragma unroll
-                        for (int r = 0; r < 4; ++r) {
-                            const int d = l ^ r;
-                            const uint32_t a_off = (uint32_t)(d * (128 * FKP * 2) + j * 32) >> 4, b_off = (uint32_t)(l * (128 * FKP * 2) + j * 32) >> 4;
-                            mma_f16_ss_words(tmem_base + r * 128, a_lo + a_off, a_hi, b_lo + b_off, b_hi, quat_negative(l, d) ? idesc_neg : idesc_pos,
-                                             (it > 0 || j > 0 || l > 0) ? 1u : 0u);
+                            for (int r = 0; r < 4; ++r) {
+                                const int d = l ^ r;
+                                const uint32_t a_off = (uint32_t)(d * (128 * FKP * 2) + j * 32) >> 4, b_off = (uint32_t)(l * (128 * FKP * 2) + j * 32) >> 4;
+                                mma_f16_ss_words(tmem_base + r * 128, a_lo + a_off, a_hi, b_lo + b_off, b_hi, quat_negative(l, d) ? idesc_neg : idesc_pos,
+                                                 (it > 0 || j > 0 || l > 0) ? 1u : 0u);
+                            }
                         }
                     }
+                    mma_commit(empty_bar + 8 * s);
+                    if (it == n_steps - 1) mma_commit(tmem_full);
                 }
-                mma_commit(empty_bar + 8 * s);
-                if (it == n_steps - 1) mma_commit(tmem_full);
                 if (++s == U_STAGES) { s = 0; par ^= 1u; }
             }
-            if (n_steps == 0) mbar_arrive(tmem_full);
+            if (n_steps == 0 && el) mbar_arrive(tmem_full);
         }
         __syncwarp();
     } else {
