@@ -153,9 +153,9 @@ __device__ __forceinline__ void plane_pack_exact(const uint32_t (&v)[32], int co
     }
 }
 
-// 192 KB of operand stages, at most 12
+// 192 KB of operand stages, at most 12. HALVES: DUAL and PAIR each halve the pixels of a stage
 constexpr int H_MAX_SLOTS = 22, H_MAX_TILES = 3;               // halo form: filter slices and halo tiles in flight
-template <int KS, bool DUAL> constexpr int G_MAX_STAGES = KS == 64 ? (DUAL ? 6 : 4) : (KS == 32 ? (DUAL ? 12 : 8) : 12);
+template <int KS, int HALVES> constexpr int G_MAX_STAGES = KS == 64 ? (HALVES == 2 ? 8 : (HALVES == 1 ? 6 : 4)) : (KS == 32 ? (HALVES ? 12 : 8) : 12);
 
 // HALO (KS == 32, stride-1 correlation, tile = 8 x PH pixels of one image): for every 32-channel slice of one component the halo
 // tile [Ht][Wt][32 channels] of the output tile is loaded once, and every tap's MMAs read it at a shifted start address; the filter
@@ -173,7 +173,7 @@ template <int KS, bool DUAL> constexpr int G_MAX_STAGES = KS == 64 ? (DUAL ? 6 :
 // (a convolution of a zero-inserted dy executes four times as many) from one compact copy of dy, in one launch. Bound by the
 // operand traffic from L2: 32 KB per four MMAs of 128 x 128 x 16.
 //
-// PAIR (not DUAL): a cluster of two CTAs takes two neighbouring row tiles and half of the pixels of the tile box each (cta_group::2): per SM
+// PAIR: a cluster of two CTAs takes two neighbouring row tiles and half of the pixels of the tile box each (cta_group::2): per SM
 // 32 KB instead of 48 KB from L2 for four MMAs of 128 x 256 x 16, and 7.5 instead of 11 KB of operands from shared memory per MMA of the halo
 // form. Without / with, under the power limit: 1x1 256 at 14, bf16, forward 94 / 82 us; 3x3 stride 2, 128 at 28, forward 184 / 157; forward +
 // backward of 3x3 64 at 56 1471 / 1362, channels-last 1164 / 1116.
@@ -181,9 +181,8 @@ template <int KS, bool HALO, bool DUAL, bool PAIR>
 __global__ void __launch_bounds__(G_THREADS, 1)
 qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x, GParams p,
                         const uint16_t* bias, uint16_t* __restrict__ out, int* __restrict__ status) {
-    static_assert(!(DUAL && PAIR), "forms");
-    constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = (DUAL || PAIR ? GN / 2 : GN) * KS * 2;
-    constexpr int MAX_STAGES = HALO ? H_MAX_SLOTS : G_MAX_STAGES<KS, DUAL || PAIR>;
+    constexpr uint32_t A_BYTES = GM * KS * 2, B_BYTES = GN / ((DUAL ? 2 : 1) * (PAIR ? 2 : 1)) * KS * 2;
+    constexpr int MAX_STAGES = HALO ? H_MAX_SLOTS : G_MAX_STAGES<KS, DUAL + PAIR>;
     const int rank = PAIR ? (int)cluster_ctarank() : 0, first = PAIR ? blockIdx.x / 2 : blockIdx.x, step = PAIR ? gridDim.x / 2 : gridDim.x;
     const uint32_t STAGE = HALO ? A_BYTES * p.a_taps : A_BYTES + B_BYTES;      // HALO: one slot of the filter ring
     const int STAGES = HALO ? p.a_slots : p.n_stages;
@@ -240,9 +239,9 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                 const int th = rest % p.tiles_h;
                 const int tn = rest / p.tiles_h;
                 if (DUAL) {
-                    const int cls = tn / p.tiles_n, a = first_class ^ cls, n0 = (tn - cls * p.tiles_n) * p.PN, m0 = tm * GM;
+                    const int cls = tn / p.tiles_n, a = first_class ^ cls, n0 = (tn - cls * p.tiles_n) * p.PN + rank * p.split_n, m0 = tm * GM;
                     for (int kh = (a + p.PT) & 1; kh < p.KH && ok; kh += 2) {
-                        const int row = th * p.PH + ((a + p.PT) >> 1) - (kh >> 1);
+                        const int row = th * p.PH + rank * p.split_h + ((a + p.PT) >> 1) - (kh >> 1);
                         for (int kw = 0; kw < p.KW && ok; ++kw) {
                             const int b = (kw + p.PL) & 1, col = tw * p.PW + ((b + p.PL) >> 1) - (kw >> 1);
                             const int tap = taps - 1 - (kh * p.KW + kw);             // the packed filters hold the taps flipped
@@ -251,7 +250,12 @@ qconv_general_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_
                                     ok = warp_wait_bounded(empty_bar + 8 * s, phase, status, ST_G_PRODUCER);
                                     if (!ok) break;
                                     const uint32_t a_dst = tiles_addr + s * STAGE, bar = full_bar + 8 * s;
-                                    if (el) {
+                                    if (el && PAIR) {
+                                        const uint32_t lead = map_to_cta(bar, 0);
+                                        if (rank == 0) mbar_arrive_expect_tx(bar, 2 * (A_BYTES + p.b_tx));
+                                        tma_load_3d_pair(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, lead);
+                                        tma_load_5d_pair(a_dst + A_BYTES, &map_x, cs * KS, col, row, n0, l, lead);
+                                    } else if (el) {
                                         mbar_arrive_expect_tx(bar, A_BYTES + p.b_tx);
                                         tma_load_3d(a_dst, &map_w, l * p.Cp + cs * KS, m0, tap, bar);
                                         tma_load_5d(a_dst + A_BYTES, &map_x, cs * KS, col, row, n0, l, bar);
@@ -1615,8 +1619,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& layer, const void* w, const
     const int epi_bytes = cl32 ? CL32_BYTES : (unaligned_rows ? ROWS_BYTES : 0);
     bool halo = false;
     // pairs of SMs: two row tiles at a time
-    bool pair = !pl.dual && (pl.Mp / GM) % 2 == 0 &&
-                worth_pairs((double)g.Nb * pl.Hout * pl.Wout / 256 * (pl.Mp / GM) * taps * pl.LK * (pl.Cp / 16));
+    bool pair = (pl.Mp / GM) % 2 == 0 && worth_pairs((double)g.Nb * Hc * Wc / 256 * (pl.Mp / GM) * taps * pl.LK * (pl.Cp / 16));
     p.split_w = p.split_h = p.split_n = p.half_valid = 0;
     p.n_cols = 256; p.Wt = p.Ht = 0; p.n_stages = 0; p.stage_bytes = 0; p.a_slots = 0; p.a_taps = 1; p.halo_bytes = 0;
     if (!pl.dual && pl.Cp % 32 == 0 && pl.SH == 1 && pl.SW == 1 && taps >= 4 && pl.Wout >= 8) {
@@ -1691,11 +1694,11 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& layer, const void* w, const
         else p.split_w = p.PW / 2;
     }
     p.rows_epi = (unaligned_rows && !p.o_generic && !p.plane_mode) ? 1 : 0;
-    const int b_rows = pl.dual || pair ? GN / 2 : GN;
+    const int halves = pl.dual + (pair ? 1 : 0), b_rows = GN >> halves;
     p.b_tx = (uint32_t)(p.exact ? (pair ? p.half_valid : p.PW * p.PH * p.PN) : b_rows) * (uint32_t)pl.KS * 2u;
     const int tail_bytes = p.plane_mode ? (int)G_PLANE_BYTES : (p.o_cl32 ? CL32_BYTES : (p.rows_epi ? ROWS_BYTES : 0));
     if (!halo) {
-        const int small = pl.dual || pair, max_stages = pl.KS == 64 ? G_MAX_STAGES<64, false> + 2 * small : (pl.KS == 32 ? G_MAX_STAGES<32, false> + 4 * small : G_MAX_STAGES<16, false>);
+        const int max_stages = pl.KS == 64 ? G_MAX_STAGES<64, 0> + 2 * halves : (pl.KS == 32 && !halves ? G_MAX_STAGES<32, 0> : G_MAX_STAGES<16, 0>);
         const int fit = (int)((227 * 1024 - 1024 - 512 - tail_bytes) / ((GM + b_rows) * pl.KS * 2));
         p.n_stages = fit < max_stages ? fit : max_stages;
         p.stage_bytes = (uint32_t)(GM + b_rows) * pl.KS * 2;
@@ -1748,7 +1751,8 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& layer, const void* w, const
     };
     auto by_slice = [&](auto* k64, auto* k32, auto* k16) -> int { return pl.KS == 64 ? run(k64) : (pl.KS == 32 ? run(k32) : run(k16)); };
     int rc;
-    if (pl.dual) rc = by_slice(qconv_general_tc_kernel<64, false, true, false>, qconv_general_tc_kernel<32, false, true, false>, qconv_general_tc_kernel<16, false, true, false>);
+    if (pl.dual && pair) rc = by_slice(qconv_general_tc_kernel<64, false, true, true>, qconv_general_tc_kernel<32, false, true, true>, qconv_general_tc_kernel<16, false, true, true>);
+    else if (pl.dual) rc = by_slice(qconv_general_tc_kernel<64, false, true, false>, qconv_general_tc_kernel<32, false, true, false>, qconv_general_tc_kernel<16, false, true, false>);
     else if (halo) rc = pair ? run(qconv_general_tc_kernel<32, true, false, true>) : run(qconv_general_tc_kernel<32, true, false, false>);
     else if (pair) rc = by_slice(qconv_general_tc_kernel<64, false, false, true>, qconv_general_tc_kernel<32, false, false, true>, qconv_general_tc_kernel<16, false, false, true>);
     else rc = by_slice(qconv_general_tc_kernel<64, false, false, false>, qconv_general_tc_kernel<32, false, false, false>, qconv_general_tc_kernel<16, false, false, false>);
