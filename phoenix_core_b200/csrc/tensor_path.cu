@@ -703,12 +703,13 @@ bool forward_keeps_staged_input(int dtype, int variant, const Geom& g) {
 
 bool backward_shares_staged_dy(int dtype, int variant, const Geom& g, StagedView* view, size_t* bytes) {
     if ((dtype != PCB_F16 && dtype != PCB_BF16) || variant != PCB_VARIANT_16_PRODUCT || !g.plain || g.groups != 1 || g.real_in) return false;
-    if (g.KH * g.KW == 1) return false;
+    const bool point = g.KH * g.KW == 1;
+    if (point && (!conv_filter_tc_flat(g) || pointwise_tc_supported(PASS_BWD_DATA, dtype, variant, g))) return false;
     if ((g.SH != 1 || g.SW != 1) && (!conv_tc_dual_classes(PASS_BWD_DATA, g) || strided_classes_supported(dtype, variant, g))) return false;
     // the same order of preference as tensor_launch, for both passes
     if (pointwise_filter_tc_supported(dtype, variant, g)) return false;
     const bool narrow_dat = narrow_tc_supported(PASS_BWD_DATA, dtype, variant, g), narrow_flt = narrow_filter_tc_supported(dtype, variant, g);
-    if (narrow_dat || narrow_flt) return narrow_dat && narrow_flt && narrow_tc_staged_dy_view(g, view, bytes);
+    if (narrow_dat || narrow_flt) return !point && narrow_dat && narrow_flt && narrow_tc_staged_dy_view(g, view, bytes);
     return conv_tc_supported(PASS_BWD_DATA, dtype, variant, g) && conv_filter_tc_supported(dtype, variant, g) && conv_tc_staged_dy_view(g, view, bytes);
 }
 

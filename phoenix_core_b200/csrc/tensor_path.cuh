@@ -97,6 +97,7 @@ int conv_filter_tc_launch(int dtype, const Geom& g, const void* dy, const void* 
                           cudaStream_t stream, const void* kept_x = nullptr, const StagedView* kept_dy = nullptr, StatusClear* sc = nullptr);
 // Geometry of the copy of dy that the general backward-data kernel stages; false when it inserts zeros (strided layers) or
 // the filter gradient would block its channels.
+bool conv_filter_tc_flat(const Geom& g);
 bool conv_tc_staged_dy_view(const Geom& g, StagedView* view, size_t* bytes);
 // The filter gradient stages x as [component][image][h][w][channels], the layout of the forward pass.
 bool conv_filter_tc_stages_like_forward(const Geom& g);
