@@ -318,7 +318,8 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
     const int q = warp & 3, half = warp >> 2;                          // TMEM lane quadrant, half of the columns (warps 0 .. 7)
     if (warp < 8) {
         if (n_stages > 0) ok = mbar_wait_bounded(done_bar, 0, status, ST_Q_EPILOGUE) && ok;
-        ok = warp_may_store(ok, read_status(status));
+        const int seen = read_status(status);                          // the CTA's own word, in shared memory: asked after the wait
+        ok = warp_may_store(ok, seen);
         tc_fence_after_sync();
         const int row = q * 32 + lane, m = m0 + row;
 #pragma unroll 1
