@@ -971,12 +971,14 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
             const int blk = blockA0 + row / p.cbA;
             const int d = blk / bpcA, co = (blk % bpcA) * p.cbA + row % p.cbA;
             const bool row_ok = d < p.nc && co < p.Co;
+            const bool any_row = __any_sync(0xffffffffu, row_ok);
             const size_t comp_stride = (size_t)p.Co * p.Ci;
+            const uint32_t rbuf = tiles_addr + (uint32_t)(warp - 2) * ADD_ROWS_BYTES<32>;      // the operand ring: all MMAs have read it
             float* tap_base = dw32 + (size_t)tap * p.nc * comp_stride;
 #pragma unroll
             for (int cb = 0; cb < 4; ++cb) {
                 const int col0 = chalf * 128 + cb * 32;
-                if (col0 >= p.n_tile_cols) break;
+                if (col0 >= p.n_tile_cols || !any_row) break;
                 uint32_t v[32];
                 tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + 256 + col0, v);
                 tmem_ld_wait();
@@ -984,27 +986,21 @@ qconv_filter_tf32_kernel(const __grid_constant__ CUtensorMap map_dy_hi, const __
                 for (int e = 0; e < 32; ++e) part[cb][e] += __uint_as_float(v[e]);
                 tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + lbuf * 128 + col0, v);
                 tmem_ld_wait();
-                if (!row_ok) continue;
 #pragma unroll
                 for (int e = 0; e < 32; ++e) v[e] = __float_as_uint(__uint_as_float(v[e]) + part[cb][e]);
-#pragma unroll
-                for (int g4 = 0; g4 < 8; ++g4) {
-                    const int col = col0 + g4 * 4;
-                    if (col >= p.n_tile_cols) continue;
-                    const int nblk = blockB0 + col / p.cbB;
+                auto add = [&](auto quads) {
+                    constexpr bool Q = decltype(quads)::value;
+                    const int col = col0 + add_rows_column<32, Q>(lane), nblk = blockB0 + col / p.cbB;      // (l, ci) of this lane's columns
                     const int l = nblk / bpcB, ci = (nblk % bpcB) * p.cbB + col % p.cbB;
-                    if (l >= p.nc || ci >= p.Ci) continue;
-                    const float sgn = alg_negative(p.neg, l, d) ? -1.f : 1.f;
-                    float* dst = tap_base + (size_t)alg_pair(p.ga, l, d) * comp_stride + (size_t)co * p.Ci + ci;
-                    if ((p.Ci & 3) == 0) {
-                        red_add_f32x4(dst, sgn * __uint_as_float(v[4 * g4]), sgn * __uint_as_float(v[4 * g4 + 1]),
-                                      sgn * __uint_as_float(v[4 * g4 + 2]), sgn * __uint_as_float(v[4 * g4 + 3]));
-                    } else {
-#pragma unroll
-                        for (int e = 0; e < 4; ++e)
-                            if (ci + e < p.Ci) atomicAdd(dst + e, sgn * __uint_as_float(v[4 * g4 + e]));
-                    }
-                }
+                    const bool col_ok = col < p.n_tile_cols && l < p.nc && ci < p.Ci;
+                    add_rows<32, Q>(rbuf, v, lane, [&](int r, float& sgn) -> float* {
+                        const int rd = __shfl_sync(0xffffffffu, row_ok ? d : -1, r), rco = __shfl_sync(0xffffffffu, co, r);
+                        if (rd < 0 || !col_ok) return nullptr;
+                        if (alg_negative(p.neg, l, rd)) sgn = -1.f;
+                        return tap_base + (size_t)alg_pair(p.ga, l, rd) * comp_stride + (size_t)rco * p.Ci + ci;
+                    });
+                };
+                if ((p.Ci & 3) == 0) add(Bool<true>()); else add(Bool<false>());
             }
         }
     }

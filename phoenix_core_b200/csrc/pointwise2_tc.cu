@@ -392,7 +392,7 @@ qconv_pointwise_filter_pair_tc_kernel(const __grid_constant__ CUtensorMap map_dy
         ok = warp_may_store(ok, seen);
         tc_fence_after_sync();
         if (ok && n_steps > 0) {
-            const int co = co0 + q * 32 + lane;
+            const uint32_t rbuf = tiles_addr + (uint32_t)(warp - 2) * ADD_ROWS_BYTES<32>;      // the operand ring: all MMAs have read it
 #pragma unroll 1
             for (int rr = 0; rr < 2; ++rr) {
                 const int r = 2 * half + rr;
@@ -401,14 +401,11 @@ qconv_pointwise_filter_pair_tc_kernel(const __grid_constant__ CUtensorMap map_dy
                     uint32_t v[32];
                     tmem_ld_32x32b_x32(tmem_base + ((uint32_t)(q * 32) << 16) + r * 128 + cb * 32, v);
                     tmem_ld_wait();
-                    if (co >= p.Co) continue;
-                    float* dst = dw32 + ((size_t)r * p.Co + co) * p.Ci + ci0 + cb * 32;
-#pragma unroll
-                    for (int g4 = 0; g4 < 8; ++g4) {
-                        if (ci0 + cb * 32 + g4 * 4 < p.Ci)
-                            red_add_f32x4(dst + g4 * 4, __uint_as_float(v[4 * g4]), __uint_as_float(v[4 * g4 + 1]),
-                                          __uint_as_float(v[4 * g4 + 2]), __uint_as_float(v[4 * g4 + 3]));
-                    }
+                    const int ci = ci0 + cb * 32 + add_rows_column<32, true>(lane);
+                    add_rows<32, true>(rbuf, v, lane, [&](int row, float&) -> float* {
+                        const int co = co0 + q * 32 + row;
+                        return co < p.Co && ci < p.Ci ? dw32 + ((size_t)r * p.Co + co) * p.Ci + ci : nullptr;
+                    });
                 }
             }
         }

@@ -72,6 +72,7 @@ def test_pairs_channels_last(gpu, oracle, co, h, w):
     ("f16", (17, 64, 128, 28, 28, 3, 2)), ("bf16", (9, 64, 64, 40, 24, 3, 1)), ("f16", (7, 48, 64, 31, 44, 3, 1)), ("f16", (5, 96, 64, 26, 57, 5, 1)),
     ("f16", (40, 64, 128, 28, 28, 3, 2)), ("f16", (33, 64, 96, 41, 30, 3, 2)), ("bf16", (14, 64, 64, 29, 52, 5, 2)), ("f16", (41, 96, 64, 20, 18, 3, 2)), ("f16", (33, 128, 192, 23, 20, 1, 1)), ("bf16", (7, 128, 192, 61, 51, 1, 1)), ("f16", (80, 128, 128, 5, 9, 3, 1)),
     ("f16", (64, 16, 64, 24, 24, 3, 1)), ("f16", (9, 48, 40, 41, 47, 1, 1)), ("bf16", (50, 24, 56, 12, 11, 1, 1)),
+    ("f16", (9, 37, 56, 15, 13, 3, 1)), ("f32", (9, 21, 40, 15, 13, 3, 1)), ("bf16", (9, 42, 64, 15, 13, 1, 1)),
     ("f16", (9, 24, 56, 15, 13, 1, 1)), ("bf16", (41, 64, 256, 14, 14, 1, 1)), ("f16", (1, 256, 64, 9, 9, 1, 1)), ("f16", (31, 256, 128, 18, 18, 1, 1)), ("f16", (11, 16, 64, 9, 7, 1, 1)),
     ("f32", (5, 64, 64, 56, 28, 3, 1)), ("f32", (40, 64, 64, 14, 15, 3, 1)), ("f32", (21, 128, 128, 19, 17, 1, 1)), ("f32", (12, 40, 48, 33, 41, 3, 1)),
     ("f32", (9, 40, 24, 41, 47, 1, 1)), ("f32", (33, 96, 64, 24, 20, 3, 2)), ("f32", (3, 16, 24, 101, 37, 3, 1)), ("f32", (5, 24, 32, 40, 51, 1, 1)),
