@@ -1169,9 +1169,7 @@ static int conv_tf32_filter_launch(const Geom& layer, const float* dy, const flo
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
     const bool pair = p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0 && worth_pairs((double)taps * p.m_tiles * p.n_tiles * steps_total * 4 * p.n_tile_cols / TN);
     const int items = taps * p.m_tiles * p.n_tiles / (pair ? 2 : 1);
-    int splits = split_count(items, pair ? sm_count() / 2 : sm_count());
-    if (splits > steps_total) splits = steps_total;
-    if (splits < 1) splits = 1;
+    const int splits = split_count(items, pair ? sm_count() / 2 : sm_count(), steps_total, 16);
     p.steps_per_split = (steps_total + splits - 1) / splits;
     p.splits = (steps_total + p.steps_per_split - 1) / p.steps_per_split;
 
