@@ -14,7 +14,7 @@
 // crop / insert / accumulate kernels (src/conv2d.hpp:167-275, :433-562; src/backend/cudnn/conv2d.hpp:280-309,
 // :447-488; src/backend/cudnn/kernels.cu:39-156).
 //
-// Kernel: persistent, one CTA per SM. Tile = 128 rows (d,co) x 256 pixels (a PW x PH x PN box of the output);
+// Kernel: persistent, one CTA per SM, or a pair of SMs per tile of 256 rows. Tile = 128 rows (d,co) x 256 pixels (a PW x PH x PN box);
 // K slice per stage = one tap, one input component, KS channels; A and B both K-major, both by TMA;
 // tcgen05.mma M=128 N=256 K=16; the accumulator is double-buffered in TMEM (2 x 256 columns) so the epilogue
 // (8 warps: TMEM -> bias -> cast -> NCHW stores) of tile i overlaps the main loop of tile i+1.

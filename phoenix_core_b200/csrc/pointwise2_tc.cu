@@ -6,8 +6,8 @@
 // resident in its shared memory) and HALF of the 128 pixels of the streamed activation tile; the tensor cores of both SMs read
 // the two halves across the pair. Per MMA and SM that is 4 KB + 2 KB of shared-memory operand reads instead of 8 KB, and each
 // activation tile is fetched from L2 once per 256 channels instead of once per 128.
-// What it buys, measured on the 128 -> 256 channel layer at 56 x 56: with one pass over the K slices per tile, 3-4 % (the steady
-// 75-80 clocks per MMA are the tensor pipe's own rate for 128-column MMAs, not a shared-memory limit). The larger gain is the
+// What it buys, measured on the 128 -> 256 channel layer at 56 x 56: with one pass over the K slices per tile, 3-4 % (the
+// tensor pipe takes 64-66 clocks per 128-column MMA here as there: shared memory does not limit it). The larger gain is the
 // schedule the four-stage activation ring allows: all K slices of a tile are resident at once, so a tile is issued in TWO
 // PHASES (accumulators 0,1 over every slice, then 2,3 over every slice) and the epilogue's drain of one accumulator pair always
 // overlaps the MMAs of the other: forward 0.185 -> 0.165 ms.

@@ -187,8 +187,7 @@ qconv_pointwise_tc_kernel(const __grid_constant__ CUtensorMap map_w, const __gri
                     //    drained it;
                     //  - the last K step of the last slice: the first pair is complete (and signalled) while the second still
                     //    computes, so its drain overlaps those MMAs.
-                    // Inside a pair the MMAs alternate between the two accumulators (back-to-back MMAs into one accumulator run at
-                    // two thirds of the rate of independent ones).
+                    // Inside a pair the MMAs alternate between the two accumulators.
                     constexpr int J = KS / 16;
                     const bool first = k == 0, last = k == n_k - 1;
                     if (first) {

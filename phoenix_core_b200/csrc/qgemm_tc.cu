@@ -15,10 +15,10 @@
 // Three groups of four warps load (plain loads: feature counts need no alignment, which a tensor map would ask for), expand and store
 // the operands in the tcgen05 layouts, each group its own stages;
 // one thread of a thirteenth warp issues the MMAs. fp32 operands are split into hi + lo TF32 numbers on their way
-// (three MMAs per product, as in conv_tf32.cu). The reduced dimension of a tile is cut over the CTAs of a cluster, which add
+// (three MMAs per product). The reduced dimension of a tile is cut over the CTAs of a cluster, which add
 // their partial tiles through distributed shared memory in a fixed order (results do not depend on timing, nothing is zeroed or
 // cast in a second pass). What bounds a dense layer of a few hundred features is the latency of this chain (load, expand, MMA,
-// exchange, store), not bandwidth: hence one kernel per call (behind the reset of the status word), no staging
+// exchange, store), not bandwidth: hence one kernel per call (its first CTA resets the call's status word), no staging
 // kernels, and a cluster split that fills the machine.
 // All mbarrier waits are bounded.
 #include "tc_common.cuh"
