@@ -803,7 +803,9 @@ bool narrow_tc_supported(Pass pass, int dtype, int variant, const Geom& g) {
     if (pass == PASS_FWD && (g.SH != 1 || g.SW != 1) && !s2d_layer(g)) return false;   // backward-data is a stride-1 correlation of the zero-inserted dy
     if (pass == PASS_BWD_DATA && (g.SH > 2 || g.SW > 2)) return false;
     if (pass == PASS_BWD_DATA && ((g.KH - 1) * g.DH < g.PT || (g.KW - 1) * g.DW < g.PL)) return false;
-    const NPlan pl = make_nplan(pass, g);
+    // (the tile of 8 pixels has to fit: outputs that are not 32-byte aligned take it. Where only the tile of 16 does -- quaternion 2x6, 19 rows,
+    // 230 656 bytes of shared memory against 234 752 -- the layer is the general kernel's.)
+    const NPlan pl = make_nplan(pass, g, false);
     if (pl.Cin > 16 || g.nc * pl.Cout > NM) return false;
     if (pl.Wt > 32 || pl.Ht > 255 || pl.smem > 226 * 1024) return false;
     if (pl.Wout < 8 || pl.Hout < 8) return false;                             // tiny images: the general kernel packs several per tile
