@@ -410,7 +410,7 @@ __device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
     const __nv_bfloat162 h = __floats2bfloat162_rn(a, b);
     return *reinterpret_cast<const uint32_t*>(&h);
 }
-// N (4 or 8) channels of a pixel: hi at hi, the bf16 parts at xb and lb, aligned to 4 N and 2 N bytes.
+// N (4 or 8) channels of a pixel: hi at hi, the bf16 parts at xb and lb, aligned to 16 and 2 N bytes.
 template <int N>
 __device__ __forceinline__ void store_split(const float (&f)[N], float* hi, uint16_t* xb, uint16_t* lb) {
     float h[N];
@@ -435,7 +435,11 @@ __device__ __forceinline__ void store_split(const float (&f)[N], float* hi, uint
         uint32_t w[8];
 #pragma unroll
         for (int e = 0; e < 8; ++e) w[e] = __float_as_uint(h[e < N ? e : 0]);
-        st_global_v8(hi, w);                         // (whole sectors)
+        if (reinterpret_cast<uintptr_t>(hi) % 32 == 0) st_global_v8(hi, w);      // (whole sectors)
+        else {                                       // the workspace is only 16-byte aligned
+            *reinterpret_cast<uint4*>(hi) = make_uint4(w[0], w[1], w[2], w[3]);
+            *reinterpret_cast<uint4*>(hi + 4) = make_uint4(w[4], w[5], w[6], w[7]);
+        }
         *reinterpret_cast<uint4*>(xb) = make_uint4(x[0], x[1], x[N / 2 - 2], x[N / 2 - 1]);
         *reinterpret_cast<uint4*>(lb) = make_uint4(l[0], l[1], l[N / 2 - 2], l[N / 2 - 1]);
     } else {
