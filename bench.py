@@ -395,9 +395,9 @@ def sweep_leg(torch, pcb, _lib, peaks, reps=5, batch=128, only=None, layouts=("n
                    "tflops": round(fl / (ms * 1e-3) / 1e12, 1), "gbs": round(nbytes / (ms * 1e-3) / 1e9, 0),
                    "f_hbm": round(nbytes / (ms * 1e-3) / 1e9 / peaks["hbm_gbs"], 3),
                    "engine": L.pcb_qconv2d_engine_for(ctypes.byref(d), pid)}
-            if dtype == "f32":       # the fp32 kernels execute one TF32 and two bf16 products, in clocks two TF32 ones
+            if dtype == "f32":       # the fp32 kernels execute three TF32 MMAs per product
                 if tf32_peak:
-                    row["f_tf32_executed"] = round(2 * fl / (ms * 1e-3) / 1e12 / tf32_peak, 3)
+                    row["f_tf32_executed"] = round(3 * fl / (ms * 1e-3) / 1e12 / tf32_peak, 3)
             else:
                 row["f_tensor"] = round(fl / (ms * 1e-3) / 1e12 / peaks["tflops_sustained"], 3)
             rows.append(row)
@@ -405,8 +405,8 @@ def sweep_leg(torch, pcb, _lib, peaks, reps=5, batch=128, only=None, layouts=("n
         del x, w, y, dy, dw, dx
         torch.cuda.empty_cache()
     return {"config": "batch %d, %s, 16-product, U[-1,1]; layout nchw = NCHW activations + OIHW filters, nhwc = channels-last activations "
-                      "+ OHWI filters; f_tensor against the sustained tensor peak (fp16), f_tf32_executed = 2 x FLOPs / time against a TF32 "
-                      "cuBLAS GEMM timed in this run (fp32: one TF32 and two bf16 products, in clocks two TF32 ones), f_hbm = algorithmic bytes / time against the "
+                      "+ OHWI filters; f_tensor against the sustained tensor peak (fp16), f_tf32_executed = 3 x FLOPs / time against a TF32 "
+                      "cuBLAS GEMM timed in this run (fp32: three TF32 MMAs per product), f_hbm = algorithmic bytes / time against the "
                       "copy bandwidth; engine 2 = tcgen05, 1 = CUDA cores" % (batch, "fp32" if dtype == "f32" else "fp16"),
             "reps": reps, "rows": rows}
 

@@ -1,6 +1,6 @@
-"""fp32 convolutions on the tensor cores: hi * hi in TF32 and the two cross terms in bf16, with accumulators of their own. The forms of the
-kernels (halo tiles; 128 and 256 columns; one and several chunks of the K loop; filter gradients on pairs of SMs and on single ones), the
-exponent range (the split may neither overflow nor lose small tensors), and the 16-bit filter gradient on pairs of SMs."""
+"""fp32 convolutions on the tensor cores: hi * hi and the two cross terms in TF32. The forms of the kernels (halo tiles; 128 and 256 columns; one and
+several chunks of the K loop; filter gradients of one and several row tiles), the exponent range (the split may neither overflow nor lose small
+tensors), what a single product, a constant plane and a tiny tensor may be off by, and the 16-bit filter gradient of the same layers."""
 import numpy as np
 import pytest
 import torch
@@ -53,8 +53,7 @@ def test_filter_gradient_row_tiles(gpu, oracle, dtype, tol, case):
 
 
 # Powers of two scale every product exactly, so the results are those of the unscaled tensors, scaled, as long as the low parts (2^-12 of a
-# value and less) stay normal numbers: filters of 2^-103, whose low parts are 2^-115 and some octaves less. Further down the low parts are
-# lost one by one, as they were with three TF32 products (2^-116: 2e-5, before 6e-6).
+# value and less) stay normal numbers: filters of 2^-103, whose low parts are 2^-115 and some octaves less. (Further down: test_fp32_tiny_filters.)
 @pytest.mark.parametrize("ex,ew", [(100, -100), (-100, 90), (60, 40)])
 def test_fp32_exponent_range(gpu, ex, ew):
     n, ci, co, h, w = 4, 20, 24, 26, 17
@@ -84,3 +83,48 @@ def test_fp32_values_next_to_the_largest(gpu):
     assert np.max(np.abs(y[0, 5] / want - 1)) <= 4e-6
     x[0, 3, 0, 0] = np.inf
     assert not np.isfinite(gpu.run_conv_fwd(x, f, None, (1, 1), (0, 0, 0, 0), "f32", "16p", "tensor")[0, 5, 0, 0])
+
+
+# What the split drops of a product: lo * lo, at most 2^-22 of it, and of either lo the bits behind the eleven that TF32 holds, at most 2^-23 each. The sum
+# of one product and zeros adds no more than the rounding of the result (the additions of the MMAs are exact). Measured: 4.0e-7.
+def test_fp32_single_products(gpu):
+    n, ci, co, h, w = 2, 40, 48, 12, 16
+    rng = np.random.default_rng(68)
+    x = np.zeros((4 * n, ci, h, w), np.float32)
+    comp, chan = rng.integers(0, 4, (n, h, w)), rng.integers(0, ci, (n, h, w))
+    i, a, b = np.meshgrid(np.arange(n), np.arange(h), np.arange(w), indexing="ij")
+    value = rng.normal(size=(n, h, w)).astype(np.float32)
+    x[comp * n + i, chan, a, b] = value
+    f = normal(69, (4, co, ci, 1, 1), std=0.1)
+    y = gpu.run_conv_fwd(x, f, None, (1, 1), (0, 0, 0, 0), "f32", "16p", "tensor").reshape(4, n, co, h, w)
+    for d in range(4):
+        want = np.abs(value[..., None].astype(np.float64) * f[comp ^ d, :, chan, 0, 0])            # [n, h, w, co]; the signs are the oracle tests'
+        got = np.abs(np.moveaxis(y[d], 1, -1))
+        assert np.max(np.abs(got / want - 1)) <= 2.0 ** -22 + 2 * 2.0 ** -23 + 2.0 ** -24
+
+
+# Planes and filters of one value: all errors of the products have one sign, and so have those of the additions, which cut off up to 2^-23 of an accumulator that
+# grows linearly over at most 64 MMAs: half of half of 64 * 2^-23 on average, beside 2^-21 for the products. The pairs of values have low parts and
+# bf16 roundings of one sign.
+@pytest.mark.parametrize("a,b", [(1.00146, 1.00146), (1.0024409, 1.0024409), (1 / 3, 0.7), (1.0004, 1.00487)])
+@pytest.mark.parametrize("ci,co,k", [(32, 32, 1), (64, 40, 3), (128, 64, 3)])
+def test_fp32_constant_planes(gpu, ci, co, k, a, b):
+    n, h, w = 2, 14, 16
+    x, f = np.zeros((4 * n, ci, h, w), np.float32), np.zeros((4, co, ci, k, k), np.float32)
+    x[:n], f[0] = a, b
+    y = gpu.run_conv_fwd(x, f, None, (1, 1), (k // 2,) * 4, "f32", "16p", "tensor")[:n]
+    taps = np.outer(*(np.convolve(np.ones(s), np.ones(k), "same") for s in (h, w)))
+    want = np.float64(np.float32(a)) * np.float64(np.float32(b)) * ci * taps
+    assert np.max(np.abs(y / want - 1)) <= 16 * 2.0 ** -23 + 2.0 ** -21 + 2.0 ** -24
+
+
+# Filters whose low parts are no longer normal numbers keep them to 2^-136, the last bit of a TF32 number; what is cut off is 2^-136 / sqrt(3) on average (in the
+# 2-norm), here of filters of 0.053 * 2^-116.
+def test_fp32_tiny_filters(gpu):
+    n, ci, co, h, w = 4, 20, 24, 26, 17
+    std, ew = (2.0 / (4 * ci * 9)) ** 0.5, -116
+    x, f = normal(74, (4 * n, ci, h, w)), normal(75, (4, co, ci, 3, 3), std=std)
+    pad = (1, 1, 1, 1)
+    y = gpu.run_conv_fwd(x, f, None, (1, 1), pad, "f32", "16p", "tensor").astype(np.float64)
+    ys = gpu.run_conv_fwd(x * np.float32(2.0 ** 100), f * np.float32(2.0 ** ew), None, (1, 1), pad, "f32", "16p", "tensor").astype(np.float64)
+    assert np.linalg.norm(ys * 2.0 ** -(100 + ew) - y) / np.linalg.norm(y) <= 2.0 ** -136 / (std * 2.0 ** ew)
