@@ -15,6 +15,7 @@
 // Dense layers are the 1x1 convolution of 1x1 images (pixels = batch); input-major dense filters and the
 // input-major dense filter gradient are handled while staging / unstaging. Replaces, for fp32 tensors, the scalar
 // fp32 library calls of src/backend/cudnn/conv2d.hpp:280-309, :447-488 and src/backend/cudnn/dense.hpp:102-133, :181-216.
+#include "column_halves.h"
 #include "tc_common.cuh"
 #include "tensor_path.cuh"
 
@@ -250,7 +251,7 @@ qconv_general_tf32_kernel(const __grid_constant__ CUtensorMap map_w_hi, const __
     } else {
         const int q = warp & 3, chalf = (warp - 2) >> 2;
         const int sv = p.store_vec;                  // pixels per store: 8, 4, 2 or 1
-        const int half = p.n_cols > 128 ? 128 : p.n_cols / 2;       // columns of a warp: chalf * half and on
+        const int half = columns_per_half(p.n_cols);                // columns of a warp: chalf * half and on
         const uint32_t lane_addr = tmem_base + ((uint32_t)(q * 32) << 16) + chalf * half;
         int unit = 0;
         bool ok = true;
