@@ -204,7 +204,7 @@ int pcb_qdense_engine_for(const pcb_dense_desc* desc, int pass);
 
 /* Device-side wait budget. The tensor-core kernels bound every barrier wait; when a wait expires the
  * kernel records it in a status word inside the workspace and returns. Every entry point above clears the
- * word once, before its first launch, and kernels only OR into it, so after a call the word covers all the
+ * word once, before or in its first launch, and kernels only OR into it, so after a call the word covers all the
  * launches of that call (a later launch of the same call gives up at its first slow wait once the word is
  * set). This reads the word back (synchronises the stream). Returns PCB_OK or PCB_ERR_DEVICE_TIMEOUT.
  * (Stands where the reference checks cudnnStatus_t / cudaError_t after each library call,

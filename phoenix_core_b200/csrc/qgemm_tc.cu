@@ -389,7 +389,8 @@ __device__ __forceinline__ void q_tile(const QProblem& p, int block, int cluster
 }
 
 // PAIR: prob[0] has layouts (AK, BK), prob[1] (AK1, BK1) -- both gradients of a dense layer in one launch.
-// The status word: every CTA keeps its own in shared memory (its waits look at no other), and ORs it into the call's word when it ends. The
+// The status word: every CTA keeps its own in shared memory (its waits look at no other; an epilogue asks those of all CTAs of its tile, so tiles of
+// other clusters are stored after an expired wait), and ORs it into the call's word when it ends. The
 // first CTA resets that word when it starts (p.clear), instead of a launch in front of this one, which cost 2 to 3 us of a call: a CTA
 // has something to OR only after a wait of 2^31 clocks has run out, a second behind the start of its wave, and the first CTA is of the
 // first wave.

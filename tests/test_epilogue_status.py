@@ -1,6 +1,7 @@
-"""What an expired wait must not lead to: a stored tile. Every epilogue asks the status word of the call before it stores, and a loader whose
-wait ran out does not announce its stage. No test can make a wait of these kernels run out (nothing may be taken out of them), so this
-reads the sources."""
+"""What an expired wait must not lead to: a tile stored from what it left unfinished. The epilogues of the convolution kernels ask the status word of
+the call before they store. The dense kernel's CTAs keep a word of their own, which the call's only gets when they end: an epilogue asks its own, and
+behind the exchange of partial tiles those of every CTA of the tile; other tiles are stored. A loader whose wait ran out does not announce its stage. No
+test can make a wait of these kernels run out (nothing may be taken out of them), so this reads the sources."""
 import os
 import re
 
@@ -28,3 +29,16 @@ def test_a_loader_does_not_announce_an_unfilled_stage():
     text = open(os.path.join(CSRC, "qgemm_tc.cu")).read()
     arrivals = re.findall(r"^.*mbar_arrive\(full_bar.*$", text, re.M)
     assert arrivals and all("if (ok && lane == 0)" in line for line in arrivals)
+
+
+def test_dense_tiles_ask_every_cta_that_worked_on_them():
+    text = open(os.path.join(CSRC, "qgemm_tc.cu")).read()
+    # the tile function is given the CTA's own word, never the call's, which is only ORed into
+    calls = re.findall(r"q_tile<[^>]*>\(p\.prob.*\);", text)
+    assert len(calls) == 2 and all(c.endswith(", own_status);") for c in calls)
+    assert re.findall(r"^.*\bstatus\b.*$", text[text.index("const int block = blockIdx.x;"):text.index("int q_launch(")], re.M)[-1].strip().startswith(
+        "if (t == 0 && *own_status != 0) atomicOr(status, *own_status);")
+    # behind the exchange: the words of all CTAs of the tile, in front of the stores
+    tail = text[text.index("if (split > 1 && t < Q_LOADERS) {"):]
+    asked, stored = tail.index("ld_cluster_u32(smem_u32(status), peer0 + r) == 0u"), tail.index("q_store(")
+    assert asked < stored and "for (int r = 0; r < split; ++r) good = good &&" in tail[:stored] and "if (good && m < p.M)" in tail[asked:stored]
