@@ -15,7 +15,7 @@ LIB = os.path.join(HERE, "libphoenix_core_b200.so")
 OBJ_DIR = os.path.join(HERE, "build")
 SOURCES = ["api.cu", "simt_qgemm.cu", "tensor_path.cu", "pointwise_tc.cu", "pointwise2_tc.cu", "pointwise8_tc.cu", "conv_tc.cu", "narrow_tc.cu",
            "conv_tf32.cu", "qgemm_tc.cu", "aux_bn.cu", "probe.cu"]
-HEADERS = ["common.cuh", "tensor_path.cuh", "umma.cuh", "tc_common.cuh", "unaligned_chunk.h", "column_halves.h", os.path.join("..", "..", "include", "phoenix_core_b200.h")]
+HEADERS = ["common.cuh", "tensor_path.cuh", "umma.cuh", "tc_common.cuh", "unaligned_chunk.h", "column_halves.h", "sm_share.h", os.path.join("..", "..", "include", "phoenix_core_b200.h")]
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
     "-Xcompiler", "-fPIC", "-Xcompiler", "-Wall",

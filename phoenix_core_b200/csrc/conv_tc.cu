@@ -1742,7 +1742,7 @@ int conv_tc_launch(Pass pass, int dtype, const Geom& layer, const void* w, const
     }
 
     const int n_tiles = p.tiles_w * p.tiles_h * p.tiles_n * p.tiles_m * (pl.dual ? 2 : 1) / (pair ? 2 : 1);
-    const int most = pair ? sm_count() / 2 : sm_count(), grid = (n_tiles < most ? n_tiles : most) * (pair ? 2 : 1);
+    const int most = pair ? sm_pairs() : sm_count(), grid = (n_tiles < most ? n_tiles : most) * (pair ? 2 : 1);
     const size_t operand_bytes = halo ? (size_t)p.a_slots * p.a_taps * GM * 64 + (size_t)p.n_stages * p.halo_bytes : (size_t)p.n_stages * p.stage_bytes;
     size_t smem = 1024 + operand_bytes + 512 + tail_bytes;
     if (smem < ONE_CTA_SMEM) smem = ONE_CTA_SMEM;
@@ -1915,7 +1915,7 @@ int conv_filter_tc_launch(int dtype, const Geom& layer, const void* dy, const vo
     const bool pair = !xmajor && p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0 &&
                       worth_pairs((double)taps * p.m_tiles * p.n_tiles * steps_total * (FK / 16) * p.n_tile_cols / GN);
     const int items = xmajor ? (taps + p.TPG - 1) / p.TPG : taps * p.m_tiles * p.n_tiles / (pair ? 2 : 1);
-    const int splits = split_count(items, pair ? sm_count() / 2 : sm_count(), steps_total, 24);
+    const int splits = split_count(items, pair ? sm_pairs() : sm_count(), steps_total, 24);
     p.steps_per_split = (steps_total + splits - 1) / splits;
     p.splits = (steps_total + p.steps_per_split - 1) / p.steps_per_split;
 

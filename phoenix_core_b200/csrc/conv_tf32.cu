@@ -1122,7 +1122,7 @@ static int conv_tf32_filter_launch(const Geom& layer, const float* dy, const flo
     const int steps_total = p.tiles_w * p.tiles_h * p.tiles_n;
     const bool pair = p.m_tiles % 2 == 0 && (p.n_tile_cols / p.cbB) % 2 == 0 && worth_pairs((double)taps * p.m_tiles * p.n_tiles * steps_total * 6 * p.n_tile_cols / TN);
     const int items = taps * p.m_tiles * p.n_tiles / (pair ? 2 : 1);
-    const int splits = split_count(items, pair ? sm_count() / 2 : sm_count(), steps_total, 16);
+    const int splits = split_count(items, pair ? sm_pairs() : sm_count(), steps_total, 16);
     p.steps_per_split = (steps_total + splits - 1) / splits;
     p.splits = (steps_total + p.steps_per_split - 1) / p.steps_per_split;
 
@@ -1297,7 +1297,7 @@ int conv_tf32_launch(Pass pass, const Geom& layer, const void* a, const void* b,
         if (rc != PCB_OK) return rc;
         if (p.splits > 1 && !cleared) PCB_CUDA_TRY(cudaMemsetAsync(out, 0, out_bytes, stream));
     }
-    const int n_items = n_tiles * p.splits / (pair ? 2 : 1), most = pair ? sm_count() / 2 : sm_count();
+    const int n_items = n_tiles * p.splits / (pair ? 2 : 1), most = pair ? sm_pairs() : sm_count();
     const int grid = (n_items < most ? n_items : most) * (pair ? 2 : 1);
     p.apart = p.n_cols <= TN / 2 ? TN / 2 : 0;
     const int chunk = p.apart ? T_CHUNK_APART : T_CHUNK;

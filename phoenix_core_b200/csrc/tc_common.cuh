@@ -1,6 +1,7 @@
 // Helpers shared by the TMA-fed tcgen05 kernels: TMA load wrappers, wide stores, the tensor-map encoder
 // (fetched from the driver at run time, so the library does not link against libcuda), small host utilities.
 #pragma once
+#include "sm_share.h"
 #include <cstdlib>
 
 #include <cuda.h>
@@ -405,17 +406,18 @@ inline int make_tensor_map(CUtensorMap* map, CUtensorMapDataType dt, const void*
 }
 
 // SMs the persistent kernels size their grids for: the device's count minus the margin set through pcb_set_sm_margin (SMs left
-// free so that another kernel, e.g. a collective's, can run beside them), never fewer than two.
-inline int sm_count() {
+// free so that another kernel, e.g. a collective's, can run beside them).
+inline int device_sms() {
     static int sms = 0;
     if (sms == 0) {
         int dev = 0;
         if (cudaGetDevice(&dev) != cudaSuccess || cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0)
             sms = 148;
     }
-    const int left = sms - pcb::g_sm_margin;
-    return left < 2 ? 2 : left;
+    return sms;
 }
+inline int sm_count() { return sms_beside(device_sms(), pcb::g_sm_margin); }
+inline int sm_pairs() { return pairs_beside(device_sms(), pcb::g_sm_margin); }
 
 // Whether a main kernel is chained to a prologue of that many CTAs: only behind a short one. Behind a longer prologue the gap does not
 // matter, and the main kernel, started CTA by CTA beside the last wave, can be the slower for it. Chained / not, us: fp32 3x3, 128
