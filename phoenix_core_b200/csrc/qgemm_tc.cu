@@ -21,6 +21,8 @@
 // exchange, store), not bandwidth: hence one kernel per call (its first CTA resets the call's status word), no staging
 // kernels, and a cluster split that fills the machine.
 // All mbarrier waits are bounded.
+#include <atomic>
+
 #include "tc_common.cuh"
 #include "tensor_path.cuh"
 #include "unaligned_chunk.h"
@@ -478,10 +480,40 @@ uint32_t q_signs(Pass pass) {
         }
     return neg;
 }
+// SMs that clusters of `cl` CTAs of these kernels (one CTA per SM) fill at once. A cluster lies inside one group of 14 to 20 SMs, and how many SMs a group has
+// differs between devices, so the runtime is asked: 16 clusters of 8 did not fit a device of 148 SMs, and the layers that were cut into 16 of them
+// took two rounds (forward in 16 bits, 144 -> 946 features at batch 42, as two rounds of 8 / one of 4: 14.7 / 8.4 us). Beside an SM margin, a cluster less for
+// each SM of it.
+int q_slots(int cl) {
+    static std::atomic<int> clusters[4];                               // of 1, 2, 4 and 8 CTAs, plus one; 0: not asked yet
+    if (cl == 1) return sm_count();
+    std::atomic<int>& known = clusters[cl == 2 ? 1 : (cl == 4 ? 2 : 3)];
+    int n = known.load(std::memory_order_relaxed) - 1;
+    if (n < 0) {
+        auto* kernel = qgemm_tc_kernel<false, 32, false, true, false, false, false>;
+        const size_t smem = QLayout<false, 32>::SMEM;
+        cudaLaunchConfig_t cfg = {};
+        cfg.gridDim = dim3((unsigned)(device_sms() / cl * cl));
+        cfg.blockDim = dim3(Q_THREADS);
+        cfg.dynamicSmemBytes = smem;
+        cudaLaunchAttribute attr[1];
+        attr[0].id = cudaLaunchAttributeClusterDimension;
+        attr[0].val.clusterDim.x = (unsigned)cl; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+        cfg.attrs = attr;
+        cfg.numAttrs = 1;
+        if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) != cudaSuccess ||
+            cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) {
+            cudaGetLastError();                                        // (no device, as where only a route is asked for: an estimate, not kept)
+            n = (cl > 2 ? device_sms() * 7 / 8 : device_sms()) / cl;
+        } else {
+            known.store(n + 1, std::memory_order_relaxed);
+        }
+    }
+    return (n - g_sm_margin) * cl;
+}
 // Picks the slices of the stages of the one or two problems of a launch, and the cluster that holds them: powers of
 // two up to 8 (a portable cluster). The cost of a choice is rounds of the machine x (stages of the longest CTA + the fixed part
-// of a CTA, about as long as 6 stages). A cluster lies inside one group of 16 to 20 SMs and every CTA takes an SM, so clusters
-// of 4 and 8 fill only about 7/8 of the SMs at once. fp32: every slice short enough for its accumulators.
+// of a CTA, about as long as 6 stages). fp32: every slice short enough for its accumulators.
 int q_plan(QParams& p, bool two, int f32) {
     long long best = -1;
     int blocks = 0;
@@ -495,7 +527,7 @@ int q_plan(QParams& p, bool two, int f32) {
             if ((sa > 1 && sa > a.stages) || (two && sb > 1 && sb > b.stages)) continue;
             if (f32 && (la > most || lb > most)) continue;
             const int cl = sa > sb ? sa : sb;
-            const int na = round_up(ta * sa, cl), nb = round_up(tb * sb, cl), slots = cl > 2 ? sm_count() * 7 / 8 / cl * cl : sm_count() / cl * cl;
+            const int na = round_up(ta * sa, cl), nb = round_up(tb * sb, cl), slots = q_slots(cl);
             if (slots < cl) continue;
             const long long cost = (long long)((na + nb + slots - 1) / slots) * ((la > lb ? la : lb) + 6 + (cl > 1 ? 1 : 0));
             if (best < 0 || cost < best) { best = cost; sa_best = sa; sb_best = sb; p.cluster = cl; p.first_blocks = na; blocks = na + nb; }
