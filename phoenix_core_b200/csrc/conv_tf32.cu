@@ -1188,7 +1188,8 @@ int conv_tf32_launch(Pass pass, const Geom& layer, const void* a, const void* b,
     const bool deep = worth_pairs((double)g.Nb * pl.Hout * pl.Wout / 256 * (pl.Mp / TM) * n_k * 6);
     // Clocks of a form, from which the fastest is taken. Of a stage: 680 with tiles of 256 pixels, 610 with 128, in halo form 22 per row of up to 32 or
     // 525. Of storing 256 pixels of 128 rows: aligned rows, and rows that go through shared memory, 4, 2 or 1 pixels per lane. A tile is stored
-    // beside the stages of the next one, a tile of 256 in several chunks beside two of those at most, and the chunks cost 3000 more. Constants with
+    // beside the stages of the next one, a tile of 256 in several chunks beside two of those at most, and the chunks cost 3000 more, 8000 where rows are aligned
+    // (1x1, 24 -> 16, 112 x 112, batch 20, tiles of 256 / 128 135.3 / 129.7 us; 64 -> 64, 28 x 28, batch 40 60.1 / 53.4). Constants with
     // which the choice lost 0.7 % on average over the forms of 32 forward layers, each timed in every form, us, 256 / 128 / halo of 32 / of 16: 3x3, 16
     // channels, 32 x 32, batch 8 26.1 / 18.4 / 31.7 / 23.6; 16 -> 24, 101 x 101, batch 32 296 / 315 / 349 / 342; 24 -> 40, 30 x 30, batch 60 173 / 201 / 175 / 160;
     // 64 -> 64, 56 x 56, batch 32 523 / 658 / 541 / 578; 1x1, 24 -> 16, 112 x 112, batch 10 82 / 69.
@@ -1198,7 +1199,7 @@ int conv_tf32_launch(Pass pass, const Geom& layer, const void* a, const void* b,
     auto wide_clocks = [&](long long rounds, long long stages, long long stage) {
         if (stages <= T_CHUNK) return rounds * (stages * stage > epilogue ? stages * stage : epilogue) + epilogue;
         const long long hidden = (stages < 2 * T_CHUNK ? stages : 2 * T_CHUNK) * stage;
-        return rounds * (stages * stage + (epilogue > hidden ? epilogue - hidden : 0) + 3000) + epilogue;
+        return rounds * (stages * stage + (epilogue > hidden ? epilogue - hidden : 0) + (p.store_vec == 8 ? 8000 : 3000)) + epilogue;
     };
     auto narrow_clocks = [&](long long rounds, long long stages, long long stage) {
         return rounds * (stages * stage > epilogue / 2 ? stages * stage : epilogue / 2) + epilogue / 2;
