@@ -427,9 +427,12 @@ inline int sm_pairs() { return pairs_beside(device_sms(), pcb::g_sm_margin); }
 inline bool chain_behind(unsigned prologue_blocks, unsigned per_sm) { return prologue_blocks <= per_sm * (unsigned)sm_count(); }
 
 // Whether a kernel of row tiles of 128 takes them two at a time on pairs of SMs (clusters of two): only where an SM has some 64 MMAs of
-// 256 columns (8192 clocks) to issue. A cluster launch starts later than a plain one. 1x1 layers, fp16, forward + backward, pairs / single, us:
-// 48 -> 56 channels, 10 x 10, batch 15 39.0 / 37.6; 56 -> 56, 30 x 30, batch 5 40.7 / 39.1; 24 -> 45, 55 x 59, batch 5 54.6 / 52.4; above the line
-// 3x3 24 -> 40, 45 x 37, batch 10, forward 24.9 / 25.7.
+// 256 columns (8192 clocks) to issue. A cluster launch starts later than a plain one, which shallow layers pay for; the halved operand traffic is what it
+// buys. No count of MMAs divides the two exactly. Forward, fp16, (MMAs per SM) single / pairs, us: 1x1, 256 -> 128, 14 x 14, batch 20 (27) 17.4 / 18.6; 64 -> 64,
+// 30 x 30, batch 48 (37) 24.7 / 25.0; 3x3 stride 2, 48 -> 64, 40 x 40, batch 12 (37) 22.9 / 23.5; above the line 3x3, 512 -> 128, 7 x 7, batch 16 (95) 106.9 / 86.2;
+// 48 -> 64, 45 x 37, batch 9 (114) 38.5 / 35.7; 24 -> 40, 45 x 37, batch 24 (152) 42.6 / 39.3. Misplaced by it: 3x3, 24 -> 40, 45 x 37, batch 10 (63) 25.6 / 25.0; 128 -> 128,
+// 7 x 7, batch 30 (45) 39.0 / 34.7; 5x5, 20 -> 64, 37 x 41, batch 8 (128) 38.3 / 39.1; channels-last 3x3, 128 -> 128, 14 x 14, batch 24 (143) 37.1 / 38.4. Filter
+// gradients, with the other passes: 3x3, 24 -> 40, 45 x 37, batch 24 123.9 / 120.0; 512 -> 128, 7 x 7, batch 16 191.0 / 192.8.
 inline bool worth_pairs(double mmas) { return mmas >= 64.0 * sm_count(); }
 
 inline int round_up(int v, int m) { return (v + m - 1) / m * m; }
