@@ -1,6 +1,7 @@
 """fp32 convolutions on the tensor cores: hi * hi and the two cross terms in TF32. The forms of the kernels (halo tiles; 128 and 256 columns; one and
 several chunks of the K loop; filter gradients of one and several row tiles), the exponent range (the split may neither overflow nor lose small
-tensors), what a single product, a constant plane and a tiny tensor may be off by, and the 16-bit filter gradient of the same layers."""
+tensors), what a single product, a constant plane and a tiny tensor may be off by, and the 16-bit filter gradient of
+a few row and column tiles (on single SMs; on pairs: test_gpu_pair_forms.py)."""
 import numpy as np
 import pytest
 import torch
@@ -34,7 +35,7 @@ def _check(gpu, oracle, dtype, tol, n, ci, co, h, w, kh, kw, stride=(1, 1), pad=
 
 
 # n, ci, co, h, w, kh, kw: halo tiles of 24 to 32 rows with aligned and unaligned rows, one and several chunks, several row tiles; plain tiles of
-# both widths; filter gradients of one to four row tiles (pairs for two and four) and of one to three column tiles
+# both widths; filter gradients of one to four row tiles and of one to three column tiles
 @pytest.mark.parametrize("case", [(16, 32, 32, 24, 32, 3, 3), (8, 48, 40, 31, 21, 3, 3), (6, 16, 36, 56, 26, 2, 2), (5, 24, 33, 28, 30, 5, 3), (3, 100, 64, 14, 15, 3, 3),
                                   (2, 33, 96, 9, 8, 1, 1), (40, 8, 8, 16, 16, 1, 1), (2, 72, 130, 7, 7, 3, 3), (9, 130, 72, 6, 5, 1, 1)])
 def test_fp32_forms(gpu, oracle, case):

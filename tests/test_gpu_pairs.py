@@ -1,6 +1,7 @@
-"""General kernels on pairs of SMs (an even number of 128-row tiles and enough work; smaller layers stay on single SMs): whole planes in each half of a tile, half a plane, planes of an odd
-number of rows (which stay on single SMs), power-of-two boxes split by images and by rows, halo tiles; batches that leave halves empty; odd
-and even planes; slices of 16, 32 and 64 channels; strides, bias, channels-last."""
+"""General kernels of layers with an even number of 128-row tiles: whole planes in a tile, planes of an odd number of rows, power-of-two boxes, halo
+tiles; batches that leave part of a tile empty; odd and even planes; slices of 16, 32 and 64 channels; strides, bias, channels-last. The layers of test_pairs
+and test_pairs_channels_last are too small for pairs of SMs and run on single ones; those of test_large_layers take pairs where they have two row tiles.
+The other forms on pairs, with a check of which kernel ran: test_gpu_pair_forms.py."""
 import numpy as np
 import pytest
 import torch
